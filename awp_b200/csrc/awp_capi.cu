@@ -66,6 +66,8 @@ struct awp_ctx {
   float coeff[16] = {}, tau8[8] = {}, w8[8] = {};
   float taumax = 0.f, taumin = 0.f;
   float qthr = 0.f;
+  unsigned thr = 0;    // bits of 2*qthr (StrArgs::thr)
+  AwpRelaxTab rel{};   // update constants of the Cartesian stress kernels
   float c1 = 9.0 / 8.0, c2 = -1.0 / 24.0;
   float dth = 0.f, dh1 = 0.f;
   int xls = 0, xre = 0, yls = 0, yre = 0;  // stress / output window (pmcl3d.c:573-631)
@@ -110,6 +112,7 @@ struct awp_ctx {
   bool tma_ok = false;            // tensor maps encoded for this context
   int tma_promo = -1;             // L2 promotion the maps were encoded with
   TmaMaps vel_maps{}, str_maps{};
+  TmaMaps topo_vel_maps{}, topo_str_maps{};  // of a curvilinear top grid
   long long cur_step = 0;
   bool initial_src_done = false;
   RecvState* recv = nullptr;     // RECVFILE receivers
@@ -168,7 +171,7 @@ StrArgs make_str_args(awp_ctx* c) {
   a.lam = f[AWP_LAM]; a.mu = f[AWP_MU]; a.qp = f[AWP_QP]; a.qs = f[AWP_QS];
   a.dcrjx = c->dcrjx; a.dcrjy = c->dcrjy; a.dcrjz = c->dcrjz; a.lam_mu = c->lam_mu;
   a.tex = c->tex;
-  memcpy(a.coeff, c->coeff, sizeof(a.coeff));
+  a.rel = c->rel;
   a.slice = c->g.slice;
   a.yline = c->g.yline;
   a.lam_mu_ld = (int)c->g.ny_pad();
@@ -183,7 +186,7 @@ StrArgs make_str_args(awp_ctx* c) {
   a.gx_lim = (c->sub_nxg ? c->sub_nxg - c->sub_x0 : c->p.nx) + AWP_NGSL + 1;
   a.gy_min = (c->p.npc == 2) ? INT_MIN : AWP_NGSL + 3;     // g_j > 1 || NPC == 2
   a.dth = c->dth; a.dh1 = c->dh1; a.dt = c->p.dt; a.c1 = c->c1; a.c2 = c->c2;
-  a.qthr = c->qthr;
+  a.thr = c->thr;
   return a;
 }
 
@@ -297,6 +300,26 @@ bool build_tma_maps(awp_ctx* c) {
   for (int q = 0; q < 3; ++q) bad |= awp_tma_encode(&c->str_maps.halo[q], f[vo[q]], c->g, hx, hy);
   for (int q = 0; q < 4; ++q) bad |= awp_tma_encode(&c->str_maps.media[q], f[sm[q]], c->g, mx, my);
   for (int q = 0; q < 12; ++q) bad |= awp_tma_encode(&c->str_maps.own[q], f[so[q]], c->g, ox, oy);
+  if (c->topo) {
+    // the curvilinear kernels' tiles: the same fields with their own boxes, and
+    // no k halo (the neighbouring levels come from the neighbouring lanes)
+    awp_topo_box(0, &hx, &hy);
+    awp_topo_box(1, &mx, &my);
+    awp_topo_box(2, &ox, &oy);
+    const bool jh[6] = {false, true, false, true, false, true};
+    for (int q = 0; q < 6; ++q)
+      bad |= awp_tma_encode(&c->topo_vel_maps.halo[q], f[vh[q]], c->g, jh[q] ? hx : ox,
+                            jh[q] ? hy : oy);
+    bad |= awp_tma_encode(&c->topo_vel_maps.media[0], f[AWP_D1], c->g, mx, my);
+    for (int q = 0; q < 3; ++q) {
+      bad |= awp_tma_encode(&c->topo_vel_maps.own[q], f[vo[q]], c->g, ox, oy);
+      bad |= awp_tma_encode(&c->topo_str_maps.halo[q], f[vo[q]], c->g, hx, hy);
+    }
+    for (int q = 0; q < 4; ++q)
+      bad |= awp_tma_encode(&c->topo_str_maps.media[q], f[sm[q]], c->g, mx, my);
+    for (int q = 0; q < 12; ++q)
+      bad |= awp_tma_encode(&c->topo_str_maps.own[q], f[so[q]], c->g, ox, oy);
+  }
   return bad == 0;
 }
 
@@ -373,8 +396,7 @@ TopoArgs topo_args(awp_ctx* c) {
   a.d1 = f[AWP_D1]; a.lam = f[AWP_LAM]; a.mu = f[AWP_MU]; a.qp = f[AWP_QP]; a.qs = f[AWP_QS];
   a.dcrjx = c->dcrjx; a.dcrjy = c->dcrjy; a.dcrjz = c->dcrjz;
   a.tex = c->tex;
-  memcpy(a.coeff, c->coeff, sizeof(a.coeff));
-  a.qthr = c->qthr;
+  a.thr = c->thr;
   a.slice = c->g.slice; a.yline = c->g.yline;
   a.nx = c->g.nxt; a.ny = c->g.nyt; a.nz = c->g.nzt;
   return a;
@@ -403,8 +425,10 @@ VelArgs make_vel_args(awp_ctx* c) {
 int phase_velocity(awp_ctx* c) {
   const VelArgs v = make_vel_args(c);
   if (c->topo) {  // topo_velocity_*_H replace dvelc[xy] on the top grid (pmcl3d.c:1661-1698)
+    if (!tma_ready(c)) return set_error(AWP_ERR_CUDA, "tensor maps of the curvilinear grid");
     PhaseScope ps(c, 0);
-    CU_TRY(awp_launch_topo_velocity(topo_args(c), c->stream));
+    CU_TRY(awp_launch_topo_velocity(topo_args(c), c->topo_vel_maps, awp_tuning_get("ichunk"),
+                                    c->d_err, c->stream));
     c->launches++;
     return AWP_OK;
   }
@@ -466,8 +490,10 @@ bool stress_split(const awp_ctx* c) {
 int phase_stress(awp_ctx* c) {
   if (c->topo && c->p.nve == 3 && !c->topo_plastic_consistent) return AWP_OK;
   if (c->topo) {  // topo_stress_*_H replace dstrqc on the top grid (pmcl3d.c:1843-1924)
+    if (!tma_ready(c)) return set_error(AWP_ERR_CUDA, "tensor maps of the curvilinear grid");
     PhaseScope ps(c, 1);
-    CU_TRY(awp_launch_topo_stress(topo_args(c), c->elastic, c->stream));
+    CU_TRY(awp_launch_topo_stress(topo_args(c), c->topo_str_maps, c->elastic,
+                                  awp_tuning_get("ichunk"), c->d_err, c->stream));
     c->launches++;
     return AWP_OK;
   }
@@ -929,6 +955,10 @@ int awp_ctx_create(const awp_params* p, awp_ctx** out) {
   c->dth = p->dt / p->dh;
   c->dh1 = 1.0 / p->dh;
   c->qthr = awp::qf_threshold();
+  {
+    const float thr = 2.0f * c->qthr;
+    memcpy(&c->thr, &thr, sizeof(c->thr));
+  }
   int st;
   cudaError_t e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
   if (e != cudaSuccess) {
@@ -977,6 +1007,7 @@ int awp_ctx_create(const awp_params* p, awp_ctx** out) {
     awp::tausub(c->taumin, c->taumax, c->tau8);
     awp::weights_sub(p->ex, p->fac, c->w8, c->coeff);
     awp::texture_tables(c->tau8, c->w8, p->dt, &c->tex);
+    awp::relax_table(c->tex, c->coeff, p->dt, c->dh1, &c->rel);
     c->tex.xls = c->xls;
     c->tex.yls = c->yls;
     c->tex.ny = c->yre - c->yls + 1;
@@ -2489,12 +2520,14 @@ int awp_topography_init(awp_ctx* c, const char* intopo) {
   t.DT = t.nu * h;
   t.dth = t.DT / h;
   t.dh1 = (float)(1.0 / (double)h);
+  awp::relax_table(c->tex, c->coeff, t.DT, t.dh1, &t.rel);
   // stress window of a rank on every domain boundary: ngsl/2 cells in from
   // each side (topo_set_stress_bounds_*, topography.c:379-420)
   t.s_i = std::max(AWP_NGSL / 2 - x0, 0); t.e_i = std::min(nxg - AWP_NGSL / 2 - x0, nx);
   t.s_j = AWP_NGSL / 2; t.e_j = ny - AWP_NGSL / 2;
   c->d_topo = d;
   c->topo = m;
+  c->tma_promo = -1;  // encode the curvilinear kernels' maps too
   return AWP_OK;
 }
 

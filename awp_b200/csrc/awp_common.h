@@ -68,6 +68,12 @@ struct AwpTexture {
   int f_ny, f_nzt; // the finer grid's interior cells in y and z
 };
 
+// Constants of the memory-variable update per texture entry (awp_stencil.cuh,
+// AwpRelax), formed by awp::relax_table for a step's DT and 1/h.
+struct AwpRelaxTab {
+  float vx2[8], wwo[8], kv[8], kr[8], kr2[8], kf[8], c0[8], c1[8], c2[8];
+};
+
 // Parity index of init_texture's visit counters (mesh.c:1103-1137) for the
 // cell (di, dj, kk) relative to the loop start: itx = parity of di + 1, ity =
 // parity of di*ny + dj + 1, itz = parity of nzt*(di*ny + dj + 1) + kk.  Only

@@ -109,7 +109,8 @@ void stress_common(float* xx, float* yy, float* zz, float* xy, float* xz, float*
   a.gx_lim = NX + AWP_NGSL + 1 - gc.nxt * rankx;
   a.gy_min = (NPC == 2) ? INT_MIN : AWP_NGSL + 3 - gc.nyt * ranky;
   a.dth = gc.dth; a.dh1 = gc.dh1; a.dt = s.DT; a.c1 = s.c1; a.c2 = s.c2;
-  a.qthr = s.qthr;
+  const float thr = 2.0f * s.qthr;
+  memcpy(&a.thr, &thr, sizeof(a.thr));
   check(awp_launch_stress(a, false, St), func);
 }
 

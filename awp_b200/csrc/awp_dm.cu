@@ -132,30 +132,22 @@ __global__ void k_dstrqc2(const DmStr2Args a) {
   const float h1w = qf2(__fmul_rn(0.25f, __fadd_rn(qs[pos], qs[pos - 1])), f_wwo, c0, c1);
   const float h2w = qf2(__fmul_rn(0.25f, __fadd_rn(qs[pos], qs[pos - Y])), f_wwo, c0, c1);
   const float h3w = qf2(__fmul_rn(0.25f, __fadd_rn(qs[pos], qs[pos + S])), f_wwo, c0, c1);
-  AwpStrCoef cf;
-  float h = __fmul_rn(__fmul_rn(-xm, hw), a.dh1);
-  float h1 = __fmul_rn(__fmul_rn(-xmu1, h1w), a.dh1);
-  float h2 = __fmul_rn(__fmul_rn(-xmu2, h2w), a.dh1);
-  float h3 = __fmul_rn(__fmul_rn(-xmu3, h3w), a.dh1);
-  qpa = __fmul_rn(__fmul_rn(-qpaw, xl), a.dh1);
-  xm = __fmul_rn(xm, a.dth);
-  xmu1 = __fmul_rn(xmu1, a.dth);
-  xmu2 = __fmul_rn(xmu2, a.dth);
-  xmu3 = __fmul_rn(xmu3, a.dth);
-  xl = __fmul_rn(xl, a.dth);
-  h = __fmul_rn(h, f_vx1);
-  h1 = __fmul_rn(h1, f_vx1);
-  h2 = __fmul_rn(h2, f_vx1);
-  h3 = __fmul_rn(h3, f_vx1);
-  qpa = __fmul_rn(qpa, f_vx1);
-  const float DT = a.dt;
-  cf.xl = xl;
-  cf.xm = __fmaf_rn(DT, h, xm);
-  cf.xmu1 = __fmaf_rn(DT, h1, xmu1);
-  cf.xmu2 = __fmaf_rn(DT, h2, xmu2);
-  cf.xmu3 = __fmaf_rn(DT, h3, xmu3);
-  cf.h = h; cf.h1 = h1; cf.h2 = h2; cf.h3 = h3; cf.qpa = qpa;
-  cf.vx1 = __fmul_rn(DT, __fmaf_rn(f_vx2, f_vx1, 1.0f));
+  // the weights scaled by -vx1/h (awp_stencil.cuh)
+  const float K = -__fmul_rn(a.dh1, f_vx1), DT = a.dt;
+  const float wh = __fmul_rn(hw, K), wq = __fmul_rn(qpaw, K);
+  const float wm[3] = {__fmul_rn(h1w, K), __fmul_rn(h2w, K), __fmul_rn(h3w, K)};
+  const float raw[3] = {xmu1, xmu2, xmu3};
+  AwpStrCoef<float> cf;
+  cf.nh = __fmul_rn(-xm, wh);
+  cf.nxm = __fmul_rn(-xm, __fmaf_rn(DT, wh, a.dth));
+  cf.Q = __fmul_rn(xl, wq);
+  cf.A = __fmul_rn(xl, __fmaf_rn(DT, wq, a.dth));
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+    cf.h[q] = __fmul_rn(raw[q], wm[q]);
+    cf.m[q] = __fmul_rn(raw[q], __fmaf_rn(DT, wm[q], a.dth));
+  }
+  const AwpRelax<float> rx = awp_relax_from(f_vx1, f_vx2, f_wwo, c0, c1, DT, a.dh1);
 
   const DmGrid& g = a.g;
   float d[9];
@@ -170,7 +162,7 @@ __global__ void k_dstrqc2(const DmStr2Args a) {
   d[8] = __fsub_rn(g.w1[pos + Y], g.w1[pos]);
   float sg[6] = {g.xx[pos], g.yy[pos], g.zz[pos], g.xy[pos], g.xz[pos], g.yz[pos]};
   float rr[6] = {a.r1[pos], a.r2[pos], a.r3[pos], a.r4[pos], a.r5[pos], a.r6[pos]};
-  awp_stress_update<false>(sg, rr, cf, f_vx1, f_vx2, f_wwo, DT, dcrj, d);
+  awp_stress_update<false>(sg, rr, cf, rx, dcrj, d);
   g.xx[pos] = sg[0]; g.yy[pos] = sg[1]; g.zz[pos] = sg[2];
   g.xy[pos] = sg[3]; g.xz[pos] = sg[4]; g.yz[pos] = sg[5];
   a.r1[pos] = rr[0]; a.r2[pos] = rr[1]; a.r3[pos] = rr[2];

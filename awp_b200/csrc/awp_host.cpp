@@ -133,6 +133,23 @@ void texture_tables(const float tau8[8], const float w8[8], float dt, AwpTexture
   }
 }
 
+void relax_table(const AwpTexture& t, const float coeff16[16], float DT, float dh1,
+                 AwpRelaxTab* out) {
+  for (int n = 0; n < 8; ++n) {
+    const double v1 = t.tau1[n], v2 = t.tau2[n], w = t.wwo8[n], dt = DT;
+    const double K = -(double)dh1 * v1;
+    out->vx2[n] = t.tau2[n];
+    out->wwo[n] = t.wwo8[n];
+    out->kv[n] = (float)(dt * (1.0 + v2 * v1));
+    out->kr2[n] = (float)(dt * v2 * (1.0 - v1));
+    out->kr[n] = (float)(dt * (1.0 + v2 * v1) + dt * v2 * (1.0 - v1));
+    out->kf[n] = (float)(dt * (w - 1.0));
+    out->c0[n] = (float)(0.25 * coeff16[2 * n] / w * K);
+    out->c1[n] = (float)(0.5 * coeff16[2 * n + 1] / w * K);
+    out->c2[n] = (float)(0.5 * K);
+  }
+}
+
 void inicrj(float arbc, int nxt, int nyt, int nzt, int NX, int NY, int ND,
             int islowest, int npc, float* dcrjx, float* dcrjy, float* dcrjz) {
   (void)nzt;

@@ -20,6 +20,12 @@ bool weights_sub(float ex, float fac, float w8[8], float coeff16[16]);
 // tau1/tau2 of pmcl3d.c:1036-1049 and the texture tables of init_texture.
 void texture_tables(const float tau8[8], const float w8[8], float dt, AwpTexture* t);
 
+// Products of the relaxation tables, the Q(f) coefficients, DT and 1/h that the
+// memory-variable update uses (AwpRelax of awp_stencil.cuh), in double and
+// rounded once.
+void relax_table(const AwpTexture& t, const float coeff16[16], float DT, float dh1,
+                 AwpRelaxTab* out);
+
 // inicrj (cerjan.c:5-64) for a single rank (coords 0,0).
 void inicrj(float arbc, int nxt, int nyt, int nzt, int NX, int NY, int ND,
             int islowest, int npc, float* dcrjx, float* dcrjy, float* dcrjz);

@@ -79,9 +79,9 @@ __device__ __forceinline__ void vel_tile(const VelArgs& a, const int bx, const i
     const float d_0jk = LDG(D + o - Y - 1);
     const float yz_0 = LDG(YZ + o);
 
-    const float fd1 = awp_vel_factor(dth, d_0, d_0j, d_0k, d_0jk);
-    const float fd2 = awp_vel_factor(dth, d_0, d_p, d_0k, d_pk);
-    const float fd3 = awp_vel_factor(dth, d_0, d_p, d_0j, d_pj);
+    const float fd1 = awp_vel_factor(dth, vadd(d_0, d_0j), vadd(d_0k, d_0jk));
+    const float fd2 = awp_vel_factor(dth, vadd(d_0, d_p), vadd(d_0k, d_pk));
+    const float fd3 = awp_vel_factor(dth, vadd(d_0, d_p), vadd(d_0j, d_pj));
     const float dcrj = LDG(a.dcrjx + i) * dcy * dcz;
 
     U[o] = awp_vel_update(U[o], fd1, c1, c2, xx_0 - xx_m1, xx_p1 - xx_m2,
@@ -111,23 +111,21 @@ __global__ void __launch_bounds__(32 * TY)
 // Stress + attenuation (dstrqc, kernel.cu:880-1197)
 // ===========================================================================
 
-struct Plane4 {  // one field at (j,k), (j-1,k), (j,k-1), (j-1,k-1) of a plane
-  float a, b, c, d;
+// One material field in one x plane at a cell's column: the value, the sums
+// over j, j-1 at k and over the four values at k, k-1.
+struct MatPlane {
+  float m, t, q;  // (j, k); (j, k) + (j-1, k); t(k) + t(k-1)
+  float pk;       // (j, k) + (j, k-1)
 };
 
-__device__ __forceinline__ Plane4 load4(const float* __restrict__ p, int Y) {
-  Plane4 r;
-  r.a = LDG(p);
-  r.b = LDG(p - Y);
-  r.c = LDG(p - 1);
-  r.d = LDG(p - Y - 1);
+__device__ __forceinline__ MatPlane mat_plane(const float* __restrict__ p, int Y) {
+  MatPlane r;
+  const float a = LDG(p), b = LDG(p - Y), c = LDG(p - 1), d = LDG(p - Y - 1);
+  r.m = a;
+  r.t = vadd(a, b);
+  r.q = awp_quad(r.t, vadd(c, d));
+  r.pk = vadd(a, c);
   return r;
-}
-
-// Sum of the 8 cell values around an edge in the reference's order:
-// pos, ip1, jm1, ijk, km1, ik1, jk1, ijk1.
-__device__ __forceinline__ float sum8(const Plane4& c, const Plane4& n) {
-  return c.a + n.a + c.b + n.b + c.c + n.c + c.d + n.d;
 }
 
 template <bool ELASTIC, bool TEXARR, int TY>
@@ -162,11 +160,11 @@ __device__ __forceinline__ void str_tile(const StrArgs& a, const int bx, const i
   float u_m1 = LDG(U + o - S), u_0 = LDG(U + o), u_p1 = LDG(U + o + S);
   float v_m2 = LDG(V + o - 2 * S), v_m1 = LDG(V + o - S), v_0 = LDG(V + o);
   float w_m2 = LDG(W + o - 2 * S), w_m1 = LDG(W + o - S), w_0 = LDG(W + o);
-  Plane4 lam_c = load4(LAM + o, Y), mu_c = load4(MU + o, Y);
-  Plane4 qp_c{0.f, 0.f, 0.f, 0.f}, qs_c{0.f, 0.f, 0.f, 0.f};
+  MatPlane lam_c = mat_plane(LAM + o, Y), mu_c = mat_plane(MU + o, Y);
+  MatPlane qp_c{0.f, 0.f, 0.f, 0.f}, qs_c{0.f, 0.f, 0.f, 0.f};
   if (!ELASTIC) {
-    qp_c = load4(QP + o, Y);
-    qs_c = load4(QS + o, Y);
+    qp_c = mat_plane(QP + o, Y);
+    qs_c = mat_plane(QS + o, Y);
   }
 
   for (int i = ib; i <= ie; ++i, o += S) {
@@ -181,11 +179,11 @@ __device__ __forceinline__ void str_tile(const StrArgs& a, const int bx, const i
     const float u_p2 = LDG(U + o + 2 * S);
     const float v_p1 = LDG(V + o + S);
     const float w_p1 = LDG(W + o + S);
-    const Plane4 lam_n = load4(LAM + o + S, Y), mu_n = load4(MU + o + S, Y);
-    Plane4 qp_n{0.f, 0.f, 0.f, 0.f}, qs_n{0.f, 0.f, 0.f, 0.f};
+    const MatPlane lam_n = mat_plane(LAM + o + S, Y), mu_n = mat_plane(MU + o + S, Y);
+    MatPlane qp_n{0.f, 0.f, 0.f, 0.f}, qs_n{0.f, 0.f, 0.f, 0.f};
     if (!ELASTIC) {
-      qp_n = load4(QP + o + S, Y);
-      qs_n = load4(QS + o + S, Y);
+      qp_n = mat_plane(QP + o + S, Y);
+      qs_n = mat_plane(QS + o + S, Y);
     }
     const float u_jp1 = LDG(U + o + Y), u_jp2 = LDG(U + o + 2 * Y), u_jm1 = LDG(U + o - Y);
     const float u_km1 = LDG(U + o - 1);
@@ -196,38 +194,24 @@ __device__ __forceinline__ void str_tile(const StrArgs& a, const int bx, const i
     float uk1 = LDG(U + o + 1), vk1 = LDG(V + o + 1), wk1 = LDG(W + o + 1);
     float uk2 = LDG(U + o + 2), vk2 = LDG(V + o + 2);
 
-    // memory-variable coefficients for this cell
-    float f_vx1, f_vx2, f_wwo;
-    int cidx;
-    if (TEXARR) {
-      const long long p = col + o;
-      f_vx1 = LDG(a.vx1 + p);
-      f_vx2 = LDG(a.vx2 + p);
-      f_wwo = LDG(a.wwo + p);
-      cidx = 2 * LDG(a.ww + p) - 2;
-    } else {
-      const int t = awp_tex_index(a.tex, i, j, k);
-      f_vx1 = a.tex.tau1[t];
-      f_vx2 = a.tex.tau2[t];
-      f_wwo = a.tex.wwo8[t];
-      cidx = 2 * t;
-    }
-    const float dcrj = LDG(a.dcrjx + i) * dcy * dcz;
-
-    float cc0 = 0.f, cc1 = 0.f;
+    // memory-variable constants of this cell
+    AwpRelax<float> rx{};
     if (!ELASTIC) {
-      if (a.coeff_dev) {
-        cc0 = LDG(a.coeff_dev + cidx);
-        cc1 = LDG(a.coeff_dev + cidx + 1);
+      if (TEXARR) {
+        const long long p = col + o;
+        const int e = 2 * LDG(a.ww + p) - 2;
+        rx = awp_relax_from(LDG(a.vx1 + p), LDG(a.vx2 + p), LDG(a.wwo + p),
+                            LDG(a.coeff_dev + e), LDG(a.coeff_dev + e + 1), DT, dh1);
       } else {
-        cc0 = a.coeff[cidx];
-        cc1 = a.coeff[cidx + 1];
+        rx = awp_relax_at(a.rel, awp_tex_index(a.tex, i, j, k));
       }
     }
-    const AwpStrCoef cf = awp_stress_coef<ELASTIC>(
-        sum8(lam_c, lam_n), sum8(mu_c, mu_n), mu_c.a, mu_c.c, mu_c.b, mu_n.a,
-        sum8(qp_c, qp_n), sum8(qs_c, qs_n), qs_c.a, qs_c.c, qs_c.b, qs_n.a, f_vx1, f_vx2, f_wwo,
-        cc0, cc1, a.qthr, dth, dh1, DT);
+    const float dcrj = LDG(a.dcrjx + i) * dcy * dcz;
+    const float P[3] = {mu_c.pk, mu_c.t, vadd(mu_c.m, mu_n.m)};
+    const float R[3] = {qs_c.pk, qs_c.t, vadd(qs_c.m, qs_n.m)};
+    const AwpStrCoef<float> cf = awp_stress_coef<ELASTIC>(
+        vadd(lam_c.q, lam_n.q), vadd(mu_c.q, mu_n.q), P, vadd(qp_c.q, qp_n.q),
+        vadd(qs_c.q, qs_n.q), R, rx, a.thr, dth, DT);
 
     // velocities at k+1 / k+2 that fall on the free-surface image layer
     // (computed here in registers; kernel.cu:1087-1112)
@@ -261,7 +245,7 @@ __device__ __forceinline__ void str_tile(const StrArgs& a, const int bx, const i
     d[7] = awp_d4(c1, c2, vk1, v_0, vk2, v_km1);
     d[8] = awp_d4(c1, c2, w_jp1, w_0, w_jp2, w_jm1);
 
-    awp_stress_update<ELASTIC>(sg, rr, cf, f_vx1, f_vx2, f_wwo, DT, dcrj, d);
+    awp_stress_update<ELASTIC>(sg, rr, cf, rx, dcrj, d);
 #pragma unroll
     for (int q = 0; q < 6; ++q) SG[q][o] = sg[q];
     if (!ELASTIC) {

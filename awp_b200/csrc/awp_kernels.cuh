@@ -34,8 +34,8 @@ struct StrArgs {
   const float *vx1, *vx2, *wwo;
   const int* ww;
   AwpTexture tex;
-  float coeff[16];
-  const float* coeff_dev;  // when set, the Q(f) table is read from device memory
+  AwpRelaxTab rel;         // per texture entry, with the step's DT and 1/h
+  const float* coeff_dev;  // with the explicit arrays: the Q(f) table (8 pairs)
   int slice, yline, lam_mu_ld;
   int i0, i1, j0, j1, k0, k1;
   int fs;        // 1: free-surface images at k = ktop (grid 0)
@@ -43,7 +43,9 @@ struct StrArgs {
   int gx_lim;    // image at i+1 exists while i < gx_lim   (kernel.cu:1092)
   int gy_min;    // image at j-1 exists while j >= gy_min  (kernel.cu:1097)
   float dth, dh1, dt, c1, c2;
-  float qthr;    // smallest float x with 1/(double)x <= 200 (Q(f) switch)
+  // bit pattern of 2*qthr, qthr the smallest float x with 1/(double)x <= 200:
+  // the Q(f) switch on a pair sum of Q^-1
+  unsigned thr;
 };
 
 // ---------------------------------------------------------------------------

@@ -1,573 +1,509 @@
 // TMA-pipelined stencil kernels for the context API (sm_100a).
 //
 // Each CTA owns a tile of 32 k (one 128-byte line) x 8 j and marches a chunk of
-// x planes.  Per plane, one elected thread issues cp.async.bulk.tensor loads of
-// the plane's tiles (with the j/k halo the stencil needs) into shared-memory
-// rings; completion is tracked by one mbarrier per ring slot.  The loads run
-// several planes ahead of the arithmetic, so the HBM latency is hidden by the
-// pipeline rather than by occupancy, and every x plane of every field is read
-// from HBM once per chunk.  Results are stored straight from registers with
-// coalesced 128-byte rows.
+// x planes.  A producer warp issues cp.async.bulk.tensor loads of each plane's
+// tiles (with the j/k halo the stencil needs) into shared-memory rings, one
+// or two planes ahead of the arithmetic; four consumer warps compute, each
+// thread two vertically adjacent cells with packed arithmetic (awp_f2.cuh).
+// What the x stencil needs of a cell's own column travels in registers, so a
+// tile stays in shared memory only while its neighbours in j and k are read.
+// Results are stored straight from registers, one full 128-byte line per half
+// warp.
+//
+// Measured at 512 x 512 x 256, anelastic (us per launch, share of the measured
+// copy bandwidth on the algorithmic bytes), against the form before (256
+// threads, one cell each, every x neighbour from shared memory, one barrier of
+// the CTA per plane, 554 thread instructions a cell in the stress update):
+//   velocity  800 -> 556 (0.66 -> 0.96),  stress 1815 -> 1385 (0.70 -> 0.92).
 //
 // Tile boxes (x = k fastest, y = j, z = i), all 16-byte aligned in x:
-//   halo   : k in [kb-4, kb+36), j in [jb-2, jb+10)   40 x 12 floats
-//   media  : k in [kb-4, kb+32), j in [jb-1, jb+8)    36 x  9 floats
-//   own    : k in [kb,   kb+32), j in [jb,   jb+8)    32 x  8 floats
+//   halo   : 40 x 11 floats, k in [kb-4, kb+36), j from jb-1 or jb-2
+//   media  : 36 x  9 floats, k in [kb-4, kb+32), j in [jb-1, jb+8)
+//   own    : 32 x  8 floats; with a j halo 32 x 11, with a k halo 40 x 8
 //
-// Every wait on an mbarrier is bounded; a wait that runs out sets the
-// context's error word and the whole CTA leaves the march together.
+// Synchronisation: a full mbarrier per ring stage (the copies' bytes), and a
+// ring of "step done" mbarriers on which the consumer warps arrive and the
+// producer waits before it refills what that step read last; no barrier of
+// the whole CTA in the march.  Every wait is bounded; a wait that runs out
+// sets the context's error word, its warp leaves the march, the others follow
+// when their own waits run out, and the producer drains the copies in flight
+// before the CTA ends.
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <cudaTypedefs.h>
 #include <math.h>
 #include <stdint.h>
 
+#include <algorithm>
+#include <atomic>
+
 #include "awp_kernels.cuh"
+#include "awp_pipe.cuh"
 #include "awp_stencil.cuh"
 #include "awp_tma.cuh"
 
 #define LDG(p) __ldg(p)
 
+using namespace awp_pipe;
+
 namespace {
 
-constexpr int TZ = 32, TY = 8, NT = TZ * TY;
-constexpr int HX = 40, HY = 12, HTILE = HX * HY;     // halo tile (floats)
-constexpr int MX = 36, MY = 9, MTILE_B = MX * MY * 4; // media tile bytes (1296)
-constexpr int MTILE = 352;                            // media tile stride (floats, 1408 B)
-constexpr int OTILE = TZ * TY;                        // own tile (floats)
-constexpr int DH_ = 7;                                // halo ring depth (planes i-2..i+2 + 2)
-constexpr int DM_ = 4;                                // media ring depth (planes i, i+1 + 2)
-constexpr int DO_ = 3;                                // own ring depth (plane i + 2)
-// Poll limit of the pipeline waits: the default, and the one the drain of an
-// aborted march always uses (copies already issued must land before the CTA
-// releases its shared memory, whatever limit the march itself ran with).
-constexpr unsigned kSpinLimit = 1u << 26;
-// velocity kernel: each stress field is staged with only the halo its
-// differences read (xx none, yy and xy j, zz and xz k, yz both), one slot of
-// the ring holding the six tiles at 128-byte multiples
-constexpr int VT_XX = 0, VT_YY = 256, VT_ZZ = 640, VT_XY = 960, VT_XZ = 1344, VT_YZ = 1664,
-              VT_SLOT = 2144;
-constexpr int VJ = TZ;  // row stride of the j-halo tiles (32 x 12)
-constexpr int VK = HX;  // row stride of the k-halo tiles (40 x 8) and of yz (40 x 12)
-
-__device__ __forceinline__ unsigned smem_u32(const void* p) {
-  return static_cast<unsigned>(__cvta_generic_to_shared(p));
-}
-__device__ __forceinline__ void mbar_init(uint64_t* bar, unsigned count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count)
-               : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, unsigned bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)),
-               "r"(bytes)
-               : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, unsigned parity) {
-  unsigned ok;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-      " selp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-// bounded wait: false when the limit ran out
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity,
-                                          unsigned limit = kSpinLimit) {
-  for (unsigned n = 0; n < limit; ++n)
-    if (mbar_try_wait(bar, parity)) return true;
-  return false;
-}
-__device__ __forceinline__ void tma_load3(void* dst, const CUtensorMap* map, uint64_t* bar,
-                                          int x, int y, int z) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(smem_u32(dst)),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
-      : "memory");
-}
-
-// One ring of per-plane slots with their mbarriers.
-struct Ring {
-  float* buf;
-  uint64_t* bar;
-  int depth, slot_floats, base;  // base = first plane of the march for this ring
-  __device__ int slot(int p) const { return (p - base) % depth; }
-  __device__ unsigned parity(int p) const { return ((p - base) / depth) & 1; }
-  __device__ uint64_t* b(int p) const { return bar + slot(p); }
-};
-
-// Slot and mbarrier phase of one plane in a ring: plane p of a march lives in
-// slot (p - base) % depth with phase ((p - base) / depth) & 1; the march
-// advances these incrementally instead of dividing.
-struct Cursor {
-  int slot;
-  unsigned phase;
-  __device__ void next(int depth) {
-    if (++slot == depth) {
-      slot = 0;
-      phase ^= 1u;
-    }
-  }
-};
-__device__ __forceinline__ int wrap_add(int s, int d, int depth) {
-  s += d;
-  return s >= depth ? s - depth : s;
-}
-
+constexpr int TZ = 32, TY = 8;
+constexpr int NC = TZ * TY / 2;       // consumer threads (two cells each)
+constexpr int NT = NC + 32;           // and the producer warp
+constexpr int HX = 40, HY = 11;       // halo box
+constexpr int HTILE = 448;            // its slot (floats, a multiple of 128 B)
+constexpr int MX = 36, MY = 9, MTILE = 352;  // media box and slot
+constexpr int OTILE = TZ * TY;        // own box and slot
+constexpr int JTILE = TZ * HY;        // j-halo box (32 x 11) and slot (352)
+constexpr int KTILE = HX * TY;        // k-halo box (40 x 8) and slot (320)
 // ===========================================================================
-// Stress + memory variables (dstrqc, kernel.cu:880-1197), same arithmetic as
+// Stress + memory variables (dstrqc, kernel.cu:880-1197), same bits as
 // k_stress in awp_kernels.cu (see there for the term-by-term citation).
+//
+// Bound by DRAM: 124 bytes a cell and the halo.  Halo/media stages run two
+// planes ahead, the cell's own twelve fields one: 63 KB of rings, three CTAs
+// (twelve computing warps) per SM.
 // ===========================================================================
 template <bool ELASTIC>
-__global__ void __launch_bounds__(NT, 2)
-    k_stress_tma(const StrArgs a, const __grid_constant__ TmaMaps tm, const int ichunk,
+struct StrCfg {
+  static constexpr int NM = ELASTIC ? 2 : 4;   // lam, mu (, qp, qs)
+  static constexpr int NO_ = ELASTIC ? 6 : 12;  // xx..yz (, r1..r6)
+  static constexpr int LH = 2, LO = 1;         // planes ahead
+  static constexpr int NH = 1 + LH, NO = 1 + LO;
+  static constexpr int DU = 3 + LH;            // u: planes i .. i+2 and the ones ahead
+  static constexpr int DV = 2 + LH;            // v, w: planes i, i+1 and the ones ahead
+  static constexpr int F_U = 0, F_V = F_U + DU * HTILE, F_W = F_V + DV * HTILE,
+                       F_M = F_W + DV * HTILE, F_O = F_M + NH * NM * MTILE,
+                       F_T = F_O + NO * NO_ * OTILE;  // relaxation table
+  static constexpr int kTab = ELASTIC ? 0 : 4 * 20;
+  static constexpr size_t bytes = sizeof(float) * (F_T + kTab) + sizeof(Pipe<NH, NO, NC / 32>);
+};
+
+template <bool ELASTIC>
+__global__ void __launch_bounds__(NT, ELASTIC ? 4 : 3)
+    k_stress_tma(const __grid_constant__ StrArgs a, const __grid_constant__ TmaMaps tm, const int ichunk,
                  int* err, const unsigned spin) {
-  constexpr int NM = ELASTIC ? 2 : 4;   // lam, mu (, qp, qs)
-  constexpr int NO = ELASTIC ? 6 : 12;  // xx..yz (, r1..r6)
+  using C = StrCfg<ELASTIC>;
+  constexpr int NM = C::NM, NO = C::NO_;
   extern __shared__ __align__(128) float smem[];
-  const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TZ + tx;
+  auto& pipe = *reinterpret_cast<Pipe<C::NH, C::NO, NC / 32>*>(smem + C::F_T + C::kTab);
+  const int tid = threadIdx.x;
   const int kb = AWP_ALIGN + blockIdx.x * TZ;
   const int jb = a.j0 + blockIdx.y * TY;
-  const int k = kb + tx, j = jb + ty;
   const int ib = a.i0 + blockIdx.z * ichunk;
   const int ie = min(ib + ichunk - 1, a.i1);
-  const bool active = (k >= a.k0) && (k <= a.k1) && (j <= a.j1);
+  const int n = ie - ib + 1;
 
-  Ring rh{smem, nullptr, DH_, 3 * HTILE, ib - 2};
-  Ring rm{rh.buf + DH_ * 3 * HTILE, nullptr, DM_, NM * MTILE, ib};
-  Ring ro{rm.buf + DM_ * NM * MTILE, nullptr, DO_, NO * OTILE, ib};
-  uint64_t* bars = reinterpret_cast<uint64_t*>(ro.buf + DO_ * NO * OTILE);
-  rh.bar = bars;
-  rm.bar = bars + DH_;
-  ro.bar = bars + DH_ + DM_;
-
-  // producer: one thread issues a plane's tiles and arms its barrier
-  // producer (thread 0): slot of the next plane each ring receives
-  int ish = 0, ism = 0, iso = 0;
-  auto issue_halo = [&](int p) {
-    if (p > ie + 2) return;
-    uint64_t* b = rh.bar + ish;
-    mbar_expect_tx(b, 3 * HTILE * 4);
-    float* d = rh.buf + ish * rh.slot_floats;
-    for (int f = 0; f < 3; ++f) tma_load3(d + f * HTILE, &tm.halo[f], b, kb - 4, jb - 2, p);
-    ish = wrap_add(ish, 1, DH_);
-  };
-  auto issue_media = [&](int p) {
-    if (p > ie + 1) return;
-    uint64_t* b = rm.bar + ism;
-    mbar_expect_tx(b, NM * MTILE_B);
-    float* d = rm.buf + ism * rm.slot_floats;
-    for (int f = 0; f < NM; ++f) tma_load3(d + f * MTILE, &tm.media[f], b, kb - 4, jb - 1, p);
-    ism = wrap_add(ism, 1, DM_);
-  };
-  auto issue_own = [&](int p) {
-    if (p > ie) return;
-    uint64_t* b = ro.bar + iso;
-    mbar_expect_tx(b, NO * OTILE * 4);
-    float* d = ro.buf + iso * ro.slot_floats;
-    for (int f = 0; f < NO; ++f) tma_load3(d + f * OTILE, &tm.own[f], b, kb, jb, p);
-    iso = wrap_add(iso, 1, DO_);
-  };
-
-  if (tid == 0) {
-    for (int q = 0; q < DH_ + DM_ + DO_; ++q) mbar_init(bars + q, 1);
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  if (tid == 0) pipe.init();
+  if (!ELASTIC) {
+    // relaxation constants of the entry pairs (e, e + 1), e even, that two
+    // adjacent levels take: nine float2 per pair in 20 floats
+    float* tab = smem + C::F_T;
+    const float* const src[9] = {a.rel.vx2, a.rel.wwo, a.rel.kv, a.rel.kr, a.rel.kr2,
+                                 a.rel.kf,  a.rel.c0,  a.rel.c1, a.rel.c2};
+#pragma unroll
+    for (int q = 0; q < 9; ++q)
+      if (tid < 8) tab[(tid >> 1) * 20 + 2 * q + (tid & 1)] = src[q][tid];
   }
   __syncthreads();
-  // next plane to issue per ring (meaningful in the producer thread only)
-  int nh = ib - 2, nm = ib, no = ib;
-  if (tid == 0) {
-    for (; nh < ib - 2 + DH_; ++nh) issue_halo(nh);
-    for (; nm < ib + DM_; ++nm) issue_media(nm);
-    for (; no < ib + DO_; ++no) issue_own(no);
+
+  if (tid >= NC) {  // producer warp
+    if (tid == NC) {
+      pipe.produce(
+          n,
+          [&](int s, uint64_t* b) {
+            // the first stage also brings the planes the later ones find there
+            const int u0 = s == 0 ? 0 : s + 2, v0 = s == 0 ? 0 : s + 1;
+            mbar_expect_tx(b, ((s + 2 - u0 + 1) + 2 * (s + 1 - v0 + 1)) * HX * HY * 4 +
+                                  NM * MX * MY * 4);
+            for (int p = u0; p <= s + 2; ++p)
+              tma_load3(smem + C::F_U + (p % C::DU) * HTILE, &tm.halo[0], b, kb - 4, jb - 1,
+                        ib + p);
+            for (int p = v0; p <= s + 1; ++p) {
+              tma_load3(smem + C::F_V + (p % C::DV) * HTILE, &tm.halo[1], b, kb - 4, jb - 2,
+                        ib + p);
+              tma_load3(smem + C::F_W + (p % C::DV) * HTILE, &tm.halo[2], b, kb - 4, jb - 1,
+                        ib + p);
+            }
+            float* m = smem + C::F_M + (s % C::NH) * NM * MTILE;
+            for (int f = 0; f < NM; ++f)
+              tma_load3(m + f * MTILE, &tm.media[f], b, kb - 4, jb - 1, ib + s + 1);
+          },
+          [&](int s, uint64_t* b) {
+            mbar_expect_tx(b, NO * OTILE * 4);
+            float* o = smem + C::F_O + (s % C::NO) * NO * OTILE;
+            for (int f = 0; f < NO; ++f)
+              tma_load3(o + f * OTILE, &tm.own[f], b, kb, jb, ib + s);
+          },
+          err, spin);
+    }
+    return;
   }
 
+  const int row = tid >> 4, kp = (tid & 15) * 2;
+  const int k = kb + kp, j = jb + row;
+  const bool jin = j <= a.j1;
+  const bool ax = jin && k >= a.k0 && k <= a.k1, ay = jin && k + 1 >= a.k0 && k + 1 <= a.k1;
   const int S = a.slice, Y = a.yline;
-  const float c1 = a.c1, c2 = a.c2, DT = a.dt, dth = a.dth, dh1 = a.dh1;
-  const float dcy = LDG(a.dcrjy + min(j, a.j1)), dcz = LDG(a.dcrjz + min(max(k, a.k0), a.k1));
+  const float c1 = a.c1, c2 = a.c2;
   const long long col = (long long)j * Y + k;
-  const bool top = a.fs && (k == a.ktop);
-  const bool top1 = a.fs && (k == a.ktop - 1);
+  const float dcy = LDG(a.dcrjy + min(j, a.j1));
+  const float2 dcz = make_float2(LDG(a.dcrjz + min(max(k, a.k0), a.k1)),
+                                 LDG(a.dcrjz + min(max(k + 1, a.k0), a.k1)));
+  // the pair (ktop - 1, ktop): nzt is even, so the surface is a second level
+  const bool top = a.fs && (k + 1 == a.ktop);
   float* __restrict__ SG[6] = {a.xx, a.yy, a.zz, a.xy, a.xz, a.yz};
   float* __restrict__ RR[6] = {a.r1, a.r2, a.r3, a.r4, a.r5, a.r6};
-  const int hoff = (ty + 2) * HX + (tx + 4);
-  const int moff = (ty + 1) * MX + (tx + 4);
-  const int ooff = ty * TZ + tx;
-  bool ok = true, aborted = false;
-
-  // consumers: the plane each ring waits for next (halo i+2, media i+1, own i)
-  // and the slots of the oldest planes read (halo i-2, media i)
-  Cursor wh{4, 0u}, wm{1, 0u}, wo{0, 0u};
-  int sh = 0, sm = 0;
-  // media of the current x plane at (j,k), (j-1,k), (j,k-1), (j-1,k-1): the
-  // next plane's values of one step are the current plane's of the next
-  float cl[4], cmu[4], cqp[4], cqs[4];
-  // relaxation-table entries of this (j, k) column.  The table index depends
-  // on the parity of i only (period 2 along the march), so both are read once
-  // here instead of per plane, where the lanes of a warp (alternating k
-  // parity) would split each constant-bank read in two.
-  float tv1[2], tv2[2], twwo[2], tc0[2] = {0.f, 0.f}, tc1[2] = {0.f, 0.f};
+  // texture entries of the two levels at even and odd steps
+  int e0[2], e1[2];
 #pragma unroll
   for (int q = 0; q < 2; ++q) {
-    const int t = awp_tex_index(a.tex, ib + q, j, k);
-    tv1[q] = a.tex.tau1[t];
-    tv2[q] = a.tex.tau2[t];
-    twwo[q] = a.tex.wwo8[t];
+    e0[q] = awp_tex_index(a.tex, ib + q, j, k);
+    e1[q] = awp_tex_index(a.tex, ib + q, j, k + 1);
+  }
+
+  // own-column values of the planes before the ones the tiles bring, and the
+  // media sums of the first plane, straight from global memory
+  long long o = (long long)ib * S + col;
+  float2 u_m1, u_0, u_p1, v_m2, v_m1, v_0, w_m2, w_m1, w_0;
+  {
+    const float *U = a.u1 + o, *V = a.v1 + o, *W = a.w1 + o;
+    u_m1 = ldg2(U - S); u_0 = ldg2(U); u_p1 = ldg2(U + S);
+    v_m2 = ldg2(V - 2 * (long long)S); v_m1 = ldg2(V - S); v_0 = ldg2(V);
+    w_m2 = ldg2(W - 2 * (long long)S); w_m1 = ldg2(W - S); w_0 = ldg2(W);
+  }
+  // one media field in one plane: value, sum with j-1, that sum plus the one a
+  // level below, and the pair sum with the level below
+  struct Mat {
+    float2 m, t, q, pk;
+  };
+  auto mat = [&](float2 A, float Ak, float2 B, float Bk) {  // rows j, j-1; k-1 values
+    Mat r;
+    r.m = A;
+    r.t = vadd(A, B);
+    const float tk = vadd(Ak, Bk);
+    r.q = awp_quad(r.t, make_float2(tk, r.t.x));
+    r.pk = vadd(A, make_float2(Ak, A.x));
+    return r;
+  };
+  auto mat_g = [&](const float* p) { return mat(ldg2(p), p[-1], ldg2(p - Y), p[-Y - 1]); };
+  auto mat_s = [&](const float* p) { return mat(lds2(p), p[-1], lds2(p - MX), p[-MX - 1]); };
+  float2 Lq, Mq, Mt, Mm, Mk, Pq = {}, Rq = {}, Rt = {}, Rm = {}, Rk = {};
+  {
+    Lq = mat_g(a.lam + o).q;
+    const Mat m = mat_g(a.mu + o);
+    Mq = m.q; Mt = m.t; Mm = m.m; Mk = m.pk;
     if (!ELASTIC) {
-      tc0[q] = a.coeff[2 * t];
-      tc1[q] = a.coeff[2 * t + 1];
+      Pq = mat_g(a.qp + o).q;
+      const Mat r = mat_g(a.qs + o);
+      Rq = r.q; Rt = r.t; Rm = r.m; Rk = r.pk;
     }
   }
-  for (int i = ib; i <= ie; ++i) {
-    // ---- wait for the planes this step reads for the first time ------------
-    if (i == ib) {
-      for (int q = 0; q < 4 && ok; ++q) ok = mbar_wait(rh.bar + q, 0u, spin);  // ib-2..ib+1
-      if (ok) ok = mbar_wait(rm.bar, 0u, spin);                                  // plane ib
-    }
-    if (ok) ok = mbar_wait(rh.bar + wh.slot, wh.phase, spin);
-    if (ok) ok = mbar_wait(rm.bar + wm.slot, wm.phase, spin);
-    if (ok) ok = mbar_wait(ro.bar + wo.slot, wo.phase, spin);
-    // one barrier per plane: it also tells the producer that every thread is
-    // done with the previous step's oldest planes, whose slots it refills
-    if (__syncthreads_or(!ok)) {
-      aborted = true;
-      break;
-    }
-    if (tid == 0 && i > ib) {
-      issue_halo(nh++);
-      issue_media(nm++);
-      issue_own(no++);
-    }
-    const int sh1 = wrap_add(sh, 1, DH_), sh2 = wrap_add(sh, 2, DH_), sh3 = wrap_add(sh, 3, DH_),
-              sh4 = wrap_add(sh, 4, DH_), sm1 = wrap_add(sm, 1, DM_);
+  const int hu = (row + 1) * HX + kp + 4, hv = (row + 2) * HX + kp + 4;
+  const int hm = (row + 1) * MX + kp + 4, ho = row * TZ + kp;
 
-    const float* Hm2 = rh.buf + sh * rh.slot_floats + hoff;
-    const float* Hm1 = rh.buf + sh1 * rh.slot_floats + hoff;
-    const float* H0 = rh.buf + sh2 * rh.slot_floats + hoff;
-    const float* Hp1 = rh.buf + sh3 * rh.slot_floats + hoff;
-    const float* Hp2 = rh.buf + sh4 * rh.slot_floats + hoff;
-    // field f of a halo plane: + f * HTILE; neighbour (dj, dk): + dj * HX + dk
-    const float u_m1 = Hm1[0], u_0 = H0[0], u_p1 = Hp1[0], u_p2 = Hp2[0];
-    const float v_m2 = Hm2[HTILE], v_m1 = Hm1[HTILE], v_0 = H0[HTILE], v_p1 = Hp1[HTILE];
-    const float w_m2 = Hm2[2 * HTILE], w_m1 = Hm1[2 * HTILE], w_0 = H0[2 * HTILE],
-                w_p1 = Hp1[2 * HTILE];
-    const float* U0 = H0;
-    const float* V0 = H0 + HTILE;
-    const float* W0 = H0 + 2 * HTILE;
-    const float u_jp1 = U0[HX], u_jp2 = U0[2 * HX], u_jm1 = U0[-HX], u_km1 = U0[-1];
-    const float v_jm1 = V0[-HX], v_jp1 = V0[HX], v_jm2 = V0[-2 * HX], v_km1 = V0[-1];
-    const float w_km1 = W0[-1], w_km2 = W0[-2], w_jp1 = W0[HX], w_jp2 = W0[2 * HX],
-                w_jm1 = W0[-HX];
-    float uk1 = U0[1], vk1 = V0[1], wk1 = W0[1], uk2 = U0[2], vk2 = V0[2];
+  Cursor<C::NH> ch;
+  Cursor<C::NO> co;
+  Cursor<awp_pipe::ND> cd;
+  int su = 0, su2 = 2, sv = 0, sv1 = 1;  // slots of u planes i, i+2 and v, w planes i, i+1
+  bool ok = true;
+#pragma unroll 1
+  for (int s = 0; s < n; ++s) {
+    ok = mbar_wait(pipe.full_h + ch.slot, ch.phase, spin);
+    if (!__all_sync(0xffffffffu, ok)) break;
+    const float* U0 = smem + C::F_U + su * HTILE + hu;
+    const float* V0 = smem + C::F_V + sv * HTILE + hv;
+    const float* W0 = smem + C::F_W + sv * HTILE + hu;
+    const float2 u_p2 = lds2(smem + C::F_U + su2 * HTILE + hu);
+    const float2 v_p1 = lds2(smem + C::F_V + sv1 * HTILE + hv);
+    const float2 w_p1 = lds2(smem + C::F_W + sv1 * HTILE + hu);
+    const float2 u_jm1 = lds2(U0 - HX), u_jp1 = lds2(U0 + HX), u_jp2 = lds2(U0 + 2 * HX);
+    const float2 v_jm2 = lds2(V0 - 2 * HX), v_jm1 = lds2(V0 - HX), v_jp1 = lds2(V0 + HX);
+    const float2 w_jm1 = lds2(W0 - HX), w_jp1 = lds2(W0 + HX), w_jp2 = lds2(W0 + 2 * HX);
+    // k neighbours: the level below and the pair above (u, v), the pair below
+    // and the level above (w)
+    const float u_km1 = U0[-1], v_km1 = V0[-1];
+    float2 u_kp = lds2(U0 + 2), v_kp = lds2(V0 + 2);
+    const float2 w_km = lds2(W0 - 2);
+    float w_kp = W0[2];
 
-    const float* Mc = rm.buf + sm * rm.slot_floats + moff;
-    const float* Mn = rm.buf + sm1 * rm.slot_floats + moff;
-    // (j,k), (j-1,k), (j,k-1), (j-1,k-1) of a media tile
-    auto m4 = [&](const float* m, int f, float& pa, float& pb, float& pc, float& pd) {
-      const float* q = m + f * MTILE;
-      pa = q[0];
-      pb = q[-MX];
-      pc = q[-1];
-      pd = q[-MX - 1];
-    };
-    if (i == ib) {
-      m4(Mc, 0, cl[0], cl[1], cl[2], cl[3]);
-      m4(Mc, 1, cmu[0], cmu[1], cmu[2], cmu[3]);
-      if (!ELASTIC) {
-        m4(Mc, 2, cqp[0], cqp[1], cqp[2], cqp[3]);
-        m4(Mc, 3, cqs[0], cqs[1], cqs[2], cqs[3]);
-      }
-    }
-    float nl[4], nmu[4], nqp[4], nqs[4];
-    m4(Mn, 0, nl[0], nl[1], nl[2], nl[3]);
-    m4(Mn, 1, nmu[0], nmu[1], nmu[2], nmu[3]);
-    const bool odd = ((i - ib) & 1) != 0;
-    const float f_vx1 = odd ? tv1[1] : tv1[0], f_vx2 = odd ? tv2[1] : tv2[0],
-                f_wwo = odd ? twwo[1] : twwo[0];
-    float QP8 = 0.f, QS8 = 0.f;
-    const float cc0 = odd ? tc0[1] : tc0[0], cc1 = odd ? tc1[1] : tc1[0];
+    // ---- media: sums of plane i + 1, coefficients of plane i ---------------
+    const float* M = smem + C::F_M + ch.slot * NM * MTILE + hm;
+    AwpRelax<float2> rx{};
+    const int odd = s & 1;
     if (!ELASTIC) {
-      m4(Mn, 2, nqp[0], nqp[1], nqp[2], nqp[3]);
-      m4(Mn, 3, nqs[0], nqs[1], nqs[2], nqs[3]);
-      QP8 = cqp[0] + nqp[0] + cqp[1] + nqp[1] + cqp[2] + nqp[2] + cqp[3] + nqp[3];
-      QS8 = cqs[0] + nqs[0] + cqs[1] + nqs[1] + cqs[2] + nqs[2] + cqs[3] + nqs[3];
-    }
-    // eight-cell sums in the reference's order: pos, ip1, jm1, ijk, km1, ik1, jk1, ijk1
-    const AwpStrCoef cf = awp_stress_coef<ELASTIC>(
-        cl[0] + nl[0] + cl[1] + nl[1] + cl[2] + nl[2] + cl[3] + nl[3],
-        cmu[0] + nmu[0] + cmu[1] + nmu[1] + cmu[2] + nmu[2] + cmu[3] + nmu[3], cmu[0], cmu[2],
-        cmu[1], nmu[0], QP8, QS8, cqs[0], cqs[2], cqs[1], nqs[0], f_vx1, f_vx2, f_wwo, cc0, cc1,
-        a.qthr, dth, dh1, DT);
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      cl[q] = nl[q];
-      cmu[q] = nmu[q];
-      if (!ELASTIC) {
-        cqp[q] = nqp[q];
-        cqs[q] = nqs[q];
+      const float* tab = smem + C::F_T;
+      const int ea = odd ? e0[1] : e0[0], eb = odd ? e1[1] : e1[0];
+      const float4* t4 = reinterpret_cast<const float4*>(tab + (ea >> 1) * 20);
+      const float4 q0 = t4[0], q1 = t4[1], q2 = t4[2], q3 = t4[3];
+      const float2 q4 = lds2(tab + (ea >> 1) * 20 + 16);
+      rx.vx2 = make_float2(q0.x, q0.y); rx.wwo = make_float2(q0.z, q0.w);
+      rx.kv = make_float2(q1.x, q1.y); rx.kr = make_float2(q1.z, q1.w);
+      rx.kr2 = make_float2(q2.x, q2.y); rx.kf = make_float2(q2.z, q2.w);
+      rx.c0 = make_float2(q3.x, q3.y); rx.c1 = make_float2(q3.z, q3.w);
+      rx.c2 = q4;
+      if (eb != (ea | 1) || (ea & 1)) {
+        // entries that are not an even-odd pair: the level of a mesh's coarse
+        // block that takes the finer block's pattern
+        auto at = [&](int q) {
+          return make_float2(tab[(ea >> 1) * 20 + 2 * q + (ea & 1)],
+                             tab[(eb >> 1) * 20 + 2 * q + (eb & 1)]);
+        };
+        rx = {at(0), at(1), at(2), at(3), at(4), at(5), at(6), at(7), at(8)};
       }
     }
-    const float dcrj = LDG(a.dcrjx + i) * dcy * dcz;
-    const long long o = (long long)i * S;
+    AwpStrCoef<float2> cf;
+    {
+      const float2 Ln = mat_s(M).q;
+      const Mat mn = mat_s(M + MTILE);
+      const float2 P[3] = {Mk, Mt, vadd(Mm, mn.m)};
+      float2 QP8 = {}, QS8 = {}, R[3] = {};
+      if (!ELASTIC) {
+        const float2 pn = mat_s(M + 2 * MTILE).q;
+        const Mat rn = mat_s(M + 3 * MTILE);
+        QP8 = vadd(Pq, pn);
+        QS8 = vadd(Rq, rn.q);
+        R[0] = Rk; R[1] = Rt; R[2] = vadd(Rm, rn.m);
+        Pq = pn;
+        Rq = rn.q; Rt = rn.t; Rm = rn.m; Rk = rn.pk;
+      }
+      cf = awp_stress_coef<ELASTIC>(vadd(Lq, Ln), vadd(Mq, mn.q), P, QP8, QS8, R, rx, a.thr,
+                                    a.dth, a.dt);
+      Lq = Ln;
+      Mq = mn.q; Mt = mn.t; Mm = mn.m; Mk = mn.pk;
+    }
+    const int i = ib + s;
+    const float2 dcrj = vscale(LDG(a.dcrjx + i) * dcy, dcz);
 
-    if (top && active) {
-      const float uimg = u_0 - (w_0 - w_m1);
-      const float vimg = v_0 - (w_jp1 - w_0);
-      const float vs1 = (i < a.gx_lim) ? u_p1 - (w_p1 - w_0) : 0.0f;
-      const float vs2 = (j >= a.gy_min) ? v_jm1 - (w_0 - w_jm1) : 0.0f;
-      const float wimg = __fmaf_rn(
-          -LDG(a.lam_mu + (long long)i * a.lam_mu_ld + j),
-          __fadd_rn(__fadd_rn(__fadd_rn(vs1 - uimg, u_p1 - u_0), vimg - vs2), v_0 - v_jm1), w_km1);
-      a.u1[col + o + 1] = uimg;
-      a.v1[col + o + 1] = vimg;
-      a.w1[col + o + 1] = wimg;
-      uk1 = uimg;
-      vk1 = vimg;
-      wk1 = wimg;
-    } else if (top1) {
-      uk2 = uk1 - (wk1 - Hm1[2 * HTILE + 1]);
-      vk2 = vk1 - (W0[HX + 1] - wk1);
+    // ---- free-surface velocity images (kernel.cu:1087-1112) ----------------
+    if (top) {
+      const float uimg = u_0.y - (w_0.y - w_m1.y);
+      const float vimg = v_0.y - (w_jp1.y - w_0.y);
+      if (jin) {
+        const float vs1 = (i < a.gx_lim) ? u_p1.y - (w_p1.y - w_0.y) : 0.0f;
+        const float vs2 = (j >= a.gy_min) ? v_jm1.y - (w_0.y - w_jm1.y) : 0.0f;
+        const float wimg = __fmaf_rn(
+            -LDG(a.lam_mu + (long long)i * a.lam_mu_ld + j),
+            __fadd_rn(__fadd_rn(__fadd_rn(vs1 - uimg, u_p1.y - u_0.y), vimg - vs2),
+                      v_0.y - v_jm1.y),
+            w_0.x);
+        a.u1[o + 2] = uimg;
+        a.v1[o + 2] = vimg;
+        a.w1[o + 2] = wimg;
+        w_kp = wimg;
+      }
+      u_kp.x = uimg;
+      v_kp.x = vimg;
     }
 
-    float d[9];
+    float2 d[9];
     d[0] = awp_d4(c1, c2, u_p1, u_0, u_p2, u_m1);
     d[1] = awp_d4(c1, c2, v_0, v_jm1, v_jp1, v_jm2);
-    d[2] = awp_d4(c1, c2, w_0, w_km1, wk1, w_km2);
+    d[2] = make_float2(awp_d4(c1, c2, w_0.x, w_km.y, w_0.y, w_km.x),
+                       awp_d4(c1, c2, w_0.y, w_0.x, w_kp, w_km.y));
     d[3] = awp_d4(c1, c2, u_jp1, u_0, u_jp2, u_jm1);
     d[4] = awp_d4(c1, c2, v_0, v_m1, v_p1, v_m2);
-    d[5] = awp_d4(c1, c2, uk1, u_0, uk2, u_km1);
+    d[5] = make_float2(awp_d4(c1, c2, u_0.y, u_0.x, u_kp.x, u_km1),
+                       awp_d4(c1, c2, u_kp.x, u_0.y, u_kp.y, u_0.x));
     d[6] = awp_d4(c1, c2, w_0, w_m1, w_p1, w_m2);
-    d[7] = awp_d4(c1, c2, vk1, v_0, vk2, v_km1);
+    d[7] = make_float2(awp_d4(c1, c2, v_0.y, v_0.x, v_kp.x, v_km1),
+                       awp_d4(c1, c2, v_kp.x, v_0.y, v_kp.y, v_0.x));
     d[8] = awp_d4(c1, c2, w_jp1, w_0, w_jp2, w_jm1);
 
-    const float* O = ro.buf + wo.slot * ro.slot_floats + ooff;
-    float sg[6], rr[6];
+    ok = mbar_wait(pipe.full_o + co.slot, co.phase, spin);
+    if (!__all_sync(0xffffffffu, ok)) break;
+    const float* O = smem + C::F_O + co.slot * NO * OTILE + ho;
+    float2 sg[6], rr[6];
 #pragma unroll
-    for (int q = 0; q < 6; ++q) sg[q] = O[q * OTILE];
-    if (!ELASTIC) {
-#pragma unroll
-      for (int q = 0; q < 6; ++q) rr[q] = O[(6 + q) * OTILE];
+    for (int q = 0; q < 6; ++q) {
+      sg[q] = lds2(O + q * OTILE);
+      if (!ELASTIC) rr[q] = lds2(O + (6 + q) * OTILE);
     }
-    awp_stress_update<ELASTIC>(sg, rr, cf, f_vx1, f_vx2, f_wwo, DT, dcrj, d);
-    if (active) {
+    awp_stress_update<ELASTIC>(sg, rr, cf, rx, dcrj, d);
+    if (ax || ay) {
 #pragma unroll
-      for (int q = 0; q < 6; ++q) SG[q][col + o] = sg[q];
-      if (!ELASTIC) {
-#pragma unroll
-        for (int q = 0; q < 6; ++q) RR[q][col + o] = rr[q];
+      for (int q = 0; q < 6; ++q) {
+        st2(SG[q] + o, sg[q], ax, ay);
+        if (!ELASTIC) st2(RR[q] + o, rr[q], ax, ay);
       }
     }
+    warp_done(pipe.done + cd.slot, tid & 31);
 
-    wh.next(DH_);
-    wm.next(DM_);
-    wo.next(DO_);
-    sh = sh1;
-    sm = sm1;
+    o += S;
+    u_m1 = u_0; u_0 = u_p1; u_p1 = u_p2;
+    v_m2 = v_m1; v_m1 = v_0; v_0 = v_p1;
+    w_m2 = w_m1; w_m1 = w_0; w_0 = w_p1;
+    ch.next();
+    co.next();
+    cd.next();
+    su = su + 1 == C::DU ? 0 : su + 1;
+    su2 = su2 + 1 == C::DU ? 0 : su2 + 1;
+    sv = sv1;
+    sv1 = sv1 + 1 == C::DV ? 0 : sv1 + 1;
   }
-  if (aborted) {
-    if (tid == 0) {
-      atomicExch(err, 1);
-      // let copies still in flight land before the CTA's shared memory is released
-      for (int p = max(nh - DH_, ib - 2); p < nh && p <= ie + 2; ++p)
-        (void)mbar_wait(rh.b(p), rh.parity(p));
-      for (int p = max(nm - DM_, ib); p < nm && p <= ie + 1; ++p)
-        (void)mbar_wait(rm.b(p), rm.parity(p));
-      for (int p = max(no - DO_, ib); p < no && p <= ie; ++p)
-        (void)mbar_wait(ro.b(p), ro.parity(p));
-    }
-    __syncthreads();
-  }
+  if (!__all_sync(0xffffffffu, ok) && (tid & 31) == 0) atomicExch(err, 1);
 }
 
 // ===========================================================================
-// Velocity (dvelcx_opt, kernel.cu:125-268), same arithmetic as k_velocity.
-// Rings: stress halo tiles (6 fields, planes i-2..i+2), density (planes i,
-// i+1), own velocity tiles (plane i).
+// Velocity (dvelcx_opt, kernel.cu:125-268), same bits as k_velocity.  The xx
+// tile is read only at the cell's own column, one plane ahead; xy and xz at
+// their own column two planes ahead and with their j or k neighbours when the
+// march arrives; yy, zz, yz, the density and the velocities once.
 // ===========================================================================
-__global__ void __launch_bounds__(NT, 3)
+struct VelCfg {
+  static constexpr int LA = 2;          // planes ahead
+  static constexpr int NH = 1 + LA;     // stages
+  static constexpr int DS = 3 + LA;     // xy, xz: planes i .. i+2 and the ones ahead
+  // one stage: xx(i+1), yy, zz, yz(i), density(i+1), u, v, w(i)
+  static constexpr int G_XX = 0, G_YY = OTILE, G_ZZ = G_YY + JTILE, G_YZ = G_ZZ + KTILE,
+                       G_D = G_YZ + HTILE, G_O = G_D + MTILE, STAGE = G_O + 3 * OTILE;
+  static constexpr int F_XY = 0, F_XZ = F_XY + DS * JTILE, F_S = F_XZ + DS * KTILE,
+                       F_END = F_S + NH * STAGE;
+  static constexpr size_t bytes = sizeof(float) * F_END + sizeof(Pipe<NH, 0, NC / 32>);
+};
+
+__global__ void __launch_bounds__(NT, 4)
     k_velocity_tma(const VelArgs a, const __grid_constant__ TmaMaps tm, const int ichunk,
                    int* err, const unsigned spin) {
+  using C = VelCfg;
   extern __shared__ __align__(128) float smem[];
-  const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TZ + tx;
+  auto& pipe = *reinterpret_cast<Pipe<C::NH, 0, NC / 32>*>(smem + C::F_END);
+  const int tid = threadIdx.x;
   const int kb = AWP_ALIGN + blockIdx.x * TZ;
   const int jb = a.j0 + blockIdx.y * TY;
-  const int k = kb + tx, j = jb + ty;
   const int ib = a.i0 + blockIdx.z * ichunk;
   const int ie = min(ib + ichunk - 1, a.i1);
-  const bool active = (k >= a.k0) && (k <= a.k1) && (j <= a.j1);
+  const int n = ie - ib + 1;
 
-  Ring rh{smem, nullptr, DH_, VT_SLOT, ib - 2};
-  Ring rm{rh.buf + DH_ * VT_SLOT, nullptr, DM_, MTILE, ib};
-  Ring ro{rm.buf + DM_ * MTILE, nullptr, DO_, 3 * OTILE, ib};
-  uint64_t* bars = reinterpret_cast<uint64_t*>(ro.buf + DO_ * 3 * OTILE);
-  rh.bar = bars;
-  rm.bar = bars + DH_;
-  ro.bar = bars + DH_ + DM_;
-
-  // producer (thread 0): slot of the next plane each ring receives
-  int ish = 0, ism = 0, iso = 0;
-  auto issue_halo = [&](int p) {
-    if (p > ie + 2) return;
-    uint64_t* b = rh.bar + ish;
-    mbar_expect_tx(b, VT_SLOT * 4);
-    float* d = rh.buf + ish * rh.slot_floats;
-    tma_load3(d + VT_XX, &tm.halo[0], b, kb, jb, p);
-    tma_load3(d + VT_YY, &tm.halo[1], b, kb, jb - 2, p);
-    tma_load3(d + VT_ZZ, &tm.halo[2], b, kb - 4, jb, p);
-    tma_load3(d + VT_XY, &tm.halo[3], b, kb, jb - 2, p);
-    tma_load3(d + VT_XZ, &tm.halo[4], b, kb - 4, jb, p);
-    tma_load3(d + VT_YZ, &tm.halo[5], b, kb - 4, jb - 2, p);
-    ish = wrap_add(ish, 1, DH_);
-  };
-  auto issue_media = [&](int p) {
-    if (p > ie + 1) return;
-    uint64_t* b = rm.bar + ism;
-    mbar_expect_tx(b, MTILE_B);
-    tma_load3(rm.buf + ism * rm.slot_floats, &tm.media[0], b, kb - 4, jb - 1, p);
-    ism = wrap_add(ism, 1, DM_);
-  };
-  auto issue_own = [&](int p) {
-    if (p > ie) return;
-    uint64_t* b = ro.bar + iso;
-    mbar_expect_tx(b, 3 * OTILE * 4);
-    float* d = ro.buf + iso * ro.slot_floats;
-    for (int f = 0; f < 3; ++f) tma_load3(d + f * OTILE, &tm.own[f], b, kb, jb, p);
-    iso = wrap_add(iso, 1, DO_);
-  };
-
-  if (tid == 0) {
-    for (int q = 0; q < DH_ + DM_ + DO_; ++q) mbar_init(bars + q, 1);
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
+  if (tid == 0) pipe.init();
   __syncthreads();
-  // next plane to issue per ring (meaningful in the producer thread only)
-  int nh = ib - 2, nm = ib, no = ib;
-  if (tid == 0) {
-    for (; nh < ib - 2 + DH_; ++nh) issue_halo(nh);
-    for (; nm < ib + DM_; ++nm) issue_media(nm);
-    for (; no < ib + DO_; ++no) issue_own(no);
+
+  if (tid >= NC) {  // producer warp
+    if (tid == NC) {
+      pipe.produce(
+          n,
+          [&](int s, uint64_t* b) {
+            const int p0 = s == 0 ? 0 : s + 2;
+            mbar_expect_tx(b, ((s + 2 - p0 + 1) * (JTILE + KTILE) + 4 * OTILE + JTILE + KTILE +
+                               HX * HY + MX * MY) * 4);
+            for (int p = p0; p <= s + 2; ++p) {
+              tma_load3(smem + C::F_XY + (p % C::DS) * JTILE, &tm.halo[3], b, kb, jb - 2, ib + p);
+              tma_load3(smem + C::F_XZ + (p % C::DS) * KTILE, &tm.halo[4], b, kb - 4, jb, ib + p);
+            }
+            float* g = smem + C::F_S + (s % C::NH) * C::STAGE;
+            const int i = ib + s;
+            tma_load3(g + C::G_XX, &tm.halo[0], b, kb, jb, i + 1);
+            tma_load3(g + C::G_YY, &tm.halo[1], b, kb, jb - 1, i);
+            tma_load3(g + C::G_ZZ, &tm.halo[2], b, kb - 4, jb, i);
+            tma_load3(g + C::G_YZ, &tm.halo[5], b, kb - 4, jb - 2, i);
+            tma_load3(g + C::G_D, &tm.media[0], b, kb - 4, jb - 1, i + 1);
+            for (int f = 0; f < 3; ++f)
+              tma_load3(g + C::G_O + f * OTILE, &tm.own[f], b, kb, jb, i);
+          },
+          [](int, uint64_t*) {}, err, spin);
+    }
+    return;
   }
 
+  const int row = tid >> 4, kp = (tid & 15) * 2;
+  const int k = kb + kp, j = jb + row;
+  const bool jin = j <= a.j1;
+  const bool ax = jin && k >= a.k0 && k <= a.k1, ay = jin && k + 1 >= a.k0 && k + 1 <= a.k1;
   const int S = a.slice, Y = a.yline;
   const float c1 = a.c1, c2 = a.c2, dth = a.dth;
-  const float dcy = LDG(a.dcrjy + min(j, a.j1)), dcz = LDG(a.dcrjz + min(k, a.k1));
-  const long long col = (long long)j * Y + k;
-  const int o_xx = VT_XX + ty * TZ + tx;             // no halo
-  const int o_yy = VT_YY + (ty + 2) * VJ + tx;       // j halo
-  const int o_zz = VT_ZZ + ty * VK + tx + 4;         // k halo
-  const int o_xy = VT_XY + (ty + 2) * VJ + tx;
-  const int o_xz = VT_XZ + ty * VK + tx + 4;
-  const int o_yz = VT_YZ + (ty + 2) * VK + tx + 4;   // both
-  const int moff = (ty + 1) * MX + (tx + 4);
-  const int ooff = ty * TZ + tx;
-  bool ok = true, aborted = false;
-
-  // consumers: the plane each ring waits for next (halo i+2, media i+1, own i)
-  // and the slots of the oldest planes read (halo i-2, media i)
-  Cursor wh{4, 0u}, wm{1, 0u}, wo{0, 0u};
-  int sh = 0, sm = 0;
-  for (int i = ib; i <= ie; ++i) {
-    // ---- wait for the planes this step reads for the first time ------------
-    if (i == ib) {
-      for (int q = 0; q < 4 && ok; ++q) ok = mbar_wait(rh.bar + q, 0u, spin);  // ib-2..ib+1
-      if (ok) ok = mbar_wait(rm.bar, 0u, spin);                                  // plane ib
-    }
-    if (ok) ok = mbar_wait(rh.bar + wh.slot, wh.phase, spin);
-    if (ok) ok = mbar_wait(rm.bar + wm.slot, wm.phase, spin);
-    if (ok) ok = mbar_wait(ro.bar + wo.slot, wo.phase, spin);
-    // one barrier per plane: it also tells the producer that every thread is
-    // done with the previous step's oldest planes, whose slots it refills
-    if (__syncthreads_or(!ok)) {
-      aborted = true;
-      break;
-    }
-    if (tid == 0 && i > ib) {
-      issue_halo(nh++);
-      issue_media(nm++);
-      issue_own(no++);
-    }
-    const int sh1 = wrap_add(sh, 1, DH_), sh2 = wrap_add(sh, 2, DH_), sh3 = wrap_add(sh, 3, DH_),
-              sh4 = wrap_add(sh, 4, DH_), sm1 = wrap_add(sm, 1, DM_);
-
-    // halo fields: 0 xx, 1 yy, 2 zz, 3 xy, 4 xz, 5 yz
-    const float* Hm2 = rh.buf + sh * rh.slot_floats;
-    const float* Hm1 = rh.buf + sh1 * rh.slot_floats;
-    const float* H0 = rh.buf + sh2 * rh.slot_floats;
-    const float* Hp1 = rh.buf + sh3 * rh.slot_floats;
-    const float* Hp2 = rh.buf + sh4 * rh.slot_floats;
-    const float xx_m2 = Hm2[o_xx], xx_m1 = Hm1[o_xx], xx_0 = H0[o_xx], xx_p1 = Hp1[o_xx];
-    const float xy_m1 = Hm1[o_xy], xy_0 = H0[o_xy], xy_p1 = Hp1[o_xy], xy_p2 = Hp2[o_xy];
-    const float xz_m1 = Hm1[o_xz], xz_0 = H0[o_xz], xz_p1 = Hp1[o_xz], xz_p2 = Hp2[o_xz];
-    const float* YY = H0 + o_yy;
-    const float* ZZ = H0 + o_zz;
-    const float* XY = H0 + o_xy;
-    const float* XZ = H0 + o_xz;
-    const float* YZ = H0 + o_yz;
-    const float yz_0 = YZ[0];
-
-    const float* Dc = rm.buf + sm * rm.slot_floats + moff;
-    const float* Dn = rm.buf + sm1 * rm.slot_floats + moff;
-    const float d_0 = Dc[0], d_0j = Dc[-MX], d_0k = Dc[-1], d_0jk = Dc[-MX - 1];
-    const float d_p = Dn[0], d_pj = Dn[-MX], d_pk = Dn[-1];
-
-    const float fd1 = awp_vel_factor(dth, d_0, d_0j, d_0k, d_0jk);
-    const float fd2 = awp_vel_factor(dth, d_0, d_p, d_0k, d_pk);
-    const float fd3 = awp_vel_factor(dth, d_0, d_p, d_0j, d_pj);
-    const float dcrj = LDG(a.dcrjx + i) * dcy * dcz;
-
-    const float* O = ro.buf + wo.slot * ro.slot_floats + ooff;
-    const float u = awp_vel_update(O[0], fd1, c1, c2, xx_0 - xx_m1, xx_p1 - xx_m2,
-                                   xy_0 - XY[-VJ], XY[VJ] - XY[-2 * VJ], xz_0 - XZ[-1],
-                                   XZ[1] - XZ[-2], dcrj);
-    const float v = awp_vel_update(O[OTILE], fd2, c1, c2, xy_p1 - xy_0, xy_p2 - xy_m1,
-                                   YY[VJ] - YY[0], YY[2 * VJ] - YY[-VJ], yz_0 - YZ[-1],
-                                   YZ[1] - YZ[-2], dcrj);
-    const float w = awp_vel_update(O[2 * OTILE], fd3, c1, c2, xz_p1 - xz_0, xz_p2 - xz_m1,
-                                   yz_0 - YZ[-VK], YZ[VK] - YZ[-2 * VK], ZZ[1] - ZZ[0],
-                                   ZZ[2] - ZZ[-1], dcrj);
-    if (active) {
-      const long long o = (long long)i * S + col;
-      a.u1[o] = u;
-      a.v1[o] = v;
-      a.w1[o] = w;
-    }
-    wh.next(DH_);
-    wm.next(DM_);
-    wo.next(DO_);
-    sh = sh1;
-    sm = sm1;
+  const float dcy = LDG(a.dcrjy + min(j, a.j1));
+  const float2 dcz = make_float2(LDG(a.dcrjz + min(k, a.k1)), LDG(a.dcrjz + min(k + 1, a.k1)));
+  long long o = (long long)ib * S + (long long)j * Y + k;
+  float2 xx_m2, xx_m1, xx_0, xy_m1, xy_0, xy_p1, xz_m1, xz_0, xz_p1;
+  // density of the current plane: value, and the level below; rows j and j-1
+  float2 d_0, d_0j;
+  float d_0k, d_0jk;
+  {
+    const float *X = a.xx + o, *P = a.xy + o, *Q = a.xz + o, *D = a.d1 + o;
+    xx_m2 = ldg2(X - 2 * (long long)S); xx_m1 = ldg2(X - S); xx_0 = ldg2(X);
+    xy_m1 = ldg2(P - S); xy_0 = ldg2(P); xy_p1 = ldg2(P + S);
+    xz_m1 = ldg2(Q - S); xz_0 = ldg2(Q); xz_p1 = ldg2(Q + S);
+    d_0 = ldg2(D); d_0j = ldg2(D - Y); d_0k = D[-1]; d_0jk = D[-Y - 1];
   }
-  if (aborted) {
-    if (tid == 0) {
-      atomicExch(err, 1);
-      for (int p = max(nh - DH_, ib - 2); p < nh && p <= ie + 2; ++p)
-        (void)mbar_wait(rh.b(p), rh.parity(p));
-      for (int p = max(nm - DM_, ib); p < nm && p <= ie + 1; ++p)
-        (void)mbar_wait(rm.b(p), rm.parity(p));
-      for (int p = max(no - DO_, ib); p < no && p <= ie; ++p)
-        (void)mbar_wait(ro.b(p), ro.parity(p));
+  const int o_own = row * TZ + kp;                    // no halo
+  const int o_yy = (row + 1) * TZ + kp;               // j halo from jb - 1
+  const int o_xy = (row + 2) * TZ + kp;               // j halo from jb - 2
+  const int o_k = row * HX + kp + 4;                  // k halo
+  const int o_yz = (row + 2) * HX + kp + 4;           // both, from jb - 2
+  const int o_d = (row + 1) * MX + kp + 4;
+
+  Cursor<C::NH> ch;
+  Cursor<awp_pipe::ND> cd;
+  int ss = 0, ss2 = 2;  // slots of the xy, xz planes i, i+2
+  bool ok = true;
+#pragma unroll 1
+  for (int s = 0; s < n; ++s) {
+    ok = mbar_wait(pipe.full_h + ch.slot, ch.phase, spin);
+    if (!__all_sync(0xffffffffu, ok)) break;
+    const float* G = smem + C::F_S + ch.slot * C::STAGE;
+    const float* XY = smem + C::F_XY + ss * JTILE + o_xy;
+    const float* XZ = smem + C::F_XZ + ss * KTILE + o_k;
+    const float* YY = G + C::G_YY + o_yy;
+    const float* ZZ = G + C::G_ZZ + o_k;
+    const float* YZ = G + C::G_YZ + o_yz;
+    const float* D = G + C::G_D + o_d;
+    const float2 xx_p1 = lds2(G + C::G_XX + o_own);
+    const float2 xy_p2 = lds2(smem + C::F_XY + ss2 * JTILE + o_xy);
+    const float2 xz_p2 = lds2(smem + C::F_XZ + ss2 * KTILE + o_k);
+    const float2 xy_jm1 = lds2(XY - TZ), xy_jm2 = lds2(XY - 2 * TZ), xy_jp1 = lds2(XY + TZ);
+    const float2 xz_km = lds2(XZ - 2);
+    const float xz_kp = XZ[2];
+    const float2 yy_0 = lds2(YY), yy_jp1 = lds2(YY + TZ), yy_jp2 = lds2(YY + 2 * TZ),
+                 yy_jm1 = lds2(YY - TZ);
+    const float2 zz_0 = lds2(ZZ), zz_kp = lds2(ZZ + 2);
+    const float zz_km1 = ZZ[-1];
+    const float2 yz_0 = lds2(YZ), yz_km = lds2(YZ - 2), yz_jm1 = lds2(YZ - HX),
+                 yz_jm2 = lds2(YZ - 2 * HX), yz_jp1 = lds2(YZ + HX);
+    const float yz_kp = YZ[2];
+    const float2 d_p = lds2(D), d_pj = lds2(D - MX);
+    const float d_pk = D[-1], d_pjk = D[-MX - 1];
+    const float2 u_old = lds2(G + C::G_O + o_own), v_old = lds2(G + C::G_O + OTILE + o_own),
+                 w_old = lds2(G + C::G_O + 2 * OTILE + o_own);
+
+    // density factors: pair sums at the level and at the one below
+    const float2 dj = vadd(d_0, d_0j), dx = vadd(d_0, d_p);
+    const float2 fd1 = awp_vel_factor(dth, dj, make_float2(vadd(d_0k, d_0jk), dj.x));
+    const float2 fd2 = awp_vel_factor(dth, dx, make_float2(vadd(d_0k, d_pk), dx.x));
+    const float2 fd3 = awp_vel_factor(dth, dx, vadd(d_0j, d_pj));
+    const float2 dcrj = vscale(LDG(a.dcrjx + ib + s) * dcy, dcz);
+
+    const float2 u = awp_vel_update(
+        u_old, fd1, c1, c2, vsub(xx_0, xx_m1), vsub(xx_p1, xx_m2), vsub(xy_0, xy_jm1),
+        vsub(xy_jp1, xy_jm2), make_float2(xz_0.x - xz_km.y, xz_0.y - xz_0.x),
+        make_float2(xz_0.y - xz_km.x, xz_kp - xz_km.y), dcrj);
+    const float2 v = awp_vel_update(
+        v_old, fd2, c1, c2, vsub(xy_p1, xy_0), vsub(xy_p2, xy_m1), vsub(yy_jp1, yy_0),
+        vsub(yy_jp2, yy_jm1), make_float2(yz_0.x - yz_km.y, yz_0.y - yz_0.x),
+        make_float2(yz_0.y - yz_km.x, yz_kp - yz_km.y), dcrj);
+    const float2 w = awp_vel_update(
+        w_old, fd3, c1, c2, vsub(xz_p1, xz_0), vsub(xz_p2, xz_m1), vsub(yz_0, yz_jm1),
+        vsub(yz_jp1, yz_jm2), make_float2(zz_0.y - zz_0.x, zz_kp.x - zz_0.y),
+        make_float2(zz_kp.x - zz_km1, zz_kp.y - zz_0.x), dcrj);
+    if (ax || ay) {
+      st2(a.u1 + o, u, ax, ay);
+      st2(a.v1 + o, v, ax, ay);
+      st2(a.w1 + o, w, ax, ay);
     }
-    __syncthreads();
+    warp_done(pipe.done + cd.slot, tid & 31);
+    o += S;
+    xx_m2 = xx_m1; xx_m1 = xx_0; xx_0 = xx_p1;
+    xy_m1 = xy_0; xy_0 = xy_p1; xy_p1 = xy_p2;
+    xz_m1 = xz_0; xz_0 = xz_p1; xz_p1 = xz_p2;
+    d_0 = d_p; d_0j = d_pj; d_0k = d_pk; d_0jk = d_pjk;
+    ch.next();
+    cd.next();
+    ss = ss + 1 == C::DS ? 0 : ss + 1;
+    ss2 = ss2 + 1 == C::DS ? 0 : ss2 + 1;
   }
+  if (!__all_sync(0xffffffffu, ok) && (tid & 31) == 0) atomicExch(err, 1);
 }
 
-inline unsigned cdiv_u(long long a, long long b) { return (unsigned)((a + b - 1) / b); }
-
-// Poll limit the next launches give their pipeline waits (process-wide).
-unsigned g_spin_limit = kSpinLimit;
-
-size_t stress_smem(bool elastic) {
-  const int nm = elastic ? 2 : 4, no = elastic ? 6 : 12;
-  return sizeof(float) * ((size_t)DH_ * 3 * HTILE + (size_t)DM_ * nm * MTILE +
-                          (size_t)DO_ * no * OTILE) +
-         sizeof(uint64_t) * (DH_ + DM_ + DO_);
-}
-size_t velocity_smem() {
-  return sizeof(float) * ((size_t)DH_ * VT_SLOT + (size_t)DM_ * MTILE + (size_t)DO_ * 3 * OTILE) +
-         sizeof(uint64_t) * (DH_ + DM_ + DO_);
-}
 
 PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
   static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
@@ -586,8 +522,10 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
 
 // L2 promotion of the tensor maps' fetches (process-wide; a context encodes
 // its maps with the value of the moment and re-encodes them when it changes):
-// 0 none, 1 64 B, 2 128 B, 3 256 B.
-static int g_l2_promotion = 3;
+// 0 none, 1 64 B, 2 128 B, 3 256 B.  A column's rows are not multiples of 256
+// bytes, so the wide granule fetches padding and rows no box asks for
+// (k_stress_tma at 512 x 512 x 256: 1618 us with 256 B, 1515 none or 128 B).
+static int g_l2_promotion = 0;
 
 int awp_tma_set_l2_promotion(int mode) {
   if (mode < 0 || mode > 3) return 1;
@@ -618,7 +556,7 @@ int awp_tma_encode(CUtensorMap* map, const float* base, const AwpGeom& g, int bo
 
 int awp_tma_box(int group, int* bx, int* by) {
   switch (group) {
-    case 0: *bx = HX; *by = HY; return 0;   // halo
+    case 0: *bx = HX; *by = HY; return 0;   // j and k halo
     case 1: *bx = MX; *by = MY; return 0;   // media
     case 2: *bx = TZ; *by = TY; return 0;   // own
     case 3: *bx = TZ; *by = HY; return 0;   // j halo only
@@ -627,25 +565,29 @@ int awp_tma_box(int group, int* bx, int* by) {
   return 1;
 }
 
+namespace {
+
+Shape g_shape_str[2][kMaxDev], g_shape_vel[kMaxDev];
+constexpr int kMost = 6;  // planes of a march (march_planes)
+
+}  // namespace
+
 cudaError_t awp_launch_stress_tma(const StrArgs& a, const TmaMaps& tm, bool elastic, int ichunk,
                                   int* err, cudaStream_t st) {
   const int nk = a.k1 - AWP_ALIGN + 1, nj = a.j1 - a.j0 + 1, ni = a.i1 - a.i0 + 1;
   if (nk <= 0 || nj <= 0 || ni <= 0) return cudaSuccess;
-  const dim3 block(TZ, TY, 1);
-  const dim3 grid(cdiv_u(nk, TZ), cdiv_u(nj, TY), cdiv_u(ni, ichunk));
-  const size_t sm = stress_smem(elastic);
-  cudaError_t e;
-  if (elastic) {
-    e = cudaFuncSetAttribute(k_stress_tma<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)sm);
-    if (e != cudaSuccess) return e;
-    k_stress_tma<true><<<grid, block, sm, st>>>(a, tm, ichunk, err, g_spin_limit);
-  } else {
-    e = cudaFuncSetAttribute(k_stress_tma<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)sm);
-    if (e != cudaSuccess) return e;
-    k_stress_tma<false><<<grid, block, sm, st>>>(a, tm, ichunk, err, g_spin_limit);
-  }
+  const dim3 tile(cdiv_u(nk, TZ), cdiv_u(nj, TY));
+  const size_t sm = elastic ? StrCfg<true>::bytes : StrCfg<false>::bytes;
+  const void* f = elastic ? (const void*)k_stress_tma<true> : (const void*)k_stress_tma<false>;
+  int resident = 0;
+  const cudaError_t e = resident_ctas(f, sm, NT, g_shape_str[elastic ? 1 : 0], &resident);
+  if (e != cudaSuccess) return e;
+  const int c = march_planes((long long)tile.x * tile.y, ni, resident, ichunk, kMost);
+  const dim3 grid(tile.x, tile.y, cdiv_u(ni, c));
+  if (elastic)
+    k_stress_tma<true><<<grid, NT, sm, st>>>(a, tm, c, err, awp_pipe_spin_limit);
+  else
+    k_stress_tma<false><<<grid, NT, sm, st>>>(a, tm, c, err, awp_pipe_spin_limit);
   return cudaGetLastError();
 }
 
@@ -653,20 +595,24 @@ cudaError_t awp_launch_velocity_tma(const VelArgs& a, const TmaMaps& tm, int ich
                                     cudaStream_t st) {
   const int nk = a.k1 - AWP_ALIGN + 1, nj = a.j1 - a.j0 + 1, ni = a.i1 - a.i0 + 1;
   if (nk <= 0 || nj <= 0 || ni <= 0) return cudaSuccess;
-  const dim3 block(TZ, TY, 1);
-  const dim3 grid(cdiv_u(nk, TZ), cdiv_u(nj, TY), cdiv_u(ni, ichunk));
-  const size_t sm = velocity_smem();
-  cudaError_t e =
-      cudaFuncSetAttribute(k_velocity_tma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  const dim3 tile(cdiv_u(nk, TZ), cdiv_u(nj, TY));
+  int resident = 0;
+  const cudaError_t e =
+      resident_ctas((const void*)k_velocity_tma, VelCfg::bytes, NT, g_shape_vel, &resident);
   if (e != cudaSuccess) return e;
-  k_velocity_tma<<<grid, block, sm, st>>>(a, tm, ichunk, err, g_spin_limit);
+  const int c = march_planes((long long)tile.x * tile.y, ni, resident, ichunk, kMost);
+  const dim3 grid(tile.x, tile.y, cdiv_u(ni, c));
+  k_velocity_tma<<<grid, NT, VelCfg::bytes, st>>>(a, tm, c, err, awp_pipe_spin_limit);
   return cudaGetLastError();
 }
 
+// the pipeline waits' poll limit
+unsigned awp_pipe_spin_limit = kSpinLimit;
+
 int awp_tma_set_spin_limit(long long polls) {
   if (polls < 0 || polls > (1ll << 30)) return 1;
-  g_spin_limit = (unsigned)polls;
+  awp_pipe_spin_limit = (unsigned)polls;
   return 0;
 }
 
-long long awp_tma_get_spin_limit() { return g_spin_limit; }
+long long awp_tma_get_spin_limit() { return awp_pipe_spin_limit; }

@@ -7,26 +7,28 @@
 //             dtopo_vel_112 (kernels/optimized_velocity.cu:1040-1629),
 //   stress:   dtopo_str_111 / dtopo_str_112 (kernels/stress_attenuation.cu:73-1415),
 // launched by topo_velocity_*_H (velocity.cu) and topo_stress_*_H
-// (stress_attenuation.cu).  Here each half-step is one kernel.  A warp owns 64
-// consecutive levels of one (i, j) column, two adjacent levels per lane, and
-// every lane loads the values of its own two levels only (one 8-byte access
-// per field where the layout is 8-byte aligned): the vertical operators
-// (7-point differences of horizontal interpolants, 4-point differences) take
-// the neighbouring levels from the neighbouring lanes by warp shuffles -- six
-// shuffles give a 7-point difference at both of a lane's levels -- so each
-// value crosses the memory system once per column instead of once per stencil
-// point.  Warps overlap by two lanes (four levels, the operators reach three)
-// on each side: tiles of 56 output levels, the top tile outputting its 60
-// levels under the surface.  The boundary-closure rows r = nz-1-k of the
-// summation-by-parts tables (awp_topo_tables.h) read the top levels of the
-// column, which all sit in the top tile's last lanes, by broadcast shuffles.
+// (stress_attenuation.cu).  Here each half-step is one TMA-pipelined kernel
+// (awp_pipe.cuh): a CTA marches along x with a tile of 64 levels x kCol
+// columns, a producer warp keeping the next planes' tiles in shared memory.
 //
-// Latency: a CTA (four warps = four j columns) takes AWP_TOPO_MARCH
-// consecutive x planes one after another, so x-neighbour reads find the
-// earlier planes in L1.  The values a thread reads only once are copied to
-// shared memory by cp.async when the thread starts on a plane: in the
-// velocity kernel all 31 of its 3-D operands, in the stress kernel the
-// stresses and memory variables the update reads at the end.
+// A warp owns the 64 levels of one column, two adjacent levels per lane, and
+// computes with packed arithmetic (awp_f2.cuh).  The vertical operators
+// (7-point differences of horizontal interpolants, 4-point differences) take
+// the neighbouring levels from the neighbouring lanes by warp shuffles: six
+// shuffles give a 7-point difference at both of a lane's levels.  Warps
+// overlap by two lanes (four levels, the operators reach three) on each side:
+// tiles of 56 output levels, the top tile outputting its 60 levels under the
+// surface.  The boundary-closure rows r = nz-1-k of the summation-by-parts
+// tables (awp_topo_tables.h) read the top levels of the column, which all sit
+// in the top tile's last lanes, by broadcast shuffles; each of the lanes 29..31
+// keeps its two rows' coefficients in shared memory.
+//
+// What makes the operators cheap: the vertical differences are linear and the
+// surface metrics f do not depend on k, so the x and y terms of a component
+// share one difference (three of them for the velocity, five for the stress);
+// a column's surface metrics, already multiplied by the operators' weights,
+// are formed by the warp's lanes in parallel once per plane and read back as
+// broadcasts; the vertical metrics' reciprocals are formed once per march.
 //
 // Term structure (f = surface function interpolants, g = vertical metric;
 // relative indices, k = 0 the bottom point of the grid):
@@ -34,14 +36,15 @@
 //                              - f1 * Dz(g P_x sigma_x) - f2 * Dz(g P_y sigma_y) ]
 //   sigma_t from strain rates  D_x u - J^-1 g P_x(f1 Dz u)  etc.
 // and the memory-variable / sponge update shared with the Cartesian kernels
-// (awp_stress_coef / awp_stress_update).  Every level evaluates the same
-// expressions in the same order (products and sums left to right as the
-// reference's operators); the reference build contracts them into FMAs at its
-// compiler's choice, so agreement with it is to rounding, not bitwise.
+// (awp_stress_coef / awp_stress_update).  The sums are associated differently
+// from the reference's, so agreement with it is to rounding.
 #include "awp_topo_kern.cuh"
 
+#include "awp_pipe.cuh"
 #include "awp_stencil.cuh"
 #include "awp_topo_tables.h"
+
+using namespace awp_pipe;
 
 namespace {
 
@@ -54,149 +57,93 @@ constexpr float kZ0 = (float)-0.0026041666666667, kZ1 = (float)0.093750000000000
 constexpr unsigned kAll = 0xffffffffu;
 constexpr int kSpan = 64;     // levels of a warp
 constexpr int kTileOut = 56;  // output levels of a tile below the top one
+constexpr int kCol = 7;       // columns (computing warps) of a CTA: 8 warps with the producer
+constexpr int kThreads = 32 * (kCol + 1);
+constexpr int kMost = 32;    // planes of a march (march_planes)
+// tiles: own 64 x kCol, j halo 64 x (kCol + 3), media 64 x (kCol + 1)
+constexpr int kOwn = kSpan * kCol, kHalo = kSpan * (kCol + 3), kMed = kSpan * (kCol + 1);
 
-// Component-wise float2 arithmetic: each of a lane's two levels evaluates the
-// scalar expression, with C++'s left-to-right grouping, unchanged.
-__device__ __forceinline__ float2 operator+(float2 a, float2 b) {
-  return make_float2(a.x + b.x, a.y + b.y);
-}
-__device__ __forceinline__ float2 operator-(float2 a, float2 b) {
-  return make_float2(a.x - b.x, a.y - b.y);
-}
-__device__ __forceinline__ float2 operator*(float2 a, float2 b) {
-  return make_float2(a.x * b.x, a.y * b.y);
-}
-__device__ __forceinline__ float2 operator*(float a, float2 b) {
-  return make_float2(a * b.x, a * b.y);
-}
-
-// The reference forms these reciprocals and quotients in double and rounds
-// the result to float.  For float operands the double quotient (53 bits)
-// rounded again to 24 bits equals the correctly rounded float quotient
-// (double rounding is innocuous for division when the wider format has at
-// least 2p + 2 bits; Figueroa, "When is double rounding innocuous?", 1995),
-// so the IEEE float division gives the same bits without the FP64 pipe.
-__device__ __forceinline__ float inv(float x) { return __frcp_rn(x); }
-__device__ __forceinline__ float quot(float x, float y) { return __fdiv_rn(x, y); }
-
-// Asynchronous copies global -> shared (cp.async) of a lane's two levels,
-// issued when a thread starts on a plane for the values it reads once, so
-// their latency overlaps the stencil arithmetic.  Each thread reads back its
-// own slots after cp.async.wait_all; no block barrier is needed.  V2: one
-// 8-byte copy (both addresses 8-byte aligned), else two 4-byte copies.
-__device__ __forceinline__ void cpa(void* s, const float* g, int bytes_is_8) {
-  const unsigned sa = (unsigned)__cvta_generic_to_shared(s);
-  if (bytes_is_8)
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sa), "l"(g) : "memory");
-  else
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(sa), "l"(g) : "memory");
-}
-template <bool V2>
-__device__ __forceinline__ void cpa2(float2* s, const float* g) {
-  if (V2) {
-    cpa(s, g, 1);
-  } else {
-    cpa(&s->x, g, 0);
-    cpa(&s->y, g + 1, 0);
-  }
-}
-__device__ __forceinline__ void cpa_wait() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
-
-template <bool V2>
-__device__ __forceinline__ float2 ld2(const float* __restrict__ p) {
-  if (V2) return __ldg(reinterpret_cast<const float2*>(p));
-  return make_float2(__ldg(p), __ldg(p + 1));
-}
-
-// 1-D vertical metric at a level, and at the lane's two levels
-__device__ __forceinline__ float gk(const float* __restrict__ g, int k) {
-  return __ldg(g + k + AWP_ALIGN);
-}
-__device__ __forceinline__ float2 gk2(const float* __restrict__ g, int k) {
-  return make_float2(__ldg(g + k + AWP_ALIGN), __ldg(g + k + 1 + AWP_ALIGN));
-}
+__device__ __forceinline__ float2 dup(float a) { return make_float2(a, a); }
 
 // Column position of a warp: tile t = 0 holds the top 64 levels, tile t > 0
 // the 64 levels starting 56 t lower; lane L holds levels kb + 2L and
 // kb + 2L + 1.  A level is output when its lane is not a halo lane (two at
 // each end; the top tile has no upper halo) and k >= 3 (the reference leaves
-// the three bottom points to the mesh coupling, dm_offset = 3).  Loads read
-// level max(kb + 2L, -32): the levels below the grid are padding and only
-// ever feed halo lanes, and the clamp keeps a short grid's reads inside it.
+// the three bottom points to the mesh coupling, dm_offset = 3).  Loads from
+// global memory read level max(kb + 2L, -32): the levels below the grid are
+// padding and only ever feed halo lanes, and the clamp keeps a short grid's
+// reads inside it (its tiles' copies are zero-filled there).
 struct ColPos2 {
-  int k, ld, lane, r0, r1;
+  int k, ld, lane;
   bool top, out0, out1;
   __device__ ColPos2(int nz, int tile) {
-    lane = threadIdx.x;
+    lane = threadIdx.x & 31;
     top = (tile == 0);
     k = nz - kSpan - kTileOut * tile + 2 * lane;
     ld = k < -AWP_ALIGN ? -AWP_ALIGN : k;
     const bool in = lane >= 2 && (top || lane <= 29);
     out0 = in && k >= 3;
     out1 = in && k + 1 >= 3;
-    // boundary rows nz-1-k of the top six levels (lanes 29..31)
-    r0 = (top && lane >= 29) ? nz - 1 - k : -1;
-    r1 = (top && lane >= 29) ? nz - 2 - k : -1;
   }
 };
 
-// Boundary-closure rows of the top tile: row r of T applied to the top NT
-// levels (level nz-1-m = lane 31 - m/2, .y for even m).  Every row is formed
-// with compile-time table indices (constant-bank operands, no per-lane indexed
-// constant loads) and each level of lanes 29..31 picks its own row.
+// Boundary-closure rows of one table for the lanes 29..31 of the top tile:
+// c[m][31 - lane] = the coefficients of level nz-1-m in the rows of the
+// lane's two levels (rows 2(31-lane) + 1 and 2(31-lane)).
+struct Closure {
+  float2 c[9][3];
+};
 template <int NT>
-__device__ __forceinline__ void closure(float2 v, const ColPos2& c, const float (&T)[6][NT],
-                                        float2& s) {
-  float top[NT];
-#pragma unroll
-  for (int m = 0; m < NT; ++m) top[m] = __shfl_sync(kAll, (m & 1) ? v.x : v.y, 31 - (m >> 1));
-#pragma unroll
-  for (int rr = 0; rr < 6; ++rr) {
-    float b = 0.f;
-#pragma unroll
-    for (int m = NT - 1; m >= 0; --m) b += T[rr][m] * top[m];
-    if (c.r0 == rr) s.x = b;
-    if (c.r1 == rr) s.y = b;
+__device__ __forceinline__ void closure_load(Closure& cl, const float (&T)[6][NT], int t) {
+  if (t < 27) {
+    const int m = t / 3, q = t % 3;
+    cl.c[m][q] = m < NT ? make_float2(T[2 * q + 1][m], T[2 * q][m]) : make_float2(0.f, 0.f);
   }
+}
+template <int NT>
+__device__ __forceinline__ float2 closure(float2 v, const ColPos2& c, const Closure& cl,
+                                          float2 s) {
+  const int q = c.lane >= 29 ? 31 - c.lane : 0;
+  float2 b = make_float2(0.f, 0.f);
+#pragma unroll
+  for (int m = NT - 1; m >= 0; --m)
+    b = vfma(cl.c[m][q], dup(__shfl_sync(kAll, (m & 1) ? v.x : v.y, 31 - (m >> 1))), b);
+  return c.lane >= 29 ? b : s;
 }
 
 // 7-point vertical difference at the lane's two levels l, l+1 of a value held
-// two levels per lane (interior coefficients), or the boundary rows of T in
-// the top tile.  Summation order as the reference's operators.
-template <int NT>
-__device__ __forceinline__ float2 zd7(float2 v, const ColPos2& c, const float (&T)[6][NT]) {
+// two levels per lane (interior coefficients), or the boundary rows in the
+// top tile.
+__device__ __forceinline__ float2 zd7(float2 v, const ColPos2& c, const Closure& cl) {
   const float m3 = __shfl_up_sync(kAll, v.y, 2);    // l-3
   const float m2 = __shfl_up_sync(kAll, v.x, 1);    // l-2
   const float m1 = __shfl_up_sync(kAll, v.y, 1);    // l-1
   const float p2 = __shfl_down_sync(kAll, v.x, 1);  // l+2
   const float p3 = __shfl_down_sync(kAll, v.y, 1);  // l+3
   const float p4 = __shfl_down_sync(kAll, v.x, 2);  // l+4
-  float2 s;
-  s.x = kZ0 * m3 + kZ1 * m2 + kZ2 * m1 - kZ2 * v.y - kZ1 * p2 - kZ0 * p3;
-  s.y = kZ0 * m2 + kZ1 * m1 + kZ2 * v.x - kZ2 * p2 - kZ1 * p3 - kZ0 * p4;
-  if (c.top) closure(v, c, T, s);  // warp-uniform branch
-  return s;
+  const float2 a = make_float2(m3 - p3, m2 - p4), b = make_float2(m2 - p2, m1 - p3),
+               d = make_float2(m1 - v.y, v.x - p2);
+  const float2 s = vfma(dup(kZ0), a, vfma(dup(kZ1), b, vscale(kZ2, d)));
+  return c.top ? closure<9>(v, c, cl, s) : s;  // warp-uniform branch
 }
 
 // 4-point vertical difference: half-point form (k-2..k+1) or node form
-// (k-1..k+2), or the boundary rows.
-template <int NT>
-__device__ __forceinline__ float2 zd4(float2 v, const ColPos2& c, bool half,
-                                      const float (&T)[6][NT]) {
-  float2 s;
-  if (half) {
-    const float m2 = __shfl_up_sync(kAll, v.x, 1), m1 = __shfl_up_sync(kAll, v.y, 1),
-                p2 = __shfl_down_sync(kAll, v.x, 1);
-    s.x = kD0 * m2 + kD1 * m1 - kD1 * v.x - kD0 * v.y;
-    s.y = kD0 * m1 + kD1 * v.x - kD1 * v.y - kD0 * p2;
+// (k-1..k+2), or the boundary rows (NT of them).
+template <bool HALF, int NT>
+__device__ __forceinline__ float2 zd4(float2 v, const ColPos2& c, const Closure& cl) {
+  const float m1 = __shfl_up_sync(kAll, v.y, 1), p2 = __shfl_down_sync(kAll, v.x, 1);
+  float2 a, b;
+  if (HALF) {
+    const float m2 = __shfl_up_sync(kAll, v.x, 1);
+    a = make_float2(m2 - v.y, m1 - p2);
+    b = make_float2(m1 - v.x, v.x - v.y);
   } else {
-    const float m1 = __shfl_up_sync(kAll, v.y, 1), p2 = __shfl_down_sync(kAll, v.x, 1),
-                p3 = __shfl_down_sync(kAll, v.y, 1);
-    s.x = kD0 * m1 + kD1 * v.x - kD1 * v.y - kD0 * p2;
-    s.y = kD0 * v.x + kD1 * v.y - kD1 * p2 - kD0 * p3;
+    const float p3 = __shfl_down_sync(kAll, v.y, 1);
+    a = make_float2(m1 - p2, v.x - p3);
+    b = make_float2(v.x - v.y, v.y - p2);
   }
-  if (c.top) closure(v, c, T, s);
-  return s;
+  const float2 s = vfma(dup(kD0), a, vscale(kD1, b));
+  return c.top ? closure<NT>(v, c, cl, s) : s;
 }
 
 // The value at level - 1 of each of a lane's two levels
@@ -204,394 +151,579 @@ __device__ __forceinline__ float2 below(float2 v) {
   return make_float2(__shfl_up_sync(kAll, v.y, 1), v.x);
 }
 
-struct Cell {
-  long long o;   // padded index of (i, j, ld): the lane's first load level
-  long long of;  // index of (i, j) in the 2-D metric arrays
-  int S, Y, F;
-  __device__ Cell(const TopoArgs& a, int i, int j, int ld)
-      : o((long long)(i + AWP_NGSL + 2) * a.slice + (long long)(j + AWP_NGSL + 2) * a.yline +
-          (ld + AWP_ALIGN)),
-        of((long long)(i + AWP_NGSL + 2) * a.fld + (j + AWP_NGSL + 2 + AWP_ALIGN)),
-        S(a.slice), Y(a.yline), F(a.fld) {}
-  // 2-D metric at (i+di, j+dj)
-  __device__ __forceinline__ float fm(const float* __restrict__ f, int di, int dj) const {
-    return __ldg(f + of + (di * F + dj));
+// 1-D vertical metric (or sponge) at a lane's two levels
+__device__ __forceinline__ float2 gk2(const float* __restrict__ g, int k) {
+  return make_float2(__ldg(g + k + AWP_ALIGN), __ldg(g + k + 1 + AWP_ALIGN));
+}
+
+// One weight of a column: scale * metric(i + di, j + dj), or scale / metric.
+struct Weight {
+  const float* p;
+  float scale;
+  bool inv;
+  __device__ float at(long long off) const {
+    const float f = __ldg(p + off);
+    return inv ? __fdividef(scale, f) : scale * f;
   }
 };
 
-// Store a lane's two output levels at p (8-byte store where aligned and both
-// are output).
-template <bool V2>
-__device__ __forceinline__ void st2(float* p, float2 v, bool o0, bool o1) {
-  if (V2 && o0 && o1) {
-    *reinterpret_cast<float2*>(p) = v;
-  } else {
-    if (o0) p[0] = v.x;
-    if (o1) p[1] = v.y;
-  }
+// Per-warp table of a plane's weights, duplicated for packed arithmetic, two
+// planes deep.
+template <int N>
+struct Table {
+  float2 w[2][N];
+};
+
+// kD (difference) and kP (interpolation) weights of a 4-point operator
+__device__ __forceinline__ float dw(int q) { return q == 0 ? kD0 : q == 1 ? kD1 : q == 2 ? -kD1 : -kD0; }
+__device__ __forceinline__ float pw(int q) { return (q == 0 || q == 3) ? kP0 : kP1; }
+
+__device__ __forceinline__ float2 dot4(const float2* w, float2 a, float2 b, float2 c, float2 d,
+                                       float2 s) {
+  s = vfma(w[0], a, s);
+  s = vfma(w[1], b, s);
+  s = vfma(w[2], c, s);
+  return vfma(w[3], d, s);
 }
-
-}  // namespace
-
-// CTAs per SM the register allocation is held to, and x planes per CTA;
-// chosen by timing at 512 x 512 x 256 with a hill.
-#ifndef AWP_TOPO_VEL_MINB
-#define AWP_TOPO_VEL_MINB 6
-#endif
-#ifndef AWP_TOPO_STR_MINB
-#define AWP_TOPO_STR_MINB 6
-#endif
-#ifndef AWP_TOPO_MARCH
-#define AWP_TOPO_MARCH 4
-#endif
+__device__ __forceinline__ float2 dot4(const float2* w, float2 a, float2 b, float2 c, float2 d) {
+  float2 s = vmul(w[0], a);
+  s = vfma(w[1], b, s);
+  s = vfma(w[2], c, s);
+  return vfma(w[3], d, s);
+}
+// interior 4-point difference with constant weights
+__device__ __forceinline__ float2 diff4(float2 a, float2 b, float2 c, float2 d) {
+  return vfma(dup(kD0), vsub(a, d), vscale(kD1, vsub(b, c)));
+}
+// interpolant P0 (a + d) + P1 (b + c)
+__device__ __forceinline__ float2 itp4(float2 a, float2 b, float2 c, float2 d) {
+  return vfma(dup(kP0), vadd(a, d), vscale(kP1, vadd(b, c)));
+}
 
 // ===========================================================================
 // Velocity
 // ===========================================================================
-// every 3-D value a velocity thread reads, staged by cp.async in one batch
-enum VelSlot {
-  kU, kV, kW, kR00, kR0m, kRm0, kRmm,
-  kX11_0, kX11_m2, kX11_m1, kX11_p1,
-  kY12_0, kY12_m2, kY12_m1, kY12_p1, kX12_m1, kX12_p1, kX12_p2,
-  kX13_0, kX13_m1, kX13_p1, kX13_p2,
-  kY22_0, kY22_m1, kY22_p1, kY22_p2,
-  kY23_0, kY23_m2, kY23_m1, kY23_p1,
-  kZ33, kVelPre
+// weights of a column: four-point differences of f X, then the slopes of the
+// interpolants, then nu / f of the three components
+enum VelW { kAx = 0, kAy = 4, kBx = 8, kBy = 12, kCy = 16, kCx = 20, kS = 24, kN = 30, kVelW = 33 };
+constexpr int kVelWPad = 40;
+
+struct TopoVelCfg {
+  static constexpr int LA = 1, NH = 1 + LA, DS = 3 + LA;
+  // one stage: xx(i+1), xz(i+2), yy, yz (j halo), zz, density, u, v, w (i)
+  static constexpr int G_XX = 0, G_XZ = kOwn, G_YY = 2 * kOwn, G_YZ = G_YY + kHalo,
+                       G_ZZ = G_YZ + kHalo, G_D = G_ZZ + kOwn, G_O = G_D + kMed,
+                       STAGE = G_O + 3 * kOwn;
+  static constexpr int F_S = DS * kHalo, F_W = F_S + NH * STAGE,
+                       F_C = F_W + kCol * 2 * kVelWPad * 2, F_END = F_C + 4 * 9 * 3 * 2;
+  static constexpr size_t bytes = sizeof(float) * F_END + sizeof(Pipe<NH, 0, kCol>) + 8;
 };
 
-// One column tile of plane i, column j.
-template <bool V2>
-__device__ __forceinline__ void velocity_column(const TopoArgs& a, const ColPos2& c, int i,
-                                                int j, float2 (&pre)[kVelPre][128]) {
-  const Cell X(a, i, j, c.ld);
-  const int tid = threadIdx.y * 32 + threadIdx.x;
-  {
-    auto cp = [&](int slot, const float* f, int di, int dj) {
-      cpa2<V2>(&pre[slot][tid], f + X.o + ((long long)di * X.S + dj * X.Y));
-    };
-    cp(kU, a.u1, 0, 0); cp(kV, a.v1, 0, 0); cp(kW, a.w1, 0, 0);
-    cp(kR00, a.d1, 0, 0); cp(kR0m, a.d1, 0, -1); cp(kRm0, a.d1, -1, 0); cp(kRmm, a.d1, -1, -1);
-    cp(kX11_0, a.xx, 0, 0); cp(kX11_m2, a.xx, -2, 0); cp(kX11_m1, a.xx, -1, 0);
-    cp(kX11_p1, a.xx, 1, 0);
-    cp(kY12_0, a.xy, 0, 0); cp(kY12_m2, a.xy, 0, -2); cp(kY12_m1, a.xy, 0, -1);
-    cp(kY12_p1, a.xy, 0, 1); cp(kX12_m1, a.xy, -1, 0); cp(kX12_p1, a.xy, 1, 0);
-    cp(kX12_p2, a.xy, 2, 0);
-    cp(kX13_0, a.xz, 0, 0); cp(kX13_m1, a.xz, -1, 0); cp(kX13_p1, a.xz, 1, 0);
-    cp(kX13_p2, a.xz, 2, 0);
-    cp(kY22_0, a.yy, 0, 0); cp(kY22_m1, a.yy, 0, -1); cp(kY22_p1, a.yy, 0, 1);
-    cp(kY22_p2, a.yy, 0, 2);
-    cp(kY23_0, a.yz, 0, 0); cp(kY23_m2, a.yz, 0, -2); cp(kY23_m1, a.yz, 0, -1);
-    cp(kY23_p1, a.yz, 0, 1);
-    cp(kZ33, a.zz, 0, 0);
-  }
-  auto P = [&](int slot) { return pre[slot][tid]; };
-  const int k = c.ld;
-  const float2 g3c = gk2(a.g3_c, k), g3 = gk2(a.g3, k), gc = gk2(a.g_c, k), gg = gk2(a.g, k);
-  const float fc = X.fm(a.f_c, 0, 0), ff = X.fm(a.f, 0, 0), f1 = X.fm(a.f_1, 0, 0),
-              f2 = X.fm(a.f_2, 0, 0);
-  const float dcx = __ldg(a.dcrjx + i + AWP_NGSL + 2) * __ldg(a.dcrjy + j + AWP_NGSL + 2);
-  const float2 dcrj = dcx * gk2(a.dcrjz, k);
-  cpa_wait();
-
-  // density at the staggered velocity points (velocity_unroll.cu:140-152)
-  const float2 r00 = P(kR00), r0m = P(kR0m), rm0 = P(kRm0), rmm = P(kRmm);
-  const float2 r00k = below(r00), r0mk = below(r0m), rm0k = below(rm0);
-  const float2 rho1 = 0.25f * (r00k + r0mk) + 0.25f * (r00 + r0m);
-  const float2 rho2 = 0.25f * (r00k + rm0k) + 0.25f * (r00 + rm0);
-  const float2 rho3 = 0.25f * (r00 + rm0) + 0.25f * (r0m + rmm);
-  const float2 d1a = f1 * g3c * rho1, d2a = f2 * g3c * rho2, d3a = fc * g3 * rho3;
-  const float2 Ai1 = make_float2(quot(a.nu, d1a.x), quot(a.nu, d1a.y));
-  const float2 Ai2 = make_float2(quot(a.nu, d2a.x), quot(a.nu, d2a.y));
-  const float2 Ai3 = make_float2(quot(a.nu, d3a.x), quot(a.nu, d3a.y));
-
-  // --- u1 -------------------------------------------------------------------
-  float2 s1 = -kD1 * fc * g3c * P(kX11_0) + kD0 * X.fm(a.f_c, -2, 0) * g3c * P(kX11_m2) +
-              kD1 * X.fm(a.f_c, -1, 0) * g3c * P(kX11_m1) -
-              kD0 * X.fm(a.f_c, 1, 0) * g3c * P(kX11_p1);
-  s1 = s1 + (-kD1 * ff * g3c * P(kY12_0) + kD0 * X.fm(a.f, 0, -2) * g3c * P(kY12_m2) +
-             kD1 * X.fm(a.f, 0, -1) * g3c * P(kY12_m1) - kD0 * X.fm(a.f, 0, 1) * g3c * P(kY12_p1));
-  s1 = s1 + zd4(P(kX13_0), c, true, kTopoVelDhz4r);
-  {
-    const float2 px =
-        gc * (kP1 * P(kX11_0) + kP0 * P(kX11_m2) + kP1 * P(kX11_m1) + kP0 * P(kX11_p1));
-    const float2 py =
-        gc * (kP1 * P(kY12_0) + kP0 * P(kY12_m2) + kP1 * P(kY12_m1) + kP0 * P(kY12_p1));
-    s1 = s1 - X.fm(a.f1_1, 0, 0) * zd7(px, c, kTopoVelDhpz4r);
-    s1 = s1 - X.fm(a.f2_1, 0, 0) * zd7(py, c, kTopoVelDhpz4r);
-  }
-  // --- u2 -------------------------------------------------------------------
-  float2 s2 = zd4(P(kY23_0), c, true, kTopoVelDhz4r);
-  s2 = s2 + (kD1 * ff * g3c * P(kY12_0) + kD0 * X.fm(a.f, -1, 0) * g3c * P(kX12_m1) -
-             kD1 * X.fm(a.f, 1, 0) * g3c * P(kX12_p1) - kD0 * X.fm(a.f, 2, 0) * g3c * P(kX12_p2));
-  s2 = s2 + (kD1 * fc * g3c * P(kY22_0) + kD0 * X.fm(a.f_c, 0, -1) * g3c * P(kY22_m1) -
-             kD1 * X.fm(a.f_c, 0, 1) * g3c * P(kY22_p1) -
-             kD0 * X.fm(a.f_c, 0, 2) * g3c * P(kY22_p2));
-  {
-    const float2 px =
-        gc * (kP1 * P(kY12_0) + kP0 * P(kX12_m1) + kP1 * P(kX12_p1) + kP0 * P(kX12_p2));
-    const float2 py =
-        gc * (kP1 * P(kY22_0) + kP0 * P(kY22_m1) + kP1 * P(kY22_p1) + kP0 * P(kY22_p2));
-    s2 = s2 - X.fm(a.f1_2, 0, 0) * zd7(px, c, kTopoVelDhpz4r);
-    s2 = s2 - X.fm(a.f2_2, 0, 0) * zd7(py, c, kTopoVelDhpz4r);
-  }
-  // --- u3 -------------------------------------------------------------------
-  float2 s3 = -kD1 * f2 * g3 * P(kY23_0) + kD0 * X.fm(a.f_2, 0, -2) * g3 * P(kY23_m2) +
-              kD1 * X.fm(a.f_2, 0, -1) * g3 * P(kY23_m1) -
-              kD0 * X.fm(a.f_2, 0, 1) * g3 * P(kY23_p1);
-  s3 = s3 + (kD1 * f1 * g3 * P(kX13_0) + kD0 * X.fm(a.f_1, -1, 0) * g3 * P(kX13_m1) -
-             kD1 * X.fm(a.f_1, 1, 0) * g3 * P(kX13_p1) - kD0 * X.fm(a.f_1, 2, 0) * g3 * P(kX13_p2));
-  s3 = s3 + zd4(P(kZ33), c, false, kTopoVelDz4r);
-  {
-    const float2 px =
-        gg * (kP1 * P(kX13_0) + kP0 * P(kX13_m1) + kP1 * P(kX13_p1) + kP0 * P(kX13_p2));
-    const float2 py =
-        gg * (kP1 * P(kY23_0) + kP0 * P(kY23_m2) + kP1 * P(kY23_m1) + kP0 * P(kY23_p1));
-    s3 = s3 - X.fm(a.f1_c, 0, 0) * zd7(px, c, kTopoVelDphz4r);
-    s3 = s3 - X.fm(a.f2_c, 0, 0) * zd7(py, c, kTopoVelDphz4r);
-  }
-
-  if (!(c.out0 || c.out1)) return;
-  st2<V2>(a.u1 + X.o, (P(kU) + Ai1 * s1) * dcrj, c.out0, c.out1);
-  st2<V2>(a.v1 + X.o, (P(kV) + Ai2 * s2) * dcrj, c.out0, c.out1);
-  st2<V2>(a.w1 + X.o, (P(kW) + Ai3 * s3) * dcrj, c.out0, c.out1);
-}
-
-// A CTA takes four columns of AWP_TOPO_MARCH consecutive x planes, one plane
-// after another, so that the x-neighbour reads of a plane find the previous
-// planes' values in L1.
-template <bool V2>
-__global__ void __launch_bounds__(128, AWP_TOPO_VEL_MINB) k_topo_velocity(const TopoArgs a) {
+__global__ void __launch_bounds__(kThreads, 2)
+    k_topo_velocity(const __grid_constant__ TopoArgs a, const __grid_constant__ TmaMaps tm,
+                    const int ichunk, int* err, const unsigned spin) {
+  using C = TopoVelCfg;
+  extern __shared__ __align__(128) float smem[];
+  Closure* const cl = reinterpret_cast<Closure*>(smem + C::F_C);
+  auto& pipe = *reinterpret_cast<Pipe<C::NH, 0, kCol>*>(smem + C::F_END);
+  const int tid = threadIdx.x, warp = tid >> 5;
   const ColPos2 c(a.nz, blockIdx.x);
-  const int j = blockIdx.y * 4 + threadIdx.y;
-  if (j >= a.ny) return;  // whole warps
-  __shared__ float2 pre[kVelPre][128];
-  const int i0 = blockIdx.z * AWP_TOPO_MARCH, i1 = min(i0 + AWP_TOPO_MARCH, a.nx);
+  const int kb = AWP_ALIGN + a.nz - kSpan - kTileOut * (int)blockIdx.x;
+  const int j0 = blockIdx.y * kCol, jb = j0 + AWP_NGSL + 2;
+  const int i0 = blockIdx.z * ichunk, n = min(ichunk, a.nx - i0), ib = i0 + AWP_NGSL + 2;
+  if (tid == 0) pipe.init();
+  closure_load(cl[0], kTopoVelDhpz4r, tid);
+  closure_load(cl[1], kTopoVelDphz4r, tid);
+  closure_load(cl[2], kTopoVelDhz4r, tid);
+  closure_load(cl[3], kTopoVelDz4r, tid);
+  __syncthreads();
+
+  if (warp == kCol) {  // producer warp
+    if (c.lane == 0) {
+      pipe.produce(
+          n,
+          [&](int s, uint64_t* b) {
+            const int p0 = s == 0 ? 0 : s + 2;
+            mbar_expect_tx(b, ((s + 2 - p0 + 1) * kHalo + C::STAGE) * 4);
+            for (int p = p0; p <= s + 2; ++p)
+              tma_load3(smem + (p % C::DS) * kHalo, &tm.halo[3], b, kb, jb - 2, ib + p);
+            float* g = smem + C::F_S + (s % C::NH) * C::STAGE;
+            const int i = ib + s;
+            tma_load3(g + C::G_XX, &tm.halo[0], b, kb, jb, i + 1);
+            tma_load3(g + C::G_XZ, &tm.halo[4], b, kb, jb, i + 2);
+            tma_load3(g + C::G_YY, &tm.halo[1], b, kb, jb - 1, i);
+            tma_load3(g + C::G_YZ, &tm.halo[5], b, kb, jb - 2, i);
+            tma_load3(g + C::G_ZZ, &tm.halo[2], b, kb, jb, i);
+            tma_load3(g + C::G_D, &tm.media[0], b, kb, jb - 1, i);
+            for (int f = 0; f < 3; ++f)
+              tma_load3(g + C::G_O + f * kOwn, &tm.own[f], b, kb, jb, i);
+          },
+          [](int, uint64_t*) {}, err, spin);
+    }
+    return;
+  }
+
+  const int j = j0 + warp;
+  const bool jin = j < a.ny;
+  const bool o0 = c.out0 && jin, o1 = c.out1 && jin;
+  const int S = a.slice, Y = a.yline, FL = a.fld;
+  const int ja = jb + warp;  // a warp past the grid computes on its padding
+  const int jm = min(j, a.ny - 1);
+  long long o = (long long)ib * S + (long long)ja * Y + (c.ld + AWP_ALIGN);
+  // this lane's two weights of the column (weight index lane, lane + 32)
+  Table<kVelWPad>& tab = reinterpret_cast<Table<kVelWPad>*>(smem + C::F_W)[warp];
+  auto weight = [&](int w) {
+    // arrays of the six differences, six slopes and three quotients
+    const float* const D[6] = {a.f_c, a.f, a.f, a.f_c, a.f_2, a.f_1};
+    const float* const SL[6] = {a.f1_1, a.f2_1, a.f1_2, a.f2_2, a.f1_c, a.f2_c};
+    const float* const Q[3] = {a.f_1, a.f_2, a.f_c};
+    // first offset and axis (x: true) of the differences, in VelW's order
+    constexpr int first[6] = {-2, -2, -1, -1, -2, -1};
+    constexpr bool alongx[6] = {true, false, true, false, false, true};
+    Weight r{a.f, 0.f, false};
+    int di = 0, dj = 0;
+    if (w < kS) {
+      const int q = w >> 2, m = w & 3;
+      r.p = D[q];
+      r.scale = dw(m);
+      (alongx[q] ? di : dj) = first[q] + m;
+    } else if (w < kN) {
+      r.p = SL[w - kS];
+      r.scale = 1.0f;
+    } else if (w < kVelW) {
+      r.p = Q[w - kN];
+      r.scale = a.nu;
+      r.inv = true;
+    }
+    r.p += (long long)(ib + di) * FL + (jm + dj + AWP_NGSL + 2 + AWP_ALIGN);
+    return r;
+  };
+  const Weight w0 = weight(c.lane), w1 = weight(c.lane + 32);
+  float n0 = w0.at(0), n1 = c.lane < 1 ? w1.at(0) : 0.f;
+
+  const float2 g3c = gk2(a.g3_c, c.ld), g3 = gk2(a.g3, c.ld), gc = gk2(a.g_c, c.ld),
+               gg = gk2(a.g, c.ld);
+  const float2 ig3c = vquot(1.0f, g3c), ig3 = vquot(1.0f, g3);
+  const float2 dcz = vscale(__ldg(a.dcrjy + ja), gk2(a.dcrjz, c.ld));
+  // own-column values of the planes before the ones the tiles bring
+  float2 xx_m2, xx_m1, xx_0, xy_m1, xy_0, xy_p1, xz_m1, xz_0, xz_p1, d_m, t_m;
+  {
+    const float *X = a.xx + o, *P = a.xy + o, *Q = a.xz + o, *D = a.d1 + o - S;
+    xx_m2 = ldg2(X - 2 * (long long)S); xx_m1 = ldg2(X - S); xx_0 = ldg2(X);
+    xy_m1 = ldg2(P - S); xy_0 = ldg2(P); xy_p1 = ldg2(P + S);
+    xz_m1 = ldg2(Q - S); xz_0 = ldg2(Q); xz_p1 = ldg2(Q + S);
+    d_m = ldg2(D);
+    t_m = vadd(d_m, ldg2(D - Y));
+  }
+  const int l = 2 * c.lane;
+  const int h0 = warp * kSpan + l, h1 = (warp + 1) * kSpan + l, h2 = (warp + 2) * kSpan + l;
+
+  Cursor<C::NH> ch;
+  Cursor<awp_pipe::ND> cd;
+  int ss = 0, ss2 = 2;
+  bool ok = true;
 #pragma unroll 1
-  for (int i = i0; i < i1; ++i) velocity_column<V2>(a, c, i, j, pre);
+  for (int s = 0; s < n; ++s) {
+    // the plane's weights, then the next plane's loads
+    float2* const W = tab.w[s & 1];
+    W[c.lane] = dup(n0);
+    if (c.lane < 1) W[32] = dup(n1);
+    if (s + 1 < n) {
+      n0 = w0.at((long long)(s + 1) * FL);
+      if (c.lane < 1) n1 = w1.at((long long)(s + 1) * FL);
+    }
+    const float dcx = __ldg(a.dcrjx + ib + s);
+    __syncwarp();
+    ok = mbar_wait(pipe.full_h + ch.slot, ch.phase, spin);
+    if (!__all_sync(kAll, ok)) break;
+    const float* G = smem + C::F_S + ch.slot * C::STAGE;
+    const float* XY = smem + ss * kHalo + h2;
+    const float* YY = G + C::G_YY + h1;
+    const float* YZ = G + C::G_YZ + h2;
+    const float2 xx_p1 = lds2(G + C::G_XX + h0), xz_p2 = lds2(G + C::G_XZ + h0);
+    const float2 xy_p2 = lds2(smem + ss2 * kHalo + h2);
+    const float2 d_0 = lds2(G + C::G_D + h1), t_0 = vadd(d_0, lds2(G + C::G_D + h0));
+    const float2 dcrj = vscale(dcx, dcz);
+
+    // --- u1 -----------------------------------------------------------------
+    {
+      const float2 y2 = lds2(XY - 2 * kSpan), y1 = lds2(XY - kSpan), yp = lds2(XY + kSpan);
+      float2 e = dot4(W + kAx, xx_m2, xx_m1, xx_0, xx_p1);
+      e = dot4(W + kAy, y2, y1, xy_0, yp, e);
+      e = vfma(g3c, e, zd4<true, 8>(xz_0, c, cl[2]));
+      float2 q = vmul(W[kS], itp4(xx_m2, xx_m1, xx_0, xx_p1));
+      q = vfma(W[kS + 1], itp4(y2, y1, xy_0, yp), q);
+      e = vsub(e, zd7(vmul(gc, q), c, cl[0]));
+      const float2 A = vmul(vmul(W[kN], ig3c), vquot(1.0f, vscale(0.25f, vadd(t_0, below(t_0)))));
+      st2(a.u1 + o, vmul(vfma(A, e, lds2(G + C::G_O + h0)), dcrj), o0, o1);
+    }
+    const float2 yz_0 = lds2(YZ);
+    // --- u2 -----------------------------------------------------------------
+    {
+      const float2 y0 = lds2(YY), ym = lds2(YY - kSpan), y1 = lds2(YY + kSpan),
+                   y2 = lds2(YY + 2 * kSpan);
+      float2 e = dot4(W + kBx, xy_m1, xy_0, xy_p1, xy_p2);
+      e = dot4(W + kBy, ym, y0, y1, y2, e);
+      e = vfma(g3c, e, zd4<true, 8>(yz_0, c, cl[2]));
+      float2 q = vmul(W[kS + 2], itp4(xy_m1, xy_0, xy_p1, xy_p2));
+      q = vfma(W[kS + 3], itp4(ym, y0, y1, y2), q);
+      e = vsub(e, zd7(vmul(gc, q), c, cl[0]));
+      const float2 x = vadd(d_0, d_m);
+      const float2 A = vmul(vmul(W[kN + 1], ig3c), vquot(1.0f, vscale(0.25f, vadd(x, below(x)))));
+      st2(a.v1 + o, vmul(vfma(A, e, lds2(G + C::G_O + kOwn + h0)), dcrj), o0, o1);
+    }
+    // --- u3 -----------------------------------------------------------------
+    {
+      const float2 y2 = lds2(YZ - 2 * kSpan), y1 = lds2(YZ - kSpan), yp = lds2(YZ + kSpan);
+      float2 e = dot4(W + kCy, y2, y1, yz_0, yp);
+      e = dot4(W + kCx, xz_m1, xz_0, xz_p1, xz_p2, e);
+      e = vfma(g3, e, zd4<false, 7>(lds2(G + C::G_ZZ + h0), c, cl[3]));
+      float2 q = vmul(W[kS + 4], itp4(xz_m1, xz_0, xz_p1, xz_p2));
+      q = vfma(W[kS + 5], itp4(y2, y1, yz_0, yp), q);
+      e = vsub(e, zd7(vmul(gg, q), c, cl[1]));
+      const float2 A = vmul(vmul(W[kN + 2], ig3), vquot(1.0f, vscale(0.25f, vadd(t_0, t_m))));
+      st2(a.w1 + o, vmul(vfma(A, e, lds2(G + C::G_O + 2 * kOwn + h0)), dcrj), o0, o1);
+    }
+    warp_done(pipe.done + cd.slot, c.lane);
+
+    o += S;
+    xx_m2 = xx_m1; xx_m1 = xx_0; xx_0 = xx_p1;
+    xy_m1 = xy_0; xy_0 = xy_p1; xy_p1 = xy_p2;
+    xz_m1 = xz_0; xz_0 = xz_p1; xz_p1 = xz_p2;
+    d_m = d_0; t_m = t_0;
+    ch.next();
+    cd.next();
+    ss = ss + 1 == C::DS ? 0 : ss + 1;
+    ss2 = ss2 + 1 == C::DS ? 0 : ss2 + 1;
+  }
+  if (!__all_sync(kAll, ok) && c.lane == 0) atomicExch(err, 1);
 }
 
 // ===========================================================================
 // Stress and memory variables
 // ===========================================================================
-// A stress thread stages the stresses and memory variables of its two levels
-// by cp.async when it starts on a plane (read only by the update at its end);
-// the velocity stencil and the media are read where they are used, through L1.
+// weights of a column: the interpolants of f-weighted velocities, then 1 / f
+enum StrW { kIu = 0, kIv = 4, kJu = 8, kJv = 12, kKw = 16, kLw = 20, kF = 24, kStrW = 28 };
+
 template <bool ELASTIC>
-struct StrStage {
-  static constexpr int kRows = ELASTIC ? 6 : 12;
+struct TopoStrCfg {
+  static constexpr int NM = ELASTIC ? 2 : 4, NF = ELASTIC ? 6 : 12;
+  static constexpr int LH = 1, LO = 1, NH = 1 + LH, NO = 1 + LO, DU = 3 + LH, DV = 2 + LH;
+  static constexpr int F_U = 0, F_V = F_U + DU * kHalo, F_W = F_V + DV * kHalo,
+                       F_M = F_W + DV * kHalo, F_O = F_M + NH * NM * kMed,
+                       F_T = F_O + NO * NF * kOwn, F_X = F_T + (ELASTIC ? 0 : 80),
+                       F_C = F_X + kCol * 2 * 32 * 2, F_END = F_C + 4 * 9 * 3 * 2;
+  static constexpr size_t bytes = sizeof(float) * F_END + sizeof(Pipe<NH, NO, kCol>) + 8;
 };
 
-template <bool ELASTIC, bool V2>
-__device__ __forceinline__ void stress_column(const TopoArgs& a, const ColPos2& c, int i, int j,
-                                              float2 (&pre)[StrStage<ELASTIC>::kRows][128]) {
-  const Cell X(a, i, j, c.ld);
-  const int k = c.ld;
-  const int S1 = a.slice, Y1 = a.yline;
-  const long long o = X.o;
-  const int tid = threadIdx.y * 32 + threadIdx.x;
-  float* const SG[6] = {a.xx, a.yy, a.zz, a.xy, a.xz, a.yz};
-  float* const RR[6] = {a.r1, a.r2, a.r3, a.r4, a.r5, a.r6};
+template <bool ELASTIC>
+__global__ void __launch_bounds__(kThreads, 2)
+    k_topo_stress(const __grid_constant__ TopoArgs a, const __grid_constant__ TmaMaps tm,
+                  const int ichunk, int* err, const unsigned spin) {
+  using C = TopoStrCfg<ELASTIC>;
+  constexpr int NM = C::NM, NF = C::NF;
+  extern __shared__ __align__(128) float smem[];
+  Closure* const cl = reinterpret_cast<Closure*>(smem + C::F_C);
+  auto& pipe = *reinterpret_cast<Pipe<C::NH, C::NO, kCol>*>(smem + C::F_END);
+  const int tid = threadIdx.x, warp = tid >> 5;
+  const ColPos2 c(a.nz, blockIdx.x);
+  const int kb = AWP_ALIGN + a.nz - kSpan - kTileOut * (int)blockIdx.x;
+  const int j0 = a.s_j + blockIdx.y * kCol, jb = j0 + AWP_NGSL + 2;
+  const int i0 = a.s_i + blockIdx.z * ichunk, n = min(ichunk, a.e_i - i0),
+            ib = i0 + AWP_NGSL + 2;
+  if (tid == 0) pipe.init();
+  closure_load(cl[0], kTopoStrPhdz4r, tid);
+  closure_load(cl[1], kTopoStrPdhz4r, tid);
+  closure_load(cl[2], kTopoStrDhz4r, tid);
+  closure_load(cl[3], kTopoStrDz4r, tid);
+  if (!ELASTIC) {  // relaxation constants of the entry pairs (as k_stress_tma)
+    float* t = smem + C::F_T;
+    const float* const src[9] = {a.rel.vx2, a.rel.wwo, a.rel.kv, a.rel.kr, a.rel.kr2,
+                                 a.rel.kf,  a.rel.c0,  a.rel.c1, a.rel.c2};
 #pragma unroll
-  for (int q = 0; q < 6; ++q) cpa2<V2>(&pre[q][tid], SG[q] + o);
-  if (!ELASTIC) {
-#pragma unroll
-    for (int q = 0; q < 6; ++q) cpa2<V2>(&pre[6 + q][tid], RR[q] + o);
+    for (int q = 0; q < 9; ++q)
+      if (tid < 8) t[(tid >> 1) * 20 + 2 * q + (tid & 1)] = src[q][tid];
   }
-  // the 21 velocity stencil points: (field, di, dj)
-  constexpr signed char kStencil[21][3] = {
-      {0, 0, 0}, {0, -1, 0}, {0, 1, 0}, {0, 2, 0}, {0, 0, -1}, {0, 0, 1}, {0, 0, 2},
-      {1, 0, 0}, {1, 0, -2}, {1, 0, -1}, {1, 0, 1}, {1, -2, 0}, {1, -1, 0}, {1, 1, 0},
-      {2, 0, 0}, {2, -2, 0}, {2, -1, 0}, {2, 1, 0}, {2, 0, -1}, {2, 0, 1}, {2, 0, 2}};
-  const float* const V[3] = {a.u1, a.v1, a.w1};
-  auto P = [&](int n) {
-    return ld2<V2>(V[kStencil[n][0]] + o + (kStencil[n][1] * S1 + kStencil[n][2] * Y1));
-  };
-  const float2 gc = gk2(a.g_c, k), g = gk2(a.g, k);
+  __syncthreads();
 
-  // every vertical difference of a horizontal interpolant is one difference
-  // of the interpolated column (the metric weights do not depend on k)
-  float2 d[9];
-  // ---- normal components: Jii = 1 / (f_c g3_c) (stress_attenuation.cu:340-431)
-  const float2 jii = X.fm(a.f_c, 0, 0) * gk2(a.g3_c, k);
-  const float2 Jii = make_float2(inv(jii.x), inv(jii.y));
-  const float2 u_0 = P(0), u_xm1 = P(1), u_xp1 = P(2), u_xp2 = P(3);
-  const float2 v_0 = P(7), v_ym2 = P(8), v_ym1 = P(9), v_yp1 = P(10);
-  const float2 w_0 = P(14);
-  {
-    const float2 iu = kP0 * X.fm(a.f1_1, -1, 0) * u_xm1 + kP1 * X.fm(a.f1_1, 0, 0) * u_0 +
-                      kP1 * X.fm(a.f1_1, 1, 0) * u_xp1 + kP0 * X.fm(a.f1_1, 2, 0) * u_xp2;
-    d[0] = kD1 * u_0 + kD0 * u_xm1 - kD1 * u_xp1 - kD0 * u_xp2 -
-           Jii * gc * zd7(iu, c, kTopoStrPhdz4r);
-    const float2 iv = kP1 * X.fm(a.f2_2, 0, 0) * v_0 + kP0 * X.fm(a.f2_2, 0, -2) * v_ym2 +
-                      kP1 * X.fm(a.f2_2, 0, -1) * v_ym1 + kP0 * X.fm(a.f2_2, 0, 1) * v_yp1;
-    d[1] = -kD1 * v_0 + kD0 * v_ym2 + kD1 * v_ym1 - kD0 * v_yp1 -
-           Jii * gc * zd7(iv, c, kTopoStrPhdz4r);
-    d[2] = Jii * zd4(w_0, c, true, kTopoStrDhz4r);
-  }
-  // ---- xy: J12i = 1 / (f g3_c); the interior rows read g3_c six points
-  // higher (stress_attenuation.cu:471), the boundary rows at k (:1149)
-  {
-    const float f0 = X.fm(a.f, 0, 0);
-    const float2 J12i = make_float2(inv(f0 * gk(a.g3_c, c.r0 < 0 ? k + 6 : k)),
-                                    inv(f0 * gk(a.g3_c, c.r1 < 0 ? k + 7 : k + 1)));
-    const float2 u_ym1 = P(4), u_yp1 = P(5), u_yp2 = P(6);
-    const float2 iu = kP1 * X.fm(a.f2_1, 0, 0) * u_0 + kP0 * X.fm(a.f2_1, 0, -1) * u_ym1 +
-                      kP1 * X.fm(a.f2_1, 0, 1) * u_yp1 + kP0 * X.fm(a.f2_1, 0, 2) * u_yp2;
-    d[3] = kD1 * u_0 + kD0 * u_ym1 - kD1 * u_yp1 - kD0 * u_yp2 -
-           J12i * gc * zd7(iu, c, kTopoStrPhdz4r);
-    const float2 v_xm2 = P(11), v_xm1 = P(12), v_xp1 = P(13);
-    const float2 iv = kP1 * X.fm(a.f1_2, 0, 0) * v_0 + kP0 * X.fm(a.f1_2, -2, 0) * v_xm2 +
-                      kP1 * X.fm(a.f1_2, -1, 0) * v_xm1 + kP0 * X.fm(a.f1_2, 1, 0) * v_xp1;
-    d[4] = -kD1 * v_0 + kD0 * v_xm2 + kD1 * v_xm1 - kD0 * v_xp1 -
-           J12i * gc * zd7(iv, c, kTopoStrPhdz4r);
-  }
-  // ---- xz: J13i = 1 / (f_1 g3) (:550-598, :1254-1317)
-  {
-    const float2 j13 = X.fm(a.f_1, 0, 0) * gk2(a.g3, k);
-    const float2 J13i = make_float2(inv(j13.x), inv(j13.y));
-    d[5] = J13i * zd4(u_0, c, false, kTopoStrDz4r);
-    const float2 w_xm2 = P(15), w_xm1 = P(16), w_xp1 = P(17);
-    const float2 iw = kP1 * X.fm(a.f1_c, 0, 0) * w_0 + kP0 * X.fm(a.f1_c, -2, 0) * w_xm2 +
-                      kP1 * X.fm(a.f1_c, -1, 0) * w_xm1 + kP0 * X.fm(a.f1_c, 1, 0) * w_xp1;
-    d[6] = -kD1 * w_0 + kD0 * w_xm2 + kD1 * w_xm1 - kD0 * w_xp1 -
-           J13i * g * zd7(iw, c, kTopoStrPdhz4r);
-  }
-  // ---- yz: J23i = 1 / (f_2 g3) (:600-650, :1319-1380)
-  {
-    const float2 j23 = X.fm(a.f_2, 0, 0) * gk2(a.g3, k);
-    const float2 J23i = make_float2(inv(j23.x), inv(j23.y));
-    d[7] = J23i * zd4(v_0, c, false, kTopoStrDz4r);
-    const float2 w_ym1 = P(18), w_yp1 = P(19), w_yp2 = P(20);
-    const float2 iw = kP1 * X.fm(a.f2_c, 0, 0) * w_0 + kP0 * X.fm(a.f2_c, 0, -1) * w_ym1 +
-                      kP1 * X.fm(a.f2_c, 0, 1) * w_yp1 + kP0 * X.fm(a.f2_c, 0, 2) * w_yp2;
-    d[8] = kD1 * w_0 + kD0 * w_ym1 - kD1 * w_yp1 - kD0 * w_yp2 -
-           J23i * g * zd7(iw, c, kTopoStrPdhz4r);
-  }
-
-  // ---- material coefficients and the update (as the Cartesian dstrqc); the
-  // level-1 neighbours of the eight-cell sums from the lane's first level and
-  // the lane below
-  const float* const MT[4] = {a.lam, a.mu, a.qp, a.qs};
-  const long long corner[4] = {o, o + S1, o - Y1, o + S1 - Y1};
-  auto mat = [&](int m, int q) { return ld2<V2>(MT[m] + corner[q]); };
-  auto sum8 = [&](int m) {
-    const float2 q0 = mat(m, 0), q1 = mat(m, 1), q2 = mat(m, 2), q3 = mat(m, 3);
-    return q0 + q1 + q2 + q3 + below(q0) + below(q1) + below(q2) + below(q3);
-  };
-  const float2 L8 = sum8(0), M8 = sum8(1);
-  const float2 QP8 = ELASTIC ? make_float2(0.f, 0.f) : sum8(2);
-  const float2 QS8 = ELASTIC ? make_float2(0.f, 0.f) : sum8(3);
-  const float2 mu0 = mat(1, 0), muk = below(mu0);
-  const float2 qs0 = ELASTIC ? make_float2(0.f, 0.f) : mat(3, 0);
-  const float2 qsk = below(qs0);
-  cpa_wait();
-  if (!(c.out0 || c.out1)) return;
-  const float2 mu_j = mat(1, 2), mu_i = mat(1, 1);
-  const float2 qs_j = ELASTIC ? make_float2(0.f, 0.f) : mat(3, 2);
-  const float2 qs_i = ELASTIC ? make_float2(0.f, 0.f) : mat(3, 1);
-  const int ia = i + AWP_NGSL + 2, ja = j + AWP_NGSL + 2;
-  const float dcx = __ldg(a.dcrjx + ia) * __ldg(a.dcrjy + ja);
-  float2 sg2[6], rr2[6];
-#pragma unroll
-  for (int q = 0; q < 6; ++q) {
-    sg2[q] = pre[q][tid];
-    rr2[q] = ELASTIC ? make_float2(0.f, 0.f) : pre[6 + q][tid];
-  }
-#pragma unroll
-  for (int e = 0; e < 2; ++e) {
-    auto el = [e](float2 v) { return e ? v.y : v.x; };
-    const int ka = k + e + AWP_ALIGN;
-    const int t = awp_tex_index(a.tex, ia, ja, ka);
-    const float f_vx1 = a.tex.tau1[t], f_vx2 = a.tex.tau2[t], f_wwo = a.tex.wwo8[t];
-    const float cc0 = ELASTIC ? 0.f : a.coeff[2 * t], cc1 = ELASTIC ? 0.f : a.coeff[2 * t + 1];
-    const AwpStrCoef cf = awp_stress_coef<ELASTIC>(
-        el(L8), el(M8), el(mu0), el(muk), el(mu_j), el(mu_i), el(QP8), el(QS8), el(qs0),
-        el(qsk), el(qs_j), el(qs_i), f_vx1, f_vx2, f_wwo, cc0, cc1, a.qthr, a.dth, a.dh1, a.DT);
-    const float dcrj = dcx * __ldg(a.dcrjz + ka);
-    float sg[6], rr[6], de[9];
-#pragma unroll
-    for (int q = 0; q < 6; ++q) {
-      sg[q] = el(sg2[q]);
-      rr[q] = el(rr2[q]);
+  if (warp == kCol) {  // producer warp
+    if (c.lane == 0) {
+      pipe.produce(
+          n,
+          [&](int s, uint64_t* b) {
+            const int u0 = s == 0 ? 0 : s + 2, v0 = s == 0 ? 0 : s + 1;
+            mbar_expect_tx(
+                b, ((s + 2 - u0 + 1) * kHalo + 2 * (s + 1 - v0 + 1) * kHalo + NM * kMed) * 4);
+            for (int p = u0; p <= s + 2; ++p)
+              tma_load3(smem + C::F_U + (p % C::DU) * kHalo, &tm.halo[0], b, kb, jb - 1, ib + p);
+            for (int p = v0; p <= s + 1; ++p) {
+              tma_load3(smem + C::F_V + (p % C::DV) * kHalo, &tm.halo[1], b, kb, jb - 2, ib + p);
+              tma_load3(smem + C::F_W + (p % C::DV) * kHalo, &tm.halo[2], b, kb, jb - 1, ib + p);
+            }
+            float* m = smem + C::F_M + (s % C::NH) * NM * kMed;
+            for (int f = 0; f < NM; ++f)
+              tma_load3(m + f * kMed, &tm.media[f], b, kb, jb - 1, ib + s + 1);
+          },
+          [&](int s, uint64_t* b) {
+            mbar_expect_tx(b, NF * kOwn * 4);
+            float* q = smem + C::F_O + (s % C::NO) * NF * kOwn;
+            for (int f = 0; f < NF; ++f)
+              tma_load3(q + f * kOwn, &tm.own[f], b, kb, jb, ib + s);
+          },
+          err, spin);
     }
-#pragma unroll
-    for (int q = 0; q < 9; ++q) de[q] = el(d[q]);
-    awp_stress_update<ELASTIC>(sg, rr, cf, f_vx1, f_vx2, f_wwo, a.DT, dcrj, de);
+    return;
+  }
+
+  const int j = j0 + warp;
+  const bool jin = j < a.e_j;
+  const bool o0 = c.out0 && jin, o1 = c.out1 && jin;
+  const int S = a.slice, Y = a.yline, FL = a.fld;
+  const int ja = jb + warp, jm = min(j, a.ny - 1);
+  long long o = (long long)ib * S + (long long)ja * Y + (c.ld + AWP_ALIGN);
+  float* __restrict__ SG[6] = {a.xx, a.yy, a.zz, a.xy, a.xz, a.yz};
+  float* __restrict__ RR[6] = {a.r1, a.r2, a.r3, a.r4, a.r5, a.r6};
+  Table<32>& tab = reinterpret_cast<Table<32>*>(smem + C::F_X)[warp];
+  Weight wt{a.f, 0.f, false};
+  {
+    // interpolants: f1_1 u (x), f2_2 v (y), f2_1 u (y), f1_2 v (x), f1_c w (x),
+    // f2_c w (y); then 1/f_c, 1/f, 1/f_1, 1/f_2
+    const float* const I[6] = {a.f1_1, a.f2_2, a.f2_1, a.f1_2, a.f1_c, a.f2_c};
+    const float* const Q[4] = {a.f_c, a.f, a.f_1, a.f_2};
+    constexpr int first[6] = {-1, -2, -1, -2, -2, -1};
+    constexpr bool alongx[6] = {true, false, false, true, true, false};
+    int di = 0, dj = 0;
+    if (c.lane < kF) {
+      const int q = c.lane >> 2, m = c.lane & 3;
+      wt.p = I[q];
+      wt.scale = pw(m);
+      (alongx[q] ? di : dj) = first[q] + m;
+    } else if (c.lane < kStrW) {
+      wt.p = Q[c.lane - kF];
+      wt.scale = 1.0f;
+      wt.inv = true;
+    }
+    wt.p += (long long)(ib + di) * FL + (jm + dj + AWP_NGSL + 2 + AWP_ALIGN);
+  }
+  float nw = wt.at(0);
+
+  const float2 ig3c = vquot(1.0f, gk2(a.g3_c, c.ld)), ig3 = vquot(1.0f, gk2(a.g3, c.ld));
+  // the xy Jacobian's interior rows read g3_c six points higher
+  // (stress_attenuation.cu:471), the boundary rows at k (:1149)
+  const bool bnd = c.top && c.lane >= 29;
+  const float2 ig12 = vquot(1.0f, gk2(a.g3_c, bnd ? c.ld : c.ld + 6));
+  const float2 gc = gk2(a.g_c, c.ld), gg = gk2(a.g, c.ld);
+  const float2 dcz = vscale(__ldg(a.dcrjy + ja), gk2(a.dcrjz, c.ld));
+  // texture entry pairs at even and odd steps (two adjacent levels starting at
+  // an even one: entries e, e + 1)
+  const int e0 = awp_tex_index(a.tex, ib, ja, c.k + AWP_ALIGN) >> 1,
+            e1 = awp_tex_index(a.tex, ib + 1, ja, c.k + AWP_ALIGN) >> 1;
+  float2 u_m1, u_0, u_p1, v_m2, v_m1, v_0, w_m2, w_m1, w_0;
+  {
+    const float *U = a.u1 + o, *V = a.v1 + o, *W = a.w1 + o;
+    u_m1 = ldg2(U - S); u_0 = ldg2(U); u_p1 = ldg2(U + S);
+    v_m2 = ldg2(V - 2 * (long long)S); v_m1 = ldg2(V - S); v_0 = ldg2(V);
+    w_m2 = ldg2(W - 2 * (long long)S); w_m1 = ldg2(W - S); w_0 = ldg2(W);
+  }
+  // media sums of the current plane: over j, j-1 and the level below
+  auto quad = [&](float2 t) { return awp_quad(t, below(t)); };
+  float2 Lq, Mq, Mt, Mm, Mk, Pq = {}, Rq = {}, Rt = {}, Rm = {}, Rk = {};
+  {
+    auto rows = [&](const float* p, float2& m) {
+      m = ldg2(p);
+      return vadd(m, ldg2(p - Y));
+    };
+    float2 m;
+    Lq = quad(rows(a.lam + o, m));
+    Mt = rows(a.mu + o, Mm);
+    Mq = quad(Mt);
+    Mk = vadd(Mm, below(Mm));
+    if (!ELASTIC) {
+      Pq = quad(rows(a.qp + o, m));
+      Rt = rows(a.qs + o, Rm);
+      Rq = quad(Rt);
+      Rk = vadd(Rm, below(Rm));
+    }
+  }
+  const int l = 2 * c.lane;
+  const int h0 = warp * kSpan + l, h1 = (warp + 1) * kSpan + l, h2 = (warp + 2) * kSpan + l;
+
+  Cursor<C::NH> ch;
+  Cursor<C::NO> co;
+  Cursor<awp_pipe::ND> cd;
+  int su = 0, su2 = 2, sv = 0, sv1 = 1;
+  bool ok = true;
+#pragma unroll 1
+  for (int s = 0; s < n; ++s) {
+    float2* const W = tab.w[s & 1];
+    W[c.lane] = dup(nw);
+    if (s + 1 < n) nw = wt.at((long long)(s + 1) * FL);
+    const float dcx = __ldg(a.dcrjx + ib + s);
+    __syncwarp();
+    ok = mbar_wait(pipe.full_h + ch.slot, ch.phase, spin);
+    if (!__all_sync(kAll, ok)) break;
+    const float* U0 = smem + C::F_U + su * kHalo + h1;
+    const float* V0 = smem + C::F_V + sv * kHalo + h2;
+    const float* W0 = smem + C::F_W + sv * kHalo + h1;
+    const float2 u_p2 = lds2(smem + C::F_U + su2 * kHalo + h1);
+    const float2 v_p1 = lds2(smem + C::F_V + sv1 * kHalo + h2);
+    const float2 w_p1 = lds2(smem + C::F_W + sv1 * kHalo + h1);
+    const float2 zero = make_float2(0.f, 0.f);
+
+    // ---- strain rates: every vertical difference of a horizontal interpolant
+    // is one difference of the interpolated column
+    float2 d[9];
+    {
+      // normal components: Jii = 1 / (f_c g3_c) (stress_attenuation.cu:340-431)
+      const float2 J = vmul(W[kF], ig3c), Jg = vmul(J, gc);
+      const float2 v2 = lds2(V0 - 2 * kSpan), v1 = lds2(V0 - kSpan), vp = lds2(V0 + kSpan);
+      d[0] = vsub(diff4(u_m1, u_0, u_p1, u_p2),
+                  vmul(Jg, zd7(dot4(W + kIu, u_m1, u_0, u_p1, u_p2), c, cl[0])));
+      d[1] = vsub(diff4(v2, v1, v_0, vp), vmul(Jg, zd7(dot4(W + kIv, v2, v1, v_0, vp), c, cl[0])));
+      d[2] = vmul(J, zd4<true, 8>(w_0, c, cl[2]));
+    }
+    {
+      // xy: J12i = 1 / (f g3_c)
+      const float2 J = vmul(vmul(W[kF + 1], ig12), gc);
+      const float2 um = lds2(U0 - kSpan), u1 = lds2(U0 + kSpan), u2 = lds2(U0 + 2 * kSpan);
+      const float2 q = dot4(W + kJv, v_m2, v_m1, v_0, v_p1, dot4(W + kJu, um, u_0, u1, u2));
+      d[3] = diff4(um, u_0, u1, u2);
+      d[4] = vsub(diff4(v_m2, v_m1, v_0, v_p1), vmul(J, zd7(q, c, cl[0])));
+    }
+    {
+      // xz: J13i = 1 / (f_1 g3) (:550-598, :1254-1317)
+      const float2 J = vmul(W[kF + 2], ig3);
+      const float2 z = zd7(dot4(W + kKw, w_m2, w_m1, w_0, w_p1), c, cl[1]);
+      d[5] = vmul(J, vsub(zd4<false, 7>(u_0, c, cl[3]), vmul(gg, z)));
+      d[6] = diff4(w_m2, w_m1, w_0, w_p1);
+    }
+    {
+      // yz: J23i = 1 / (f_2 g3) (:600-650, :1319-1380)
+      const float2 J = vmul(W[kF + 3], ig3);
+      const float2 wm = lds2(W0 - kSpan), w1 = lds2(W0 + kSpan), w2 = lds2(W0 + 2 * kSpan);
+      const float2 z = zd7(dot4(W + kLw, wm, w_0, w1, w2), c, cl[1]);
+      d[7] = vmul(J, vsub(zd4<false, 7>(v_0, c, cl[3]), vmul(gg, z)));
+      d[8] = diff4(wm, w_0, w1, w2);
+    }
+
+    // ---- material coefficients and the update (as the Cartesian dstrqc) -----
+    AwpRelax<float2> rx{};
+    if (!ELASTIC) {
+      const float* t = smem + C::F_T + ((s & 1) ? e1 : e0) * 20;
+      const float4* t4 = reinterpret_cast<const float4*>(t);
+      const float4 q0 = t4[0], q1 = t4[1], q2 = t4[2], q3 = t4[3];
+      rx.vx2 = make_float2(q0.x, q0.y); rx.wwo = make_float2(q0.z, q0.w);
+      rx.kv = make_float2(q1.x, q1.y); rx.kr = make_float2(q1.z, q1.w);
+      rx.kr2 = make_float2(q2.x, q2.y); rx.kf = make_float2(q2.z, q2.w);
+      rx.c0 = make_float2(q3.x, q3.y); rx.c1 = make_float2(q3.z, q3.w);
+      rx.c2 = lds2(t + 16);
+    }
+    AwpStrCoef<float2> cf;
+    {
+      const float* M = smem + C::F_M + ch.slot * NM * kMed;
+      auto rows = [&](int f, float2& m) {
+        m = lds2(M + f * kMed + h1);
+        return vadd(m, lds2(M + f * kMed + h0));
+      };
+      float2 m, mm;
+      const float2 Ln = quad(rows(0, m)), mt = rows(1, mm), mq = quad(mt);
+      const float2 P[3] = {Mk, Mt, vadd(Mm, mm)};
+      float2 QP8 = zero, QS8 = zero, R[3] = {zero, zero, zero};
+      if (!ELASTIC) {
+        float2 rm;
+        const float2 pq = quad(rows(2, m)), rt = rows(3, rm), rq = quad(rt);
+        QP8 = vadd(Pq, pq);
+        QS8 = vadd(Rq, rq);
+        R[0] = Rk; R[1] = Rt; R[2] = vadd(Rm, rm);
+        Pq = pq;
+        Rq = rq; Rt = rt; Rm = rm; Rk = vadd(rm, below(rm));
+      }
+      cf = awp_stress_coef<ELASTIC>(vadd(Lq, Ln), vadd(Mq, mq), P, QP8, QS8, R, rx, a.thr, a.dth,
+                                    a.DT);
+      Lq = Ln;
+      Mq = mq; Mt = mt; Mm = mm; Mk = vadd(mm, below(mm));
+    }
+    const float2 dcrj = vscale(dcx, dcz);
+    ok = mbar_wait(pipe.full_o + co.slot, co.phase, spin);
+    if (!__all_sync(kAll, ok)) break;
+    const float* O = smem + C::F_O + co.slot * NF * kOwn + h0;
+    float2 sg[6], rr[6];
 #pragma unroll
     for (int q = 0; q < 6; ++q) {
-      if (e) {
-        sg2[q].y = sg[q];
-        rr2[q].y = rr[q];
-      } else {
-        sg2[q].x = sg[q];
-        rr2[q].x = rr[q];
+      sg[q] = lds2(O + q * kOwn);
+      if (!ELASTIC) rr[q] = lds2(O + (6 + q) * kOwn);
+    }
+    awp_stress_update<ELASTIC>(sg, rr, cf, rx, dcrj, d);
+    if (o0 || o1) {
+#pragma unroll
+      for (int q = 0; q < 6; ++q) {
+        st2(SG[q] + o, sg[q], o0, o1);
+        if (!ELASTIC) st2(RR[q] + o, rr[q], o0, o1);
       }
     }
-  }
-#pragma unroll
-  for (int q = 0; q < 6; ++q) {
-    st2<V2>(SG[q] + o, sg2[q], c.out0, c.out1);
-    if (!ELASTIC) st2<V2>(RR[q] + o, rr2[q], c.out0, c.out1);
-  }
-}
+    warp_done(pipe.done + cd.slot, c.lane);
 
-template <bool ELASTIC, bool V2>
-__global__ void __launch_bounds__(128, AWP_TOPO_STR_MINB) k_topo_stress(const TopoArgs a) {
-  const ColPos2 c(a.nz, blockIdx.x);
-  const int j = a.s_j + blockIdx.y * 4 + threadIdx.y;
-  if (j >= a.e_j) return;  // whole warps
-  __shared__ float2 pre[StrStage<ELASTIC>::kRows][128];
-  const int i0 = a.s_i + blockIdx.z * AWP_TOPO_MARCH, i1 = min(i0 + AWP_TOPO_MARCH, a.e_i);
-#pragma unroll 1
-  for (int i = i0; i < i1; ++i) stress_column<ELASTIC, V2>(a, c, i, j, pre);
+    o += S;
+    u_m1 = u_0; u_0 = u_p1; u_p1 = u_p2;
+    v_m2 = v_m1; v_m1 = v_0; v_0 = v_p1;
+    w_m2 = w_m1; w_m1 = w_0; w_0 = w_p1;
+    ch.next();
+    co.next();
+    cd.next();
+    su = su + 1 == C::DU ? 0 : su + 1;
+    su2 = su2 + 1 == C::DU ? 0 : su2 + 1;
+    sv = sv1;
+    sv1 = sv1 + 1 == C::DV ? 0 : sv1 + 1;
+  }
+  if (!__all_sync(kAll, ok) && c.lane == 0) atomicExch(err, 1);
 }
 
 // Tiles of a column: the top one (outputs nz-60 .. nz-1), then one per 56
 // levels below it until a tile outputs level 3.
-static unsigned column_tiles(int nz) {
+unsigned column_tiles(int nz) {
   return 1u + (nz > 63 ? (unsigned)((nz - 63 + kTileOut - 1) / kTileOut) : 0u);
 }
 
-// 8-byte accesses need an even column length (yline = nz + 64, so every
-// level pair starts on an even index) and 8-byte aligned fields.
-static bool pairs_aligned(const TopoArgs& a) {
-  const void* p[] = {a.u1, a.v1, a.w1, a.xx, a.yy, a.zz, a.xy, a.xz, a.yz, a.r1, a.r2,
-                     a.r3, a.r4, a.r5, a.r6, a.d1, a.lam, a.mu, a.qp, a.qs};
-  if (a.yline % 2 || a.slice % 2) return false;
-  for (const void* q : p)
-    if (q && ((size_t)q & 7)) return false;
-  return true;
+Shape g_shape_vel[kMaxDev], g_shape_str[2][kMaxDev];
+
+}  // namespace
+
+int awp_topo_box(int group, int* bx, int* by) {
+  *bx = kSpan;
+  *by = group == 0 ? kCol + 3 : group == 1 ? kCol + 1 : kCol;
+  return 0;
 }
 
-cudaError_t awp_launch_topo_velocity(const TopoArgs& a, cudaStream_t st) {
+cudaError_t awp_launch_topo_velocity(const TopoArgs& a, const TmaMaps& tm, int ichunk, int* err,
+                                     cudaStream_t st) {
   if (a.nz < 12 || a.nx < 1 || a.ny < 1) return cudaErrorInvalidValue;
-  const dim3 block(32, 4, 1);
-  const dim3 grid(column_tiles(a.nz), (a.ny + 3) / 4,
-                  (a.nx + AWP_TOPO_MARCH - 1) / AWP_TOPO_MARCH);
-  if (pairs_aligned(a))
-    k_topo_velocity<true><<<grid, block, 0, st>>>(a);
-  else
-    k_topo_velocity<false><<<grid, block, 0, st>>>(a);
+  const dim3 tile(column_tiles(a.nz), cdiv_u(a.ny, kCol));
+  int resident = 0;
+  const cudaError_t e = resident_ctas((const void*)k_topo_velocity, TopoVelCfg::bytes, kThreads,
+                                      g_shape_vel, &resident);
+  if (e != cudaSuccess) return e;
+  const int ch = march_planes((long long)tile.x * tile.y, a.nx, resident, ichunk, kMost);
+  k_topo_velocity<<<dim3(tile.x, tile.y, cdiv_u(a.nx, ch)), kThreads, TopoVelCfg::bytes, st>>>(
+      a, tm, ch, err, awp_pipe_spin_limit);
   return cudaGetLastError();
 }
 
-cudaError_t awp_launch_topo_stress(const TopoArgs& a, bool elastic, cudaStream_t st) {
+cudaError_t awp_launch_topo_stress(const TopoArgs& a, const TmaMaps& tm, bool elastic, int ichunk,
+                                   int* err, cudaStream_t st) {
   if (a.nz < 12) return cudaErrorInvalidValue;
-  if (a.e_i <= a.s_i || a.e_j <= a.s_j) return cudaSuccess;
-  const dim3 block(32, 4, 1);
-  const dim3 grid(column_tiles(a.nz), (a.e_j - a.s_j + 3) / 4,
-                  (a.e_i - a.s_i + AWP_TOPO_MARCH - 1) / AWP_TOPO_MARCH);
-  const bool v2 = pairs_aligned(a);
-  if (elastic) {
-    if (v2)
-      k_topo_stress<true, true><<<grid, block, 0, st>>>(a);
-    else
-      k_topo_stress<true, false><<<grid, block, 0, st>>>(a);
-  } else {
-    if (v2)
-      k_topo_stress<false, true><<<grid, block, 0, st>>>(a);
-    else
-      k_topo_stress<false, false><<<grid, block, 0, st>>>(a);
-  }
+  const int ni = a.e_i - a.s_i, nj = a.e_j - a.s_j;
+  if (ni <= 0 || nj <= 0) return cudaSuccess;
+  const dim3 tile(column_tiles(a.nz), cdiv_u(nj, kCol));
+  const size_t sm = elastic ? TopoStrCfg<true>::bytes : TopoStrCfg<false>::bytes;
+  const void* f = elastic ? (const void*)k_topo_stress<true> : (const void*)k_topo_stress<false>;
+  int resident = 0;
+  const cudaError_t e = resident_ctas(f, sm, kThreads, g_shape_str[elastic ? 1 : 0], &resident);
+  if (e != cudaSuccess) return e;
+  const int ch = march_planes((long long)tile.x * tile.y, ni, resident, ichunk, kMost);
+  const dim3 grid(tile.x, tile.y, cdiv_u(ni, ch));
+  if (elastic)
+    k_topo_stress<true><<<grid, kThreads, sm, st>>>(a, tm, ch, err, awp_pipe_spin_limit);
+  else
+    k_topo_stress<false><<<grid, kThreads, sm, st>>>(a, tm, ch, err, awp_pipe_spin_limit);
   return cudaGetLastError();
 }

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include "awp_common.h"
+#include "awp_tma.cuh"
 
 struct TopoArgs {
   // wavefield and memory variables (padded layout of awp_common.h)
@@ -15,15 +16,21 @@ struct TopoArgs {
   const float *f, *f_1, *f_2, *f_c, *f1_1, *f1_2, *f1_c, *f2_1, *f2_2, *f2_c;
   const float *g, *g_c, *g3, *g3_c;
   AwpTexture tex;
-  float coeff[16];
+  AwpRelaxTab rel;  // per texture entry, with this struct's DT and 1/h
   int nx, ny, nz, slice, yline, fld;
   float nu;              // velocity: dt/h (topo_t.dth)
   float DT, dth, dh1;    // stress: (dt/h)*h, DT/h, 1/h (topo_set_constants)
-  float qthr;            // smallest float x with 1/(double)x <= 200 (Q(f) switch)
+  unsigned thr;          // Q(f) switch on a pair sum of Q^-1 (StrArgs::thr)
   int s_i, e_i, s_j, e_j;  // stress window, relative indices, ends exclusive
 };
 
 // dtopo_vel_111_unroll + dtopo_vel_112 (velocity_unroll.cu, optimized_velocity.cu:1040-1629)
-cudaError_t awp_launch_topo_velocity(const TopoArgs& a, cudaStream_t st);
+// tensor maps: the TmaMaps groups of the velocity and stress kernels with the
+// boxes of awp_topo_box (group 0: j halo, 1: media, 2: own); ichunk: x planes a
+// CTA marches at most
+int awp_topo_box(int group, int* box_x, int* box_y);
+cudaError_t awp_launch_topo_velocity(const TopoArgs& a, const TmaMaps& tm, int ichunk, int* err,
+                                     cudaStream_t st);
 // dtopo_str_111 + dtopo_str_112 (kernels/stress_attenuation.cu:73-1415)
-cudaError_t awp_launch_topo_stress(const TopoArgs& a, bool elastic, cudaStream_t st);
+cudaError_t awp_launch_topo_stress(const TopoArgs& a, const TmaMaps& tm, bool elastic, int ichunk,
+                                   int* err, cudaStream_t st);

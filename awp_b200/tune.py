@@ -15,12 +15,12 @@ import itertools
 
 CANDIDATES = {
     "tma": (1, 0),
-    # longer marches re-read fewer x-halo planes per chunk and keep the CTAs
-    # that share j/k halos closer in time; 512 covers a whole 512-plane grid
+    # the most planes a CTA marches: the TMA kernels take fewer by the grid's
+    # size, the read-only-path ones march as many
     "ichunk": (16, 32, 64, 128, 256, 512),
 }
-# L2 promotion of the TMA tiles: 3 = 256 B (the library default), 2 = 128 B,
-# 1 = 64 B, 0 = none
+# L2 promotion of the TMA tiles: 3 = 256 B, 2 = 128 B, 1 = 64 B, 0 = none (the
+# library default)
 PROMOTIONS = (3, 2, 1, 0)
 KEYS = ("tma_vel", "tma_str", "ichunk", "l2_promotion")
 

@@ -508,14 +508,15 @@ int awp_check_finite_noalloc(const float* const* fields, int nfields, long long 
 int awp_profile_phases(awp_ctx* ctx, int enable);
 int awp_phase_times(awp_ctx* ctx, double ms[AWP_NPHASES], long long launches[AWP_NPHASES]);
 /* Launch-shape tuning of the stencil kernels (process-wide): key "ichunk"
- * (x planes marched per CTA, 4..1024), "tma_vel" / "tma_str" (1: the context
+ * (x planes marched per CTA at most, 4..1024: the TMA kernels take fewer where
+ * the grid asks for it), "tma_vel" / "tma_str" (1: the context
  * API runs the TMA-pipelined velocity / stress kernel, 0: the read-only-path
  * one; results are bit-identical), "tma" (sets both; reads -1 when they
  * differ) and "spin_limit" (0 .. 2^30, default 2^26: polls of each pipeline
  * wait of the TMA kernels before it gives up, 0 = give up at once; a wait that
  * gives up makes the CTA drain its issued copies and leave, and the next
  * awp_synchronize of the context returns AWP_ERR_CUDA once) and
- * "l2_promotion" (0 none, 1 64 B, 2 128 B, 3 256 B (default): the L2 fetch
+ * "l2_promotion" (0 none (default), 1 64 B, 2 128 B, 3 256 B: the L2 fetch
  * granule of the TMA tiles; a context re-encodes its tensor maps before its
  * next TMA launch after a change; results do not change).  Returns AWP_OK or
  * AWP_ERR_ARG;

@@ -1,0 +1,125 @@
+"""Time steps against a float64 restatement, at the sizes where tiles end.
+
+perf/cases.py restates every phase of the step in float64 with plain torch
+operations (``exact``); here its inputs are run at sizes around the kernels'
+tile edges: z columns of the 32-level Cartesian and the 64/56-level
+curvilinear tiles, y rows around 8 and 7, x ranges shorter than a march and
+one plane past it.  A float32 step rounds each update a few times; over the
+2-3 steps run here the accumulated relative L2 difference is a few 1e-7
+(measured 0.5-9e-7 over these cases), so 3e-6 leaves a factor of three."""
+import importlib.util
+import os
+
+import numpy as np
+import pytest
+import torch
+
+from awp_b200 import _lib, tune
+
+pytestmark = pytest.mark.gpu
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+
+def cases():
+    spec = importlib.util.spec_from_file_location(
+        "perf_cases", os.path.join(ROOT, "perf", "cases.py"))
+    m = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(m)
+    return m
+
+
+def leaves(v):
+    if isinstance(v, dict):
+        for k in sorted(v):
+            yield from ((f"{k}.{n}", x) for n, x in leaves(v[k]))
+    elif isinstance(v, (list, tuple)):
+        for i, x in enumerate(v):
+            yield from ((f"{i}.{n}", y) for n, y in leaves(x))
+    else:
+        yield "", v
+
+
+def grid(nx, ny, nz, q=True, steps=3, **kw):
+    return dict(dict(kind="grid", nx=nx, ny=ny, nz=nz, q=q, steps=steps, fault=False,
+                     gather=False), **kw)
+
+
+CASES = [
+    grid(24, 24, 8), grid(25, 31, 32), grid(33, 33, 36, q=False), grid(27, 41, 64, gather=True),
+    grid(39, 26, 100, fault=True),
+    dict(kind="hill", nx=24, ny=25, nz=12, q=True, steps=2),
+    dict(kind="hill", nx=29, ny=31, nz=60, q=False, steps=2),
+    dict(kind="hill", nx=26, ny=36, nz=64, q=True, steps=2),
+    dict(kind="hill", nx=41, ny=30, nz=68, q=True, steps=2),
+    dict(kind="hill", nx=25, ny=28, nz=120, q=False, steps=2),
+    dict(kind="hill", nx=37, ny=27, nz=124, q=True, steps=2),
+    dict(kind="plastic", nx=41, ny=43, nz=36, q=True, steps=3),
+    dict(kind="plastic", nx=44, ny=40, nz=64, q=False, steps=3),
+    dict(kind="mesh", nx=20, ny=21, nz=32, nzc=24, steps=3, hill=False, plastic=False),
+    dict(kind="mesh", nx=22, ny=20, nz=68, nzc=36, steps=3, hill=True, plastic=True),
+    dict(kind="ensemble", n=3, lo=40, hi=70, steps=3, mode=0, draw=3),
+    dict(kind="ensemble", n=3, lo=40, hi=70, steps=3, mode=1, draw=4),
+    dict(kind="gradient", nx=36, ny=33, nz=32, steps=14, q=True, nrec=9, nsnap=0),
+    dict(kind="gradient", nx=33, ny=36, nz=36, steps=13, q=False, nrec=9, nsnap=3),
+]
+
+
+@pytest.mark.parametrize("case", CASES, ids=lambda c: f"{c['kind']}-{c.get('nx', c.get('n'))}-"
+                         f"{c.get('nz', c.get('mode'))}")
+def test_steps_match_float64(case):
+    m = cases()
+    st = m.prepare(case, 5)
+    got = dict(leaves(m.run(st)))
+    torch.cuda.synchronize()
+    want = dict(leaves(m.exact(case, 5)))
+    assert set(got) == set(want)
+    for name, x in got.items():
+        x, y = torch.as_tensor(x).double(), torch.as_tensor(want[name]).double()
+        ref = float(y.norm())
+        assert float((x.to(y.device) - y).norm()) <= 3e-6 * ref, (name, ref)
+
+
+@pytest.mark.parametrize("kind", ["grid", "hill"])
+def test_marches_beside_another_context(kind):
+    """Two contexts on their own streams share the SMs; each must leave the
+    fields it leaves alone, bit for bit (the producer may refill a slot only
+    when every lane has its values, however long its warp waits)."""
+    m = cases()
+    case = grid(150, 120, 96, steps=6) if kind == "grid" else \
+        dict(kind="hill", nx=120, ny=100, nz=96, q=True, steps=4)
+    alone = m.prepare(case, 1)
+    m.run(alone)
+    torch.cuda.synchronize()
+    want = {f: v.clone() for f, v in alone["out"].items()}
+    for _ in range(3):
+        a, b = m.prepare(case, 1), m.prepare(case, 2)
+        b2 = m.prepare(case, 3)
+        m.run(b)
+        m.run(a)
+        m.run(b2)
+        torch.cuda.synchronize()
+        for f, v in a["out"].items():
+            assert torch.equal(v.view(torch.int32), want[f].view(torch.int32)), f
+
+
+def test_march_length_does_not_change_curvilinear_fields():
+    lib = _lib.load()
+    saved = tune.get_tuning(lib)
+    m = cases()
+    case = dict(kind="hill", nx=45, ny=30, nz=68, q=True, steps=3)
+    want = None
+    try:
+        for ich in (4, 7, 32):
+            tune.set_tuning(lib, "ichunk", ich)
+            st = m.prepare(case, 2)
+            out = m.run(st)
+            torch.cuda.synchronize()
+            got = {f: v.cpu().numpy().view(np.uint32).copy() for f, v in out.items()}
+            if want is None:
+                want = got
+            for f in got:
+                assert np.array_equal(got[f], want[f]), (f, ich)
+    finally:
+        for k, v in saved.items():
+            tune.set_tuning(lib, k, v)
