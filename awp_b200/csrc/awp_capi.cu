@@ -75,6 +75,7 @@ struct awp_ctx {
   bool elastic = false;  // Q^-1 == 0 everywhere and memory variables zero
   // sources
   int nsrc = 0, ncell = 0, src_stride = 0;
+  bool src_deep = false;  // every source cell at least three levels below the top
   int *d_cell_pos = nullptr, *d_cell_first = nullptr, *d_order = nullptr;
   float* d_src[6] = {};
   float* d_mom = nullptr;
@@ -131,6 +132,10 @@ struct awp_ctx {
   // adjoint workspace, kept between gradient calls of the same size
   float* adj_slab = nullptr;
   size_t adj_slab_floats = 0;
+  // receivers, seismograms and surface scratch of the seismogram and gradient
+  // calls, kept for the next call (grows to the largest one's need)
+  char* scratch = nullptr;
+  size_t scratch_bytes = 0;
   long long dev_bytes = 0;
   long long launches = 0;
   // phase timing
@@ -507,6 +512,8 @@ int phase_stress(awp_ctx* c) {
   return launch_cart_stress(c, i1 + 1, c->xre, c->yls, c->yre);                 // xss3
 }
 
+bool sources_with_fstr(const awp_ctx* c);
+
 int phase_sources(awp_ctx* c) {
   float** f = c->f;
   if (c->srcf) {  // sources_read + sources_add_cartesian (pmcl3d.c:1987-2004)
@@ -525,7 +532,8 @@ int phase_sources(awp_ctx* c) {
                        g_errmsg, sizeof(g_errmsg)))
       return AWP_ERR_IO;
   }
-  if ((c->p.ifault < 4 && c->cur_step < c->p.nst) || c->p.ifault == 5) {
+  if (!sources_with_fstr(c) &&
+      ((c->p.ifault < 4 && c->cur_step < c->p.nst) || c->p.ifault == 5)) {
     PhaseScope ps(c, 2);
     int st = launch_sources(c, (int)c->cur_step);
     if (st) return st;
@@ -597,8 +605,25 @@ FstrArgs make_fstr_args(awp_ctx* c) {
   return fs;
 }
 
+// The point sources of a step ride in fstr's launch where nothing comes
+// between the two and they touch different cells: a single grid without
+// plasticity whose sources all lie below the imaged levels (2.1 us of host
+// time and a 4 us kernel less a step).  Phase timing keeps them apart.
+bool sources_with_fstr(const awp_ctx* c) {
+  return c->src_deep && c->ncell > 0 && c->p.ngrids == 1 && c->p.nve != 3 && !c->profile &&
+         (c->p.ifault < 4 || c->p.ifault == 5);
+}
+
 int phase_fstr(awp_ctx* c) {
   if (c->p.grid != 0) return AWP_OK;  // fstr_H on grid 0 only (pmcl3d.c:2243)
+  if (sources_with_fstr(c) && (c->p.ifault == 5 || c->cur_step < c->p.nst)) {
+    const SrcArgs s = make_src_args(c, (int)c->cur_step);
+    const KinSrcArgs k = make_kin_args(c, (int)c->cur_step);
+    CU_TRY(awp_launch_fstr_sources(make_fstr_args(c), c->p.ifault == 5 ? nullptr : &s,
+                                   c->p.ifault == 5 ? &k : nullptr, nullptr, 0, 0, c->stream));
+    c->launches++;
+    return AWP_OK;
+  }
   const FstrArgs fs = make_fstr_args(c);
   PhaseScope ps(c, 4);
   CU_TRY(awp_launch_fstr(fs, c->stream));
@@ -778,6 +803,7 @@ int dm_stress(awp_ctx* c) {  // dstrqc2 over xss1..xse3 x yls..yre (pmcl3d.c:193
   memcpy(a.coeff, c->coeff, sizeof(a.coeff));
   a.i0 = c->xls; a.i1 = c->xre; a.j0 = c->yls; a.j1 = c->yre;
   a.dth = c->dth; a.dh1 = c->dh1; a.dt = c->p.dt;
+  a.thr = c->thr;
   CU_TRY(awp_launch_dstrqc2(a, c->stream));
   c->launches++;
   return AWP_OK;
@@ -903,6 +929,7 @@ int awp_ctx_destroy(awp_ctx* c) {
   delete c->topo;
   cudaFree(c->d_topo);
   cudaFree(c->adj_slab);
+  cudaFree(c->scratch);
   for (int i = 0; i < AWP_NFIELDS; ++i) cudaFree(c->f[i]);
   cudaFree(c->dcrjx); cudaFree(c->dcrjy); cudaFree(c->dcrjz); cudaFree(c->lam_mu);
   cudaFree(c->d_cell_pos); cudaFree(c->d_cell_first); cudaFree(c->d_order);
@@ -1197,6 +1224,8 @@ int awp_upload_sources(awp_ctx* c, int nsrc, const int* pos, const float* data) 
     for (int s : kv.second) order.push_back(s);
   }
   cfirst.push_back((int)order.size());
+  c->src_deep = true;
+  for (int p : cpos) c->src_deep = c->src_deep && p % c->g.yline <= c->g.top() - 3;
   // de-interleave the time series: [comp][nsrc][stride]
   std::vector<float> comp((size_t)6 * nsrc * stride);
   for (int s = 0; s < nsrc; ++s)
@@ -2049,71 +2078,46 @@ int awp_topo_metrics(const char* path, int nx, int ny, int nz, float h, float* o
 // ===========================================================================
 // Batched instances
 // ===========================================================================
+constexpr int kBatchSteps = 8;  // most steps in one graph of parallel branches
+
 struct awp_batch {
   std::vector<awp_ctx*> ctx;
   cudaStream_t stream = nullptr;
   cudaEvent_t ev = nullptr;
-  BatchInst* d_inst = nullptr;
-  int4 *d_vt = nullptr, *d_st = nullptr, *d_ste = nullptr;
-  int2 *d_src = nullptr, *d_rows = nullptr;
-  int* d_cnt = nullptr;   // [3] tile counters
   int* d_step = nullptr;  // steps taken (device copy of cur_step)
-  BatchLaunch L{};
   int ty = 8, ichunk = 16;
-  int mode = 0;  // 0: persistent tile-queue launches; 1: graph of each instance's own launches
-  int branches = 0;  // mode 1: parallel graph branches (0: one per instance)
-  std::vector<cudaStream_t> cs;   // mode 1: one capture stream per instance
-  std::vector<cudaEvent_t> join;  // mode 1: branch joins
+  int mode = 0;
+  int branches = 0;  // parallel branches (0: one per instance)
+  std::vector<cudaStream_t> cs;   // one branch stream per instance
+  std::vector<cudaEvent_t> join;  // branch joins
   cudaEvent_t fork = nullptr;
   long long launches_per_step = 0;
   bool use_graph = true;
-  bool dirty = true;  // tile lists / graph to rebuild
+  bool dirty = true;  // graphs to rebuild
   long long step = 0;
   long long cells = 0;
-  cudaGraph_t graph = nullptr;
-  cudaGraphExec_t exec = nullptr;
+  cudaGraphExec_t branch_exec[kBatchSteps + 1] = {};  // n steps of parallel branches
+  bool stepped = false;                      // branches have run before
 };
 
 namespace {
 
-void batch_free_lists(awp_batch* b) {
-  cudaFree(b->d_vt); cudaFree(b->d_st); cudaFree(b->d_ste);
-  b->d_vt = b->d_st = b->d_ste = nullptr;
-  if (b->exec) cudaGraphExecDestroy(b->exec);
-  if (b->graph) cudaGraphDestroy(b->graph);
-  b->exec = nullptr;
-  b->graph = nullptr;
-}
-
-template <class T>
-int upload_vec(T** d, const std::vector<T>& h) {
-  *d = nullptr;
-  if (h.empty()) return AWP_OK;
-  CU_TRY(cudaMalloc((void**)d, sizeof(T) * h.size()));
-  CU_TRY(cudaMemcpy(*d, h.data(), sizeof(T) * h.size(), cudaMemcpyHostToDevice));
-  return AWP_OK;
-}
-
-// Mode 1: one step of every instance as parallel branches of one graph, each
-// branch the instance's own tuned launches (velocity, stress, sources at the
-// device step, free-surface images); the step counter advances after the join.
-int batch_capture_instances(awp_batch* b) {
-  if (b->cs.empty()) {
-    b->cs.assign(b->ctx.size(), nullptr);
-    b->join.assign(b->ctx.size(), nullptr);
-    for (size_t q = 0; q < b->ctx.size(); ++q) {
-      CU_TRY(cudaStreamCreateWithFlags(&b->cs[q], cudaStreamNonBlocking));
-      CU_TRY(cudaEventCreateWithFlags(&b->join[q], cudaEventDisableTiming));
-    }
-    CU_TRY(cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming));
+void batch_free_graphs(awp_batch* b) {
+  for (auto& e : b->branch_exec) {
+    if (e) cudaGraphExecDestroy(e);
+    e = nullptr;
   }
-  CU_TRY(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
+}
+
+// nsteps steps of every instance as parallel branches off the batch's stream,
+// each branch its instances' own tuned launches (velocity, stress, sources at
+// the device step, free-surface images); the step counter advances by nsteps
+// after the join.  Enqueued directly or into a capture of the stream.
+int batch_enqueue_branches(awp_batch* b, int nsteps) {
   int st = AWP_OK;
-  long long l0 = 0;
-  for (awp_ctx* c : b->ctx) l0 += c->launches;
   cudaError_t ce = cudaEventRecord(b->fork, b->stream);
   // branches in decreasing size: the largest instances start first, so the
-  // small ones fill the tail (capture order is the graph's launch order)
+  // small ones fill the tail
   std::vector<size_t> ord(b->ctx.size());
   for (size_t q = 0; q < ord.size(); ++q) ord[q] = q;
   std::stable_sort(ord.begin(), ord.end(), [&](size_t x, size_t y) {
@@ -2122,119 +2126,119 @@ int batch_capture_instances(awp_batch* b) {
   // instances dealt round-robin (largest first) onto nb branches
   const size_t nb = b->branches > 0 ? std::min((size_t)b->branches, ord.size()) : ord.size();
   std::vector<char> used(nb, 0);
-  for (size_t n = 0; n < ord.size() && !st && ce == cudaSuccess; ++n) {
-    const size_t q = ord[n], br = n % nb;
-    awp_ctx* c = b->ctx[q];
-    cudaStream_t saved = c->stream;
-    const bool prof = c->profile;
-    c->stream = b->cs[br];
-    c->profile = false;
-    if (!used[br]) {
-      ce = cudaStreamWaitEvent(b->cs[br], b->fork, 0);
-      used[br] = 1;
-    }
-    if (ce == cudaSuccess) st = phase_velocity(c);
-    if (!st && ce == cudaSuccess) st = phase_stress(c);
-    if (!st && ce == cudaSuccess && c->ncell > 0) {
-      if (c->p.ifault == 5) {
-        const KinSrcArgs k = make_kin_args(c, 0);
-        ce = awp_launch_sources_dev(nullptr, &k, b->d_step, 0, c->stream);
-        c->launches++;
-      } else if (c->p.ifault < 4) {
-        const SrcArgs a = make_src_args(c, 0);
-        ce = awp_launch_sources_dev(&a, nullptr, b->d_step, c->p.nst, c->stream);
-        c->launches++;
+  for (int t = 0; t < nsteps; ++t)
+    for (size_t n = 0; n < ord.size() && !st && ce == cudaSuccess; ++n) {
+      const size_t q = ord[n], br = n % nb;
+      awp_ctx* c = b->ctx[q];
+      cudaStream_t saved = c->stream;
+      const bool prof = c->profile;
+      c->stream = b->cs[br];
+      c->profile = false;
+      if (!used[br]) {
+        ce = cudaStreamWaitEvent(b->cs[br], b->fork, 0);
+        used[br] = 1;
       }
+      if (ce == cudaSuccess) st = phase_velocity(c);
+      if (!st && ce == cudaSuccess) st = phase_stress(c);
+      const bool with_fstr = sources_with_fstr(c);
+      if (!st && ce == cudaSuccess && with_fstr) {
+        const SrcArgs a = make_src_args(c, 0);
+        const KinSrcArgs k = make_kin_args(c, 0);
+        const bool kin = c->p.ifault == 5;
+        ce = awp_launch_fstr_sources(make_fstr_args(c), kin ? nullptr : &a, kin ? &k : nullptr,
+                                     b->d_step, t, c->p.nst, c->stream);
+        c->launches++;
+      } else if (!st && ce == cudaSuccess && c->ncell > 0) {
+        if (c->p.ifault == 5) {
+          const KinSrcArgs k = make_kin_args(c, 0);
+          ce = awp_launch_sources_dev(nullptr, &k, b->d_step, t, 0, c->stream);
+          c->launches++;
+        } else if (c->p.ifault < 4) {
+          const SrcArgs a = make_src_args(c, 0);
+          ce = awp_launch_sources_dev(&a, nullptr, b->d_step, t, c->p.nst, c->stream);
+          c->launches++;
+        }
+      }
+      if (!st && ce == cudaSuccess && !with_fstr) st = phase_fstr(c);
+      c->stream = saved;
+      c->profile = prof;
     }
-    if (!st && ce == cudaSuccess) st = phase_fstr(c);
-    c->stream = saved;
-    c->profile = prof;
-  }
-  for (size_t br = 0; br < nb && !st && ce == cudaSuccess; ++br) {
+  for (size_t br = 0; br < nb; ++br) {  // rejoin even after an error (a capture must)
     if (!used[br]) continue;
-    ce = cudaEventRecord(b->join[br], b->cs[br]);
-    if (ce == cudaSuccess) ce = cudaStreamWaitEvent(b->stream, b->join[br], 0);
+    cudaError_t e = cudaEventRecord(b->join[br], b->cs[br]);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(b->stream, b->join[br], 0);
+    if (ce == cudaSuccess) ce = e;
   }
   if (!st && ce == cudaSuccess) {
-    ce = awp_launch_step_advance(b->d_step, b->stream);
+    ce = awp_launch_step_advance(b->d_step, nsteps, b->stream);
     b->ctx[0]->launches++;
   }
-  cudaGraph_t g = nullptr;
-  const cudaError_t ee = cudaStreamEndCapture(b->stream, &g);
-  long long l1 = 0;
-  for (awp_ctx* c : b->ctx) l1 += c->launches;
-  b->ctx[0]->launches -= (l1 - l0);  // counted per replay instead
-  b->launches_per_step = l1 - l0;
-  if (st || ce != cudaSuccess || ee != cudaSuccess) {
-    if (g) cudaGraphDestroy(g);
-    if (st) return st;
-    return set_error(AWP_ERR_CUDA, "batch graph capture: %s",
-                     cudaGetErrorString(ce != cudaSuccess ? ce : ee));
+  if (!st && ce != cudaSuccess)
+    st = set_error(AWP_ERR_CUDA, "batch step: %s", cudaGetErrorString(ce));
+  return st;
+}
+
+int batch_streams(awp_batch* b) {
+  if (!b->cs.empty()) return AWP_OK;
+  b->cs.assign(b->ctx.size(), nullptr);
+  b->join.assign(b->ctx.size(), nullptr);
+  for (size_t q = 0; q < b->ctx.size(); ++q) {
+    CU_TRY(cudaStreamCreateWithFlags(&b->cs[q], cudaStreamNonBlocking));
+    CU_TRY(cudaEventCreateWithFlags(&b->join[q], cudaEventDisableTiming));
   }
-  b->graph = g;
-  CU_TRY(cudaGraphInstantiate(&b->exec, g, 0));
+  CU_TRY(cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming));
   return AWP_OK;
 }
 
-// Tile lists for the current shape (tile 32 k x ty j x ichunk i), the
-// persistent grid sizes, and the captured one-step graph.
-int batch_build(awp_batch* b) {
-  batch_free_lists(b);
-  if (b->mode == 1) {
-    const int e = batch_capture_instances(b);
-    if (!e) b->dirty = false;
-    return e;
+long long batch_launches(const awp_batch* b) {
+  long long n = 0;
+  for (const awp_ctx* c : b->ctx) n += c->launches;
+  return n;
+}
+
+// The graph of n steps of branches.
+int batch_capture_branches(awp_batch* b, int n) {
+  const long long l0 = batch_launches(b);
+  CU_TRY(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
+  const int st = batch_enqueue_branches(b, n);
+  cudaGraph_t g = nullptr;
+  const cudaError_t ee = cudaStreamEndCapture(b->stream, &g);
+  const long long l1 = batch_launches(b);
+  b->ctx[0]->launches -= (l1 - l0);  // counted per replay instead
+  b->launches_per_step = (l1 - l0 - 1) / n;
+  cudaError_t ie = ee;
+  if (!st && ee == cudaSuccess) ie = cudaGraphInstantiate(&b->branch_exec[n], g, 0);
+  if (g) cudaGraphDestroy(g);
+  if (st) return st;
+  if (ie != cudaSuccess) {
+    b->branch_exec[n] = nullptr;
+    return set_error(AWP_ERR_CUDA, "batch graph capture: %s", cudaGetErrorString(ie));
   }
-  std::vector<int4> vt, st, ste;
-  for (size_t n = 0; n < b->ctx.size(); ++n) {
-    awp_ctx* c = b->ctx[n];
-    const VelArgs v = make_vel_args(c);
-    const int gx = (v.k1 - v.k0 + 32) / 32, gy = (v.j1 - v.j0 + b->ty) / b->ty,
-              gz = (v.i1 - v.i0 + b->ichunk) / b->ichunk;
-    for (int z = 0; z < gz; ++z)
-      for (int y = 0; y < gy; ++y)
-        for (int x = 0; x < gx; ++x) vt.push_back(make_int4((int)n, x, y, z));
-    const StrArgs a = make_str_args(c);
-    const int sx = (a.k1 - a.k0 + 32) / 32, sy = (a.j1 - a.j0 + b->ty) / b->ty,
-              sz = (a.i1 - a.i0 + b->ichunk) / b->ichunk;
-    std::vector<int4>& dst = c->elastic ? ste : st;
-    for (int z = 0; z < sz; ++z)
-      for (int y = 0; y < sy; ++y)
-        for (int x = 0; x < sx; ++x) dst.push_back(make_int4((int)n, x, y, z));
+  return AWP_OK;
+}
+
+// Branches: graphs of up to kBatchSteps steps, in which an instance runs on
+// into its next step without waiting for the others.  A batch's first few
+// steps are enqueued directly: capturing and instantiating costs more than
+// launching them.
+int batch_step_branches(awp_batch* b, int nsteps) {
+  int e = batch_streams(b);
+  if (e) return e;
+  const bool graph = b->use_graph || b->mode == 1;  // mode 1 always replays graphs
+  if (!graph || (!b->stepped && nsteps <= kBatchSteps)) {
+    b->stepped = true;
+    for (int n = 0; n < nsteps; n += kBatchSteps)
+      if ((e = batch_enqueue_branches(b, std::min(kBatchSteps, nsteps - n)))) return e;
+    return AWP_OK;
   }
-  int e;
-  if ((e = upload_vec(&b->d_vt, vt)) || (e = upload_vec(&b->d_st, st)) ||
-      (e = upload_vec(&b->d_ste, ste)))
-    return e;
-  int bv = 0, bs = 0;
-  if (awp_batch_blocks_per_sm(b->ty, &bv, &bs))
-    return set_error(AWP_ERR_CUDA, "batch occupancy query failed");
-  int dev = 0, nsm = 0;
-  CU_TRY(cudaGetDevice(&dev));
-  CU_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-  BatchLaunch& L = b->L;
-  L.inst = b->d_inst;
-  L.vtiles = b->d_vt; L.stiles = b->d_st; L.stiles_el = b->d_ste;
-  L.nvtiles = (int)vt.size(); L.nstiles = (int)st.size(); L.nstiles_el = (int)ste.size();
-  L.counters = b->d_cnt; L.step = b->d_step;
-  L.ty = b->ty; L.ichunk = b->ichunk;
-  L.grid_vel = std::max(1, std::min(nsm * std::max(bv, 1), L.nvtiles));
-  L.grid_str = std::max(1, std::min(nsm * std::max(bs, 1), std::max(L.nstiles, L.nstiles_el)));
-  b->launches_per_step = 1 + (L.nstiles > 0) + (L.nstiles_el > 0) + (L.nsrc > 0) + 1;
-  if (b->use_graph) {
-    CU_TRY(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
-    cudaError_t le = awp_launch_batch_step(L, b->stream);
-    cudaGraph_t g = nullptr;
-    cudaError_t ce = cudaStreamEndCapture(b->stream, &g);
-    if (le != cudaSuccess || ce != cudaSuccess) {
-      if (g) cudaGraphDestroy(g);
-      return set_error(AWP_ERR_CUDA, "batch graph capture: %s",
-                       cudaGetErrorString(le != cudaSuccess ? le : ce));
-    }
-    b->graph = g;
-    CU_TRY(cudaGraphInstantiate(&b->exec, g, 0));
+  b->stepped = true;
+  for (int n = 0; n < nsteps;) {
+    const int k = std::min(kBatchSteps, nsteps - n);
+    if (!b->branch_exec[k] && (e = batch_capture_branches(b, k))) return e;
+    CU_TRY(cudaGraphLaunch(b->branch_exec[k], b->stream));
+    b->ctx[0]->launches += b->launches_per_step * k + 1;
+    n += k;
   }
-  b->dirty = false;
   return AWP_OK;
 }
 
@@ -2245,9 +2249,8 @@ extern "C" {
 int awp_batch_destroy(awp_batch* b) {
   if (!b) return AWP_OK;
   if (b->stream) cudaStreamSynchronize(b->stream);
-  batch_free_lists(b);
-  cudaFree(b->d_inst); cudaFree(b->d_src); cudaFree(b->d_rows);
-  cudaFree(b->d_cnt); cudaFree(b->d_step);
+  batch_free_graphs(b);
+  cudaFree(b->d_step);
   for (cudaStream_t x : b->cs) if (x) cudaStreamDestroy(x);
   for (cudaEvent_t x : b->join) if (x) cudaEventDestroy(x);
   if (b->fork) cudaEventDestroy(b->fork);
@@ -2283,40 +2286,11 @@ int awp_batch_create(awp_ctx* const* ctxs, int n, awp_batch** out) {
     awp_batch_destroy(b);
     return set_error(AWP_ERR_CUDA, "batch stream/event creation failed");
   }
-  std::vector<BatchInst> inst(n);
-  std::vector<int2> src, rows;
-  for (int q = 0; q < n; ++q) {
-    awp_ctx* c = ctxs[q];
-    BatchInst& I = inst[q];
-    memset(&I, 0, sizeof(I));
-    I.v = make_vel_args(c);
-    I.s = make_str_args(c);
-    I.f = make_fstr_args(c);
-    I.src = make_src_args(c, 0);
-    I.kin = make_kin_args(c, 0);
-    I.elastic = c->elastic ? 1 : 0;
-    I.ifault = c->p.ifault;
-    I.nst = c->p.nst;
-    if (c->ncell > 0 && (c->p.ifault < 4 || c->p.ifault == 5))
-      for (int k = 0; k < c->ncell; ++k) src.push_back(make_int2(q, k));
-    for (int i = I.f.i0; i <= I.f.i1; ++i) rows.push_back(make_int2(q, i));
-    b->cells += (long long)c->p.nx * c->p.ny * c->p.nz;
-  }
-  int e;
-  if ((e = upload_vec(&b->d_inst, inst)) || (e = upload_vec(&b->d_src, src)) ||
-      (e = upload_vec(&b->d_rows, rows))) {
+  for (const awp_ctx* c : b->ctx) b->cells += (long long)c->p.nx * c->p.ny * c->p.nz;
+  if (cudaMalloc((void**)&b->d_step, sizeof(int)) != cudaSuccess) {
     awp_batch_destroy(b);
-    return e;
+    return set_error(AWP_ERR_NOMEM, "batch step counter");
   }
-  if (cudaMalloc((void**)&b->d_cnt, 3 * sizeof(int)) != cudaSuccess ||
-      cudaMalloc((void**)&b->d_step, sizeof(int)) != cudaSuccess) {
-    awp_batch_destroy(b);
-    return set_error(AWP_ERR_NOMEM, "batch counters");
-  }
-  b->L.src_cells = b->d_src;
-  b->L.nsrc = (int)src.size();
-  b->L.rows = b->d_rows;
-  b->L.nrows = (int)rows.size();
   const int st = (int)b->step;
   if (cudaMemcpy(b->d_step, &st, sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess) {
     awp_batch_destroy(b);
@@ -2398,21 +2372,18 @@ int awp_batch_step(awp_batch* b, int nsteps) {
     CU_TRY(cudaStreamWaitEvent(b->stream, b->ev, 0));
   }
   if (b->dirty) {
-    int e = batch_build(b);
-    if (e) return e;
+    batch_free_graphs(b);
+    b->dirty = false;
   }
-  for (int n = 0; n < nsteps; ++n) {
-    if (b->use_graph || b->mode == 1)
-      CU_TRY(cudaGraphLaunch(b->exec, b->stream));
-    else
-      CU_TRY(awp_launch_batch_step(b->L, b->stream));
+  {
+    const int e = batch_step_branches(b, nsteps);
+    if (e) return e;
   }
   CU_TRY(cudaEventRecord(b->ev, b->stream));
   for (awp_ctx* c : b->ctx) {
     CU_TRY(cudaStreamWaitEvent(c->stream, b->ev, 0));
     c->cur_step += nsteps;
   }
-  b->ctx[0]->launches += b->launches_per_step * nsteps;
   b->step += nsteps;
   return AWP_OK;
 }
@@ -2425,16 +2396,24 @@ int awp_batch_synchronize(awp_batch* b) {
 
 int awp_batch_info(awp_batch* b, long long info[6]) {
   if (!b || !info) return set_error(AWP_ERR_ARG, "null argument");
-  if (b->dirty) {
-    int e = batch_build(b);
-    if (e) return e;
+  // tiles of 32 k x ty j x ichunk i over every instance's update ranges
+  long long nv = 0, ns = 0;
+  auto tiles = [&](int i0, int i1, int j0, int j1, int k0, int k1) {
+    return (long long)((k1 - k0 + 32) / 32) * ((j1 - j0 + b->ty) / b->ty) *
+           ((i1 - i0 + b->ichunk) / b->ichunk);
+  };
+  for (awp_ctx* c : b->ctx) {
+    const VelArgs v = make_vel_args(c);
+    const StrArgs a = make_str_args(c);
+    nv += tiles(v.i0, v.i1, v.j0, v.j1, v.k0, v.k1);
+    ns += tiles(a.i0, a.i1, a.j0, a.j1, a.k0, a.k1);
   }
   info[0] = (long long)b->ctx.size();
   info[1] = b->cells;
-  info[2] = b->L.nvtiles;
-  info[3] = (long long)b->L.nstiles + b->L.nstiles_el;
-  info[4] = b->L.grid_vel;
-  info[5] = b->L.grid_str;
+  info[2] = nv;
+  info[3] = ns;
+  info[4] = nv;
+  info[5] = ns;
   return AWP_OK;
 }
 
@@ -2556,9 +2535,36 @@ int check_adjoint_ctx(awp_ctx* c) {
   return AWP_OK;
 }
 
+// Pieces of the context's scratch on 256-byte boundaries, reserved once per
+// call (an allocation and a free each were up to 0.1 ms and a device-wide wait).
+struct Scratch {
+  awp_ctx* c;
+  size_t used = 0;
+  static size_t round(size_t bytes) { return (bytes + 255) / 256 * 256; }
+  int reserve(size_t bytes) {
+    if (c->scratch_bytes >= bytes) return AWP_OK;
+    CU_TRY(cudaStreamSynchronize(c->stream));
+    cudaFree(c->scratch);
+    c->scratch = nullptr;
+    c->scratch_bytes = 0;
+    if (cudaMalloc((void**)&c->scratch, bytes) != cudaSuccess) {
+      c->scratch = nullptr;
+      return set_error(AWP_ERR_NOMEM, "scratch of %zu bytes", bytes);
+    }
+    c->scratch_bytes = bytes;
+    return AWP_OK;
+  }
+  template <class T>
+  T* take(size_t n) {
+    T* p = reinterpret_cast<T*>(c->scratch + used);
+    used += round(n * sizeof(T));
+    return p;
+  }
+};
+
 // device copies of receiver positions (padded linear index) and components
-int upload_receivers(awp_ctx* c, int nrec, const int* xyz, const int* comp, long long** d_idx,
-                     int** d_comp) {
+int upload_receivers(awp_ctx* c, int nrec, const int* xyz, const int* comp, long long* d_idx,
+                     int* d_comp) {
   std::vector<long long> idx(nrec);
   for (int r = 0; r < nrec; ++r) {
     const int x = xyz[3 * r], y = xyz[3 * r + 1], z = xyz[3 * r + 2];
@@ -2568,10 +2574,10 @@ int upload_receivers(awp_ctx* c, int nrec, const int* xyz, const int* comp, long
     idx[r] = (long long)(x + 2 + AWP_NGSL) * c->g.slice +
              (long long)(y + 2 + AWP_NGSL) * c->g.yline + (c->g.top() - z);
   }
-  CU_TRY(cudaMalloc((void**)d_idx, sizeof(long long) * std::max(nrec, 1)));
-  CU_TRY(cudaMalloc((void**)d_comp, sizeof(int) * std::max(nrec, 1)));
-  CU_TRY(cudaMemcpy(*d_idx, idx.data(), sizeof(long long) * nrec, cudaMemcpyHostToDevice));
-  CU_TRY(cudaMemcpy(*d_comp, comp, sizeof(int) * nrec, cudaMemcpyHostToDevice));
+  // pageable sources: each call returns once the data has left the host arrays
+  CU_TRY(cudaMemcpyAsync(d_idx, idx.data(), sizeof(long long) * nrec, cudaMemcpyHostToDevice,
+                         c->stream));
+  CU_TRY(cudaMemcpyAsync(d_comp, comp, sizeof(int) * nrec, cudaMemcpyHostToDevice, c->stream));
   return AWP_OK;
 }
 
@@ -2597,13 +2603,21 @@ int awp_set_moduli(awp_ctx* c, const float* lambda, const float* mu, const float
   if (!c->media_ready) return set_error(AWP_ERR_STATE, "upload media first (Q and layout)");
   const size_t n = (size_t)c->g.nxt * c->g.nyt * c->g.nzt;
   DevBuf b;
-  float *dl = b.f(n), *dm = b.f(n), *dr = b.f(n);
-  if (!dl || !dm || !dr) return set_error(AWP_ERR_NOMEM, "moduli staging");
-  // host or device arrays alike (unified addressing picks the direction)
-  CU_TRY(cudaMemcpyAsync(dl, lambda, n * sizeof(float), cudaMemcpyDefault, c->stream));
-  CU_TRY(cudaMemcpyAsync(dm, mu, n * sizeof(float), cudaMemcpyDefault, c->stream));
-  CU_TRY(cudaMemcpyAsync(dr, rho, n * sizeof(float), cudaMemcpyDefault, c->stream));
-  CU_TRY(awp_launch_set_moduli(dl, dm, dr, c->f[AWP_LAM], c->f[AWP_MU], c->f[AWP_D1], c->g,
+  // arrays in this device's memory are read in place; others are staged
+  const float* src[3] = {lambda, mu, rho};
+  int dev = 0;
+  CU_TRY(cudaGetDevice(&dev));
+  for (const float*& p : src) {
+    cudaPointerAttributes at{};
+    const bool known = cudaPointerGetAttributes(&at, p) == cudaSuccess;
+    if (!known) (void)cudaGetLastError();
+    if (known && at.type == cudaMemoryTypeDevice && at.device == dev) continue;
+    float* d = b.f(n);
+    if (!d) return set_error(AWP_ERR_NOMEM, "moduli staging");
+    CU_TRY(cudaMemcpyAsync(d, p, n * sizeof(float), cudaMemcpyDefault, c->stream));
+    p = d;
+  }
+  CU_TRY(awp_launch_set_moduli(src[0], src[1], src[2], c->f[AWP_LAM], c->f[AWP_MU], c->f[AWP_D1], c->g,
                                c->stream));
   CU_TRY(awp_launch_lam_mu(c->f[AWP_LAM], c->f[AWP_MU], c->lam_mu, c->g, c->xls, c->xre, c->yls,
                            c->yre, c->stream));
@@ -2646,15 +2660,15 @@ int awp_seismograms(awp_ctx* c, int nsteps, int nrec, const int* rec_xyz, const 
   if (e) return e;
   if (nsteps < 0 || nrec < 1 || !rec_xyz || !rec_comp || !seis)
     return set_error(AWP_ERR_ARG, "bad receiver arguments");
-  long long* d_idx = nullptr;
-  int* d_comp = nullptr;
-  e = upload_receivers(c, nrec, rec_xyz, rec_comp, &d_idx, &d_comp);
-  DevBuf b;
-  b.p.push_back(d_idx);
-  b.p.push_back(d_comp);
-  if (e) return e;
-  float* d_seis = b.f((size_t)std::max(nsteps, 1) * nrec);
-  if (!d_seis) return set_error(AWP_ERR_NOMEM, "seismogram buffer");
+  const size_t nseis = (size_t)std::max(nsteps, 1) * nrec;
+  Scratch sc{c};
+  if ((e = sc.reserve(Scratch::round(sizeof(long long) * nrec) +
+                      Scratch::round(sizeof(int) * nrec) + Scratch::round(sizeof(float) * nseis))))
+    return e;
+  long long* d_idx = sc.take<long long>(nrec);
+  int* d_comp = sc.take<int>(nrec);
+  float* d_seis = sc.take<float>(nseis);
+  if ((e = upload_receivers(c, nrec, rec_xyz, rec_comp, d_idx, d_comp))) return e;
   for (int n = 0; n < nsteps; ++n) {
     if ((e = one_step(c))) return e;
     CU_TRY(awp_launch_sample(c->f[AWP_U1], c->f[AWP_V1], c->f[AWP_W1], d_idx, d_comp, nrec,
@@ -2817,16 +2831,20 @@ int awp_misfit_gradient_q(awp_ctx* c, int nsteps, int nrec, const int* rec_xyz,
   };
   auto take = [&]() -> float* { return take_n(cp); };
   auto take_v = [&]() -> float* { return take_n(cv); };
-  DevBuf b;
-  long long* d_idx = nullptr;
-  int* d_comp = nullptr;
-  e = upload_receivers(c, nrec, rec_xyz, rec_comp, &d_idx, &d_comp);
-  b.p.push_back(d_idx);
-  b.p.push_back(d_comp);
-  if (e) return e;
-  float* d_seis = b.f((size_t)nsteps * nrec);
-  float* d_res = b.f((size_t)nsteps * nrec);
-  if (!d_seis || !d_res) return set_error(AWP_ERR_NOMEM, "seismogram buffers");
+  const size_t nseis = (size_t)nsteps * nrec, nsurf = (size_t)c->g.nx_pad() * c->g.ny_pad(),
+               nimg = (size_t)4 * (sa.i1 - sa.i0 + 3) * (sa.j1 - sa.j0 + 3);
+  Scratch sc{c};
+  if ((e = sc.reserve(Scratch::round(sizeof(long long) * nrec) +
+                      3 * Scratch::round(sizeof(int) * (nrec + 1)) +
+                      2 * Scratch::round(sizeof(float) * nseis) +
+                      Scratch::round(sizeof(float) * nsurf) +
+                      Scratch::round(sizeof(float) * nimg))))
+    return e;
+  long long* d_idx = sc.take<long long>(nrec);
+  int* d_comp = sc.take<int>(nrec + 1);
+  float* d_seis = sc.take<float>(nseis);
+  float* d_res = sc.take<float>(nseis);
+  if ((e = upload_receivers(c, nrec, rec_xyz, rec_comp, d_idx, d_comp))) return e;
   cudaStream_t st = c->stream;
 
   // ---- forward pass with snapshots X_{sL} and the final state ---------------------
@@ -2893,9 +2911,8 @@ int awp_misfit_gradient_q(awp_ctx* c, int nsteps, int nrec, const int* rec_xyz,
   a.gqp = take();
   a.gqs = take();
   CU_TRY(cudaMemsetAsync(zero0, 0, (size_t)(c->adj_slab + slab_next - zero0) * sizeof(float), st));
-  if (!(a.glm = b.f((size_t)c->g.nx_pad() * c->g.ny_pad())))
-    return set_error(AWP_ERR_NOMEM, "gradients");
-  CU_TRY(cudaMemsetAsync(a.glm, 0, sizeof(float) * c->g.nx_pad() * c->g.ny_pad(), st));
+  a.glm = sc.take<float>(nsurf);
+  CU_TRY(cudaMemsetAsync(a.glm, 0, sizeof(float) * nsurf, st));
   a.d1 = c->f[AWP_D1]; a.lam = c->f[AWP_LAM]; a.mu = c->f[AWP_MU];
   a.qp = c->f[AWP_QP]; a.qs = c->f[AWP_QS]; a.lam_mu = c->lam_mu;
   a.dcrjx = c->dcrjx; a.dcrjy = c->dcrjy; a.dcrjz = c->dcrjz;
@@ -2910,16 +2927,15 @@ int awp_misfit_gradient_q(awp_ctx* c, int nsteps, int nrec, const int* rec_xyz,
   a.si0 = sa.i0; a.si1 = sa.i1; a.sj0 = sa.j0; a.sj1 = sa.j1; a.sk0 = sa.k0; a.sk1 = sa.k1;
   a.gx_lim = sa.gx_lim; a.gy_min = sa.gy_min; a.lam_mu_ld = sa.lam_mu_ld;
   a.fj1 = make_fstr_args(c).j1;
-  if (!(a.img = b.f((size_t)4 * (a.si1 - a.si0 + 3) * (a.sj1 - a.sj0 + 3))))
-    return set_error(AWP_ERR_NOMEM, "image scratch");
+  a.img = sc.take<float>(nimg);
   // segment store: the velocities at the start of a segment and after each
   // of its steps (slot 0 = start)
   std::vector<float*> seg((size_t)(H > 0 ? L + 1 : 0) * 3, nullptr);
   for (auto& q : seg) q = take_v();
   float* const Lvel[3] = {a.L[0], a.L[1], a.L[2]};
   // receivers grouped by (component, cell) for the residual injection
-  int* d_first = nullptr;
-  int* d_order = nullptr;
+  int* const d_first = sc.take<int>(nrec + 1);
+  int* const d_order = sc.take<int>(nrec + 1);
   int ncell_rec = 0;
   {
     std::vector<std::pair<long long, int>> key(nrec);
@@ -2938,12 +2954,10 @@ int awp_misfit_gradient_q(awp_ctx* c, int nsteps, int nrec, const int* rec_xyz,
     }
     ncell_rec = (int)first.size();
     first.push_back(nrec);
-    CU_TRY(cudaMalloc((void**)&d_first, sizeof(int) * first.size()));
-    b.p.push_back(d_first);
-    CU_TRY(cudaMalloc((void**)&d_order, sizeof(int) * order.size()));
-    b.p.push_back(d_order);
-    CU_TRY(cudaMemcpy(d_first, first.data(), sizeof(int) * first.size(), cudaMemcpyHostToDevice));
-    CU_TRY(cudaMemcpy(d_order, order.data(), sizeof(int) * order.size(), cudaMemcpyHostToDevice));
+    CU_TRY(cudaMemcpyAsync(d_first, first.data(), sizeof(int) * first.size(),
+                           cudaMemcpyHostToDevice, st));
+    CU_TRY(cudaMemcpyAsync(d_order, order.data(), sizeof(int) * order.size(),
+                           cudaMemcpyHostToDevice, st));
   }
 
   // ---- backward sweep: the stored tail, then the recomputed segments ---------------

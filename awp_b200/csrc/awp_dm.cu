@@ -1,8 +1,7 @@
 // Discontinuous-mesh coupling kernels (reference: src/awp/kernel.cu:2289-3234,
 // src/awp/mesh.c:1404-1443).  All are 2-D over an interface (a few planes of
-// work per step), so they run one thread per horizontal point; the
-// arithmetic follows the reference expression by expression with explicit
-// rounding intrinsics.
+// work per step) and bound by the 32-byte sectors their single levels of
+// k-contiguous columns touch.
 //
 // At one rank the reference's swap-area exchanges (swap.c:549-583,
 // kernel.cu:3320-3676) return at once and bgcaccess (kernel.cu:2809-2852)
@@ -29,60 +28,71 @@ __global__ void k_dvelc2(const DmVel2Args a) {
   const int S = a.g.slice, Y = a.g.yline;
   const int k = 2 + AWP_ALIGN;
   const long long pos = at(a.g, i, j, k);
-  const float* d = a.d1;
+  // every load first (a store could alias a later load, and would make it
+  // wait): each of these values is a 32-byte sector of its own column
+  const float* d = a.d1 + pos;
+  const float *xx = a.g.xx + pos, *yy = a.g.yy + pos, *zz = a.g.zz + pos, *xy = a.g.xy + pos,
+              *xz = a.g.xz + pos, *yz = a.g.yz + pos;
+  const float d0 = d[0], dk = d[-1], dx = d[S], dxk = d[S - 1], dy = d[-Y], dyk = d[-Y - 1],
+              dxy = d[S - Y];
+  const float u0 = a.g.u1[pos], v0 = a.g.v1[pos], w0 = a.g.w1[pos];
+  const float xx0 = xx[0], xxm = xx[-S], yy0 = yy[0], yyp = yy[Y], zz0 = zz[0], zzp = zz[1];
+  const float xy0 = xy[0], xyx = xy[S], xyy = xy[-Y];
+  const float xz0 = xz[0], xzx = xz[S], xzk = xz[-1];
+  const float yz0 = yz[0], yzy = yz[-Y], yzk = yz[-1];
   const float dcrj = __fmul_rn(__fmul_rn(a.dcrjz[k], a.dcrjx[i]), a.dcrjy[j]);
-  // w along the first line
-  {
-    const float fd3 = a.dth / __fmul_rn(0.25f, __fadd_rn(__fadd_rn(__fadd_rn(d[pos], d[pos + S]),
-                                                                   d[pos - Y]),
-                                                         d[pos + S - Y]));
-    const float s = __fadd_rn(__fadd_rn(__fsub_rn(a.g.xz[pos + S], a.g.xz[pos]),
-                                        __fsub_rn(a.g.yz[pos], a.g.yz[pos - Y])),
-                              __fsub_rn(a.g.zz[pos + 1], a.g.zz[pos]));
-    a.g.w1[pos] = __fmul_rn(__fmaf_rn(fd3, s, a.g.w1[pos]), dcrj);
-  }
-  // u, v along the second line (same k in the reference)
-  {
-    const float fd1 = a.dth / __fmul_rn(0.25f, __fadd_rn(__fadd_rn(__fadd_rn(d[pos], d[pos - Y]),
-                                                                   d[pos - 1]),
-                                                         d[pos - Y - 1]));
-    const float fd2 = a.dth / __fmul_rn(0.25f, __fadd_rn(__fadd_rn(__fadd_rn(d[pos], d[pos + S]),
-                                                                   d[pos - 1]),
-                                                         d[pos + S - 1]));
-    const float su = __fadd_rn(__fadd_rn(__fsub_rn(a.g.xx[pos], a.g.xx[pos - S]),
-                                         __fsub_rn(a.g.xy[pos], a.g.xy[pos - Y])),
-                               __fsub_rn(a.g.xz[pos], a.g.xz[pos - 1]));
-    const float sv = __fadd_rn(__fadd_rn(__fsub_rn(a.g.xy[pos + S], a.g.xy[pos]),
-                                         __fsub_rn(a.g.yy[pos + Y], a.g.yy[pos])),
-                               __fsub_rn(a.g.yz[pos], a.g.yz[pos - 1]));
-    a.g.u1[pos] = __fmul_rn(__fmaf_rn(fd1, su, a.g.u1[pos]), dcrj);
-    a.g.v1[pos] = __fmul_rn(__fmaf_rn(fd2, sv, a.g.v1[pos]), dcrj);
-  }
+  auto mean = [](float p, float q, float r, float t) {
+    return __fmul_rn(0.25f, __fadd_rn(__fadd_rn(__fadd_rn(p, q), r), t));
+  };
+  const float fd1 = a.dth / mean(d0, dy, dk, dyk), fd2 = a.dth / mean(d0, dx, dk, dxk),
+              fd3 = a.dth / mean(d0, dx, dy, dxy);
+  const float sw = __fadd_rn(__fadd_rn(__fsub_rn(xzx, xz0), __fsub_rn(yz0, yzy)),
+                             __fsub_rn(zzp, zz0));
+  const float su = __fadd_rn(__fadd_rn(__fsub_rn(xx0, xxm), __fsub_rn(xy0, xyy)),
+                             __fsub_rn(xz0, xzk));
+  const float sv = __fadd_rn(__fadd_rn(__fsub_rn(xyx, xy0), __fsub_rn(yyp, yy0)),
+                             __fsub_rn(yz0, yzk));
+  a.g.w1[pos] = __fmul_rn(__fmaf_rn(fd3, sw, w0), dcrj);
+  a.g.u1[pos] = __fmul_rn(__fmaf_rn(fd1, su, u0), dcrj);
+  a.g.v1[pos] = __fmul_rn(__fmaf_rn(fd2, sv, v0), dcrj);
 }
 
 // ===========================================================================
 // dstrqc2 (kernel.cu:2564-2767), anelastic form (ELA2 undefined)
 // ===========================================================================
-// Q(f) weight of dstrqc2: double switch 1/(2q) <= 200, low-Q polynomial in
-// double, otherwise wwo*q (dstrqc uses 2*wwo*q there), then / wwo.
-__device__ __forceinline__ float qf2(float q, float wwo, float c0, float c1) {
-  float w;
-  if (1. / ((double)q * 2.0) <= 200.0) {
-    const double x = 2. * (double)q;
-    w = (float)__fma_rn(__dmul_rn((double)c0, x), x, __dmul_rn((double)c1, x));
-  } else {
-    w = __fmul_rn(wwo, q);
-  }
-  return w / wwo;
-}
-
-__global__ void k_dstrqc2(const DmStr2Args a) {
+// The switch 1/(2q) <= 200 on q = S/4 as one compare of bit patterns and the
+// low-Q polynomial in float, as awp_weight (awp_stencil.cuh); the high-Q
+// branch is wwo*q here where dstrqc has 2*wwo*q, so its constant is halved.
+// Every load is issued before the arithmetic: the kernel's time is the sectors
+// of one level of k-contiguous columns, one 32-byte sector per value (300 x
+// 300: 62 -> 33 us with the double-precision divisions of the switch gone).
+__global__ void __launch_bounds__(128) k_dstrqc2(const DmStr2Args a) {
   const int j = a.j0 + blockIdx.x * blockDim.x + threadIdx.x;
   const int i = a.i0 + blockIdx.y * blockDim.y + threadIdx.y;
   if (i > a.i1 || j > a.j1) return;
   const int S = a.g.slice, Y = a.g.yline;
   const int k = AWP_ALIGN + 2;
   const long long pos = at(a.g, i, j, k);
+  const DmGrid& g = a.g;
+  float sg[6] = {g.xx[pos], g.yy[pos], g.zz[pos], g.xy[pos], g.xz[pos], g.yz[pos]};
+  float rr[6] = {a.r1[pos], a.r2[pos], a.r3[pos], a.r4[pos], a.r5[pos], a.r6[pos]};
+  const float *u = g.u1 + pos, *v = g.v1 + pos, *w = g.w1 + pos;
+  const float u0 = u[0], ux = u[S], uy = u[Y], uk = u[1];
+  const float v0 = v[0], vx = v[-S], vy = v[-Y], vk = v[1];
+  const float w0 = w[0], wx = w[-S], wy = w[Y], wk = w[-1];
+  // a field's value, its pair sums with k-1, j-1, i+1 and its eight-cell sum
+  struct Mat {
+    float pk, pj, pi, s8;
+  };
+  auto mat = [&](const float* f) {
+    const float* p = f + pos;
+    const float m0 = p[0], mk = p[-1], mj = p[-Y], mjk = p[-Y - 1], mi = p[S], mik = p[S - 1],
+                mij = p[S - Y], mijk = p[S - Y - 1];
+    return Mat{vadd(m0, mk), vadd(m0, mj), vadd(m0, mi),
+               vadd(awp_quad(vadd(m0, mj), vadd(mk, mjk)),
+                    awp_quad(vadd(mi, mij), vadd(mik, mijk)))};
+  };
+  const Mat L = mat(a.lam), M = mat(a.mu), P = mat(a.qp), R = mat(a.qs);
   const float dcrj = __fmul_rn(__fmul_rn(a.dcrjz[k], a.dcrjx[i]), a.dcrjy[j]);
   float f_vx1, f_vx2, f_wwo;
   int cidx;
@@ -100,68 +110,15 @@ __global__ void k_dstrqc2(const DmStr2Args a) {
   }
   const float c0 = a.coeff_dev ? a.coeff_dev[cidx] : a.coeff[cidx];
   const float c1 = a.coeff_dev ? a.coeff_dev[cidx + 1] : a.coeff[cidx + 1];
-  // eight-cell sums in the reference's order: pos, ip1, jm1, ijk, km1, ik1, jk1, ijk1
-  auto sum8 = [&](const float* f) {
-    float s = __fadd_rn(f[pos], f[pos + S]);
-    s = __fadd_rn(s, f[pos - Y]);
-    s = __fadd_rn(s, f[pos + S - Y]);
-    s = __fadd_rn(s, f[pos - 1]);
-    s = __fadd_rn(s, f[pos + S - 1]);
-    s = __fadd_rn(s, f[pos - Y - 1]);
-    return __fadd_rn(s, f[pos + S - Y - 1]);
-  };
-  const float* mu = a.mu;
-  float xl = __fdiv_rn(8.0f, sum8(a.lam));   // = (float)(8.0/(double)x), see k_stress
-  float xm = __fdiv_rn(16.0f, sum8(mu));
-  float xmu1 = __fdiv_rn(2.0f, __fadd_rn(mu[pos], mu[pos - 1]));
-  float xmu2 = __fdiv_rn(2.0f, __fadd_rn(mu[pos], mu[pos - Y]));
-  float xmu3 = __fdiv_rn(2.0f, __fadd_rn(mu[pos], mu[pos + S]));
-  xl = __fadd_rn(xl, xm);
-  // qpa: float switch 1.0f/(2q) <= 200.0f
-  float qpa = __fmul_rn(0.0625f, sum8(a.qp));
-  float qpaw;
-  if (1.0f / (qpa * 2.0f) <= 200.0f) {
-    const double x = 2. * (double)qpa;
-    qpaw = (float)__fma_rn(__dmul_rn((double)c0, x), x, __dmul_rn((double)c1, x));
-  } else {
-    qpaw = __fmul_rn(f_wwo, qpa);
-  }
-  qpaw = qpaw / f_wwo;
-  const float* qs = a.qs;
-  const float hw = qf2(__fmul_rn(0.0625f, sum8(qs)), f_wwo, c0, c1);
-  const float h1w = qf2(__fmul_rn(0.25f, __fadd_rn(qs[pos], qs[pos - 1])), f_wwo, c0, c1);
-  const float h2w = qf2(__fmul_rn(0.25f, __fadd_rn(qs[pos], qs[pos - Y])), f_wwo, c0, c1);
-  const float h3w = qf2(__fmul_rn(0.25f, __fadd_rn(qs[pos], qs[pos + S])), f_wwo, c0, c1);
-  // the weights scaled by -vx1/h (awp_stencil.cuh)
-  const float K = -__fmul_rn(a.dh1, f_vx1), DT = a.dt;
-  const float wh = __fmul_rn(hw, K), wq = __fmul_rn(qpaw, K);
-  const float wm[3] = {__fmul_rn(h1w, K), __fmul_rn(h2w, K), __fmul_rn(h3w, K)};
-  const float raw[3] = {xmu1, xmu2, xmu3};
-  AwpStrCoef<float> cf;
-  cf.nh = __fmul_rn(-xm, wh);
-  cf.nxm = __fmul_rn(-xm, __fmaf_rn(DT, wh, a.dth));
-  cf.Q = __fmul_rn(xl, wq);
-  cf.A = __fmul_rn(xl, __fmaf_rn(DT, wq, a.dth));
-#pragma unroll
-  for (int q = 0; q < 3; ++q) {
-    cf.h[q] = __fmul_rn(raw[q], wm[q]);
-    cf.m[q] = __fmul_rn(raw[q], __fmaf_rn(DT, wm[q], a.dth));
-  }
-  const AwpRelax<float> rx = awp_relax_from(f_vx1, f_vx2, f_wwo, c0, c1, DT, a.dh1);
-
-  const DmGrid& g = a.g;
-  float d[9];
-  d[0] = __fsub_rn(g.u1[pos + S], g.u1[pos]);  // normal: x, y, z
-  d[1] = __fsub_rn(g.v1[pos], g.v1[pos - Y]);
-  d[2] = __fsub_rn(g.w1[pos], g.w1[pos - 1]);
-  d[3] = __fsub_rn(g.u1[pos + Y], g.u1[pos]);  // xy pair
-  d[4] = __fsub_rn(g.v1[pos], g.v1[pos - S]);
-  d[5] = __fsub_rn(g.u1[pos + 1], g.u1[pos]);  // xz pair
-  d[6] = __fsub_rn(g.w1[pos], g.w1[pos - S]);
-  d[7] = __fsub_rn(g.v1[pos + 1], g.v1[pos]);  // yz pair
-  d[8] = __fsub_rn(g.w1[pos + Y], g.w1[pos]);
-  float sg[6] = {g.xx[pos], g.yy[pos], g.zz[pos], g.xy[pos], g.xz[pos], g.yz[pos]};
-  float rr[6] = {a.r1[pos], a.r2[pos], a.r3[pos], a.r4[pos], a.r5[pos], a.r6[pos]};
+  AwpRelax<float> rx = awp_relax_from(f_vx1, f_vx2, f_wwo, c0, c1, a.dt, a.dh1);
+  rx.c2 *= 0.5f;
+  const float PM[3] = {M.pk, M.pj, M.pi}, PR[3] = {R.pk, R.pj, R.pi};
+  const AwpStrCoef<float> cf =
+      awp_stress_coef<false>(L.s8, M.s8, PM, P.s8, R.s8, PR, rx, a.thr, a.dth, a.dt);
+  const float d[9] = {__fsub_rn(ux, u0), __fsub_rn(v0, vy), __fsub_rn(w0, wk),  // x, y, z
+                      __fsub_rn(uy, u0), __fsub_rn(v0, vx),                     // xy pair
+                      __fsub_rn(uk, u0), __fsub_rn(w0, wx),                     // xz pair
+                      __fsub_rn(vk, v0), __fsub_rn(wy, w0)};                    // yz pair
   awp_stress_update<false>(sg, rr, cf, rx, dcrj, d);
   g.xx[pos] = sg[0]; g.yy[pos] = sg[1]; g.zz[pos] = sg[2];
   g.xy[pos] = sg[3]; g.xz[pos] = sg[4]; g.yz[pos] = sg[5];
@@ -172,8 +129,10 @@ __global__ void k_dstrqc2(const DmStr2Args a) {
 // ===========================================================================
 // intp3d (kernel.cu:2359-2561): bilinear weights (1, 2/3, 1/3, 0) spread each
 // coarse cell's four corners over a 4 x 4 fine patch at kh = align+1.
-// Neighbouring patches share an edge where the weight is 0 on one side, and
-// both threads store the same value there, as in the reference.
+// Neighbouring patches share an edge, where the weight is 0 on one side and
+// the reference's threads store the same value: a thread stores its patch's
+// 3 x 3 cells, the last rows and columns their edge too (each store is a
+// sector of its own).
 // ===========================================================================
 __global__ void k_intp3d(const DmPairArgs a) {
   const int j = AWP_NGSL + blockIdx.x * blockDim.x + threadIdx.x;
@@ -189,8 +148,9 @@ __global__ void k_intp3d(const DmPairArgs a) {
   // field, its fine patch offset in i and j
   auto patch = [&](const float* L, float* H, int oi, int oj) {
     const float v0 = L[pl], v1 = L[pip], v2 = L[pjp], v3 = L[pij];
-    for (int jj = 1; jj <= 4; ++jj)
-      for (int ii = 1; ii <= 4; ++ii) {
+    const int nj = j == lo.nyt + 3 + AWP_NGSL ? 4 : 3, ni = i == lo.nxt + 3 + AWP_NGSL ? 4 : 3;
+    for (int jj = 1; jj <= nj; ++jj)
+      for (int ii = 1; ii <= ni; ++ii) {
         const float wa = w[ii - 1], wb = w[jj - 1], wc = w[4 - ii], wd = w[4 - jj];
         float s = __fmul_rn(__fmul_rn(v0, wa), wb);
         s = __fmaf_rn(__fmul_rn(v1, wc), wb, s);
@@ -215,80 +175,97 @@ __global__ void k_intp3d(const DmPairArgs a) {
 
 // ===========================================================================
 // swap3 (kernel.cu:3032-3217): tent-weighted 5 x 5 x 5 window average of the
-// fine grid (WWL = 2) into the coarse grid's top two layers.  Weights and
-// products in double, each partial sum rounded to float like the reference's
-// float accumulator.
+// fine grid (WWL = 2) into the coarse grid's top two layers.
 // ===========================================================================
-// A CTA takes 2 (i) x 32 (j) coarse columns of one field (blockIdx.z): it
-// copies the fine-grid box the field's windows read
-// (9 x 99 x 8 points: fine i2-2 .. i3+2 and j2-2 .. j3+2 of its columns,
-// levels align+1 .. align+8) into shared memory with k-contiguous,
-// sector-wide loads, then each of its threads forms one window of one column
-// (a field has one or two: levels nzt-2 and nzt-1), its 125 terms in the
-// reference's order from shared memory.  Read straight from global memory the
-// windows' stride-3 j columns cost a sector per 4-byte load; the box copy
-// reads each sector once.
-constexpr int kSwTI = 2, kSwTJ = 32;
-constexpr int kSwBI = 3 * (kSwTI - 1) + 6, kSwBJ = 3 * (kSwTJ - 1) + 6, kSwBK = 8;
-constexpr int kSwKS = 9;  // padded k stride: lanes 3 j apart fall in distinct banks
+// The tent weight is a product (3-|ii|)(3-|jj|)(3-|kk|) / 729, so a window is
+// three five-point sums, one per axis: 5 + 5 + 5 terms a value where the
+// reference adds 125 in one float chain (each partial sum rounded; the three
+// short sums round less).  A CTA takes 4 (i) x 32 (j) coarse columns of one
+// field (blockIdx.z): its fine columns' levels align+1 .. align+8 are summed
+// along k as they are read (eight lanes a column: k-contiguous, sector-wide
+// loads), then along j and i from shared memory.
+// 300 x 300 over 100 x 100: 51 -> 17 us a launch against the chain of 125
+// double-precision terms.
+constexpr int kSwTI = 4, kSwTJ = 32;
+constexpr int kSwBI = 3 * (kSwTI - 1) + 5, kSwBJ = 3 * (kSwTJ - 1) + 5;
+constexpr int kSwThreads = 32 * kSwBI;  // a warp per fine row
 
-// The 125 tent weights of a window in the sum's order (jj, ii, kk), formed on
-// the host as the reference forms them on the device, in double:
-// (1 / total) * (3 - |ii|) * (3 - |jj|) * (3 - |kk|) left to right.
-struct SwapWeights {
-  double w[125];
-};
-
-__global__ void __launch_bounds__(128) k_swap3(const DmPairArgs a, const SwapWeights sw) {
-  __shared__ float box[kSwBI * kSwBJ * kSwKS];
+__global__ void __launch_bounds__(kSwThreads) k_swap3(const DmPairArgs a) {
+  __shared__ float ks[2][kSwBI][kSwBJ + 1];  // summed along k (two windows)
+  __shared__ float js[2][kSwBI][kSwTJ + 1];  // ... and along j
   const DmGrid &lo = a.lo, &hi = a.hi;
-  const int tid = threadIdx.y * 32 + threadIdx.x;
+  const int tid = threadIdx.x;
   const int i0 = AWP_NGSL + blockIdx.y * kSwTI, j0 = AWP_NGSL + blockIdx.x * kSwTJ;
   const int imax = lo.nxt + AWP_NGSL + 4, jmax = lo.nyt + AWP_NGSL + 4;
-  // fine box origin (i2 - 2, j2 - 2 of the first column) and the extent the
-  // valid columns read
-  const int fi0 = (i0 - 2 - AWP_NGSL) * 3 + AWP_NGSL, fj0 = (j0 - 2 - AWP_NGSL) * 3 + AWP_NGSL;
-  const int nbi = 3 * (min(i0 + kSwTI - 1, imax) - i0) + 6;
-  const int nbj = 3 * (min(j0 + kSwTJ - 1, jmax) - j0) + 6;
-  // this thread's column and window slot (level 0 or 1)
-  const int c = tid & 63, lev = tid >> 6;
-  const int ci = c >> 5, cj = c & 31;
-  const int i = i0 + ci, j = j0 + cj;
-  const bool valid = i <= imax && j <= jmax;
+  const int nci = min(kSwTI, imax - i0 + 1), ncj = min(kSwTJ, jmax - j0 + 1);
+  float* dst;
+  const float* src;
+  int kh0, nwin, di, dj;  // level-0 window at kh0 (level 1 at 6); shifted fine columns
+  switch (blockIdx.z) {
+    case 0: dst = lo.u1; src = hi.u1; kh0 = 3; nwin = 2; di = 0; dj = 0; break;
+    case 1: dst = lo.v1; src = hi.v1; kh0 = 3; nwin = 2; di = 1; dj = 1; break;
+    case 2: dst = lo.xy; src = hi.xy; kh0 = 3; nwin = 2; di = 0; dj = 1; break;
+    case 3: dst = lo.xx; src = hi.xx; kh0 = 3; nwin = 2; di = 1; dj = 0; break;
+    case 4: dst = lo.yy; src = hi.yy; kh0 = 3; nwin = 2; di = 1; dj = 0; break;
+    case 5: dst = lo.zz; src = hi.zz; kh0 = 3; nwin = 2; di = 1; dj = 0; break;
+    case 6: dst = lo.xz; src = hi.xz; kh0 = 4; nwin = 1; di = 0; dj = 0; break;
+    case 7: dst = lo.w1; src = hi.w1; kh0 = 4; nwin = 1; di = 1; dj = 0; break;
+    default: dst = lo.yz; src = hi.yz; kh0 = 4; nwin = 1; di = 1; dj = 1; break;
+  }
+  // the window of coarse column c centres on fine column 3 (c - 2 - ngsl) + 2 + ngsl + d
+  const int fi0 = (i0 - 2 - AWP_NGSL) * 3 + AWP_NGSL + di,
+            fj0 = (j0 - 2 - AWP_NGSL) * 3 + AWP_NGSL + dj;
+  const int nbi = 3 * (nci - 1) + 5, nbj = 3 * (ncj - 1) + 5;
+  // along k: lane kk of eight holds level align+1+kk; its weights in the two
+  // windows, centred on levels align + kh0 and align + 6
   {
-    const int f = blockIdx.z;  // one field per CTA
-    float* dst;
-    const float* src;
-    int kh0, nwin, di, dj;  // level-0 window at kh0 (level 1 at 6); source i3 / j3 if di / dj
-    switch (f) {
-      case 0: dst = lo.u1; src = hi.u1; kh0 = 3; nwin = 2; di = 0; dj = 0; break;
-      case 1: dst = lo.v1; src = hi.v1; kh0 = 3; nwin = 2; di = 1; dj = 1; break;
-      case 2: dst = lo.xy; src = hi.xy; kh0 = 3; nwin = 2; di = 0; dj = 1; break;
-      case 3: dst = lo.xx; src = hi.xx; kh0 = 3; nwin = 2; di = 1; dj = 0; break;
-      case 4: dst = lo.yy; src = hi.yy; kh0 = 3; nwin = 2; di = 1; dj = 0; break;
-      case 5: dst = lo.zz; src = hi.zz; kh0 = 3; nwin = 2; di = 1; dj = 0; break;
-      case 6: dst = lo.xz; src = hi.xz; kh0 = 4; nwin = 1; di = 0; dj = 0; break;
-      case 7: dst = lo.w1; src = hi.w1; kh0 = 4; nwin = 1; di = 1; dj = 0; break;
-      default: dst = lo.yz; src = hi.yz; kh0 = 4; nwin = 1; di = 1; dj = 1; break;
-    }
-    for (int t = tid; t < nbi * nbj * kSwBK; t += 128) {
-      const int bk = t % kSwBK, r = t / kSwBK, bj = r % nbj, bi = r / nbj;
-      box[(bi * kSwBJ + bj) * kSwKS + bk] = src[at(hi, fi0 + bi, fj0 + bj, AWP_ALIGN + 1 + bk)];
-    }
-    __syncthreads();
-    if (valid && lev < nwin) {
-      const int kh = lev ? 6 : kh0;
-      const int bi = 3 * ci + di + 2, bj = 3 * cj + dj + 2, bk = kh - 1;
-      float sum = 0.0f;
-      int q = 0;
-      for (int jj = -AWP_WWL; jj <= AWP_WWL; ++jj)
-        for (int ii = -AWP_WWL; ii <= AWP_WWL; ++ii)
+    const int kk = tid & 7;
+    auto tent = [](int d) { return (float)(3 - min(3, d < 0 ? -d : d)); };
+    const float w0 = tent(kk + 1 - kh0), w1 = tent(kk + 1 - 6);
+    const int warp = tid >> 5, c4 = (tid & 31) >> 3;
+    const int bi = warp;
+    if (bi < nbi) {
+      const float* p = src + at(hi, fi0 + bi, fj0, AWP_ALIGN + 1 + kk);
+      constexpr int kFly = 9;  // columns of a lane in flight (latency bound)
+      for (int b0 = 0; b0 < nbj; b0 += 4 * kFly) {
+        float h[kFly];
 #pragma unroll
-          for (int kk = -AWP_WWL; kk <= AWP_WWL; ++kk, ++q) {
-            const float h = box[((bi + ii) * kSwBJ + bj + jj) * kSwKS + bk + kk];
-            sum = (float)__fma_rn(sw.w[q], (double)h, (double)sum);
+        for (int q = 0; q < kFly; ++q) {
+          const int bj = b0 + 4 * q + c4;
+          h[q] = bj < nbj ? p[(long long)bj * hi.yline] : 0.f;
+        }
+#pragma unroll
+        for (int q = 0; q < kFly; ++q) {
+          const int bj = b0 + 4 * q + c4;
+          float s0 = w0 * h[q], s1 = w1 * h[q];
+#pragma unroll
+          for (int m = 4; m >= 1; m >>= 1) {
+            s0 += __shfl_xor_sync(0xffffffffu, s0, m);
+            s1 += __shfl_xor_sync(0xffffffffu, s1, m);
           }
-      dst[at(lo, i, j, AWP_ALIGN + lo.nzt - 2 + lev)] = sum;
+          if (kk == 0 && bj < nbj) {
+            ks[0][bi][bj] = s0;
+            ks[1][bi][bj] = s1;
+          }
+        }
+      }
+    }
+  }
+  __syncthreads();
+  for (int t = tid; t < nwin * nbi * kSwTJ; t += kSwThreads) {
+    const int cj = t & (kSwTJ - 1), r = t / kSwTJ, lev = r >= nbi ? 1 : 0, bi = r - lev * nbi;
+    if (cj < ncj) {
+      const float* p = &ks[lev][bi][3 * cj];
+      js[lev][bi][cj] = (p[0] + p[4]) + 2.f * (p[1] + p[3]) + 3.f * p[2];
+    }
+  }
+  __syncthreads();
+  for (int t = tid; t < nwin * kSwTI * kSwTJ; t += kSwThreads) {
+    const int cj = t & (kSwTJ - 1), ci = (t / kSwTJ) & (kSwTI - 1), lev = t / (kSwTJ * kSwTI);
+    if (ci < nci && cj < ncj) {
+      const float(*p)[kSwTJ + 1] = &js[lev][3 * ci];
+      const float s = (p[0][cj] + p[4][cj]) + 2.f * (p[1][cj] + p[3][cj]) + 3.f * p[2][cj];
+      dst[at(lo, i0 + ci, j0 + cj, AWP_ALIGN + lo.nzt - 2 + lev)] = __fdiv_rn(s, 729.0f);
     }
   }
 }
@@ -334,21 +311,8 @@ cudaError_t awp_launch_intp3d(const DmPairArgs& a, cudaStream_t st) {
 }
 
 cudaError_t awp_launch_swap3(const DmPairArgs& a, cudaStream_t st) {
-  double total = 0.;  // ttlwght2 = ttlwght3 = ttlwght4 for WWL = 2 (kernel.cu:3052-3061)
-  for (int jj = -AWP_WWL; jj <= AWP_WWL; jj++)
-    for (int ii = -AWP_WWL; ii <= AWP_WWL; ii++)
-      for (int kk = -AWP_WWL; kk <= AWP_WWL; kk++)
-        total += (1. + AWP_WWL - abs(jj)) * (1. + AWP_WWL - abs(ii)) * (1. + AWP_WWL - abs(kk));
-  const double inv_total = 1. / total;
-  SwapWeights sw;
-  int q = 0;
-  for (int jj = -AWP_WWL; jj <= AWP_WWL; jj++)
-    for (int ii = -AWP_WWL; ii <= AWP_WWL; ii++)
-      for (int kk = -AWP_WWL; kk <= AWP_WWL; kk++)
-        sw.w[q++] = inv_total * (1. + AWP_WWL - abs(ii)) * (1. + AWP_WWL - abs(jj)) *
-                    (1. + AWP_WWL - abs(kk));
-  k_swap3<<<dim3(cdiv(a.lo.nyt + 5, kSwTJ), cdiv(a.lo.nxt + 5, kSwTI), 9), dim3(32, 4), 0, st>>>(
-      a, sw);
+  // columns ngsl .. n + ngsl + 4 of the coarse block
+  k_swap3<<<dim3(cdiv(a.lo.nyt + 5, kSwTJ), cdiv(a.lo.nxt + 5, kSwTI), 9), kSwThreads, 0, st>>>(a);
   return cudaGetLastError();
 }
 

@@ -36,6 +36,7 @@ struct DmStr2Args {
   const float* coeff_dev;
   int i0, i1, j0, j1;
   float dth, dh1, dt;
+  unsigned thr;  // Q(f) switch on a pair sum of Q^-1 (StrArgs::thr)
 };
 
 // intp3d (kernel.cu:2359-2561) coarse -> fine and swap3 (kernel.cu:3032-3217)

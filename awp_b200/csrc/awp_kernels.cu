@@ -293,8 +293,30 @@ __device__ __forceinline__ void fstr_cell(const FstrArgs& a, const int i, const 
   a.yz[p] = 0.0f;
 }
 
+// The same with whole-sector accesses where the surface pair starts on a
+// multiple of four floats (the context's layout): a thread's column is a
+// 32-byte sector per field below and one above the surface, so the kernel's
+// time is its sectors, and one access to each replaces two or three.
+__device__ __forceinline__ void fstr_cell4(const FstrArgs& a, const int i, const int j) {
+  if (j > a.j1 || i > a.i1) return;
+  const long long p = (long long)i * a.slice + (long long)j * a.yline + a.ktop;
+  const float2 z = *reinterpret_cast<const float2*>(a.zz + p - 1);
+  const float4 x = *reinterpret_cast<const float4*>(a.xz + p - 3);
+  const float4 y = *reinterpret_cast<const float4*>(a.yz + p - 3);
+  *reinterpret_cast<float2*>(a.zz + p + 1) = make_float2(-z.y, -z.x);
+  *reinterpret_cast<float2*>(a.xz + p + 1) = make_float2(-x.z, -x.y);
+  *reinterpret_cast<float2*>(a.yz + p + 1) = make_float2(-y.z, -y.y);
+  a.xz[p] = 0.0f;
+  a.yz[p] = 0.0f;
+}
+
+template <bool V4>
 __global__ void k_fstr(const FstrArgs a) {
-  fstr_cell(a, a.i0 + blockIdx.y, a.j0 + blockIdx.x * blockDim.x + threadIdx.x);
+  const int i = a.i0 + blockIdx.y, j = a.j0 + blockIdx.x * blockDim.x + threadIdx.x;
+  if (V4)
+    fstr_cell4(a, i, j);
+  else
+    fstr_cell(a, i, j);
 }
 
 // ===========================================================================
@@ -448,6 +470,36 @@ __global__ void k_addkinsrc(const KinSrcArgs a) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= a.ncell) return;
   addkinsrc_cell(a, c, a.step);
+}
+
+// Free-surface imaging and the point sources of a step in one launch, for
+// sources below the levels the imaging touches (the caller checks): the last
+// row of CTAs adds the sources.  `step` (replayable graphs): the step is read
+// from the device, *step + 1 + off, and IFAULT < 4 stops at nst.
+__global__ void k_fstr_src(const FstrArgs f, const SrcArgs s, const int* step, const int off,
+                           const int nst) {
+  if (blockIdx.y + 1 < gridDim.y) {
+    fstr_cell4(f, f.i0 + blockIdx.y, f.j0 + blockIdx.x * blockDim.x + threadIdx.x);
+    return;
+  }
+  SrcArgs a = s;
+  if (step) {
+    a.tidx = *step + 1 + off;
+    if (a.tidx >= nst) return;
+  }
+  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < a.ncell; c += gridDim.x * blockDim.x)
+    addsrc_cell(a, c);
+}
+
+__global__ void k_fstr_kinsrc(const FstrArgs f, const KinSrcArgs k, const int* step,
+                              const int off) {
+  if (blockIdx.y + 1 < gridDim.y) {
+    fstr_cell4(f, f.i0 + blockIdx.y, f.j0 + blockIdx.x * blockDim.x + threadIdx.x);
+    return;
+  }
+  const int cur = step ? *step + 1 + off : k.step;
+  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < k.ncell; c += gridDim.x * blockDim.x)
+    addkinsrc_cell(k, c, cur);
 }
 
 // ===========================================================================
@@ -888,98 +940,25 @@ inline unsigned cdiv_u(long long a, long long b) { return (unsigned)((a + b - 1)
 
 }  // namespace
 
-// ===========================================================================
-// Batched instances (many independent simulations, one persistent launch per
-// half-step).  CTAs pull tiles (instance, tile coordinates) from a global
-// counter and run the same per-tile bodies as the one-simulation kernels, so
-// each instance's arithmetic is unchanged.
-// ===========================================================================
-__device__ __forceinline__ int next_tile(int* counter, int* s_tile) {
-  __syncthreads();  // every thread has read the previous tile
-  if (threadIdx.x == 0 && threadIdx.y == 0) *s_tile = atomicAdd(counter, 1);
-  __syncthreads();
-  return *s_tile;
-}
-
-template <int TY>
-__global__ void __launch_bounds__(32 * TY)
-    k_batch_velocity(const BatchInst* __restrict__ inst, const int4* __restrict__ tiles,
-                     const int ntiles, int* counter, const int ichunk) {
-  __shared__ int s_tile;
-  for (;;) {
-    const int t = next_tile(counter, &s_tile);
-    if (t >= ntiles) return;
-    const int4 d = tiles[t];
-    const VelArgs a = inst[d.x].v;
-    vel_tile<TY>(a, d.y, d.z, d.w, ichunk, threadIdx.x, threadIdx.y);
-  }
-}
-
-// Elastic and anelastic instances have separate tile lists and launches, so
-// each launch carries one stress variant (register pressure as k_stress).
-template <bool ELASTIC, int TY>
-__global__ void __launch_bounds__(32 * TY, TY == 8 ? 2 : 1)
-    k_batch_stress(const BatchInst* __restrict__ inst, const int4* __restrict__ tiles,
-                   const int ntiles, int* counter, const int ichunk) {
-  __shared__ int s_tile;
-  for (;;) {
-    const int t = next_tile(counter, &s_tile);
-    if (t >= ntiles) return;
-    const int4 d = tiles[t];
-    const StrArgs& a = inst[d.x].s;  // read in place (dynamically indexed tables)
-    str_tile<ELASTIC, false, TY>(a, d.y, d.z, d.w, ichunk, threadIdx.x, threadIdx.y);
-  }
-}
-
-// Sources of every instance at step *step + 1 (the step being taken), with the
-// schedule of one_step: IFAULT < 4 while the step is below NST, IFAULT 5 always.
-__global__ void k_batch_sources(const BatchInst* __restrict__ inst,
-                                const int2* __restrict__ cells, const int n,
-                                const int* __restrict__ step) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= n) return;
-  const int2 e = cells[q];
-  const BatchInst& I = inst[e.x];
-  const int cur = *step + 1;
-  if (I.ifault == 5) {
-    addkinsrc_cell(I.kin, e.y, cur);
-  } else if (I.ifault < 4 && cur < I.nst) {
-    SrcArgs a = I.src;
-    a.tidx = cur;
-    addsrc_cell(a, e.y);
-  }
-}
-
-// Sources of one instance at step *step + 1 read from device memory (replayable
-// graphs): the schedule of one_step, IFAULT < 4 while the step is below NST.
-__global__ void k_addsrc_dev(const SrcArgs a, const int* __restrict__ step, const int nst) {
+// Sources of one instance at step *step + 1 + off read from device memory
+// (replayable graphs): the schedule of one_step, IFAULT < 4 while the step is below NST.
+__global__ void k_addsrc_dev(const SrcArgs a, const int* __restrict__ step, const int off,
+                             const int nst) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  const int cur = *step + 1;
+  const int cur = *step + 1 + off;
   if (c >= a.ncell || cur >= nst) return;
   SrcArgs b = a;
   b.tidx = cur;
   addsrc_cell(b, c);
 }
 
-__global__ void k_addkinsrc_dev(const KinSrcArgs a, const int* __restrict__ step) {
+__global__ void k_addkinsrc_dev(const KinSrcArgs a, const int* __restrict__ step, const int off) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= a.ncell) return;
-  addkinsrc_cell(a, c, *step + 1);
+  addkinsrc_cell(a, c, *step + 1 + off);
 }
 
-__global__ void k_step_advance(int* step) { *step = *step + 1; }
-
-// Free-surface imaging of every instance (one CTA per (instance, x row)); the
-// first thread then advances the batch's step counter.
-__global__ void k_batch_fstr(const BatchInst* __restrict__ inst, const int2* __restrict__ rows,
-                             const int n, int* step) {
-  for (int r = blockIdx.x; r < n; r += gridDim.x) {
-    const int2 e = rows[r];
-    const FstrArgs& a = inst[e.x].f;
-    for (int j = a.j0 + threadIdx.x; j <= a.j1; j += blockDim.x) fstr_cell(a, e.y, j);
-  }
-  if (blockIdx.x == 0 && threadIdx.x == 0) *step = *step + 1;
-}
+__global__ void k_step_advance(int* step, const int n) { *step = *step + n; }
 
 // ===========================================================================
 // launchers
@@ -1040,10 +1019,33 @@ int awp_tuning_get(const char* key) {
   return -1;
 }
 
+namespace {
+bool fstr_aligned(const FstrArgs& a) {
+  const uintptr_t p = reinterpret_cast<uintptr_t>(a.zz) | reinterpret_cast<uintptr_t>(a.xz) |
+                      reinterpret_cast<uintptr_t>(a.yz);
+  return !(p & 15) && a.yline % 4 == 0 && a.slice % 4 == 0 && (a.ktop + 1) % 4 == 0;
+}
+}  // namespace
+
 cudaError_t awp_launch_fstr(const FstrArgs& a, cudaStream_t st) {
   const int nj = a.j1 - a.j0 + 1, ni = a.i1 - a.i0 + 1;
   if (nj <= 0 || ni <= 0) return cudaSuccess;
-  k_fstr<<<dim3(cdiv_u(nj, 128), ni, 1), 128, 0, st>>>(a);
+  if (fstr_aligned(a))
+    k_fstr<true><<<dim3(cdiv_u(nj, 128), ni, 1), 128, 0, st>>>(a);
+  else
+    k_fstr<false><<<dim3(cdiv_u(nj, 128), ni, 1), 128, 0, st>>>(a);
+  return cudaGetLastError();
+}
+
+cudaError_t awp_launch_fstr_sources(const FstrArgs& f, const SrcArgs* s, const KinSrcArgs* k,
+                                    const int* step, int off, int nst, cudaStream_t st) {
+  const int nj = f.j1 - f.j0 + 1, ni = f.i1 - f.i0 + 1;
+  if (nj <= 0 || ni <= 0 || !fstr_aligned(f)) return cudaErrorInvalidValue;
+  const dim3 grid(cdiv_u(nj, 128), ni + 1, 1);
+  if (s)
+    k_fstr_src<<<grid, 128, 0, st>>>(f, *s, step, off, nst);
+  else
+    k_fstr_kinsrc<<<grid, 128, 0, st>>>(f, *k, step, off);
   return cudaGetLastError();
 }
 
@@ -1202,57 +1204,15 @@ cudaError_t awp_launch_nonfinite(const float* p, long long n, unsigned int* flag
   return cudaGetLastError();
 }
 
-int awp_batch_blocks_per_sm(int ty, int* vel, int* str) {
-  cudaError_t e;
-  if (ty == 8) {
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(vel, k_batch_velocity<8>, 256, 0);
-    if (e == cudaSuccess)
-      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(str, k_batch_stress<false, 8>, 256, 0);
-  } else if (ty == 4) {
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(vel, k_batch_velocity<4>, 128, 0);
-    if (e == cudaSuccess)
-      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(str, k_batch_stress<false, 4>, 128, 0);
-  } else {
-    return 1;
-  }
-  return e == cudaSuccess ? 0 : 2;
-}
-
-template <int TY>
-static void launch_batch_halfsteps(const BatchLaunch& b, cudaStream_t st) {
-  const dim3 block(32, TY);
-  k_batch_velocity<TY><<<b.grid_vel, block, 0, st>>>(b.inst, b.vtiles, b.nvtiles, b.counters,
-                                                     b.ichunk);
-  if (b.nstiles > 0)
-    k_batch_stress<false, TY><<<b.grid_str, block, 0, st>>>(b.inst, b.stiles, b.nstiles,
-                                                            b.counters + 1, b.ichunk);
-  if (b.nstiles_el > 0)
-    k_batch_stress<true, TY><<<b.grid_str, block, 0, st>>>(b.inst, b.stiles_el, b.nstiles_el,
-                                                           b.counters + 2, b.ichunk);
-}
-
-cudaError_t awp_launch_batch_step(const BatchLaunch& b, cudaStream_t st) {
-  cudaError_t e = cudaMemsetAsync(b.counters, 0, 3 * sizeof(int), st);
-  if (e != cudaSuccess) return e;
-  if (b.ty == 8)
-    launch_batch_halfsteps<8>(b, st);
-  else
-    launch_batch_halfsteps<4>(b, st);
-  if (b.nsrc > 0)
-    k_batch_sources<<<cdiv_u(b.nsrc, 128), 128, 0, st>>>(b.inst, b.src_cells, b.nsrc, b.step);
-  k_batch_fstr<<<b.nrows > 0 ? b.nrows : 1, 128, 0, st>>>(b.inst, b.rows, b.nrows, b.step);
-  return cudaGetLastError();
-}
-
-cudaError_t awp_launch_sources_dev(const SrcArgs* a, const KinSrcArgs* k, const int* step,
+cudaError_t awp_launch_sources_dev(const SrcArgs* a, const KinSrcArgs* k, const int* step, int off,
                                    int nst, cudaStream_t st) {
   if (a && a->ncell > 0)
-    k_addsrc_dev<<<cdiv_u(a->ncell, 128), 128, 0, st>>>(*a, step, nst);
-  if (k && k->ncell > 0) k_addkinsrc_dev<<<cdiv_u(k->ncell, 128), 128, 0, st>>>(*k, step);
+    k_addsrc_dev<<<cdiv_u(a->ncell, 128), 128, 0, st>>>(*a, step, off, nst);
+  if (k && k->ncell > 0) k_addkinsrc_dev<<<cdiv_u(k->ncell, 128), 128, 0, st>>>(*k, step, off);
   return cudaGetLastError();
 }
 
-cudaError_t awp_launch_step_advance(int* step, cudaStream_t st) {
-  k_step_advance<<<1, 1, 0, st>>>(step);
+cudaError_t awp_launch_step_advance(int* step, int n, cudaStream_t st) {
+  k_step_advance<<<1, 1, 0, st>>>(step, n);
   return cudaGetLastError();
 }

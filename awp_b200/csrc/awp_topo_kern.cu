@@ -209,7 +209,7 @@ enum VelW { kAx = 0, kAy = 4, kBx = 8, kBy = 12, kCy = 16, kCx = 20, kS = 24, kN
 constexpr int kVelWPad = 40;
 
 struct TopoVelCfg {
-  static constexpr int LA = 1, NH = 1 + LA, DS = 3 + LA;
+  static constexpr int LA = 2, NH = 1 + LA, DS = 3 + LA;  // planes ahead, rings
   // one stage: xx(i+1), xz(i+2), yy, yz (j halo), zz, density, u, v, w (i)
   static constexpr int G_XX = 0, G_XZ = kOwn, G_YY = 2 * kOwn, G_YZ = G_YY + kHalo,
                        G_ZZ = G_YZ + kHalo, G_D = G_ZZ + kOwn, G_O = G_D + kMed,
@@ -304,7 +304,8 @@ __global__ void __launch_bounds__(kThreads, 2)
   const float2 g3c = gk2(a.g3_c, c.ld), g3 = gk2(a.g3, c.ld), gc = gk2(a.g_c, c.ld),
                gg = gk2(a.g, c.ld);
   const float2 ig3c = vquot(1.0f, g3c), ig3 = vquot(1.0f, g3);
-  const float2 dcz = vscale(__ldg(a.dcrjy + ja), gk2(a.dcrjz, c.ld));
+  const float dcy = __ldg(a.dcrjy + ja);
+  const float2 dcz = gk2(a.dcrjz, c.ld);
   // own-column values of the planes before the ones the tiles bring
   float2 xx_m2, xx_m1, xx_0, xy_m1, xy_0, xy_p1, xz_m1, xz_0, xz_p1, d_m, t_m;
   {
@@ -343,7 +344,7 @@ __global__ void __launch_bounds__(kThreads, 2)
     const float2 xx_p1 = lds2(G + C::G_XX + h0), xz_p2 = lds2(G + C::G_XZ + h0);
     const float2 xy_p2 = lds2(smem + ss2 * kHalo + h2);
     const float2 d_0 = lds2(G + C::G_D + h1), t_0 = vadd(d_0, lds2(G + C::G_D + h0));
-    const float2 dcrj = vscale(dcx, dcz);
+    const float2 dcrj = vscale(dcx * dcy, dcz);
 
     // --- u1 -----------------------------------------------------------------
     {
@@ -408,11 +409,12 @@ enum StrW { kIu = 0, kIv = 4, kJu = 8, kJv = 12, kKw = 16, kLw = 20, kF = 24, kS
 template <bool ELASTIC>
 struct TopoStrCfg {
   static constexpr int NM = ELASTIC ? 2 : 4, NF = ELASTIC ? 6 : 12;
-  static constexpr int LH = 1, LO = 1, NH = 1 + LH, NO = 1 + LO, DU = 3 + LH, DV = 2 + LH;
+  static constexpr int LH = 2, LO = 1, NH = 1 + LH, NO = 1 + LO, DU = 3 + LH, DV = 2 + LH;
   static constexpr int F_U = 0, F_V = F_U + DU * kHalo, F_W = F_V + DV * kHalo,
                        F_M = F_W + DV * kHalo, F_O = F_M + NH * NM * kMed,
                        F_T = F_O + NO * NF * kOwn, F_X = F_T + (ELASTIC ? 0 : 80),
-                       F_C = F_X + kCol * 2 * 32 * 2, F_END = F_C + 4 * 9 * 3 * 2;
+                       F_C = F_X + kCol * 2 * 32 * 2, F_G = F_C + 4 * 9 * 3 * 2,
+                       F_END = F_G + 6 * 64;  // vertical metrics of the lanes
   static constexpr size_t bytes = sizeof(float) * F_END + sizeof(Pipe<NH, NO, kCol>) + 8;
 };
 
@@ -443,6 +445,21 @@ __global__ void __launch_bounds__(kThreads, 2)
 #pragma unroll
     for (int q = 0; q < 9; ++q)
       if (tid < 8) t[(tid >> 1) * 20 + 2 * q + (tid & 1)] = src[q][tid];
+  }
+  // the vertical metrics depend on k alone: one copy for all the columns, read
+  // where they are used (held in registers they spilled)
+  enum { kGc, kGg, kIg3c, kIg3, kIg12, kDcz };
+  float2* const vm = reinterpret_cast<float2*>(smem + C::F_G);
+  if (warp == 0) {
+    vm[32 * kGc + c.lane] = gk2(a.g_c, c.ld);
+    vm[32 * kGg + c.lane] = gk2(a.g, c.ld);
+    vm[32 * kIg3c + c.lane] = vquot(1.0f, gk2(a.g3_c, c.ld));
+    vm[32 * kIg3 + c.lane] = vquot(1.0f, gk2(a.g3, c.ld));
+    // the xy Jacobian's interior rows read g3_c six points higher
+    // (stress_attenuation.cu:471), the boundary rows at k (:1149)
+    vm[32 * kIg12 + c.lane] =
+        vquot(1.0f, gk2(a.g3_c, c.top && c.lane >= 29 ? c.ld : c.ld + 6));
+    vm[32 * kDcz + c.lane] = gk2(a.dcrjz, c.ld);
   }
   __syncthreads();
 
@@ -507,13 +524,8 @@ __global__ void __launch_bounds__(kThreads, 2)
   }
   float nw = wt.at(0);
 
-  const float2 ig3c = vquot(1.0f, gk2(a.g3_c, c.ld)), ig3 = vquot(1.0f, gk2(a.g3, c.ld));
-  // the xy Jacobian's interior rows read g3_c six points higher
-  // (stress_attenuation.cu:471), the boundary rows at k (:1149)
-  const bool bnd = c.top && c.lane >= 29;
-  const float2 ig12 = vquot(1.0f, gk2(a.g3_c, bnd ? c.ld : c.ld + 6));
-  const float2 gc = gk2(a.g_c, c.ld), gg = gk2(a.g, c.ld);
-  const float2 dcz = vscale(__ldg(a.dcrjy + ja), gk2(a.dcrjz, c.ld));
+  auto G = [&](int q) { return vm[32 * q + c.lane]; };
+  const float dcy = __ldg(a.dcrjy + ja);
   // texture entry pairs at even and odd steps (two adjacent levels starting at
   // an even one: entries e, e + 1)
   const int e0 = awp_tex_index(a.tex, ib, ja, c.k + AWP_ALIGN) >> 1,
@@ -527,7 +539,7 @@ __global__ void __launch_bounds__(kThreads, 2)
   }
   // media sums of the current plane: over j, j-1 and the level below
   auto quad = [&](float2 t) { return awp_quad(t, below(t)); };
-  float2 Lq, Mq, Mt, Mm, Mk, Pq = {}, Rq = {}, Rt = {}, Rm = {}, Rk = {};
+  float2 Lq, Mq, Mt, Mm, Pq = {}, Rq = {}, Rt = {}, Rm = {};
   {
     auto rows = [&](const float* p, float2& m) {
       m = ldg2(p);
@@ -537,12 +549,10 @@ __global__ void __launch_bounds__(kThreads, 2)
     Lq = quad(rows(a.lam + o, m));
     Mt = rows(a.mu + o, Mm);
     Mq = quad(Mt);
-    Mk = vadd(Mm, below(Mm));
     if (!ELASTIC) {
       Pq = quad(rows(a.qp + o, m));
       Rt = rows(a.qs + o, Rm);
       Rq = quad(Rt);
-      Rk = vadd(Rm, below(Rm));
     }
   }
   const int l = 2 * c.lane;
@@ -575,7 +585,7 @@ __global__ void __launch_bounds__(kThreads, 2)
     float2 d[9];
     {
       // normal components: Jii = 1 / (f_c g3_c) (stress_attenuation.cu:340-431)
-      const float2 J = vmul(W[kF], ig3c), Jg = vmul(J, gc);
+      const float2 J = vmul(W[kF], G(kIg3c)), Jg = vmul(J, G(kGc));
       const float2 v2 = lds2(V0 - 2 * kSpan), v1 = lds2(V0 - kSpan), vp = lds2(V0 + kSpan);
       d[0] = vsub(diff4(u_m1, u_0, u_p1, u_p2),
                   vmul(Jg, zd7(dot4(W + kIu, u_m1, u_0, u_p1, u_p2), c, cl[0])));
@@ -584,7 +594,7 @@ __global__ void __launch_bounds__(kThreads, 2)
     }
     {
       // xy: J12i = 1 / (f g3_c)
-      const float2 J = vmul(vmul(W[kF + 1], ig12), gc);
+      const float2 J = vmul(vmul(W[kF + 1], G(kIg12)), G(kGc));
       const float2 um = lds2(U0 - kSpan), u1 = lds2(U0 + kSpan), u2 = lds2(U0 + 2 * kSpan);
       const float2 q = dot4(W + kJv, v_m2, v_m1, v_0, v_p1, dot4(W + kJu, um, u_0, u1, u2));
       d[3] = diff4(um, u_0, u1, u2);
@@ -592,17 +602,17 @@ __global__ void __launch_bounds__(kThreads, 2)
     }
     {
       // xz: J13i = 1 / (f_1 g3) (:550-598, :1254-1317)
-      const float2 J = vmul(W[kF + 2], ig3);
+      const float2 J = vmul(W[kF + 2], G(kIg3));
       const float2 z = zd7(dot4(W + kKw, w_m2, w_m1, w_0, w_p1), c, cl[1]);
-      d[5] = vmul(J, vsub(zd4<false, 7>(u_0, c, cl[3]), vmul(gg, z)));
+      d[5] = vmul(J, vsub(zd4<false, 7>(u_0, c, cl[3]), vmul(G(kGg), z)));
       d[6] = diff4(w_m2, w_m1, w_0, w_p1);
     }
     {
       // yz: J23i = 1 / (f_2 g3) (:600-650, :1319-1380)
-      const float2 J = vmul(W[kF + 3], ig3);
+      const float2 J = vmul(W[kF + 3], G(kIg3));
       const float2 wm = lds2(W0 - kSpan), w1 = lds2(W0 + kSpan), w2 = lds2(W0 + 2 * kSpan);
       const float2 z = zd7(dot4(W + kLw, wm, w_0, w1, w2), c, cl[1]);
-      d[7] = vmul(J, vsub(zd4<false, 7>(v_0, c, cl[3]), vmul(gg, z)));
+      d[7] = vmul(J, vsub(zd4<false, 7>(v_0, c, cl[3]), vmul(G(kGg), z)));
       d[8] = diff4(wm, w_0, w1, w2);
     }
 
@@ -627,23 +637,23 @@ __global__ void __launch_bounds__(kThreads, 2)
       };
       float2 m, mm;
       const float2 Ln = quad(rows(0, m)), mt = rows(1, mm), mq = quad(mt);
-      const float2 P[3] = {Mk, Mt, vadd(Mm, mm)};
+      const float2 P[3] = {vadd(Mm, below(Mm)), Mt, vadd(Mm, mm)};
       float2 QP8 = zero, QS8 = zero, R[3] = {zero, zero, zero};
       if (!ELASTIC) {
         float2 rm;
         const float2 pq = quad(rows(2, m)), rt = rows(3, rm), rq = quad(rt);
         QP8 = vadd(Pq, pq);
         QS8 = vadd(Rq, rq);
-        R[0] = Rk; R[1] = Rt; R[2] = vadd(Rm, rm);
+        R[0] = vadd(Rm, below(Rm)); R[1] = Rt; R[2] = vadd(Rm, rm);
         Pq = pq;
-        Rq = rq; Rt = rt; Rm = rm; Rk = vadd(rm, below(rm));
+        Rq = rq; Rt = rt; Rm = rm;
       }
       cf = awp_stress_coef<ELASTIC>(vadd(Lq, Ln), vadd(Mq, mq), P, QP8, QS8, R, rx, a.thr, a.dth,
                                     a.DT);
       Lq = Ln;
-      Mq = mq; Mt = mt; Mm = mm; Mk = vadd(mm, below(mm));
+      Mq = mq; Mt = mt; Mm = mm;
     }
-    const float2 dcrj = vscale(dcx, dcz);
+    const float2 dcrj = vscale(dcx * dcy, G(kDcz));
     ok = mbar_wait(pipe.full_o + co.slot, co.phase, spin);
     if (!__all_sync(kAll, ok)) break;
     const float* O = smem + C::F_O + co.slot * NF * kOwn + h0;

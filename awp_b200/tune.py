@@ -107,7 +107,8 @@ def autotune_batch(batch, steps: int = 3, timer=None) -> dict:
     batch.set_mode(0)
     for ty, ich in itertools.product(*BATCH_CANDIDATES.values()):
         batch.set_shape(ty, ich)
-        batch.step(1)  # build the tile lists and the graph
+        batch.step(steps)  # build the tile lists or the graphs
+        batch.step(steps)
         batch.synchronize()
         ms = timer(lambda: batch.step(steps))
         table.append({"mode": 0, "ty": ty, "ichunk": ich, "ms_per_step": ms / steps})
@@ -123,7 +124,7 @@ def autotune_batch(batch, steps: int = 3, timer=None) -> dict:
         set_tuning(lib, "ichunk", ich)
         batch.set_mode(0)
         batch.set_mode(1)  # recapture
-        batch.step(1)
+        batch.step(steps)
         batch.synchronize()
         ms = timer(lambda: batch.step(steps))
         table.append({"mode": 1, "ty": None, "ichunk": ich, "tma_vel": tv,
@@ -135,7 +136,7 @@ def autotune_batch(batch, steps: int = 3, timer=None) -> dict:
         best["branches"] = 0
         for nb in (32, 16, 8):  # fewer, longer branches
             batch.set_branches(nb)
-            batch.step(1)
+            batch.step(steps)
             batch.synchronize()
             ms = timer(lambda: batch.step(steps))
             row = {"mode": 1, "ty": None, "ichunk": best["ichunk"], "tma_vel": best["tma_vel"],

@@ -313,31 +313,31 @@ typedef struct awp_batch awp_batch;
  * pointers to them; destroy the batch before its contexts. */
 int awp_batch_create(awp_ctx* const* ctxs, int n, awp_batch** out);
 int awp_batch_destroy(awp_batch* batch);
-/* Advance every instance nsteps, each step one persistent launch per
- * half-step over a tile queue of all instances (CTAs pull 32 k x ty j x ichunk
- * i tiles from a global counter), then the sources and free-surface images of
- * all instances; the step is one CUDA graph replayed nsteps times.  Each
- * instance's arithmetic is that of awp_step, bit for bit.  Ordered after
- * earlier work on the contexts' streams and before later work on them. */
+/* Advance every instance nsteps: parallel branches of each instance's own
+ * launches (velocity, stress, sources at the device-held step, free-surface
+ * images), replayed as CUDA graphs of up to eight steps in which an instance
+ * runs on into its next step without waiting for the others; a batch's first
+ * few steps are enqueued directly.  Each instance's arithmetic is that of
+ * awp_step, bit for bit.  Ordered after earlier work on the contexts' streams
+ * and before later work on them. */
 int awp_batch_step(awp_batch* batch, int nsteps);
 int awp_batch_synchronize(awp_batch* batch);
-/* Tile shape (ty = 4 or 8 j rows, ichunk x planes per tile; default 8, 16)
- * and graph replay (1, default) or direct launches (0). */
+/* Tile shape the counts of awp_batch_info refer to (ty = 4 or 8 j rows, ichunk
+ * x planes per tile; default 8, 16), and graph replay (1, default) or, in mode
+ * 0, direct launches (0). */
 int awp_batch_set_shape(awp_batch* batch, int ty, int ichunk);
 int awp_batch_get_shape(const awp_batch* batch, int* ty, int* ichunk);
 int awp_batch_set_graph(awp_batch* batch, int use_graph);
-/* Execution mode: 0 (default) the persistent tile-queue launches above;
- * 1 one graph per step whose parallel branches are each instance's own tuned
- * launches (velocity, stress, sources at the device-held step, free-surface
- * images), the step counter advanced after the join.  Same results. */
+/* Execution mode: 0 (default) graphs or direct launches as awp_batch_set_graph
+ * says; 1 graphs whatever it says.  Same results. */
 int awp_batch_set_mode(awp_batch* batch, int mode);
 int awp_batch_get_mode(const awp_batch* batch);
-/* Mode 1: the instances' launches are dealt, largest first, round-robin onto
+/* The instances' launches are dealt, largest first, round-robin onto
  * `branches` parallel graph branches (0, the default: one branch per
  * instance). */
 int awp_batch_set_branches(awp_batch* batch, int branches);
-/* info = instances, interior cells, velocity tiles, stress tiles, persistent
- * CTAs of the velocity and stress launches. */
+/* info = instances, interior cells, velocity tiles, stress tiles, and the two
+ * tile counts again (the batch launches no persistent CTAs). */
 int awp_batch_info(awp_batch* batch, long long info[6]);
 
 /* ------------------------------------------------------------------------ */
