@@ -30,6 +30,7 @@
 //   fstr      zz(top+1) = -zz(top), ..., xz(top) = yz(top) = 0  (kernel.cu:1616-1647)
 #include "awp_adjoint.cuh"
 
+#include "awp_pipe.cuh"
 #include "awp_stencil.cuh"
 
 namespace {
@@ -37,253 +38,310 @@ namespace {
 enum { LU, LV, LW, LXX, LYY, LZZ, LXY, LXZ, LYZ, LR1, LR2, LR3, LR4, LR5, LR6 };
 enum { E1, E2, E3, E4, E5, E6, GL8, GM8, GP1, GP2, GP3, GQP8, GQS8, GQ1, GQ2, GQ3 };
 
-// d(weight)/dq of the Q(f) weight awp_qf_weight(q, ...): the polynomial
-// c0 (2q)^2 + c1 (2q) over wwo on the low-Q branch, 2 q otherwise (the branch
-// held fixed, as the forward takes it at q)
-__device__ __forceinline__ float qf_dweight(float q, float wwo, float c0, float c1,
-                                            float qthr) {
-  const float x = 2.0f * q;
-  const bool low = (x >= qthr) || (x < 0.f) || (x == 0.f && signbit(x));
-  return low ? (8.0f * c0 * q + 2.0f * c1) / wwo : 2.0f;
-}
 enum { VA, VB, VC, VEA, VEB, VEC };
 
-// Per-thread asynchronous 4-byte copy global -> shared (cp.async); a thread
-// reads back only its own slots, after cp.async.wait_all.
-__device__ __forceinline__ void cpa4(float* s, const float* g) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(
+// Two vertically adjacent cells per thread (the pair starts on an even level,
+// so every access is 8-byte aligned), computed with packed arithmetic.
+__device__ __forceinline__ float2 ld2(const float* p) {
+  return *reinterpret_cast<const float2*>(p);
+}
+__device__ __forceinline__ void st2(float* p, float2 v) { *reinterpret_cast<float2*>(p) = v; }
+__device__ __forceinline__ void st2(float* p, float2 v, bool ax, bool ay) {
+  if (ax && ay) {
+    st2(p, v);
+  } else {
+    if (ax) p[0] = v.x;
+    if (ay) p[1] = v.y;
+  }
+}
+// Per-thread asynchronous 8-byte copy global -> shared (cp.async); a thread
+// reads back only its own slots, after waiting for its group.
+__device__ __forceinline__ void cpa8(float2* s, const float* g) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(
                    (unsigned)__cvta_generic_to_shared(s)),
                "l"(g)
                : "memory");
 }
-__device__ __forceinline__ void cpa_wait() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
+__device__ __forceinline__ void cpa_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cpa_wait() {
+  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
+}
 
-#ifndef AWP_ADJ_STAGE
-#define AWP_ADJ_STAGE 1  // stage the stress transpose's once-read values
-#endif
-#ifndef AWP_ADJ_MINB
-#define AWP_ADJ_MINB 7  // CTAs per SM the stress transpose's registers allow
-#endif
+__device__ __forceinline__ void pre2(const float* p) {
+  asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p));
+}
+
+// Derivative of awp_weight (awp_stencil.cuh) with respect to S, the branch held
+// as the forward takes it.
+__device__ __forceinline__ float2 dweight(float2 S, const AwpRelax<float2>& t, unsigned thr) {
+  const float2 p = vfma(vadd(t.c0, t.c0), S, t.c1);
+  return make_float2(__float_as_uint(S.x) >= thr ? p.x : t.c2.x,
+                     __float_as_uint(S.y) >= thr ? p.y : t.c2.y);
+}
 
 // ---------------------------------------------------------------------------
 // stress^T, pointwise part: memory variables and stresses in place, adjoint
 // strain rates of the cell into E[], its material weights added to the sums
-// in E[].  Seven 128-thread CTAs per SM (72 registers) run it faster than
-// four without spills: the kernel waits on HBM latency.  The values it reads
-// once and late (the cell's adjoint stresses, memory variables and weight
-// sums) are copied to shared memory by cp.async when a thread starts, which
-// takes them out of the registers (840 against 860 ms for a 600-step
-// gradient at 256 x 256 x 128).
+// in E[].  188 bytes a cell.  A thread marches kSch x planes with the forward
+// update's coefficients and register queues for the velocities and media; the
+// cell's own adjoint stresses, memory variables and weight sums (read once and
+// late) come one plane ahead by cp.async, so a plane's copies are in flight
+// while the one before is computed; the next plane's first velocities and media
+// are called into L2 at the same time.  At its traffic (160 x 144 x 96 with Q
+// sums: 110 us); marches of 8 or 16 planes and four CTAs an SM are 5-12 %
+// slower, and without the L2 prefetch a whole gradient is 4 % slower.
 // ---------------------------------------------------------------------------
+constexpr int kSch = 4;
+
 // WANTQ: also accumulate the Q^-1 weights (anelastic runs that ask for the
 // Q^-1 gradients); without it the five Q sums are neither read nor written.
 template <bool ELASTIC, bool WANTQ>
-__global__ void __launch_bounds__(128, AWP_ADJ_MINB) k_adj_stress_cell(const AdjArgs a) {
-  // the cell's own adjoint stresses and memory variables and its weight sums,
-  // read once and late: copied to shared memory when the thread starts
-  // (slots 0-5 stresses, 6-11 memory variables, 12-16 moduli sums, 17-21 Q sums)
-  __shared__ float stg[AWP_ADJ_STAGE ? 22 : 1][128];
-  const int tid = threadIdx.y * 32 + threadIdx.x;
-  // the relaxation tables in shared memory: the lanes of a warp alternate the
-  // table entry with the parity of k, which a constant-bank read would serve
-  // in two passes
-  __shared__ float tab[40];  // tau1[8], tau2[8], wwo8[8], coeff[16]
-  {
-    if (tid < 8) {
-      tab[tid] = a.tex.tau1[tid];
-      tab[8 + tid] = a.tex.tau2[tid];
-      tab[16 + tid] = a.tex.wwo8[tid];
-    }
-    if (!ELASTIC && tid < 16) tab[24 + tid] = a.coeff[tid];
+__global__ void __launch_bounds__(128, 3) k_adj_stress_cell(const __grid_constant__ AdjArgs a) {
+  // staged, two planes: 0-5 stresses, 6-10 moduli sums, 11-16 memory
+  // variables, 17-21 Q sums
+  constexpr int NS = ELASTIC ? 11 : WANTQ ? 22 : 17;
+  __shared__ float2 stg[2][NS][128];
+  // relaxation constants of the entry pairs (e, e + 1), e even: nine float2
+  // per pair in 20 floats (as k_stress_tma)
+  __shared__ __align__(16) float tab[4 * 20];
+  const int tid = threadIdx.x;
+  awp_pipe::grid_go();
+  if (!ELASTIC) {
+    const float* const src[9] = {a.rel.vx2, a.rel.wwo, a.rel.kv, a.rel.kr, a.rel.kr2,
+                                 a.rel.kf,  a.rel.c0,  a.rel.c1, a.rel.c2};
+#pragma unroll
+    for (int q = 0; q < 9; ++q)
+      if (tid < 8) tab[(tid >> 1) * 20 + 2 * q + (tid & 1)] = src[q][tid];
     __syncthreads();
   }
-  const int k = a.sk0 + blockIdx.x * 32 + threadIdx.x;
-  const int j = a.sj0 + blockIdx.y * 4 + threadIdx.y;
-  const int i = a.si0 + blockIdx.z;
-  if (k > a.sk1 || j > a.sj1 || i > a.si1) return;
-  // stencil neighbours as 32-bit offsets from per-array pointers at the cell
+  awp_pipe::grid_wait();
+  // flat (j, level pair): pairs of levels from the even one at or below sk0
+  const int kp0 = a.sk0 & ~1, np = (a.sk1 - kp0) / 2 + 1;
+  const int idx = blockIdx.x * 128 + tid;
+  const int j = a.sj0 + idx / np, k = kp0 + 2 * (idx % np);
+  const int ib = a.si0 + blockIdx.y * kSch, ie = min(ib + kSch - 1, a.si1);
+  if (j > a.sj1) return;
+  const bool ax = k >= a.sk0, ay = k + 1 <= a.sk1;
   const int S = a.g.slice, Y = a.g.yline;
-  const long long p = (long long)i * S + (long long)j * Y + k;
-  const float c1 = a.c1, c2 = a.c2, DT = a.dt;
-  if (AWP_ADJ_STAGE) {
+  const int VS = (int)a.vb.S, VY = (int)a.vb.Y;
+  const float c1 = a.c1, c2 = a.c2;
+  long long p = (long long)ib * S + (long long)j * Y + k;
+  long long pv = (long long)ib * a.vb.S + (long long)j * a.vb.Y + k - a.vb.off;
+  auto stage = [&](int b, long long o) {
 #pragma unroll
-    for (int q = 0; q < 6; ++q) cpa4(&stg[q][tid], a.L[LXX + q] + p);
+    for (int q = 0; q < 6; ++q) cpa8(&stg[b][q][tid], a.L[LXX + q] + o);
+#pragma unroll
+    for (int q = 0; q < 5; ++q) cpa8(&stg[b][6 + q][tid], a.E[GL8 + q] + o);
     if (!ELASTIC) {
 #pragma unroll
-      for (int q = 0; q < 6; ++q) cpa4(&stg[6 + q][tid], a.L[LR1 + q] + p);
+      for (int q = 0; q < 6; ++q) cpa8(&stg[b][11 + q][tid], a.L[LR1 + q] + o);
     }
-#pragma unroll
-    for (int q = 0; q < 5; ++q) cpa4(&stg[12 + q][tid], a.E[GL8 + q] + p);
     if (!ELASTIC && WANTQ) {
 #pragma unroll
-      for (int q = 0; q < 5; ++q) cpa4(&stg[17 + q][tid], a.E[GQP8 + q] + p);
+      for (int q = 0; q < 5; ++q) cpa8(&stg[b][17 + q][tid], a.E[GQP8 + q] + o);
     }
-  }
-  // the cell's value of a staged array
-  auto own = [&](int slot, const float* f) { return AWP_ADJ_STAGE ? stg[slot][tid] : f[p]; };
-
-  // forward strain rates from the velocities after the step (VelBox layout)
-  const int VS = (int)a.vb.S, VY = (int)a.vb.Y;
-  const long long pv = (long long)i * a.vb.S + (long long)j * a.vb.Y + k - a.vb.off;
-  const float* u = a.fu + pv;
-  const float* v = a.fv + pv;
-  const float* w = a.fw + pv;
-  const float vs1 = c1 * (u[VS] - u[0]) + c2 * (u[2 * VS] - u[-VS]);
-  const float vs2 = c1 * (v[0] - v[-VY]) + c2 * (v[VY] - v[-(2 * VY)]);
-  const float vs3 = c1 * (w[0] - w[-1]) + c2 * (w[1] - w[-2]);
-  const float e4 = c1 * (u[VY] - u[0]) + c2 * (u[2 * VY] - u[-VY]) +
-                   c1 * (v[0] - v[-VS]) + c2 * (v[VS] - v[-(2 * VS)]);
-  const float e5 = c1 * (u[1] - u[0]) + c2 * (u[2] - u[-1]) +
-                   c1 * (w[0] - w[-VS]) + c2 * (w[VS] - w[-(2 * VS)]);
-  const float e6 = c1 * (v[1] - v[0]) + c2 * (v[2] - v[-1]) +
-                   c1 * (w[VY] - w[0]) + c2 * (w[2 * VY] - w[-VY]);
-
-  // materials of the cell (kernel.cu:962-1070)
-  auto sum8 = [&](const float* m0) {
-    const float* m = m0 + p;
-    return m[0] + m[S] + m[-Y] + m[S - Y] + m[-1] + m[S - 1] + m[-Y - 1] + m[S - Y - 1];
+    cpa_commit();
   };
-  const float* mu = a.mu + p;
-  const float L8 = sum8(a.lam), M8 = sum8(a.mu);
-  const float P1 = mu[0] + mu[-1], P2 = mu[0] + mu[-Y], P3 = mu[0] + mu[S];
-  const float xm_raw = 16.0f / M8;
-  const float xl_raw = 8.0f / L8 + xm_raw;
-  const float m1_raw = 2.0f / P1, m2_raw = 2.0f / P2, m3_raw = 2.0f / P3;
-  const int t = awp_tex_index(a.tex, i, j, k);
-  const float fvx1 = tab[t], fvx2 = tab[8 + t], wwo = tab[16 + t];
-  float c_xm = a.dth, c_h = 0.f, c_q = 0.f, c_m[3] = {a.dth, a.dth, a.dth}, c_hh[3] = {0, 0, 0};
-  // derivatives of the Q weights with respect to their averaged arguments
-  float dqpaw = 0.f, dhw = 0.f, dhiw[3] = {0.f, 0.f, 0.f};
-  if (!ELASTIC) {
-    const float cc0 = tab[24 + 2 * t], cc1 = tab[25 + 2 * t];
-    const float qs8 = 0.0625f * sum8(a.qs), qp8 = 0.0625f * sum8(a.qp);
-    const float hw = awp_qf_weight(qs8, wwo, cc0, cc1, a.qthr);
-    const float qpaw = awp_qf_weight(qp8, wwo, cc0, cc1, a.qthr);
-    const float* qs = a.qs + p;
-    const float qsp[3] = {0.25f * (qs[0] + qs[-1]), 0.25f * (qs[0] + qs[-Y]),
-                          0.25f * (qs[0] + qs[S])};
-    const float hiw[3] = {awp_qf_weight(qsp[0], wwo, cc0, cc1, a.qthr),
-                          awp_qf_weight(qsp[1], wwo, cc0, cc1, a.qthr),
-                          awp_qf_weight(qsp[2], wwo, cc0, cc1, a.qthr)};
-    dhw = qf_dweight(qs8, wwo, cc0, cc1, a.qthr);
-    dqpaw = qf_dweight(qp8, wwo, cc0, cc1, a.qthr);
-    for (int q = 0; q < 3; ++q) dhiw[q] = qf_dweight(qsp[q], wwo, cc0, cc1, a.qthr);
-    c_h = -hw * a.dh1 * fvx1;
-    c_xm = a.dth + DT * c_h;
-    c_q = -qpaw * a.dh1 * fvx1;
-    for (int q = 0; q < 3; ++q) {
-      c_hh[q] = -hiw[q] * a.dh1 * fvx1;
-      c_m[q] = a.dth + DT * c_hh[q];
-    }
+  stage(0, p);
+  float2 u_m1, u_0, u_p1, v_m2, v_m1, v_0, w_m2, w_m1, w_0;
+  {
+    const float *u = a.fu + pv, *v = a.fv + pv, *w = a.fw + pv;
+    u_m1 = ld2(u - VS); u_0 = ld2(u); u_p1 = ld2(u + VS);
+    v_m2 = ld2(v - 2 * VS); v_m1 = ld2(v - VS); v_0 = ld2(v);
+    w_m2 = ld2(w - 2 * VS); w_m1 = ld2(w - VS); w_0 = ld2(w);
   }
-  const float xm = xm_raw * c_xm, h = xm_raw * c_h, xl = xl_raw * a.dth, qpa = xl_raw * c_q;
-  const float xmu[3] = {m1_raw * c_m[0], m2_raw * c_m[1], m3_raw * c_m[2]};
-  const float hh[3] = {m1_raw * c_hh[0], m2_raw * c_hh[1], m3_raw * c_hh[2]};
-  const float K = a.dcrjx[i] * a.dcrjy[j] * a.dcrjz[k];
-  const float al = DT * (1.0f + fvx2 * fvx1);   // coefficient of r in sigma
-  const float be = fvx2, ga = fvx2 * (1.0f - fvx1);
-
-  // fstr^T of this column's top three cells (the imaged values above the
-  // surface are cleared later, in k_adj_vel_cell): zz(t) += -zz(t+1),
-  // zz(t-1) += -zz(t+2), xz/yz(t-1) += -xz/yz(t+1), xz/yz(t-2) += -xz/yz(t+2),
-  // xz/yz(t) after the imaging is zero
+  // a media field in one plane (as k_stress_tma)
+  struct Mat {
+    float2 m, t, q, pk;
+  };
+  auto mat = [&](const float* f) {
+    Mat r;
+    r.m = ld2(f);
+    const float mk = f[-1];
+    r.t = vadd(r.m, ld2(f - Y));
+    r.q = awp_quad(r.t, make_float2(vadd(mk, f[-Y - 1]), r.t.x));
+    r.pk = vadd(r.m, make_float2(mk, r.m.x));
+    return r;
+  };
+  const float2 zero = make_float2(0.f, 0.f);
+  float2 Lq = mat(a.lam + p).q, Pq = zero;
+  Mat mc = mat(a.mu + p), rc{zero, zero, zero, zero};
+  if (!ELASTIC) {
+    Pq = mat(a.qp + p).q;
+    rc = mat(a.qs + p);
+  }
+  const float dcy = a.dcrjy[j];
+  const float2 dcz = make_float2(a.dcrjz[k], a.dcrjz[k + 1]);
   const int top = a.g.top();
-  auto fs = [&](int f) -> float {  // adjoint of the field after the stress update
-    const float* Lf = a.L[f];
-    float v = own(f - LXX, Lf);
-    if (k == top) {
-      if (f == LZZ) v -= Lf[p + 1];
-      if (f == LXZ || f == LYZ) v = 0.f;
-    } else if (k == top - 1) {
-      if (f == LZZ) v -= Lf[p + 3];
-      if (f == LXZ || f == LYZ) v -= Lf[p + 2];
-    } else if (k == top - 2) {
-      if (f == LXZ || f == LYZ) v -= Lf[p + 4];
+  const bool tp = k + 1 == top, tp2 = k + 3 == top;  // the pair at the surface, the one below
+#pragma unroll 1
+  for (int i = ib; i <= ie; ++i) {
+    const int buf = (i - ib) & 1;
+    if (i < ie) {
+      stage(buf ^ 1, p + S);
+      // and the next plane's first reads of the velocities and media on their
+      // way into L2
+      pre2(a.fu + pv + 3 * VS);
+      pre2(a.fv + pv + 2 * VS);
+      pre2(a.fw + pv + 2 * VS);
+      pre2(a.lam + p + 2 * S);
+      pre2(a.mu + p + 2 * S);
+      if (!ELASTIC) {
+        pre2(a.qp + p + 2 * S);
+        pre2(a.qs + p + 2 * S);
+      }
     }
-    return v;
-  };
-  // every load of the adjoint state before the first store: the stores below
-  // go to other arrays (or other cells of the same array), and issuing the
-  // loads together keeps them from waiting on one another
-  if (AWP_ADJ_STAGE) cpa_wait();
-  const float lx = own(0, a.L[LXX]), ly = own(1, a.L[LYY]), lz = fs(LZZ);
-  const float ls[3] = {fs(LXY), fs(LXZ), fs(LYZ)};
-  float rv[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  if (!ELASTIC)
-    for (int q = 0; q < 6; ++q) rv[q] = own(6 + q, a.L[LR1 + q]);
-  // material weights, summed over the time steps (their spatial transposes
-  // are linear and time-invariant, so k_adj_material applies them once)
-  float wacc[5], qacc[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
-  for (int q = 0; q < 5; ++q) wacc[q] = own(12 + q, a.E[GL8 + q]);
-  if (!ELASTIC && WANTQ)
-    for (int q = 0; q < 5; ++q) qacc[q] = own(17 + q, a.E[GQP8 + q]);
-  // normal components
-  float PX, PY, PZ, QX = 0.f, QY = 0.f, QZ = 0.f;
-  PX = K * lx;
-  PY = K * K * ly;
-  PZ = K * K * lz;
-  if (!ELASTIC) {
-    QX = DT * (wwo - 1.0f) * K * lx + wwo * rv[0];
-    QY = DT * (wwo - 1.0f) * K * ly + wwo * rv[1];
-    QZ = DT * (wwo - 1.0f) * K * lz + wwo * rv[2];
-  }
-  const float sP = PX + PY + PZ, sQ = QX + QY + QZ;
-  const float A = xl + DT * qpa;
-  const float s123 = vs1 + vs2 + vs3;
-  const float G_xl = s123 * sP;
-  const float G_qpa = DT * s123 * sP + s123 * sQ;
-  const float G_xm = -((vs2 + vs3) * PX + (vs1 + vs3) * PY + (vs1 + vs2) * PZ);
-  const float G_h = -((vs2 + vs3) * QX + (vs1 + vs3) * QY + (vs1 + vs2) * QZ);
+    // ---- forward strain rates from the velocities after the step ------------
+    const float *u = a.fu + pv, *v = a.fv + pv, *w = a.fw + pv;
+    const float2 u_p2 = ld2(u + 2 * VS), v_p1 = ld2(v + VS), w_p1 = ld2(w + VS);
+    float2 vs1, vs2, vs3, es[3];
+    vs1 = awp_d4(c1, c2, u_p1, u_0, u_p2, u_m1);
+    vs2 = awp_d4(c1, c2, v_0, ld2(v - VY), ld2(v + VY), ld2(v - 2 * VY));
+    es[0] = vadd(awp_d4(c1, c2, ld2(u + VY), u_0, ld2(u + 2 * VY), ld2(u - VY)),
+                 awp_d4(c1, c2, v_0, v_m1, v_p1, v_m2));
+    {
+      const float2 wa = ld2(w - 2), ua = ld2(u + 2), va = ld2(v + 2);
+      vs3 = awp_d4(c1, c2, w_0, make_float2(wa.y, w_0.x), make_float2(w_0.y, w[2]), wa);
+      es[1] = vadd(awp_d4(c1, c2, make_float2(u_0.y, ua.x), u_0, ua, make_float2(u[-1], u_0.x)),
+                   awp_d4(c1, c2, w_0, w_m1, w_p1, w_m2));
+      es[2] = vadd(awp_d4(c1, c2, make_float2(v_0.y, va.x), v_0, va, make_float2(v[-1], v_0.x)),
+                   awp_d4(c1, c2, ld2(w + VY), w_0, ld2(w + 2 * VY), ld2(w - VY)));
+    }
+    // ---- materials of the cell (kernel.cu:962-1070) -------------------------
+    const float2 Ln = mat(a.lam + p + S).q;
+    const Mat mn = mat(a.mu + p + S);
+    const float2 lr = vquot(8.0f, vadd(Lq, Ln)), xm_raw = vquot(16.0f, vadd(mc.q, mn.q));
+    const float2 xl_raw = vadd(lr, xm_raw);
+    const float2 P[3] = {mc.pk, mc.t, vadd(mc.m, mn.m)};
+    const float2 dthv = vset<float2>(a.dth), DT = vset<float2>(a.dt);
+    AwpRelax<float2> t{};
+    float2 c_h = zero, c_q = zero, c_hh[3] = {zero, zero, zero};
+    float2 dqw = zero, dhw = zero, dhh[3] = {zero, zero, zero};
+    if (!ELASTIC) {
+      const float* e = tab + (awp_tex_index(a.tex, i, j, k) >> 1) * 20;
+      const float4* e4 = reinterpret_cast<const float4*>(e);
+      const float4 q0 = e4[0], q1 = e4[1], q2 = e4[2], q3 = e4[3];
+      t.vx2 = make_float2(q0.x, q0.y); t.wwo = make_float2(q0.z, q0.w);
+      t.kv = make_float2(q1.x, q1.y); t.kr = make_float2(q1.z, q1.w);
+      t.kr2 = make_float2(q2.x, q2.y); t.kf = make_float2(q2.z, q2.w);
+      t.c0 = make_float2(q3.x, q3.y); t.c1 = make_float2(q3.z, q3.w);
+      t.c2 = make_float2(e[16], e[17]);
+      const float2 pn = mat(a.qp + p + S).q;
+      const Mat rn = mat(a.qs + p + S);
+      const float2 qs8 = vscale(0.25f, vadd(rc.q, rn.q)), qp8 = vscale(0.25f, vadd(Pq, pn));
+      const float2 R[3] = {rc.pk, rc.t, vadd(rc.m, rn.m)};
+      c_h = awp_weight(qs8, t.c0, t.c1, t.c2, a.thr);
+      c_q = awp_weight(qp8, t.c0, t.c1, t.c2, a.thr);
+#pragma unroll
+      for (int q = 0; q < 3; ++q) c_hh[q] = awp_weight(R[q], t.c0, t.c1, t.c2, a.thr);
+      if (WANTQ) {
+        dhw = vscale(0.25f, dweight(qs8, t, a.thr));
+        dqw = vscale(0.25f, dweight(qp8, t, a.thr));
+#pragma unroll
+        for (int q = 0; q < 3; ++q) dhh[q] = dweight(R[q], t, a.thr);
+      }
+      Pq = pn;
+      rc = rn;
+    }
+    Lq = Ln;
+    mc = mn;
+    const float2 c_xm = vfma(DT, c_h, dthv);
+    const float2 nxm = vmul(vscale(-1.0f, xm_raw), c_xm), nh = vmul(vscale(-1.0f, xm_raw), c_h);
+    const float2 xl = vmul(xl_raw, dthv), qpa = vmul(xl_raw, c_q);
+    const float2 A = vfma(DT, qpa, xl);
+    const float2 K = vscale(a.dcrjx[i] * dcy, dcz);
 
-  // shear components
-  const float es[3] = {e4, e5, e6};
-  const float mraw[3] = {m1_raw, m2_raw, m3_raw};
-  float GP[3], ES[3], GQP[3];
-  for (int q = 0; q < 3; ++q) {
-    const float l = ls[q], lrv = rv[3 + q];
-    ES[q] = (xmu[q] + DT * hh[q] * (wwo - 1.0f)) * K * l + wwo * hh[q] * lrv;
-    const float G_xmu = es[q] * K * l;
-    const float G_hq = es[q] * (DT * (wwo - 1.0f) * K * l + wwo * lrv);
-    const float Pq = q == 0 ? P1 : (q == 1 ? P2 : P3);
-    GP[q] = -2.0f / (Pq * Pq) * (G_xmu * c_m[q] + G_hq * c_hh[q]);
-    // Qs^-1 pair: hh = m_raw c_hh, xmu = m_raw (dth + DT c_hh), c_hh = -hiw dh1 vx1
-    GQP[q] = (G_hq + DT * G_xmu) * mraw[q] * (-a.dh1 * fvx1) * dhiw[q] * 0.25f;
-  }
-
-  // stores: the adjoint state in place, then the temporaries
-  a.L[LXX][p] = K * lx;
-  a.L[LYY][p] = K * K * ly;
-  a.L[LZZ][p] = K * K * lz;
-  a.L[LXY][p] = K * ls[0];
-  a.L[LXZ][p] = K * ls[1];
-  a.L[LYZ][p] = K * ls[2];
-  if (!ELASTIC) {
-    a.L[LR1][p] = (al + DT * ga) * K * lx + be * rv[0];
-    a.L[LR2][p] = al * K * K * ly + DT * ga * K * ly + be * rv[1];
-    a.L[LR3][p] = al * K * K * lz + DT * ga * K * lz + be * rv[2];
-    for (int q = 0; q < 3; ++q) a.L[LR4 + q][p] = (al + DT * ga) * K * ls[q] + be * rv[3 + q];
-  }
-  float* const* E = a.E;
-  E[E1][p] = A * sP - xm * (PY + PZ) + qpa * sQ - h * (QY + QZ);
-  E[E2][p] = A * sP - xm * (PX + PZ) + qpa * sQ - h * (QX + QZ);
-  E[E3][p] = A * sP - xm * (PX + PY) + qpa * sQ - h * (QX + QY);
-  for (int q = 0; q < 3; ++q) E[E4 + q][p] = ES[q];
-  // chain to the eight-cell sums
-  const float G_xlraw = G_xl * a.dth + G_qpa * c_q;
-  const float G_xmraw = G_xm * c_xm + G_h * c_h + G_xlraw;
-  E[GL8][p] = wacc[0] + -8.0f / (L8 * L8) * G_xlraw;
-  E[GM8][p] = wacc[1] + -16.0f / (M8 * M8) * G_xmraw;
-  E[GP1][p] = wacc[2] + GP[0];
-  E[GP2][p] = wacc[3] + GP[1];
-  E[GP3][p] = wacc[4] + GP[2];
-  if (!ELASTIC && WANTQ) {
-    // Qp^-1 eight-cell sum: qpa = xl_raw c_q, c_q = -qpaw dh1 vx1
-    E[GQP8][p] = qacc[0] + G_qpa * xl_raw * (-a.dh1 * fvx1) * dqpaw * 0.0625f;
-    // Qs^-1 eight-cell sum: h = xm_raw c_h, xm = xm_raw (dth + DT c_h)
-    E[GQS8][p] = qacc[1] + (G_h + DT * G_xm) * xm_raw * (-a.dh1 * fvx1) * dhw * 0.0625f;
-    E[GQ1][p] = qacc[2] + GQP[0];
-    E[GQ2][p] = qacc[3] + GQP[1];
-    E[GQ3][p] = qacc[4] + GQP[2];
+    // ---- the adjoint state of the cell; fstr^T of the column's top three ----
+    // cells (the imaged values above the surface are cleared later, in
+    // k_adj_vel_cell): zz(t) += -zz(t+1), zz(t-1) += -zz(t+2), xz/yz(t-1) +=
+    // -xz/yz(t+1), xz/yz(t-2) += -xz/yz(t+2), xz/yz(t) after the imaging is zero
+    if (i < ie)
+      cpa_wait<1>();
+    else
+      cpa_wait<0>();
+    const float2 lx = stg[buf][0][tid], ly = stg[buf][1][tid];
+    float2 lz = stg[buf][2][tid], ls[3] = {stg[buf][3][tid], stg[buf][4][tid], stg[buf][5][tid]};
+    if (tp) {
+      const float2 z = ld2(a.L[LZZ] + p + 2);
+      lz.y -= z.x;
+      lz.x -= z.y;
+      ls[1] = make_float2(ls[1].x - a.L[LXZ][p + 2], 0.f);
+      ls[2] = make_float2(ls[2].x - a.L[LYZ][p + 2], 0.f);
+    } else if (tp2) {
+      ls[1].y -= a.L[LXZ][p + 5];
+      ls[2].y -= a.L[LYZ][p + 5];
+    }
+    float2 rv[6];
+#pragma unroll
+    for (int q = 0; q < 6; ++q) rv[q] = ELASTIC ? zero : stg[buf][ELASTIC ? 0 : 11 + q][tid];
+    // normal components
+    const float2 Ky = vmul(K, ly), Kz = vmul(K, lz);
+    const float2 PX = vmul(K, lx), PY = vmul(K, Ky), PZ = vmul(K, Kz);
+    float2 QX = zero, QY = zero, QZ = zero;
+    if (!ELASTIC) {
+      QX = vfma(t.kf, PX, vmul(t.wwo, rv[0]));
+      QY = vfma(t.kf, Ky, vmul(t.wwo, rv[1]));
+      QZ = vfma(t.kf, Kz, vmul(t.wwo, rv[2]));
+    }
+    const float2 pyz = vadd(PY, PZ), pxz = vadd(PX, PZ), pxy = vadd(PX, PY);
+    const float2 qyz = vadd(QY, QZ), qxz = vadd(QX, QZ), qxy = vadd(QX, QY);
+    const float2 sP = vadd(pxy, PZ), sQ = vadd(qxy, QZ);
+    const float2 s123 = vadd(vadd(vs1, vs2), vs3);
+    const float2 v23 = vadd(vs2, vs3), v13 = vadd(vs1, vs3), v12 = vadd(vs1, vs2);
+    const float2 G_xl = vmul(s123, sP), G_qpa = vfma(s123, sQ, vmul(DT, G_xl));
+    const float2 nG_xm = vfma(v23, PX, vfma(v13, PY, vmul(v12, PZ)));  // minus the derivative
+    const float2 nG_h = vfma(v23, QX, vfma(v13, QY, vmul(v12, QZ)));
+    const float2 com = vfma(A, sP, vmul(qpa, sQ));
+    st2(a.E[E1] + p, vfma(nxm, pyz, vfma(nh, qyz, com)), ax, ay);
+    st2(a.E[E2] + p, vfma(nxm, pxz, vfma(nh, qxz, com)), ax, ay);
+    st2(a.E[E3] + p, vfma(nxm, pxy, vfma(nh, qxy, com)), ax, ay);
+    st2(a.L[LXX] + p, PX, ax, ay);
+    st2(a.L[LYY] + p, PY, ax, ay);
+    st2(a.L[LZZ] + p, PZ, ax, ay);
+    if (!ELASTIC) {
+      st2(a.L[LR1] + p, vfma(t.kr, PX, vmul(t.vx2, rv[0])), ax, ay);
+      st2(a.L[LR2] + p, vfma(t.kv, PY, vfma(t.kr2, Ky, vmul(t.vx2, rv[1]))), ax, ay);
+      st2(a.L[LR3] + p, vfma(t.kv, PZ, vfma(t.kr2, Kz, vmul(t.vx2, rv[2]))), ax, ay);
+    }
+    // chain to the eight-cell sums
+    const float2 G_xlraw = vfma(G_qpa, c_q, vmul(G_xl, dthv));
+    const float2 G_xmraw = vsub(G_xlraw, vfma(nG_xm, c_xm, vmul(nG_h, c_h)));
+    st2(a.E[GL8] + p, vfma(vscale(-0.125f, vmul(lr, lr)), G_xlraw, stg[buf][6][tid]), ax, ay);
+    st2(a.E[GM8] + p, vfma(vscale(-0.0625f, vmul(xm_raw, xm_raw)), G_xmraw, stg[buf][7][tid]), ax,
+        ay);
+    if (!ELASTIC && WANTQ) {
+      st2(a.E[GQP8] + p, vfma(vmul(G_qpa, xl_raw), dqw, stg[buf][ELASTIC ? 0 : 17][tid]), ax, ay);
+      const float2 g = vfma(DT, nG_xm, nG_h);
+      st2(a.E[GQS8] + p,
+          vfma(vmul(g, vscale(-1.0f, xm_raw)), dhw, stg[buf][WANTQ ? 18 : 0][tid]), ax, ay);
+    }
+    // shear components
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      const float2 mr = vquot(2.0f, P[q]);
+      const float2 cm = vfma(DT, c_hh[q], dthv), xmu = vmul(mr, cm), hh = vmul(mr, c_hh[q]);
+      const float2 Kl = vmul(K, ls[q]);
+      float2 Fq = zero;
+      if (!ELASTIC) Fq = vfma(t.kf, Kl, vmul(t.wwo, rv[3 + q]));
+      st2(a.L[LXY + q] + p, Kl, ax, ay);
+      if (!ELASTIC) st2(a.L[LR4 + q] + p, vfma(t.kr, Kl, vmul(t.vx2, rv[3 + q])), ax, ay);
+      st2(a.E[E4 + q] + p, vfma(xmu, Kl, vmul(hh, Fq)), ax, ay);
+      const float2 G_xmu = vmul(es[q], Kl), G_hq = vmul(es[q], Fq);
+      st2(a.E[GP1 + q] + p,
+          vfma(vscale(-0.5f, vmul(mr, mr)), vfma(G_hq, c_hh[q], vmul(G_xmu, cm)),
+               stg[buf][8 + q][tid]),
+          ax, ay);
+      if (!ELASTIC && WANTQ)
+        st2(a.E[GQ1 + q] + p,
+            vfma(vmul(vfma(DT, G_xmu, G_hq), mr), dhh[q], stg[buf][WANTQ ? 19 + q : 0][tid]), ax,
+            ay);
+    }
+    p += S;
+    pv += VS;
+    u_m1 = u_0; u_0 = u_p1; u_p1 = u_p2;
+    v_m2 = v_m1; v_m1 = v_0; v_0 = v_p1;
+    w_m2 = w_m1; w_m1 = w_0; w_0 = w_p1;
   }
 }
 
@@ -294,46 +352,61 @@ __global__ void __launch_bounds__(128, AWP_ADJ_MINB) k_adj_stress_cell(const Adj
 // ---------------------------------------------------------------------------
 constexpr int kGch = 4;  // x planes a gather thread marches (register queues along x)
 
-__global__ void k_adj_stress_gather(const AdjArgs a) {
-  const int k = a.sk0 - 2 + blockIdx.x * 32 + threadIdx.x;
-  const int j = a.sj0 - 2 + blockIdx.y * 4 + threadIdx.y;
-  const int ib = a.si0 - 2 + blockIdx.z * kGch;
+// c1*(a - b) + c2*(c - d) added to s
+__device__ __forceinline__ float2 add4(float c1, float2 c2, float2 a, float2 b, float2 c, float2 d,
+                                       float2 s) {
+  return vfma(c2, vsub(c, d), vfma(vset<float2>(c1), vsub(a, b), s));
+}
+
+// Level pairs from the even level at or below k0: a pair may reach one level
+// past the transpose's range on either side, where E (V) is zero and the sum
+// adds nothing.
+__global__ void __launch_bounds__(128) k_adj_stress_gather(const __grid_constant__ AdjArgs a) {
+  awp_pipe::grid_start();
+  const int kp0 = (a.sk0 - 2) & ~1, np = (a.sk1 + 2 - kp0) / 2 + 1;
+  const int idx = blockIdx.x * 128 + threadIdx.x;
+  const int j = a.sj0 - 2 + idx / np, k = kp0 + 2 * (idx % np);
+  const int ib = a.si0 - 2 + blockIdx.y * kGch;
   const int ie = min(ib + kGch - 1, a.si1 + 2);
-  if (k > a.sk1 + 2 || j > a.sj1 + 2) return;
+  if (j > a.sj1 + 2) return;
   const int S = a.g.slice, Y = a.g.yline;
   const long long q = (long long)ib * S + (long long)j * Y + k;
-  const float c1 = a.c1, c2 = a.c2;
-  const float* e1 = a.E[E1] + q;
-  const float* e2 = a.E[E2] + q;
-  const float* e3 = a.E[E3] + q;
-  const float* e4 = a.E[E4] + q;
-  const float* e5 = a.E[E5] + q;
-  const float* e6 = a.E[E6] + q;
-  float* Lu = a.L[LU] + q;
-  float* Lv = a.L[LV] + q;
-  float* Lw = a.L[LW] + q;
+  const float c1 = a.c1;
+  const float2 c2 = vset<float2>(a.c2), zero = make_float2(0.f, 0.f);
+  const float* __restrict__ e1 = a.E[E1] + q;
+  const float* __restrict__ e2 = a.E[E2] + q;
+  const float* __restrict__ e3 = a.E[E3] + q;
+  const float* __restrict__ e4 = a.E[E4] + q;
+  const float* __restrict__ e5 = a.E[E5] + q;
+  const float* __restrict__ e6 = a.E[E6] + q;
+  float* __restrict__ Lu = a.L[LU] + q;
+  float* __restrict__ Lv = a.L[LV] + q;
+  float* __restrict__ Lw = a.L[LW] + q;
   // x queues: e1 at x-2, x-1, x; e4, e5 at x-1, x, x+1
-  float e1m2 = e1[-(2 * S)], e1m1 = e1[-S], e1c = e1[0];
-  float e4m1 = e4[-S], e4c = e4[0], e4p1 = e4[S];
-  float e5m1 = e5[-S], e5c = e5[0], e5p1 = e5[S];
-#pragma unroll 1
+  float2 e1m2 = ld2(e1 - 2 * S), e1m1 = ld2(e1 - S), e1c = ld2(e1);
+  float2 e4m1 = ld2(e4 - S), e4c = ld2(e4), e4p1 = ld2(e4 + S);
+  float2 e5m1 = ld2(e5 - S), e5c = ld2(e5), e5p1 = ld2(e5 + S);
+#pragma unroll 2
   for (int i = ib; i <= ie; ++i) {
-    // the sums first, then the read-modify-writes, so that no load waits
-    // behind a store
-    const float e1p1 = e1[S], e4p2 = e4[2 * S], e5p2 = e5[2 * S];
-    const float du = c1 * (e1m1 - e1c) + c2 * (e1m2 - e1p1) +
-                     c1 * (e4[-Y] - e4c) + c2 * (e4[-(2 * Y)] - e4[Y]) +
-                     c1 * (e5[-1] - e5c) + c2 * (e5[-2] - e5[1]);
-    const float dv = c1 * (e2[0] - e2[Y]) + c2 * (e2[-Y] - e2[2 * Y]) +
-                     c1 * (e4c - e4p1) + c2 * (e4m1 - e4p2) +
-                     c1 * (e6[-1] - e6[0]) + c2 * (e6[-2] - e6[1]);
-    const float dw = c1 * (e3[0] - e3[1]) + c2 * (e3[-1] - e3[2]) +
-                     c1 * (e5c - e5p1) + c2 * (e5m1 - e5p2) +
-                     c1 * (e6[-Y] - e6[0]) + c2 * (e6[-(2 * Y)] - e6[Y]);
-    const float lu = Lu[0], lv = Lv[0], lw = Lw[0];
-    Lu[0] = lu + du;
-    Lv[0] = lv + dv;
-    Lw[0] = lw + dw;
+    const float2 lu = ld2(Lu), lv = ld2(Lv), lw = ld2(Lw);
+    const float2 e1p1 = ld2(e1 + S), e4p2 = ld2(e4 + 2 * S), e5p2 = ld2(e5 + 2 * S);
+    const float2 e4a = ld2(e4 - Y), e4b = ld2(e4 - 2 * Y), e4d = ld2(e4 + Y);
+    const float2 e2c = ld2(e2), e2a = ld2(e2 + Y), e2b = ld2(e2 - Y), e2d = ld2(e2 + 2 * Y);
+    const float2 e3c = ld2(e3), e3d = ld2(e3 + 2), e5k = ld2(e5 - 2), e6k = ld2(e6 - 2);
+    const float2 e6c = ld2(e6), e6a = ld2(e6 - Y), e6b = ld2(e6 - 2 * Y), e6d = ld2(e6 + Y);
+    const float e3m = e3[-1], e5p = e5[2], e6p = e6[2];
+    float2 s = add4(c1, c2, e1m1, e1c, e1m2, e1p1, zero);
+    s = add4(c1, c2, e4a, e4c, e4b, e4d, s);
+    s = add4(c1, c2, make_float2(e5k.y, e5c.x), e5c, e5k, make_float2(e5c.y, e5p), s);
+    st2(Lu, vadd(lu, s));
+    s = add4(c1, c2, e2c, e2a, e2b, e2d, zero);
+    s = add4(c1, c2, e4c, e4p1, e4m1, e4p2, s);
+    s = add4(c1, c2, make_float2(e6k.y, e6c.x), e6c, e6k, make_float2(e6c.y, e6p), s);
+    st2(Lv, vadd(lv, s));
+    s = add4(c1, c2, e3c, make_float2(e3c.y, e3d.x), make_float2(e3m, e3c.x), e3d, zero);
+    s = add4(c1, c2, e5c, e5p1, e5m1, e5p2, s);
+    s = add4(c1, c2, e6a, e6c, e6b, e6d, s);
+    st2(Lw, vadd(lw, s));
     e1m2 = e1m1; e1m1 = e1c; e1c = e1p1;
     e4m1 = e4c; e4c = e4p1; e4p1 = e4p2;
     e5m1 = e5c; e5c = e5p1; e5p1 = e5p2;
@@ -356,6 +429,7 @@ __device__ __forceinline__ long long img_index(const AdjArgs& a, int i, int j) {
 }
 
 __global__ void k_adj_images(const AdjArgs a) {
+  awp_pipe::grid_start();
   // targets: the imaged columns and the one-column ring the images also read
   const int j = a.sj0 - 1 + blockIdx.x * blockDim.x + threadIdx.x;
   const int i = a.si0 - 1 + blockIdx.y;
@@ -409,6 +483,7 @@ __global__ void k_adj_images(const AdjArgs a) {
 // velocity^T, pointwise part
 // ---------------------------------------------------------------------------
 __global__ void k_adj_vel_cell(const AdjArgs a) {
+  awp_pipe::grid_start();
   const int k = a.vk0 + blockIdx.x * 32 + threadIdx.x;
   const int j = a.vj0 + blockIdx.y * 4 + threadIdx.y;
   const int i = a.vi0 + blockIdx.z;
@@ -477,51 +552,55 @@ __global__ void k_adj_vel_cell(const AdjArgs a) {
 // velocity^T, gather part: weighted adjoint velocities -> adjoint stresses;
 // density weights -> the density gradient
 // ---------------------------------------------------------------------------
-__global__ void k_adj_vel_gather(const AdjArgs a) {
-  const int k = a.vk0 - 2 + blockIdx.x * 32 + threadIdx.x;
-  const int j = a.vj0 - 2 + blockIdx.y * 4 + threadIdx.y;
-  const int ib = a.vi0 - 2 + blockIdx.z * kGch;
+__global__ void __launch_bounds__(128) k_adj_vel_gather(const __grid_constant__ AdjArgs a) {
+  awp_pipe::grid_start();
+  const int kp0 = (a.vk0 - 2) & ~1, np = (a.vk1 + 2 - kp0) / 2 + 1;
+  const int idx = blockIdx.x * 128 + threadIdx.x;
+  const int j = a.vj0 - 2 + idx / np, k = kp0 + 2 * (idx % np);
+  const int ib = a.vi0 - 2 + blockIdx.y * kGch;
   const int ie = min(ib + kGch - 1, a.vi1 + 2);
-  if (k > a.vk1 + 2 || j > a.vj1 + 2) return;
+  if (j > a.vj1 + 2) return;
   const int S = a.g.slice, Y = a.g.yline;
   const long long q = (long long)ib * S + (long long)j * Y + k;
-  const float c1 = a.c1, c2 = a.c2;
-  const float* A = a.V[VA] + q;
-  const float* B = a.V[VB] + q;
-  const float* C = a.V[VC] + q;
-  float* L[6] = {a.L[LXX] + q, a.L[LXY] + q, a.L[LXZ] + q,
-                 a.L[LYY] + q, a.L[LYZ] + q, a.L[LZZ] + q};
+  const float c1 = a.c1;
+  const float2 c2 = vset<float2>(a.c2), zero = make_float2(0.f, 0.f);
+  const float* __restrict__ A = a.V[VA] + q;
+  const float* __restrict__ B = a.V[VB] + q;
+  const float* __restrict__ C = a.V[VC] + q;
+  float* __restrict__ Lxx = a.L[LXX] + q;
+  float* __restrict__ Lxy = a.L[LXY] + q;
+  float* __restrict__ Lxz = a.L[LXZ] + q;
+  float* __restrict__ Lyy = a.L[LYY] + q;
+  float* __restrict__ Lyz = a.L[LYZ] + q;
+  float* __restrict__ Lzz = a.L[LZZ] + q;
   // x queues: A at x-1, x, x+1; B, C at x-2, x-1, x
-  float Am1 = A[-S], Ac = A[0], Ap1 = A[S];
-  float Bm2 = B[-(2 * S)], Bm1 = B[-S], Bc = B[0];
-  float Cm2 = C[-(2 * S)], Cm1 = C[-S], Cc = C[0];
-#pragma unroll 1
+  float2 Am1 = ld2(A - S), Ac = ld2(A), Ap1 = ld2(A + S);
+  float2 Bm2 = ld2(B - 2 * S), Bm1 = ld2(B - S), Bc = ld2(B);
+  float2 Cm2 = ld2(C - 2 * S), Cm1 = ld2(C - S), Cc = ld2(C);
+#pragma unroll 2
   for (int i = ib; i <= ie; ++i) {
-    // the sums first, then the read-modify-writes (no load behind a store)
-    const float Ap2 = A[2 * S], Bp1 = B[S], Cp1 = C[S];
-    const float dxx = c1 * (Ac - Ap1) + c2 * (Am1 - Ap2);
-    const float dxy = c1 * (Ac - A[Y]) + c2 * (A[-Y] - A[2 * Y]) +
-                      c1 * (Bm1 - Bc) + c2 * (Bm2 - Bp1);
-    const float dxz = c1 * (Ac - A[1]) + c2 * (A[-1] - A[2]) +
-                      c1 * (Cm1 - Cc) + c2 * (Cm2 - Cp1);
-    const float dyy = c1 * (B[-Y] - Bc) + c2 * (B[-(2 * Y)] - B[Y]);
-    const float dyz = c1 * (Bc - B[1]) + c2 * (B[-1] - B[2]) +
-                      c1 * (Cc - C[Y]) + c2 * (C[-Y] - C[2 * Y]);
-    const float dzz = c1 * (C[-1] - Cc) + c2 * (C[-2] - C[1]);
-    const float l0 = L[0][0], l1 = L[1][0], l2 = L[2][0];
-    const float l3 = L[3][0], l4 = L[4][0], l5 = L[5][0];
-    L[0][0] = l0 + dxx;
-    L[1][0] = l1 + dxy;
-    L[2][0] = l2 + dxz;
-    L[3][0] = l3 + dyy;
-    L[4][0] = l4 + dyz;
-    L[5][0] = l5 + dzz;
+    const float2 l0 = ld2(Lxx), l1 = ld2(Lxy), l2 = ld2(Lxz), l3 = ld2(Lyy), l4 = ld2(Lyz),
+                 l5 = ld2(Lzz);
+    const float2 Ap2 = ld2(A + 2 * S), Bp1 = ld2(B + S), Cp1 = ld2(C + S);
+    const float2 Aa = ld2(A + Y), Ab = ld2(A - Y), Ad = ld2(A + 2 * Y), Ak = ld2(A + 2);
+    const float2 Ba = ld2(B + Y), Bb = ld2(B - Y), Bd = ld2(B - 2 * Y), Bk = ld2(B + 2);
+    const float2 Ca = ld2(C + Y), Cb = ld2(C - Y), Cd = ld2(C + 2 * Y), Ck = ld2(C - 2);
+    const float Am = A[-1], Bm = B[-1], Cp = C[2];
+    st2(Lxx, vadd(l0, add4(c1, c2, Ac, Ap1, Am1, Ap2, zero)));
+    st2(Lxy, vadd(l1, add4(c1, c2, Bm1, Bc, Bm2, Bp1, add4(c1, c2, Ac, Aa, Ab, Ad, zero))));
+    st2(Lxz, vadd(l2, add4(c1, c2, Cm1, Cc, Cm2, Cp1,
+                           add4(c1, c2, Ac, make_float2(Ac.y, Ak.x), make_float2(Am, Ac.x), Ak,
+                                zero))));
+    st2(Lyy, vadd(l3, add4(c1, c2, Bb, Bc, Bd, Ba, zero)));
+    st2(Lyz, vadd(l4, add4(c1, c2, Cc, Ca, Cb, Cd,
+                           add4(c1, c2, Bc, make_float2(Bc.y, Bk.x), make_float2(Bm, Bc.x), Bk,
+                                zero))));
+    st2(Lzz, vadd(l5, add4(c1, c2, make_float2(Ck.y, Cc.x), Cc, Ck, make_float2(Cc.y, Cp), zero)));
     Am1 = Ac; Ac = Ap1; Ap1 = Ap2;
     Bm2 = Bm1; Bm1 = Bc; Bc = Bp1;
     Cm2 = Cm1; Cm1 = Cc; Cc = Cp1;
     A += S; B += S; C += S;
-#pragma unroll
-    for (int f = 0; f < 6; ++f) L[f] += S;
+    Lxx += S; Lxy += S; Lxz += S; Lyy += S; Lyz += S; Lzz += S;
   }
 }
 
@@ -567,6 +646,7 @@ __global__ void k_adj_material(const AdjArgs a, int i0, int j0, int k0, int ni, 
 __global__ void k_adj_inject(float* Lu, float* Lv, float* Lw, const long long* idx,
                              const int* comp, const int* first, const int* order, int ncell,
                              const float* res) {
+  awp_pipe::grid_start();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= ncell) return;
   const int r0 = order[first[c]];
@@ -578,6 +658,7 @@ __global__ void k_adj_inject(float* Lu, float* Lv, float* Lw, const long long* i
 
 __global__ void k_sample(const float* u, const float* v, const float* w, const long long* idx,
                          const int* comp, int n, float* out) {
+  awp_pipe::grid_start();
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= n) return;
   const float* f = comp[r] == 0 ? u : (comp[r] == 1 ? v : w);
@@ -694,19 +775,21 @@ __global__ void k_set_moduli(const float* lambda, const float* mu_, const float*
 }
 
 // padded velocities -> VelBox rows; rows beyond nk (up to ld) are not read
+// level pairs: the box starts on a multiple of four levels
 __global__ void k_pack_vel(const float* __restrict__ u, const float* __restrict__ v,
                            const float* __restrict__ w, float* __restrict__ du,
                            float* __restrict__ dv, float* __restrict__ dw, const VelBox b,
                            long long S, long long Y) {
-  const int kk = blockIdx.x * 32 + threadIdx.x;
-  const int jj = blockIdx.y * 4 + threadIdx.y;
-  const int ii = blockIdx.z;
-  if (kk >= b.nk || jj >= b.nj) return;
+  awp_pipe::grid_start();
+  const int np = (b.nk + 1) / 2, idx = blockIdx.x * 128 + threadIdx.x;
+  const int jj = idx / np, kk = 2 * (idx % np), ii = blockIdx.y;
+  if (jj >= b.nj) return;
   const long long p = (long long)(b.i0 + ii) * S + (long long)(b.j0 + jj) * Y + b.k0 + kk;
   const long long q = (long long)ii * b.S + (long long)jj * b.Y + kk;
-  du[q] = u[p];
-  dv[q] = v[p];
-  dw[q] = w[p];
+  const float2 x = ld2(u + p), y = ld2(v + p), z = ld2(w + p);
+  st2(du + q, x);
+  st2(dv + q, y);
+  st2(dw + q, z);
 }
 
 inline unsigned cdiv(long long a, long long b) { return (unsigned)((a + b - 1) / b); }
@@ -717,47 +800,48 @@ cudaError_t awp_launch_pack_vel(const float* u, const float* v, const float* w, 
                                 float* dv, float* dw, const VelBox& b, const AwpGeom& g,
                                 cudaStream_t st) {
   if (b.ni <= 0 || b.nj <= 0 || b.nk <= 0) return cudaSuccess;
-  k_pack_vel<<<dim3(cdiv(b.nk, 32), cdiv(b.nj, 4), b.ni), dim3(32, 4), 0, st>>>(
-      u, v, w, du, dv, dw, b, g.slice, g.yline);
-  return cudaGetLastError();
+  return awp_pipe::launch_after(k_pack_vel, dim3(cdiv((long long)b.nj * ((b.nk + 1) / 2), 128), b.ni), dim3(128), 0, st,  u, v, w, du, dv, dw, b, g.slice, g.yline);
 }
 
 cudaError_t awp_launch_adjoint_step(const AdjArgs& a, cudaStream_t st) {
-  const int si = a.si1 - a.si0 + 1, sj = a.sj1 - a.sj0 + 1, sk = a.sk1 - a.sk0 + 1;
-  const dim3 blk(32, 4);
+  const int si = a.si1 - a.si0 + 1, sj = a.sj1 - a.sj0 + 1;
   // the imaging (fstr) transpose runs inside k_adj_stress_cell
-  const dim3 sgrid(cdiv(sk, 32), cdiv(sj, 4), si);
-  if (a.elastic)
-    k_adj_stress_cell<true, false><<<sgrid, blk, 0, st>>>(a);
-  else if (a.want_q)
-    k_adj_stress_cell<false, true><<<sgrid, blk, 0, st>>>(a);
-  else
-    k_adj_stress_cell<false, false><<<sgrid, blk, 0, st>>>(a);
-  k_adj_stress_gather<<<dim3(cdiv(sk + 4, 32), cdiv(sj + 4, 4), cdiv(si + 4, kGch)), blk, 0,
-                        st>>>(a);
-  k_adj_images<<<dim3(cdiv(sj + 2, 128), si + 2), 128, 0, st>>>(a);
+  auto pairs = [](int k0, int k1) { return (long long)((k1 - (k0 & ~1)) / 2 + 1); };
+  const dim3 sgrid(cdiv(sj * pairs(a.sk0, a.sk1), 128), cdiv(si, kSch));
+  const auto cell = a.elastic  ? k_adj_stress_cell<true, false>
+                    : a.want_q ? k_adj_stress_cell<false, true>
+                               : k_adj_stress_cell<false, false>;
   const int vi = a.vi1 - a.vi0 + 1, vj = a.vj1 - a.vj0 + 1, vk = a.vk1 - a.vk0 + 1;
-  k_adj_vel_cell<<<dim3(cdiv(vk, 32), cdiv(vj, 4), vi), blk, 0, st>>>(a);
-  k_adj_vel_gather<<<dim3(cdiv(vk + 4, 32), cdiv(vj + 4, 4), cdiv(vi + 4, kGch)), blk, 0,
-                     st>>>(a);
-  return cudaGetLastError();
+  const dim3 b(128);
+  cudaError_t e;
+  using awp_pipe::launch_after;
+  if ((e = launch_after(cell, sgrid, b, 0, st, a))) return e;
+  if ((e = launch_after(k_adj_stress_gather,
+                        dim3(cdiv((sj + 4) * pairs(a.sk0 - 2, a.sk1 + 2), 128),
+                             cdiv(si + 4, kGch)),
+                        b, 0, st, a)))
+    return e;
+  if ((e = launch_after(k_adj_images, dim3(cdiv(sj + 2, 128), si + 2), b, 0, st, a))) return e;
+  if ((e = launch_after(k_adj_vel_cell, dim3(cdiv(vk, 32), cdiv(vj, 4), vi), dim3(32, 4), 0, st,
+                        a)))
+    return e;
+  return launch_after(k_adj_vel_gather,
+                      dim3(cdiv((vj + 4) * pairs(a.vk0 - 2, a.vk1 + 2), 128), cdiv(vi + 4, kGch)),
+                      b, 0, st, a);
 }
 
 cudaError_t awp_launch_adjoint_inject(float* const L[3], const long long* idx, const int* comp,
                                       const int* first, const int* order, int ncell,
                                       const float* res, cudaStream_t st) {
   if (ncell <= 0) return cudaSuccess;
-  k_adj_inject<<<cdiv(ncell, 128), 128, 0, st>>>(L[0], L[1], L[2], idx, comp, first, order,
-                                                 ncell, res);
-  return cudaGetLastError();
+  return awp_pipe::launch_after(k_adj_inject, dim3(cdiv(ncell, 128)), dim3(128), 0, st, L[0], L[1], L[2], idx, comp, first, order, ncell, res);
 }
 
 cudaError_t awp_launch_sample(const float* u, const float* v, const float* w,
                               const long long* idx, const int* comp, int nrec, float* out,
                               cudaStream_t st) {
   if (nrec <= 0) return cudaSuccess;
-  k_sample<<<cdiv(nrec, 128), 128, 0, st>>>(u, v, w, idx, comp, nrec, out);
-  return cudaGetLastError();
+  return awp_pipe::launch_after(k_sample, dim3(cdiv(nrec, 128)), dim3(128), 0, st, u, v, w, idx, comp, nrec, out);
 }
 
 cudaError_t awp_launch_adjoint_fold(const AdjArgs& a, float* g_lambda, float* g_mu,

@@ -42,8 +42,9 @@ struct AdjArgs {
   const float *d1, *lam, *mu, *qp, *qs, *lam_mu;
   const float *dcrjx, *dcrjy, *dcrjz;
   AwpTexture tex;
-  float coeff[16];
-  float dth, dh1, dt, c1, c2, qthr;
+  AwpRelaxTab rel;  // the forward update's constants and Q(f) switch
+  unsigned thr;
+  float dth, dt, c1, c2;
   int elastic;
   int want_q;  // accumulate the Q^-1 weights (the caller asked for g_qpinv / g_qsinv)
   AwpGeom g;

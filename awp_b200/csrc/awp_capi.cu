@@ -2917,8 +2917,9 @@ int awp_misfit_gradient_q(awp_ctx* c, int nsteps, int nrec, const int* rec_xyz,
   a.qp = c->f[AWP_QP]; a.qs = c->f[AWP_QS]; a.lam_mu = c->lam_mu;
   a.dcrjx = c->dcrjx; a.dcrjy = c->dcrjy; a.dcrjz = c->dcrjz;
   a.tex = c->tex;
-  memcpy(a.coeff, c->coeff, sizeof(a.coeff));
-  a.dth = c->dth; a.dh1 = c->dh1; a.dt = c->p.dt; a.c1 = c->c1; a.c2 = c->c2; a.qthr = c->qthr;
+  a.rel = c->rel;
+  a.thr = c->thr;
+  a.dth = c->dth; a.dt = c->p.dt; a.c1 = c->c1; a.c2 = c->c2;
   a.elastic = c->elastic ? 1 : 0;
   a.want_q = (!c->elastic && (g_qpinv || g_qsinv)) ? 1 : 0;
   a.g = c->g;
