@@ -308,18 +308,21 @@ bool build_tma_maps(awp_ctx* c) {
   if (c->topo) {
     // the curvilinear kernels' tiles: the same fields with their own boxes, and
     // no k halo (the neighbouring levels come from the neighbouring lanes)
-    awp_topo_box(0, &hx, &hy);
-    awp_topo_box(1, &mx, &my);
-    awp_topo_box(2, &ox, &oy);
+    awp_topo_box(0, 0, &hx, &hy);
+    awp_topo_box(0, 1, &mx, &my);
+    awp_topo_box(0, 2, &ox, &oy);
     const bool jh[6] = {false, true, false, true, false, true};
     for (int q = 0; q < 6; ++q)
       bad |= awp_tma_encode(&c->topo_vel_maps.halo[q], f[vh[q]], c->g, jh[q] ? hx : ox,
                             jh[q] ? hy : oy);
     bad |= awp_tma_encode(&c->topo_vel_maps.media[0], f[AWP_D1], c->g, mx, my);
-    for (int q = 0; q < 3; ++q) {
+    for (int q = 0; q < 3; ++q)
       bad |= awp_tma_encode(&c->topo_vel_maps.own[q], f[vo[q]], c->g, ox, oy);
+    awp_topo_box(1, 0, &hx, &hy);
+    awp_topo_box(1, 1, &mx, &my);
+    awp_topo_box(1, 2, &ox, &oy);
+    for (int q = 0; q < 3; ++q)
       bad |= awp_tma_encode(&c->topo_str_maps.halo[q], f[vo[q]], c->g, hx, hy);
-    }
     for (int q = 0; q < 4; ++q)
       bad |= awp_tma_encode(&c->topo_str_maps.media[q], f[sm[q]], c->g, mx, my);
     for (int q = 0; q < 12; ++q)
@@ -388,6 +391,11 @@ int phase_begin(awp_ctx* c) {
   return AWP_OK;
 }
 
+// The interface layer of a mesh block over a coarser one (dvelc2, dstrqc2: the
+// level below the block's own range) rides in the TMA kernels, whose tiles hold
+// it anyway: on its own it is a sector of every field per column.
+bool mesh_layer(const awp_ctx* c) { return c->p.grid < c->p.ngrids - 1; }
+
 // Kernel arguments of the curvilinear half-steps: the wavefield, media and
 // texture of the context plus the metric arrays of awp_topography_init.
 TopoArgs topo_args(awp_ctx* c) {
@@ -404,6 +412,7 @@ TopoArgs topo_args(awp_ctx* c) {
   a.thr = c->thr;
   a.slice = c->g.slice; a.yline = c->g.yline;
   a.nx = c->g.nxt; a.ny = c->g.nyt; a.nz = c->g.nzt;
+  a.layer = mesh_layer(c) ? 1 : 0;
   return a;
 }
 
@@ -424,11 +433,13 @@ VelArgs make_vel_args(awp_ctx* c) {
   v.k1 = AWP_ALIGN + round_up(c->g.nzt, 4) - 1;
   if (c->p.grid > 0) v.k1 = std::min(v.k1, c->g.nzt + AWP_ALIGN - 3);
   v.dth = c->dth; v.c1 = c->c1; v.c2 = c->c2;
+  v.layer = 0;
+  v.layer_j1 = c->yre;
   return v;
 }
 
 int phase_velocity(awp_ctx* c) {
-  const VelArgs v = make_vel_args(c);
+  VelArgs v = make_vel_args(c);
   if (c->topo) {  // topo_velocity_*_H replace dvelc[xy] on the top grid (pmcl3d.c:1661-1698)
     if (!tma_ready(c)) return set_error(AWP_ERR_CUDA, "tensor maps of the curvilinear grid");
     PhaseScope ps(c, 0);
@@ -439,6 +450,7 @@ int phase_velocity(awp_ctx* c) {
   }
   const bool tma = awp_tuning_get("tma_vel") == 1 && tma_ready(c);
   PhaseScope ps(c, 0);
+  if (tma) v.layer = mesh_layer(c) ? 1 : 0;
   if (tma)
     CU_TRY(awp_launch_velocity_tma(v, c->vel_maps, awp_tuning_get("ichunk"), c->d_err,
                                    c->stream));
@@ -466,11 +478,13 @@ void middle_band(const awp_ctx* c, int* i0, int* i1, int* j0, int* j1) {
 
 // Cartesian stress (+ memory variables) over i0..i1 x j0..j1 of the stress
 // window, with the kernel family the tuning selects.
-int launch_cart_stress(awp_ctx* c, int i0, int i1, int j0, int j1) {
+// `layer` (TMA kernel): the interface layer too.
+int launch_cart_stress(awp_ctx* c, int i0, int i1, int j0, int j1, bool layer = false) {
   if (i1 < i0 || j1 < j0) return AWP_OK;
   const bool tma = awp_tuning_get("tma_str") == 1 && tma_ready(c);
   StrArgs s = make_str_args(c);
   s.i0 = i0; s.i1 = i1; s.j0 = j0; s.j1 = j1;
+  s.layer = layer ? 1 : 0;
   if (tma)
     CU_TRY(awp_launch_stress_tma(s, c->str_maps, c->elastic, awp_tuning_get("ichunk"),
                                  c->d_err, c->stream));
@@ -492,8 +506,23 @@ bool stress_split(const awp_ctx* c) {
   return c->p.nve == 3 && (!c->topo || !c->topo_plastic_consistent);
 }
 
+// Whether the stress launch itself takes the interface layer: not where the
+// stress is split around the plasticity section (the layer belongs before the
+// sources, whole).
+bool stress_layer(awp_ctx* c) {
+  return mesh_layer(c) && !c->topo && !stress_split(c) && awp_tuning_get("tma_str") == 1 &&
+         tma_ready(c);
+}
+bool velocity_layer(awp_ctx* c) {
+  return mesh_layer(c) && !c->topo && awp_tuning_get("tma_vel") == 1 && tma_ready(c);
+}
+
+bool topo_stress_runs(const awp_ctx* c) {
+  return c->topo && !(c->p.nve == 3 && !c->topo_plastic_consistent);
+}
+
 int phase_stress(awp_ctx* c) {
-  if (c->topo && c->p.nve == 3 && !c->topo_plastic_consistent) return AWP_OK;
+  if (c->topo && !topo_stress_runs(c)) return AWP_OK;
   if (c->topo) {  // topo_stress_*_H replace dstrqc on the top grid (pmcl3d.c:1843-1924)
     if (!tma_ready(c)) return set_error(AWP_ERR_CUDA, "tensor maps of the curvilinear grid");
     PhaseScope ps(c, 1);
@@ -503,7 +532,8 @@ int phase_stress(awp_ctx* c) {
     return AWP_OK;
   }
   PhaseScope ps(c, 1);
-  if (!stress_split(c)) return launch_cart_stress(c, c->xls, c->xre, c->yls, c->yre);
+  if (!stress_split(c))
+    return launch_cart_stress(c, c->xls, c->xre, c->yls, c->yre, stress_layer(c));
   int i0, i1, j0, j1, st;
   middle_band(c, &i0, &i1, &j0, &j1);
   if ((st = launch_cart_stress(c, i0, i1, c->yls, j0 - 1))) return st;  // xss2, front
@@ -765,14 +795,19 @@ DmGrid dm_grid(awp_ctx* c) {
   return g;
 }
 
-int dm_interfaces(awp_ctx* const* g, int n, cudaStream_t st) {
+// `set`: the fields to trade.  The reference trades all nine after the
+// velocity and again after the stress update; the exchange of a field that
+// nothing has written since its last exchange stores what is there already
+// (intp3d reads the coarse level nzt-3 and swap3 writes nzt-2 and nzt-1), so
+// those are left out (53 x 41 coarse columns: 33 -> 17 us a step).
+int dm_interfaces(awp_ctx* const* g, int n, int set, cudaStream_t st) {
   for (int p = 1; p < n; ++p) {  // coarse -> fine (pmcl3d.c:1767-1772, 2057-2062)
-    DmPairArgs a{dm_grid(g[p]), dm_grid(g[p - 1])};
+    DmPairArgs a{dm_grid(g[p]), dm_grid(g[p - 1]), set};
     CU_TRY(awp_launch_intp3d(a, st));
     g[p]->launches++;
   }
   for (int p = 0; p < n - 1; ++p) {  // fine -> coarse (pmcl3d.c:1802-1806, 2085-2090)
-    DmPairArgs a{dm_grid(g[p + 1]), dm_grid(g[p])};
+    DmPairArgs a{dm_grid(g[p + 1]), dm_grid(g[p]), set};
     CU_TRY(awp_launch_swap3(a, st));
     g[p]->launches++;
   }
@@ -780,6 +815,7 @@ int dm_interfaces(awp_ctx* const* g, int n, cudaStream_t st) {
 }
 
 int dm_velocity(awp_ctx* c) {  // dvelc2 (pmcl3d.c:1729-1732)
+  if (velocity_layer(c) || c->topo) return AWP_OK;  // the velocity launch took it
   DmVel2Args a;
   a.g = dm_grid(c);
   a.d1 = c->f[AWP_D1];
@@ -791,6 +827,7 @@ int dm_velocity(awp_ctx* c) {  // dvelc2 (pmcl3d.c:1729-1732)
 }
 
 int dm_stress(awp_ctx* c) {  // dstrqc2 over xss1..xse3 x yls..yre (pmcl3d.c:1936-1948)
+  if (stress_layer(c)) return AWP_OK;  // the stress launch took it
   DmStr2Args a;
   memset(&a, 0, sizeof(a));
   float** f = c->f;
@@ -804,6 +841,11 @@ int dm_stress(awp_ctx* c) {  // dstrqc2 over xss1..xse3 x yls..yre (pmcl3d.c:193
   a.i0 = c->xls; a.i1 = c->xre; a.j0 = c->yls; a.j1 = c->yre;
   a.dth = c->dth; a.dh1 = c->dh1; a.dt = c->p.dt;
   a.thr = c->thr;
+  a.ex_i0 = a.ex_j0 = 1;
+  if (topo_stress_runs(c)) {  // the curvilinear launch took its window's columns
+    a.ex_i0 = c->targs.s_i + AWP_NGSL + 2; a.ex_i1 = c->targs.e_i + AWP_NGSL + 1;
+    a.ex_j0 = c->targs.s_j + AWP_NGSL + 2; a.ex_j1 = c->targs.e_j + AWP_NGSL + 1;
+  }
   CU_TRY(awp_launch_dstrqc2(a, c->stream));
   c->launches++;
   return AWP_OK;
@@ -856,17 +898,26 @@ int mesh_prepare(awp_mesh* m) {
 }
 
 // One time step of the whole stack in pmcl3d's order (pmcl3d.c:1628-2490).
-int mesh_step(awp_mesh* m) {
+// `first`: the first step of a call (the caller may have written any field).
+int mesh_step(awp_mesh* m, bool first) {
   awp_ctx* const* g = m->g;
   const int n = m->ngrids;
   int st;
+  // velocities change after their exchange only by prescribed velocities and
+  // boundary forces; stresses after theirs by the plastic return (the sources
+  // come before it, the free surface is far from every interface)
+  bool vel_later = g[0]->d_frc_pos != nullptr, str_later = first;
+  for (int p = 0; p < n; ++p) {
+    vel_later = vel_later || g[p]->forcef;
+    str_later = str_later || g[p]->p.nve == 3;
+  }
   for (int p = 0; p < n; ++p)
     if ((st = phase_begin(g[p]))) return st;
   for (int p = 0; p < n; ++p)
     if ((st = phase_velocity(g[p]))) return st;
   for (int p = 0; p < n - 1; ++p)
     if ((st = dm_velocity(g[p]))) return st;
-  if ((st = dm_interfaces(g, n, m->stream))) return st;
+  if ((st = dm_interfaces(g, n, str_later ? AWP_DM_ALL : AWP_DM_VELOCITY, m->stream))) return st;
   if ((st = phase_forcing(g[0]))) return st;
   for (int p = 0; p < n; ++p)
     if ((st = phase_stress(g[p]))) return st;
@@ -874,7 +925,7 @@ int mesh_step(awp_mesh* m) {
     if ((st = dm_stress(g[p]))) return st;
   for (int p = 0; p < n; ++p)
     if ((st = phase_sources(g[p]))) return st;
-  if ((st = dm_interfaces(g, n, m->stream))) return st;
+  if ((st = dm_interfaces(g, n, vel_later ? AWP_DM_ALL : AWP_DM_STRESS, m->stream))) return st;
   for (int p = 0; p < n; ++p)
     if ((st = phase_plasticity(g[p]))) return st;
   if ((st = phase_fstr(g[0]))) return st;
@@ -1869,7 +1920,7 @@ int awp_mesh_step(awp_mesh* m, int nsteps) {
     if (m->g[p]->p.nve == 3 && !m->g[p]->plast_ready)
       return set_error(AWP_ERR_STATE, "grid %d: NVE=3 needs awp_upload_plasticity first", p);
   for (int s = 0; s < nsteps; ++s) {
-    int st = mesh_step(m);
+    int st = mesh_step(m, s == 0);
     if (st) return st;
   }
   return AWP_OK;

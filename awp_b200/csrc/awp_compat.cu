@@ -430,6 +430,7 @@ void dstrqc2_H(float* xx, float* yy, float* zz, float* xy, float* xz, float* yz,
   a.coeff_dev = coeff;
   a.i0 = s_i; a.i1 = e_i; a.j0 = s_j; a.j1 = e_j;
   a.dth = gc.dth; a.dh1 = gc.dh1; a.dt = s.DT;
+  a.ex_i0 = a.ex_j0 = 1;  // no columns left out
   const float thr = 2.0f * s.qthr;
   memcpy(&a.thr, &thr, sizeof(a.thr));
   check(awp_launch_dstrqc2(a, St), "dstrqc2_H");

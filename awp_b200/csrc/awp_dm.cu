@@ -10,6 +10,7 @@
 #include <cuda_runtime.h>
 
 #include "awp_dm.cuh"
+#include "awp_pipe.cuh"
 #include "awp_stencil.cuh"
 
 namespace {
@@ -22,6 +23,7 @@ __device__ __forceinline__ long long at(const DmGrid& g, int i, int j, int k) {
 // dvelc2 (kernel.cu:2289-2343)
 // ===========================================================================
 __global__ void k_dvelc2(const DmVel2Args a) {
+  awp_pipe::grid_start();
   const int j = 2 + AWP_NGSL + blockIdx.x * blockDim.x + threadIdx.x;
   const int i = 2 + AWP_NGSL + blockIdx.y * blockDim.y + threadIdx.y;
   if (i >= a.g.nxt + 2 + AWP_NGSL || j >= a.g.nyt + 2 + AWP_NGSL) return;
@@ -65,11 +67,15 @@ __global__ void k_dvelc2(const DmVel2Args a) {
 // branch is wwo*q here where dstrqc has 2*wwo*q, so its constant is halved.
 // Every load is issued before the arithmetic: the kernel's time is the sectors
 // of one level of k-contiguous columns, one 32-byte sector per value (300 x
-// 300: 62 -> 33 us with the double-precision divisions of the switch gone).
+// 300: 58 us), so a mesh block leaves it only the ring outside the exclusion
+// rectangle (14 us): inside, the stress kernel that has the lines above in
+// shared memory updates the layer too.
 __global__ void __launch_bounds__(128) k_dstrqc2(const DmStr2Args a) {
+  awp_pipe::grid_start();
   const int j = a.j0 + blockIdx.x * blockDim.x + threadIdx.x;
   const int i = a.i0 + blockIdx.y * blockDim.y + threadIdx.y;
   if (i > a.i1 || j > a.j1) return;
+  if (i >= a.ex_i0 && i <= a.ex_i1 && j >= a.ex_j0 && j <= a.ex_j1) return;
   const int S = a.g.slice, Y = a.g.yline;
   const int k = AWP_ALIGN + 2;
   const long long pos = at(a.g, i, j, k);
@@ -135,6 +141,7 @@ __global__ void __launch_bounds__(128) k_dstrqc2(const DmStr2Args a) {
 // sector of its own).
 // ===========================================================================
 __global__ void k_intp3d(const DmPairArgs a) {
+  awp_pipe::grid_start();
   const int j = AWP_NGSL + blockIdx.x * blockDim.x + threadIdx.x;
   const int i = AWP_NGSL + blockIdx.y * blockDim.y + threadIdx.y;
   if (i > a.lo.nxt + 3 + AWP_NGSL || j > a.lo.nyt + 3 + AWP_NGSL) return;
@@ -159,16 +166,17 @@ __global__ void k_intp3d(const DmPairArgs a) {
         H[ph + (long long)(ii - 1 + oi) * hi.slice + (long long)(jj - 1 + oj) * hi.yline] = s;
       }
   };
-  // one field per blockIdx.z (the nine patches of a column are independent)
-  switch (blockIdx.z) {
-    case 0: patch(lo.xz, hi.xz, 0, 0); break;
-    case 1: patch(lo.yz, hi.yz, 1, 1); break;
-    case 2: patch(lo.w1, hi.w1, 1, 0); break;
-    case 3: patch(lo.xx, hi.xx, 1, 0); break;
-    case 4: patch(lo.yy, hi.yy, 1, 0); break;
-    case 5: patch(lo.zz, hi.zz, 1, 0); break;
-    case 6: patch(lo.u1, hi.u1, 0, 0); break;
-    case 7: patch(lo.v1, hi.v1, 1, 1); break;
+  // one field per blockIdx.z (the nine patches of a column are independent):
+  // the velocities first
+  switch (blockIdx.z + (a.set == AWP_DM_STRESS ? 3 : 0)) {
+    case 0: patch(lo.w1, hi.w1, 1, 0); break;
+    case 1: patch(lo.u1, hi.u1, 0, 0); break;
+    case 2: patch(lo.v1, hi.v1, 1, 1); break;
+    case 3: patch(lo.xz, hi.xz, 0, 0); break;
+    case 4: patch(lo.yz, hi.yz, 1, 1); break;
+    case 5: patch(lo.xx, hi.xx, 1, 0); break;
+    case 6: patch(lo.yy, hi.yy, 1, 0); break;
+    case 7: patch(lo.zz, hi.zz, 1, 0); break;
     default: patch(lo.xy, hi.xy, 0, 1); break;
   }
 }
@@ -184,13 +192,14 @@ __global__ void k_intp3d(const DmPairArgs a) {
 // field (blockIdx.z): its fine columns' levels align+1 .. align+8 are summed
 // along k as they are read (eight lanes a column: k-contiguous, sector-wide
 // loads), then along j and i from shared memory.
-// 300 x 300 over 100 x 100: 51 -> 17 us a launch against the chain of 125
+// 300 x 300 over 100 x 100, all nine fields: 51 -> 26 us a launch against the chain of 125
 // double-precision terms.
 constexpr int kSwTI = 4, kSwTJ = 32;
 constexpr int kSwBI = 3 * (kSwTI - 1) + 5, kSwBJ = 3 * (kSwTJ - 1) + 5;
 constexpr int kSwThreads = 32 * kSwBI;  // a warp per fine row
 
 __global__ void __launch_bounds__(kSwThreads) k_swap3(const DmPairArgs a) {
+  awp_pipe::grid_start();
   __shared__ float ks[2][kSwBI][kSwBJ + 1];  // summed along k (two windows)
   __shared__ float js[2][kSwBI][kSwTJ + 1];  // ... and along j
   const DmGrid &lo = a.lo, &hi = a.hi;
@@ -201,15 +210,15 @@ __global__ void __launch_bounds__(kSwThreads) k_swap3(const DmPairArgs a) {
   float* dst;
   const float* src;
   int kh0, nwin, di, dj;  // level-0 window at kh0 (level 1 at 6); shifted fine columns
-  switch (blockIdx.z) {
+  switch (blockIdx.z + (a.set == AWP_DM_STRESS ? 3 : 0)) {  // the velocities first
     case 0: dst = lo.u1; src = hi.u1; kh0 = 3; nwin = 2; di = 0; dj = 0; break;
     case 1: dst = lo.v1; src = hi.v1; kh0 = 3; nwin = 2; di = 1; dj = 1; break;
-    case 2: dst = lo.xy; src = hi.xy; kh0 = 3; nwin = 2; di = 0; dj = 1; break;
+    case 2: dst = lo.w1; src = hi.w1; kh0 = 4; nwin = 1; di = 1; dj = 0; break;
     case 3: dst = lo.xx; src = hi.xx; kh0 = 3; nwin = 2; di = 1; dj = 0; break;
     case 4: dst = lo.yy; src = hi.yy; kh0 = 3; nwin = 2; di = 1; dj = 0; break;
     case 5: dst = lo.zz; src = hi.zz; kh0 = 3; nwin = 2; di = 1; dj = 0; break;
-    case 6: dst = lo.xz; src = hi.xz; kh0 = 4; nwin = 1; di = 0; dj = 0; break;
-    case 7: dst = lo.w1; src = hi.w1; kh0 = 4; nwin = 1; di = 1; dj = 0; break;
+    case 6: dst = lo.xy; src = hi.xy; kh0 = 3; nwin = 2; di = 0; dj = 1; break;
+    case 7: dst = lo.xz; src = hi.xz; kh0 = 4; nwin = 1; di = 0; dj = 0; break;
     default: dst = lo.yz; src = hi.yz; kh0 = 4; nwin = 1; di = 1; dj = 1; break;
   }
   // the window of coarse column c centres on fine column 3 (c - 2 - ngsl) + 2 + ngsl + d
@@ -289,31 +298,31 @@ __global__ void k_checkmesh(const DmCheckArgs a) {
 
 inline unsigned cdiv(int a, int b) { return (unsigned)((a + b - 1) / b); }
 
+unsigned pair_fields(const DmPairArgs& a) {
+  return a.set == AWP_DM_ALL ? 9 : a.set == AWP_DM_VELOCITY ? 3 : 6;
+}
+
 }  // namespace
 
 cudaError_t awp_launch_dvelc2(const DmVel2Args& a, cudaStream_t st) {
   const dim3 block(32, 4);
-  k_dvelc2<<<dim3(cdiv(a.g.nyt, 32), cdiv(a.g.nxt, 4)), block, 0, st>>>(a);
-  return cudaGetLastError();
+  return awp_pipe::launch_after(k_dvelc2, dim3(cdiv(a.g.nyt, 32), cdiv(a.g.nxt, 4)), block, 0, st, a);
 }
 
 cudaError_t awp_launch_dstrqc2(const DmStr2Args& a, cudaStream_t st) {
   if (a.i1 < a.i0 || a.j1 < a.j0) return cudaSuccess;
   const dim3 block(32, 4);
-  k_dstrqc2<<<dim3(cdiv(a.j1 - a.j0 + 1, 32), cdiv(a.i1 - a.i0 + 1, 4)), block, 0, st>>>(a);
-  return cudaGetLastError();
+  return awp_pipe::launch_after(k_dstrqc2, dim3(cdiv(a.j1 - a.j0 + 1, 32), cdiv(a.i1 - a.i0 + 1, 4)), block, 0, st, a);
 }
 
 cudaError_t awp_launch_intp3d(const DmPairArgs& a, cudaStream_t st) {
   const dim3 block(32, 4);
-  k_intp3d<<<dim3(cdiv(a.lo.nyt + 4, 32), cdiv(a.lo.nxt + 4, 4), 9), block, 0, st>>>(a);
-  return cudaGetLastError();
+  return awp_pipe::launch_after(k_intp3d, dim3(cdiv(a.lo.nyt + 4, 32), cdiv(a.lo.nxt + 4, 4), pair_fields(a)), block, 0, st, a);
 }
 
 cudaError_t awp_launch_swap3(const DmPairArgs& a, cudaStream_t st) {
   // columns ngsl .. n + ngsl + 4 of the coarse block
-  k_swap3<<<dim3(cdiv(a.lo.nyt + 5, kSwTJ), cdiv(a.lo.nxt + 5, kSwTI), 9), kSwThreads, 0, st>>>(a);
-  return cudaGetLastError();
+  return awp_pipe::launch_after(k_swap3, dim3(cdiv(a.lo.nyt + 5, kSwTJ), cdiv(a.lo.nxt + 5, kSwTI), pair_fields(a)), dim3(kSwThreads), 0, st, a);
 }
 
 cudaError_t awp_launch_checkmesh(const DmCheckArgs& a, cudaStream_t st) {

@@ -37,12 +37,15 @@ struct DmStr2Args {
   int i0, i1, j0, j1;
   float dth, dh1, dt;
   unsigned thr;  // Q(f) switch on a pair sum of Q^-1 (StrArgs::thr)
+  int ex_i0, ex_i1, ex_j0, ex_j1;  // without these columns (i0 > i1: none)
 };
 
 // intp3d (kernel.cu:2359-2561) coarse -> fine and swap3 (kernel.cu:3032-3217)
 // fine -> coarse across one interface.
+enum { AWP_DM_ALL, AWP_DM_VELOCITY, AWP_DM_STRESS };
 struct DmPairArgs {
   DmGrid lo, hi;
+  int set;  // AWP_DM_*: the fields of this launch
 };
 
 // checkmesh (mesh.c:1404-1443): the coarse grid's values at its top three

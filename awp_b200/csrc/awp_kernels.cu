@@ -20,6 +20,7 @@
 #include <string.h>
 
 #include "awp_kernels.cuh"
+#include "awp_pipe.cuh"
 #include "awp_stencil.cuh"
 #include "awp_tma.cuh"
 
@@ -312,6 +313,7 @@ __device__ __forceinline__ void fstr_cell4(const FstrArgs& a, const int i, const
 
 template <bool V4>
 __global__ void k_fstr(const FstrArgs a) {
+  awp_pipe::grid_start();
   const int i = a.i0 + blockIdx.y, j = a.j0 + blockIdx.x * blockDim.x + threadIdx.x;
   if (V4)
     fstr_cell4(a, i, j);
@@ -364,6 +366,7 @@ __device__ __forceinline__ void addsrc_cell(const SrcArgs& a, const int c) {
 }
 
 __global__ void k_addsrc(const SrcArgs a) {
+  awp_pipe::grid_start();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= a.ncell) return;
   addsrc_cell(a, c);
@@ -467,6 +470,7 @@ __device__ __forceinline__ void addkinsrc_cell(const KinSrcArgs& a, const int c,
 }
 
 __global__ void k_addkinsrc(const KinSrcArgs a) {
+  awp_pipe::grid_start();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= a.ncell) return;
   addkinsrc_cell(a, c, a.step);
@@ -478,6 +482,7 @@ __global__ void k_addkinsrc(const KinSrcArgs a) {
 // from the device, *step + 1 + off, and IFAULT < 4 stops at nst.
 __global__ void k_fstr_src(const FstrArgs f, const SrcArgs s, const int* step, const int off,
                            const int nst) {
+  awp_pipe::grid_start();
   if (blockIdx.y + 1 < gridDim.y) {
     fstr_cell4(f, f.i0 + blockIdx.y, f.j0 + blockIdx.x * blockDim.x + threadIdx.x);
     return;
@@ -493,6 +498,7 @@ __global__ void k_fstr_src(const FstrArgs f, const SrcArgs s, const int* step, c
 
 __global__ void k_fstr_kinsrc(const FstrArgs f, const KinSrcArgs k, const int* step,
                               const int off) {
+  awp_pipe::grid_start();
   if (blockIdx.y + 1 < gridDim.y) {
     fstr_cell4(f, f.i0 + blockIdx.y, f.j0 + blockIdx.x * blockDim.x + threadIdx.x);
     return;
@@ -532,6 +538,7 @@ __device__ __forceinline__ float pfluid_at(const PlastParams& pp, int k) {
 }
 
 __global__ void k_plast_calc(const PlastCalcArgs a) {
+  awp_pipe::grid_start();
   const int k = a.k0 + blockIdx.x * blockDim.x + threadIdx.x;
   const int j = a.j0 + blockIdx.y * blockDim.y + threadIdx.y;
   const int i = a.i0 + blockIdx.z;
@@ -595,6 +602,7 @@ __global__ void k_plast_calc(const PlastCalcArgs a) {
 }
 
 __global__ void k_plast_app(const PlastAppArgs a) {
+  awp_pipe::grid_start();
   const int k = a.k0 + blockIdx.x * blockDim.x + threadIdx.x;
   const int j = a.j0 + blockIdx.y * blockDim.y + threadIdx.y;
   const int i = a.i0 + blockIdx.z;
@@ -679,6 +687,7 @@ __global__ void k_plast_app(const PlastAppArgs a) {
 // launched rows rounded up to the shipped 2 x 2 blocks.  The reference forms
 // the increments in double.
 __global__ void k_addplanesrc(const PlaneSrcArgs a) {
+  awp_pipe::grid_start();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   if (i >= a.nx || j >= a.ny) return;
@@ -698,6 +707,7 @@ __global__ void k_addplanesrc(const PlaneSrcArgs a) {
 // Output gather (velbuffer, kernel.cu:3948-4011)
 // ===========================================================================
 __global__ void k_velbuffer(const VelBufArgs a) {
+  awp_pipe::grid_start();
   const int ix = blockIdx.x * blockDim.x + threadIdx.x;
   const int iy = blockIdx.y * blockDim.y + threadIdx.y;
   const int iz = blockIdx.z * blockDim.z + threadIdx.z;
@@ -944,6 +954,7 @@ inline unsigned cdiv_u(long long a, long long b) { return (unsigned)((a + b - 1)
 // (replayable graphs): the schedule of one_step, IFAULT < 4 while the step is below NST.
 __global__ void k_addsrc_dev(const SrcArgs a, const int* __restrict__ step, const int off,
                              const int nst) {
+  awp_pipe::grid_start();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   const int cur = *step + 1 + off;
   if (c >= a.ncell || cur >= nst) return;
@@ -953,12 +964,16 @@ __global__ void k_addsrc_dev(const SrcArgs a, const int* __restrict__ step, cons
 }
 
 __global__ void k_addkinsrc_dev(const KinSrcArgs a, const int* __restrict__ step, const int off) {
+  awp_pipe::grid_start();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= a.ncell) return;
   addkinsrc_cell(a, c, *step + 1 + off);
 }
 
-__global__ void k_step_advance(int* step, const int n) { *step = *step + n; }
+__global__ void k_step_advance(int* step, const int n) {
+  awp_pipe::grid_start();
+  *step = *step + n;
+}
 
 // ===========================================================================
 // launchers
@@ -1030,11 +1045,9 @@ bool fstr_aligned(const FstrArgs& a) {
 cudaError_t awp_launch_fstr(const FstrArgs& a, cudaStream_t st) {
   const int nj = a.j1 - a.j0 + 1, ni = a.i1 - a.i0 + 1;
   if (nj <= 0 || ni <= 0) return cudaSuccess;
-  if (fstr_aligned(a))
-    k_fstr<true><<<dim3(cdiv_u(nj, 128), ni, 1), 128, 0, st>>>(a);
-  else
-    k_fstr<false><<<dim3(cdiv_u(nj, 128), ni, 1), 128, 0, st>>>(a);
-  return cudaGetLastError();
+  const dim3 grid(cdiv_u(nj, 128), ni, 1);
+  return awp_pipe::launch_after(fstr_aligned(a) ? k_fstr<true> : k_fstr<false>, grid, dim3(128), 0,
+                                st, a);
 }
 
 cudaError_t awp_launch_fstr_sources(const FstrArgs& f, const SrcArgs* s, const KinSrcArgs* k,
@@ -1043,22 +1056,23 @@ cudaError_t awp_launch_fstr_sources(const FstrArgs& f, const SrcArgs* s, const K
   if (nj <= 0 || ni <= 0 || !fstr_aligned(f)) return cudaErrorInvalidValue;
   const dim3 grid(cdiv_u(nj, 128), ni + 1, 1);
   if (s)
-    k_fstr_src<<<grid, 128, 0, st>>>(f, *s, step, off, nst);
-  else
-    k_fstr_kinsrc<<<grid, 128, 0, st>>>(f, *k, step, off);
-  return cudaGetLastError();
+    return awp_pipe::launch_after(k_fstr_src, grid, dim3(128), 0, st, f, *s,
+                                  step, off, nst);
+  return awp_pipe::launch_after(k_fstr_kinsrc, grid, dim3(128), 0, st, f, *k,
+                                step, off);
 }
 
 cudaError_t awp_launch_addsrc(const SrcArgs& a, cudaStream_t st) {
   if (a.ncell <= 0) return cudaSuccess;
   if (a.cell_pos)
-    k_addsrc<<<cdiv_u(a.ncell, 128), 128, 0, st>>>(a);
+    return awp_pipe::launch_after(k_addsrc, dim3(cdiv_u(a.ncell, 128)), dim3(128), 0, st, a);
   else
     k_addsrc_direct<<<cdiv_u(a.ncell, 128), 128, 0, st>>>(a);
   return cudaGetLastError();
 }
 
 __global__ void k_frcvel(const FrcvelArgs a) {
+  awp_pipe::grid_start();
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= a.npsrc) return;
   const int i = a.i - 1;
@@ -1129,42 +1143,36 @@ cudaError_t awp_launch_copy_segments(const CopySegs& s, cudaStream_t st) {
 
 cudaError_t awp_launch_frcvel(const FrcvelArgs& a, cudaStream_t st) {
   if (a.npsrc <= 0) return cudaSuccess;
-  k_frcvel<<<cdiv_u(a.npsrc, 256), 256, 0, st>>>(a);
-  return cudaGetLastError();
+  return awp_pipe::launch_after(k_frcvel, dim3(cdiv_u(a.npsrc, 256)), dim3(256), 0, st, a);
 }
 
 cudaError_t awp_launch_planesrc(const PlaneSrcArgs& a, cudaStream_t st) {
   if (a.nx <= 0 || a.ny <= 0) return cudaSuccess;
-  k_addplanesrc<<<dim3(cdiv_u(a.nx, 16), cdiv_u(a.ny, 16)), dim3(16, 16), 0, st>>>(a);
-  return cudaGetLastError();
+  return awp_pipe::launch_after(k_addplanesrc, dim3(cdiv_u(a.nx, 16), cdiv_u(a.ny, 16)), dim3(16, 16), 0, st, a);
 }
 
 cudaError_t awp_launch_addkinsrc(const KinSrcArgs& a, cudaStream_t st) {
   if (a.ncell <= 0) return cudaSuccess;
-  k_addkinsrc<<<cdiv_u(a.ncell, 128), 128, 0, st>>>(a);
-  return cudaGetLastError();
+  return awp_pipe::launch_after(k_addkinsrc, dim3(cdiv_u(a.ncell, 128)), dim3(128), 0, st, a);
 }
 
 cudaError_t awp_launch_plast_calc(const PlastCalcArgs& a, cudaStream_t st) {
   const int nk = a.k1 - a.k0 + 1, nj = a.j1 - a.j0 + 1, ni = a.i1 - a.i0 + 1;
   if (nk <= 0 || nj <= 0 || ni <= 0) return cudaSuccess;
-  k_plast_calc<<<dim3(cdiv_u(nk, 32), cdiv_u(nj, 4), ni), dim3(32, 4, 1), 0, st>>>(a);
-  return cudaGetLastError();
+  return awp_pipe::launch_after(k_plast_calc, dim3(cdiv_u(nk, 32), cdiv_u(nj, 4), ni), dim3(32, 4, 1), 0, st, a);
 }
 
 cudaError_t awp_launch_plast_app(const PlastAppArgs& a, cudaStream_t st) {
   const int nk = a.k1 - a.k0 + 1, nj = a.j1 - a.j0 + 1, ni = a.i1 - a.i0 + 1;
   if (nk <= 0 || nj <= 0 || ni <= 0) return cudaSuccess;
-  k_plast_app<<<dim3(cdiv_u(nk, 32), cdiv_u(nj, 4), ni), dim3(32, 4, 1), 0, st>>>(a);
-  return cudaGetLastError();
+  return awp_pipe::launch_after(k_plast_app, dim3(cdiv_u(nk, 32), cdiv_u(nj, 4), ni), dim3(32, 4, 1), 0, st, a);
 }
 
 cudaError_t awp_launch_velbuffer(const VelBufArgs& a, cudaStream_t st) {
   if (a.rec_nxt <= 0 || a.rec_nyt <= 0 || a.rec_nzt <= 0) return cudaSuccess;
   const dim3 block(32, 4, 1);
   const dim3 grid(cdiv_u(a.rec_nxt, 32), cdiv_u(a.rec_nyt, 4), a.rec_nzt);
-  k_velbuffer<<<grid, block, 0, st>>>(a);
-  return cudaGetLastError();
+  return awp_pipe::launch_after(k_velbuffer, grid, block, 0, st, a);
 }
 
 cudaError_t awp_launch_media(const MediaArgs& a, cudaStream_t st) {
@@ -1213,6 +1221,5 @@ cudaError_t awp_launch_sources_dev(const SrcArgs* a, const KinSrcArgs* k, const 
 }
 
 cudaError_t awp_launch_step_advance(int* step, int n, cudaStream_t st) {
-  k_step_advance<<<1, 1, 0, st>>>(step, n);
-  return cudaGetLastError();
+  return awp_pipe::launch_after(k_step_advance, dim3(1), dim3(1), 0, st, step, n);
 }

@@ -17,6 +17,9 @@ struct VelArgs {
   int slice, yline;
   int i0, i1, j0, j1, k0, k1;  // inclusive update ranges
   float dth, c1, c2;
+  // TMA kernel: > 0 on a mesh block over a coarser one: the level below k0 is
+  // the interface layer, updated to second order (dvelc2) for j <= layer_j1
+  int layer, layer_j1;
 };
 
 // ---------------------------------------------------------------------------
@@ -46,6 +49,7 @@ struct StrArgs {
   // bit pattern of 2*qthr, qthr the smallest float x with 1/(double)x <= 200:
   // the Q(f) switch on a pair sum of Q^-1
   unsigned thr;
+  int layer;     // TMA kernel: as VelArgs (dstrqc2 on the level below k0)
 };
 
 // ---------------------------------------------------------------------------

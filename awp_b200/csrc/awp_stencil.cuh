@@ -6,25 +6,6 @@
 #include "awp_common.h"
 #include "awp_f2.cuh"
 
-// Q(f) weight (kernel.cu:974-1040) before its division by wwo.  The reference
-// switches on 1./(q*2.0) <= 200.0 evaluated in double; for float q that is
-// exactly (2q >= qthr) for positive q, true for negative q and -0, false for
-// +0/NaN.  The reference evaluates the polynomial c0 (2q)^2 + c1 (2q) in
-// double; here it is float (the two differ by about one float ulp, far below
-// the 1e-5 parity bar, at a fraction of the instructions).
-__device__ __forceinline__ float awp_qf_weight_num(float q, float wwo, float c0, float c1,
-                                               float qthr) {
-  const float x = __fmul_rn(2.0f, q);
-  const bool low = (x >= qthr) || (x < 0.f) || (x == 0.f && signbit(x));
-  return low ? __fmaf_rn(__fmul_rn(c0, x), x, __fmul_rn(c1, x))
-             : __fmul_rn(__fmul_rn(2.0f, wwo), q);
-}
-
-__device__ __forceinline__ float awp_qf_weight(float q, float wwo, float c0, float c1,
-                                           float qthr) {
-  return awp_qf_weight_num(q, wwo, c0, c1, qthr) / wwo;  // the build's division mode
-}
-
 // ---------------------------------------------------------------------------
 // Rounding discipline.  The per-cell arithmetic below is written with explicit
 // rounding (intrinsics, or the packed instructions of awp_f2.cuh that round
@@ -41,13 +22,18 @@ __device__ __forceinline__ V awp_d4(float c1, float c2, V a, V b, V c, V d) {
   return vfma(vset<V>(c2), vsub(c, d), vscale(c1, vsub(a, b)));
 }
 
+// The same with a pair of weights per level.
+__device__ __forceinline__ float2 awp_d4(float2 c1, float2 c2, float2 a, float2 b, float2 c,
+                                         float2 d) {
+  return vfma(c2, vsub(c, d), vmul(c1, vsub(a, b)));
+}
+
 // Velocity update of dvelcx (kernel.cu:222-253):
 // (v + fd*(c1*x0 + c2*x1 + c1*y0 + c2*y1 + c1*z0 + c2*z1)) * dcrj, where
 // x0..z1 are the six differences of the three stress derivatives.
 template <class V>
-__device__ __forceinline__ V awp_vel_update(V v, V fd, float c1, float c2, V x0, V x1, V y0, V y1,
-                                            V z0, V z1, V dcrj) {
-  const V k1 = vset<V>(c1), k2 = vset<V>(c2);
+__device__ __forceinline__ V awp_vel_update(V v, V fd, V k1, V k2, V x0, V x1, V y0, V y1, V z0,
+                                            V z1, V dcrj) {
   V s = vmul(k1, x0);
   s = vfma(k2, x1, s);
   s = vfma(k1, y0, s);

@@ -14,7 +14,7 @@
 // copy bandwidth on the algorithmic bytes), against the form before (256
 // threads, one cell each, every x neighbour from shared memory, one barrier of
 // the CTA per plane, 554 thread instructions a cell in the stress update):
-//   velocity  800 -> 556 (0.66 -> 0.96),  stress 1815 -> 1385 (0.70 -> 0.92).
+//   velocity  800 -> 545 (0.66 -> 0.96),  stress 1815 -> 1388 (0.70 -> 0.92).
 //
 // Tile boxes (x = k fastest, y = j, z = i), all 16-byte aligned in x:
 //   halo   : 40 x 11 floats, k in [kb-4, kb+36), j from jb-1 or jb-2
@@ -80,7 +80,8 @@ struct StrCfg {
   static constexpr size_t bytes = sizeof(float) * (F_T + kTab) + sizeof(Pipe<NH, NO, NC / 32>);
 };
 
-template <bool ELASTIC>
+// LAYER: the launch takes a mesh block's interface layer too (StrArgs::layer).
+template <bool ELASTIC, bool LAYER>
 __global__ void __launch_bounds__(NT, ELASTIC ? 4 : 3)
     k_stress_tma(const __grid_constant__ StrArgs a, const __grid_constant__ TmaMaps tm, const int ichunk,
                  int* err, const unsigned spin) {
@@ -95,6 +96,7 @@ __global__ void __launch_bounds__(NT, ELASTIC ? 4 : 3)
   const int ie = min(ib + ichunk - 1, a.i1);
   const int n = ie - ib + 1;
 
+  grid_go();
   if (tid == 0) pipe.init();
   if (!ELASTIC) {
     // relaxation constants of the entry pairs (e, e + 1), e even, that two
@@ -107,6 +109,7 @@ __global__ void __launch_bounds__(NT, ELASTIC ? 4 : 3)
       if (tid < 8) tab[(tid >> 1) * 20 + 2 * q + (tid & 1)] = src[q][tid];
   }
   __syncthreads();
+  grid_wait();
 
   if (tid >= NC) {  // producer warp
     if (tid == NC) {
@@ -144,13 +147,16 @@ __global__ void __launch_bounds__(NT, ELASTIC ? 4 : 3)
   const int row = tid >> 4, kp = (tid & 15) * 2;
   const int k = kb + kp, j = jb + row;
   const bool jin = j <= a.j1;
-  const bool ax = jin && k >= a.k0 && k <= a.k1, ay = jin && k + 1 >= a.k0 && k + 1 <= a.k1;
+  // the interface layer of a mesh block: second order, weights (1, 0)
+  const bool layer = LAYER && k + 1 == a.k0;
+  const bool ax = jin && ((k >= a.k0 && k <= a.k1) || layer),
+             ay = jin && k + 1 >= a.k0 && k + 1 <= a.k1;
   const int S = a.slice, Y = a.yline;
-  const float c1 = a.c1, c2 = a.c2;
+  const float2 c1 = make_float2(layer ? 1.0f : a.c1, a.c1),
+               c2 = make_float2(layer ? 0.0f : a.c2, a.c2);
   const long long col = (long long)j * Y + k;
   const float dcy = LDG(a.dcrjy + min(j, a.j1));
-  const float2 dcz = make_float2(LDG(a.dcrjz + min(max(k, a.k0), a.k1)),
-                                 LDG(a.dcrjz + min(max(k + 1, a.k0), a.k1)));
+  const float2 dcz = ldg2(a.dcrjz + k);
   // the pair (ktop - 1, ktop): nzt is even, so the surface is a second level
   const bool top = a.fs && (k + 1 == a.ktop);
   float* __restrict__ SG[6] = {a.xx, a.yy, a.zz, a.xy, a.xz, a.yz};
@@ -252,6 +258,7 @@ __global__ void __launch_bounds__(NT, ELASTIC ? 4 : 3)
         };
         rx = {at(0), at(1), at(2), at(3), at(4), at(5), at(6), at(7), at(8)};
       }
+      if (LAYER && layer) rx.c2.x *= 0.5f;  // dstrqc2's high-Q branch is wwo*q, not 2*wwo*q
     }
     AwpStrCoef<float2> cf;
     {
@@ -300,15 +307,15 @@ __global__ void __launch_bounds__(NT, ELASTIC ? 4 : 3)
     float2 d[9];
     d[0] = awp_d4(c1, c2, u_p1, u_0, u_p2, u_m1);
     d[1] = awp_d4(c1, c2, v_0, v_jm1, v_jp1, v_jm2);
-    d[2] = make_float2(awp_d4(c1, c2, w_0.x, w_km.y, w_0.y, w_km.x),
-                       awp_d4(c1, c2, w_0.y, w_0.x, w_kp, w_km.y));
+    d[2] = make_float2(awp_d4(c1.x, c2.x, w_0.x, w_km.y, w_0.y, w_km.x),
+                       awp_d4(c1.y, c2.y, w_0.y, w_0.x, w_kp, w_km.y));
     d[3] = awp_d4(c1, c2, u_jp1, u_0, u_jp2, u_jm1);
     d[4] = awp_d4(c1, c2, v_0, v_m1, v_p1, v_m2);
-    d[5] = make_float2(awp_d4(c1, c2, u_0.y, u_0.x, u_kp.x, u_km1),
-                       awp_d4(c1, c2, u_kp.x, u_0.y, u_kp.y, u_0.x));
+    d[5] = make_float2(awp_d4(c1.x, c2.x, u_0.y, u_0.x, u_kp.x, u_km1),
+                       awp_d4(c1.y, c2.y, u_kp.x, u_0.y, u_kp.y, u_0.x));
     d[6] = awp_d4(c1, c2, w_0, w_m1, w_p1, w_m2);
-    d[7] = make_float2(awp_d4(c1, c2, v_0.y, v_0.x, v_kp.x, v_km1),
-                       awp_d4(c1, c2, v_kp.x, v_0.y, v_kp.y, v_0.x));
+    d[7] = make_float2(awp_d4(c1.x, c2.x, v_0.y, v_0.x, v_kp.x, v_km1),
+                       awp_d4(c1.y, c2.y, v_kp.x, v_0.y, v_kp.y, v_0.x));
     d[8] = awp_d4(c1, c2, w_jp1, w_0, w_jp2, w_jm1);
 
     ok = mbar_wait(pipe.full_o + co.slot, co.phase, spin);
@@ -363,6 +370,7 @@ struct VelCfg {
   static constexpr size_t bytes = sizeof(float) * F_END + sizeof(Pipe<NH, 0, NC / 32>);
 };
 
+template <bool LAYER>
 __global__ void __launch_bounds__(NT, 4)
     k_velocity_tma(const VelArgs a, const __grid_constant__ TmaMaps tm, const int ichunk,
                    int* err, const unsigned spin) {
@@ -376,8 +384,10 @@ __global__ void __launch_bounds__(NT, 4)
   const int ie = min(ib + ichunk - 1, a.i1);
   const int n = ie - ib + 1;
 
+  grid_go();
   if (tid == 0) pipe.init();
   __syncthreads();
+  grid_wait();
 
   if (tid >= NC) {  // producer warp
     if (tid == NC) {
@@ -409,11 +419,15 @@ __global__ void __launch_bounds__(NT, 4)
   const int row = tid >> 4, kp = (tid & 15) * 2;
   const int k = kb + kp, j = jb + row;
   const bool jin = j <= a.j1;
-  const bool ax = jin && k >= a.k0 && k <= a.k1, ay = jin && k + 1 >= a.k0 && k + 1 <= a.k1;
+  const bool layer = LAYER && k + 1 == a.k0;  // as in k_stress_tma (dvelc2)
+  const bool ax = layer ? j <= a.layer_j1 : jin && k >= a.k0 && k <= a.k1,
+             ay = jin && k + 1 >= a.k0 && k + 1 <= a.k1;
   const int S = a.slice, Y = a.yline;
-  const float c1 = a.c1, c2 = a.c2, dth = a.dth;
+  const float2 c1 = make_float2(layer ? 1.0f : a.c1, a.c1),
+               c2 = make_float2(layer ? 0.0f : a.c2, a.c2);
+  const float dth = a.dth;
   const float dcy = LDG(a.dcrjy + min(j, a.j1));
-  const float2 dcz = make_float2(LDG(a.dcrjz + min(k, a.k1)), LDG(a.dcrjz + min(k + 1, a.k1)));
+  const float2 dcz = ldg2(a.dcrjz + k);
   long long o = (long long)ib * S + (long long)j * Y + k;
   float2 xx_m2, xx_m1, xx_0, xy_m1, xy_0, xy_p1, xz_m1, xz_0, xz_p1;
   // density of the current plane: value, and the level below; rows j and j-1
@@ -567,7 +581,7 @@ int awp_tma_box(int group, int* bx, int* by) {
 
 namespace {
 
-Shape g_shape_str[2][kMaxDev], g_shape_vel[kMaxDev];
+Shape g_shape_str[4][kMaxDev], g_shape_vel[2][kMaxDev];
 constexpr int kMost = 6;  // planes of a march (march_planes)
 
 }  // namespace
@@ -578,17 +592,15 @@ cudaError_t awp_launch_stress_tma(const StrArgs& a, const TmaMaps& tm, bool elas
   if (nk <= 0 || nj <= 0 || ni <= 0) return cudaSuccess;
   const dim3 tile(cdiv_u(nk, TZ), cdiv_u(nj, TY));
   const size_t sm = elastic ? StrCfg<true>::bytes : StrCfg<false>::bytes;
-  const void* f = elastic ? (const void*)k_stress_tma<true> : (const void*)k_stress_tma<false>;
+  const auto f = elastic ? (a.layer ? k_stress_tma<true, true> : k_stress_tma<true, false>)
+                         : (a.layer ? k_stress_tma<false, true> : k_stress_tma<false, false>);
   int resident = 0;
-  const cudaError_t e = resident_ctas(f, sm, NT, g_shape_str[elastic ? 1 : 0], &resident);
+  const cudaError_t e = resident_ctas(
+      (const void*)f, sm, NT, g_shape_str[(elastic ? 2 : 0) + (a.layer ? 1 : 0)], &resident);
   if (e != cudaSuccess) return e;
   const int c = march_planes((long long)tile.x * tile.y, ni, resident, ichunk, kMost);
-  const dim3 grid(tile.x, tile.y, cdiv_u(ni, c));
-  if (elastic)
-    k_stress_tma<true><<<grid, NT, sm, st>>>(a, tm, c, err, awp_pipe_spin_limit);
-  else
-    k_stress_tma<false><<<grid, NT, sm, st>>>(a, tm, c, err, awp_pipe_spin_limit);
-  return cudaGetLastError();
+  return launch_after(f, dim3(tile.x, tile.y, cdiv_u(ni, c)), dim3(NT), sm, st, a, tm, c,
+                      err, awp_pipe_spin_limit);
 }
 
 cudaError_t awp_launch_velocity_tma(const VelArgs& a, const TmaMaps& tm, int ichunk, int* err,
@@ -596,14 +608,14 @@ cudaError_t awp_launch_velocity_tma(const VelArgs& a, const TmaMaps& tm, int ich
   const int nk = a.k1 - AWP_ALIGN + 1, nj = a.j1 - a.j0 + 1, ni = a.i1 - a.i0 + 1;
   if (nk <= 0 || nj <= 0 || ni <= 0) return cudaSuccess;
   const dim3 tile(cdiv_u(nk, TZ), cdiv_u(nj, TY));
+  const auto f = a.layer ? k_velocity_tma<true> : k_velocity_tma<false>;
   int resident = 0;
-  const cudaError_t e =
-      resident_ctas((const void*)k_velocity_tma, VelCfg::bytes, NT, g_shape_vel, &resident);
+  const cudaError_t e = resident_ctas((const void*)f, VelCfg::bytes, NT,
+                                      g_shape_vel[a.layer ? 1 : 0], &resident);
   if (e != cudaSuccess) return e;
   const int c = march_planes((long long)tile.x * tile.y, ni, resident, ichunk, kMost);
-  const dim3 grid(tile.x, tile.y, cdiv_u(ni, c));
-  k_velocity_tma<<<grid, NT, VelCfg::bytes, st>>>(a, tm, c, err, awp_pipe_spin_limit);
-  return cudaGetLastError();
+  return launch_after(f, dim3(tile.x, tile.y, cdiv_u(ni, c)), dim3(NT), VelCfg::bytes, st,
+                      a, tm, c, err, awp_pipe_spin_limit);
 }
 
 // the pipeline waits' poll limit

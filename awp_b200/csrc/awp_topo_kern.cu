@@ -57,11 +57,18 @@ constexpr float kZ0 = (float)-0.0026041666666667, kZ1 = (float)0.093750000000000
 constexpr unsigned kAll = 0xffffffffu;
 constexpr int kSpan = 64;     // levels of a warp
 constexpr int kTileOut = 56;  // output levels of a tile below the top one
-constexpr int kCol = 7;       // columns (computing warps) of a CTA: 8 warps with the producer
-constexpr int kThreads = 32 * (kCol + 1);
+// Columns (computing warps) of a CTA, and its tiles: own 64 x NC, j halo 64 x
+// (NC + 3), media 64 x (NC + 1).  Two CTAs of eight warps with the producer at
+// 116-128 registers; the velocity kernel's three CTAs at 80 were slower (433
+// -> 462 us at 384 x 384 x 160: spills).
+template <int NC>
+struct Tile {
+  static constexpr int kCol = NC, kThreads = 32 * (NC + 1);
+  static constexpr int kOwn = kSpan * NC, kHalo = kSpan * (NC + 3), kMed = kSpan * (NC + 1);
+};
+using VelTile = Tile<7>;
+using StrTile = Tile<7>;
 constexpr int kMost = 32;    // planes of a march (march_planes)
-// tiles: own 64 x kCol, j halo 64 x (kCol + 3), media 64 x (kCol + 1)
-constexpr int kOwn = kSpan * kCol, kHalo = kSpan * (kCol + 3), kMed = kSpan * (kCol + 1);
 
 __device__ __forceinline__ float2 dup(float a) { return make_float2(a, a); }
 
@@ -88,33 +95,48 @@ struct ColPos2 {
 };
 
 // Boundary-closure rows of one table for the lanes 29..31 of the top tile:
-// c[m][31 - lane] = the coefficients of level nz-1-m in the rows of the
-// lane's two levels (rows 2(31-lane) + 1 and 2(31-lane)).
+// c[31 - lane][p] = the coefficients of levels nz-1-2p (x, y) and nz-2-2p (z,
+// w) in the rows of the lane's two levels (rows 2(31-lane) + 1 and
+// 2(31-lane)).  The shared-memory pipe is the curvilinear kernels' busiest
+// (60 %), and the closures were 29 % of the velocity kernel's traffic as
+// broadcast shuffles: each lane now takes the top ten levels from lanes 27..31
+// as five pairs, and its coefficients four at a time.
 struct Closure {
-  float2 c[9][3];
+  float4 c[3][5];
 };
 template <int NT>
 __device__ __forceinline__ void closure_load(Closure& cl, const float (&T)[6][NT], int t) {
-  if (t < 27) {
-    const int m = t / 3, q = t % 3;
-    cl.c[m][q] = m < NT ? make_float2(T[2 * q + 1][m], T[2 * q][m]) : make_float2(0.f, 0.f);
+  if (t < 15) {
+    const int q = t / 5, m = 2 * (t % 5);
+    cl.c[q][t % 5] = make_float4(m < NT ? T[2 * q + 1][m] : 0.f, m < NT ? T[2 * q][m] : 0.f,
+                                 m + 1 < NT ? T[2 * q + 1][m + 1] : 0.f,
+                                 m + 1 < NT ? T[2 * q][m + 1] : 0.f);
   }
 }
 template <int NT>
 __device__ __forceinline__ float2 closure(float2 v, const ColPos2& c, const Closure& cl,
-                                          float2 s) {
-  const int q = c.lane >= 29 ? 31 - c.lane : 0;
+                                          float2* top, float2 s) {
+  // the warp's own scratch: this column's levels nz-10 .. nz-1
+  __syncwarp();
+  if (c.lane >= 27) top[31 - c.lane] = v;
+  __syncwarp();
+  const float4* const k = cl.c[c.lane >= 29 ? 31 - c.lane : 0];
   float2 b = make_float2(0.f, 0.f);
 #pragma unroll
-  for (int m = NT - 1; m >= 0; --m)
-    b = vfma(cl.c[m][q], dup(__shfl_sync(kAll, (m & 1) ? v.x : v.y, 31 - (m >> 1))), b);
+  for (int p = (NT + 1) / 2 - 1; p >= 0; --p) {
+    const float4 w = k[p];
+    const float2 t = top[p];  // levels nz-2-2p, nz-1-2p
+    if (2 * p + 1 < NT) b = vfma(make_float2(w.z, w.w), dup(t.x), b);
+    b = vfma(make_float2(w.x, w.y), dup(t.y), b);
+  }
   return c.lane >= 29 ? b : s;
 }
 
 // 7-point vertical difference at the lane's two levels l, l+1 of a value held
 // two levels per lane (interior coefficients), or the boundary rows in the
 // top tile.
-__device__ __forceinline__ float2 zd7(float2 v, const ColPos2& c, const Closure& cl) {
+__device__ __forceinline__ float2 zd7(float2 v, const ColPos2& c, const Closure& cl,
+                                      float2* top) {
   const float m3 = __shfl_up_sync(kAll, v.y, 2);    // l-3
   const float m2 = __shfl_up_sync(kAll, v.x, 1);    // l-2
   const float m1 = __shfl_up_sync(kAll, v.y, 1);    // l-1
@@ -124,13 +146,14 @@ __device__ __forceinline__ float2 zd7(float2 v, const ColPos2& c, const Closure&
   const float2 a = make_float2(m3 - p3, m2 - p4), b = make_float2(m2 - p2, m1 - p3),
                d = make_float2(m1 - v.y, v.x - p2);
   const float2 s = vfma(dup(kZ0), a, vfma(dup(kZ1), b, vscale(kZ2, d)));
-  return c.top ? closure<9>(v, c, cl, s) : s;  // warp-uniform branch
+  return c.top ? closure<9>(v, c, cl, top, s) : s;  // warp-uniform branch
 }
 
 // 4-point vertical difference: half-point form (k-2..k+1) or node form
 // (k-1..k+2), or the boundary rows (NT of them).
 template <bool HALF, int NT>
-__device__ __forceinline__ float2 zd4(float2 v, const ColPos2& c, const Closure& cl) {
+__device__ __forceinline__ float2 zd4(float2 v, const ColPos2& c, const Closure& cl,
+                                      float2* top) {
   const float m1 = __shfl_up_sync(kAll, v.y, 1), p2 = __shfl_down_sync(kAll, v.x, 1);
   float2 a, b;
   if (HALF) {
@@ -143,7 +166,7 @@ __device__ __forceinline__ float2 zd4(float2 v, const ColPos2& c, const Closure&
     b = make_float2(v.x - v.y, v.y - p2);
   }
   const float2 s = vfma(dup(kD0), a, vscale(kD1, b));
-  return c.top ? closure<NT>(v, c, cl, s) : s;
+  return c.top ? closure<NT>(v, c, cl, top, s) : s;
 }
 
 // The value at level - 1 of each of a lane's two levels
@@ -208,21 +231,23 @@ __device__ __forceinline__ float2 itp4(float2 a, float2 b, float2 c, float2 d) {
 enum VelW { kAx = 0, kAy = 4, kBx = 8, kBy = 12, kCy = 16, kCx = 20, kS = 24, kN = 30, kVelW = 33 };
 constexpr int kVelWPad = 40;
 
-struct TopoVelCfg {
+struct TopoVelCfg : VelTile {
   static constexpr int LA = 2, NH = 1 + LA, DS = 3 + LA;  // planes ahead, rings
   // one stage: xx(i+1), xz(i+2), yy, yz (j halo), zz, density, u, v, w (i)
   static constexpr int G_XX = 0, G_XZ = kOwn, G_YY = 2 * kOwn, G_YZ = G_YY + kHalo,
                        G_ZZ = G_YZ + kHalo, G_D = G_ZZ + kOwn, G_O = G_D + kMed,
                        STAGE = G_O + 3 * kOwn;
   static constexpr int F_S = DS * kHalo, F_W = F_S + NH * STAGE,
-                       F_C = F_W + kCol * 2 * kVelWPad * 2, F_END = F_C + 4 * 9 * 3 * 2;
+                       F_C = F_W + kCol * 2 * kVelWPad * 2, F_T = F_C + 4 * 60,
+                       F_G = F_T + kCol * 5 * 2, F_END = F_G + 7 * 64 + 4;
   static constexpr size_t bytes = sizeof(float) * F_END + sizeof(Pipe<NH, 0, kCol>) + 8;
 };
 
-__global__ void __launch_bounds__(kThreads, 2)
+__global__ void __launch_bounds__(VelTile::kThreads, 2)
     k_topo_velocity(const __grid_constant__ TopoArgs a, const __grid_constant__ TmaMaps tm,
                     const int ichunk, int* err, const unsigned spin) {
   using C = TopoVelCfg;
+  constexpr int kCol = C::kCol, kOwn = C::kOwn, kHalo = C::kHalo;
   extern __shared__ __align__(128) float smem[];
   Closure* const cl = reinterpret_cast<Closure*>(smem + C::F_C);
   auto& pipe = *reinterpret_cast<Pipe<C::NH, 0, kCol>*>(smem + C::F_END);
@@ -231,12 +256,27 @@ __global__ void __launch_bounds__(kThreads, 2)
   const int kb = AWP_ALIGN + a.nz - kSpan - kTileOut * (int)blockIdx.x;
   const int j0 = blockIdx.y * kCol, jb = j0 + AWP_NGSL + 2;
   const int i0 = blockIdx.z * ichunk, n = min(ichunk, a.nx - i0), ib = i0 + AWP_NGSL + 2;
+  grid_go();
   if (tid == 0) pipe.init();
   closure_load(cl[0], kTopoVelDhpz4r, tid);
   closure_load(cl[1], kTopoVelDphz4r, tid);
   closure_load(cl[2], kTopoVelDhz4r, tid);
   closure_load(cl[3], kTopoVelDz4r, tid);
+  // the vertical metrics depend on k alone: one copy for all the columns
+  enum { kGc, kGg, kG3c, kG3, kIg3c, kIg3, kDcz };
+  float2* const vm = reinterpret_cast<float2*>(smem + C::F_G);
+  if (warp == 0) {
+    vm[32 * kGc + c.lane] = gk2(a.g_c, c.ld);
+    vm[32 * kGg + c.lane] = gk2(a.g, c.ld);
+    vm[32 * kG3c + c.lane] = gk2(a.g3_c, c.ld);
+    vm[32 * kG3 + c.lane] = gk2(a.g3, c.ld);
+    vm[32 * kIg3c + c.lane] = vquot(1.0f, gk2(a.g3_c, c.ld));
+    vm[32 * kIg3 + c.lane] = vquot(1.0f, gk2(a.g3, c.ld));
+    vm[32 * kDcz + c.lane] = gk2(a.dcrjz, c.ld);
+  }
+  auto M = [&](int q) { return vm[32 * q + c.lane]; };
   __syncthreads();
+  grid_wait();
 
   if (warp == kCol) {  // producer warp
     if (c.lane == 0) {
@@ -269,6 +309,9 @@ __global__ void __launch_bounds__(kThreads, 2)
   const int S = a.slice, Y = a.yline, FL = a.fld;
   const int ja = jb + warp;  // a warp past the grid computes on its padding
   const int jm = min(j, a.ny - 1);
+  // the lowest tile's lane of levels 2 and 3 takes the interface layer
+  const bool low = a.layer && blockIdx.x + 1 == gridDim.x;
+  const bool lay = low && c.k == 2 && c.lane >= 2 && (c.top || c.lane <= 29) && jin;
   long long o = (long long)ib * S + (long long)ja * Y + (c.ld + AWP_ALIGN);
   // this lane's two weights of the column (weight index lane, lane + 32)
   Table<kVelWPad>& tab = reinterpret_cast<Table<kVelWPad>*>(smem + C::F_W)[warp];
@@ -301,11 +344,8 @@ __global__ void __launch_bounds__(kThreads, 2)
   const Weight w0 = weight(c.lane), w1 = weight(c.lane + 32);
   float n0 = w0.at(0), n1 = c.lane < 1 ? w1.at(0) : 0.f;
 
-  const float2 g3c = gk2(a.g3_c, c.ld), g3 = gk2(a.g3, c.ld), gc = gk2(a.g_c, c.ld),
-               gg = gk2(a.g, c.ld);
-  const float2 ig3c = vquot(1.0f, g3c), ig3 = vquot(1.0f, g3);
   const float dcy = __ldg(a.dcrjy + ja);
-  const float2 dcz = gk2(a.dcrjz, c.ld);
+  float2* const top = reinterpret_cast<float2*>(smem + C::F_T) + warp * 5;
   // own-column values of the planes before the ones the tiles bring
   float2 xx_m2, xx_m1, xx_0, xy_m1, xy_0, xy_p1, xz_m1, xz_0, xz_p1, d_m, t_m;
   {
@@ -344,19 +384,26 @@ __global__ void __launch_bounds__(kThreads, 2)
     const float2 xx_p1 = lds2(G + C::G_XX + h0), xz_p2 = lds2(G + C::G_XZ + h0);
     const float2 xy_p2 = lds2(smem + ss2 * kHalo + h2);
     const float2 d_0 = lds2(G + C::G_D + h1), t_0 = vadd(d_0, lds2(G + C::G_D + h0));
-    const float2 dcrj = vscale(dcx * dcy, dcz);
+    const float2 dcrj = vscale(dcx * dcy, M(kDcz));
 
     // --- u1 -----------------------------------------------------------------
     {
       const float2 y2 = lds2(XY - 2 * kSpan), y1 = lds2(XY - kSpan), yp = lds2(XY + kSpan);
       float2 e = dot4(W + kAx, xx_m2, xx_m1, xx_0, xx_p1);
       e = dot4(W + kAy, y2, y1, xy_0, yp, e);
-      e = vfma(g3c, e, zd4<true, 8>(xz_0, c, cl[2]));
+      e = vfma(M(kG3c), e, zd4<true, 8>(xz_0, c, cl[2], top));
       float2 q = vmul(W[kS], itp4(xx_m2, xx_m1, xx_0, xx_p1));
       q = vfma(W[kS + 1], itp4(y2, y1, xy_0, yp), q);
-      e = vsub(e, zd7(vmul(gc, q), c, cl[0]));
-      const float2 A = vmul(vmul(W[kN], ig3c), vquot(1.0f, vscale(0.25f, vadd(t_0, below(t_0)))));
-      st2(a.u1 + o, vmul(vfma(A, e, lds2(G + C::G_O + h0)), dcrj), o0, o1);
+      e = vsub(e, zd7(vmul(M(kGc), q), c, cl[0], top));
+      const float2 ir = vquot(1.0f, vscale(0.25f, vadd(t_0, below(t_0))));
+      const float2 A = vmul(vmul(W[kN], M(kIg3c)), ir), u0 = lds2(G + C::G_O + h0);
+      float2 u = vmul(vfma(A, e, u0), dcrj);
+      if (low) {  // dvelc2 (kernel.cu:2289-2343)
+        const float km = __shfl_up_sync(kAll, xz_0.y, 1);
+        const float su = (xx_0.x - xx_m1.x) + (xy_0.x - y1.x) + (xz_0.x - km);
+        if (lay) u.x = __fmul_rn(__fmaf_rn(a.nu * ir.x, su, u0.x), dcrj.x);
+      }
+      st2(a.u1 + o, u, o0 || lay, o1);
     }
     const float2 yz_0 = lds2(YZ);
     // --- u2 -----------------------------------------------------------------
@@ -365,25 +412,45 @@ __global__ void __launch_bounds__(kThreads, 2)
                    y2 = lds2(YY + 2 * kSpan);
       float2 e = dot4(W + kBx, xy_m1, xy_0, xy_p1, xy_p2);
       e = dot4(W + kBy, ym, y0, y1, y2, e);
-      e = vfma(g3c, e, zd4<true, 8>(yz_0, c, cl[2]));
+      e = vfma(M(kG3c), e, zd4<true, 8>(yz_0, c, cl[2], top));
       float2 q = vmul(W[kS + 2], itp4(xy_m1, xy_0, xy_p1, xy_p2));
       q = vfma(W[kS + 3], itp4(ym, y0, y1, y2), q);
-      e = vsub(e, zd7(vmul(gc, q), c, cl[0]));
+      e = vsub(e, zd7(vmul(M(kGc), q), c, cl[0], top));
       const float2 x = vadd(d_0, d_m);
-      const float2 A = vmul(vmul(W[kN + 1], ig3c), vquot(1.0f, vscale(0.25f, vadd(x, below(x)))));
-      st2(a.v1 + o, vmul(vfma(A, e, lds2(G + C::G_O + kOwn + h0)), dcrj), o0, o1);
+      const float2 A = vmul(vmul(W[kN + 1], M(kIg3c)), vquot(1.0f, vscale(0.25f, vadd(x, below(x)))));
+      const float2 v0 = lds2(G + C::G_O + kOwn + h0);
+      float2 v = vmul(vfma(A, e, v0), dcrj);
+      if (low) {
+        const float km = __shfl_up_sync(kAll, yz_0.y, 1), dk = __shfl_up_sync(kAll, d_0.y, 1);
+        if (lay) {
+          const float* D = a.d1 + o + S;
+          const float sv = (xy_p1.x - xy_0.x) + (y1.x - y0.x) + (yz_0.x - km);
+          const float r = __fmul_rn(0.25f, (d_0.x + D[0]) + (dk + D[-1]));
+          v.x = __fmul_rn(__fmaf_rn(__fdividef(a.nu, r), sv, v0.x), dcrj.x);
+        }
+      }
+      st2(a.v1 + o, v, o0 || lay, o1);
     }
     // --- u3 -----------------------------------------------------------------
     {
       const float2 y2 = lds2(YZ - 2 * kSpan), y1 = lds2(YZ - kSpan), yp = lds2(YZ + kSpan);
       float2 e = dot4(W + kCy, y2, y1, yz_0, yp);
       e = dot4(W + kCx, xz_m1, xz_0, xz_p1, xz_p2, e);
-      e = vfma(g3, e, zd4<false, 7>(lds2(G + C::G_ZZ + h0), c, cl[3]));
+      const float2 z = lds2(G + C::G_ZZ + h0);
+      e = vfma(M(kG3), e, zd4<false, 7>(z, c, cl[3], top));
       float2 q = vmul(W[kS + 4], itp4(xz_m1, xz_0, xz_p1, xz_p2));
       q = vfma(W[kS + 5], itp4(y2, y1, yz_0, yp), q);
-      e = vsub(e, zd7(vmul(gg, q), c, cl[1]));
-      const float2 A = vmul(vmul(W[kN + 2], ig3), vquot(1.0f, vscale(0.25f, vadd(t_0, t_m))));
-      st2(a.w1 + o, vmul(vfma(A, e, lds2(G + C::G_O + 2 * kOwn + h0)), dcrj), o0, o1);
+      e = vsub(e, zd7(vmul(M(kGg), q), c, cl[1], top));
+      const float2 A = vmul(vmul(W[kN + 2], M(kIg3)), vquot(1.0f, vscale(0.25f, vadd(t_0, t_m))));
+      const float2 w0 = lds2(G + C::G_O + 2 * kOwn + h0);
+      float2 w = vmul(vfma(A, e, w0), dcrj);
+      if (lay) {
+        const float* D = a.d1 + o + S;
+        const float sw = (xz_p1.x - xz_0.x) + (yz_0.x - y1.x) + (z.y - z.x);
+        const float r = __fmul_rn(0.25f, t_0.x + (D[0] + D[-Y]));
+        w.x = __fmul_rn(__fmaf_rn(__fdividef(a.nu, r), sw, w0.x), dcrj.x);
+      }
+      st2(a.w1 + o, w, o0 || lay, o1);
     }
     warp_done(pipe.done + cd.slot, c.lane);
 
@@ -407,23 +474,24 @@ __global__ void __launch_bounds__(kThreads, 2)
 enum StrW { kIu = 0, kIv = 4, kJu = 8, kJv = 12, kKw = 16, kLw = 20, kF = 24, kStrW = 28 };
 
 template <bool ELASTIC>
-struct TopoStrCfg {
+struct TopoStrCfg : StrTile {
   static constexpr int NM = ELASTIC ? 2 : 4, NF = ELASTIC ? 6 : 12;
   static constexpr int LH = 2, LO = 1, NH = 1 + LH, NO = 1 + LO, DU = 3 + LH, DV = 2 + LH;
   static constexpr int F_U = 0, F_V = F_U + DU * kHalo, F_W = F_V + DV * kHalo,
                        F_M = F_W + DV * kHalo, F_O = F_M + NH * NM * kMed,
                        F_T = F_O + NO * NF * kOwn, F_X = F_T + (ELASTIC ? 0 : 80),
-                       F_C = F_X + kCol * 2 * 32 * 2, F_G = F_C + 4 * 9 * 3 * 2,
-                       F_END = F_G + 6 * 64;  // vertical metrics of the lanes
+                       F_C = F_X + kCol * 2 * 32 * 2, F_L = F_C + 4 * 60,
+                       F_G = F_L + kCol * 5 * 2 + 2, F_END = F_G + 6 * 64;  // vertical metrics of the lanes
   static constexpr size_t bytes = sizeof(float) * F_END + sizeof(Pipe<NH, NO, kCol>) + 8;
 };
 
 template <bool ELASTIC>
-__global__ void __launch_bounds__(kThreads, 2)
+__global__ void __launch_bounds__(StrTile::kThreads, 2)
     k_topo_stress(const __grid_constant__ TopoArgs a, const __grid_constant__ TmaMaps tm,
                   const int ichunk, int* err, const unsigned spin) {
   using C = TopoStrCfg<ELASTIC>;
   constexpr int NM = C::NM, NF = C::NF;
+  constexpr int kCol = C::kCol, kOwn = C::kOwn, kHalo = C::kHalo, kMed = C::kMed;
   extern __shared__ __align__(128) float smem[];
   Closure* const cl = reinterpret_cast<Closure*>(smem + C::F_C);
   auto& pipe = *reinterpret_cast<Pipe<C::NH, C::NO, kCol>*>(smem + C::F_END);
@@ -433,6 +501,7 @@ __global__ void __launch_bounds__(kThreads, 2)
   const int j0 = a.s_j + blockIdx.y * kCol, jb = j0 + AWP_NGSL + 2;
   const int i0 = a.s_i + blockIdx.z * ichunk, n = min(ichunk, a.e_i - i0),
             ib = i0 + AWP_NGSL + 2;
+  grid_go();
   if (tid == 0) pipe.init();
   closure_load(cl[0], kTopoStrPhdz4r, tid);
   closure_load(cl[1], kTopoStrPdhz4r, tid);
@@ -462,6 +531,7 @@ __global__ void __launch_bounds__(kThreads, 2)
     vm[32 * kDcz + c.lane] = gk2(a.dcrjz, c.ld);
   }
   __syncthreads();
+  grid_wait();
 
   if (warp == kCol) {  // producer warp
     if (c.lane == 0) {
@@ -497,6 +567,8 @@ __global__ void __launch_bounds__(kThreads, 2)
   const bool o0 = c.out0 && jin, o1 = c.out1 && jin;
   const int S = a.slice, Y = a.yline, FL = a.fld;
   const int ja = jb + warp, jm = min(j, a.ny - 1);
+  const bool low = a.layer && blockIdx.x + 1 == gridDim.x;  // as in k_topo_velocity
+  const bool lay = low && c.k == 2 && c.lane >= 2 && (c.top || c.lane <= 29) && jin;
   long long o = (long long)ib * S + (long long)ja * Y + (c.ld + AWP_ALIGN);
   float* __restrict__ SG[6] = {a.xx, a.yy, a.zz, a.xy, a.xz, a.yz};
   float* __restrict__ RR[6] = {a.r1, a.r2, a.r3, a.r4, a.r5, a.r6};
@@ -526,6 +598,7 @@ __global__ void __launch_bounds__(kThreads, 2)
 
   auto G = [&](int q) { return vm[32 * q + c.lane]; };
   const float dcy = __ldg(a.dcrjy + ja);
+  float2* const top = reinterpret_cast<float2*>(smem + C::F_L) + warp * 5;
   // texture entry pairs at even and odd steps (two adjacent levels starting at
   // an even one: entries e, e + 1)
   const int e0 = awp_tex_index(a.tex, ib, ja, c.k + AWP_ALIGN) >> 1,
@@ -588,9 +661,17 @@ __global__ void __launch_bounds__(kThreads, 2)
       const float2 J = vmul(W[kF], G(kIg3c)), Jg = vmul(J, G(kGc));
       const float2 v2 = lds2(V0 - 2 * kSpan), v1 = lds2(V0 - kSpan), vp = lds2(V0 + kSpan);
       d[0] = vsub(diff4(u_m1, u_0, u_p1, u_p2),
-                  vmul(Jg, zd7(dot4(W + kIu, u_m1, u_0, u_p1, u_p2), c, cl[0])));
-      d[1] = vsub(diff4(v2, v1, v_0, vp), vmul(Jg, zd7(dot4(W + kIv, v2, v1, v_0, vp), c, cl[0])));
-      d[2] = vmul(J, zd4<true, 8>(w_0, c, cl[2]));
+                  vmul(Jg, zd7(dot4(W + kIu, u_m1, u_0, u_p1, u_p2), c, cl[0], top)));
+      d[1] = vsub(diff4(v2, v1, v_0, vp), vmul(Jg, zd7(dot4(W + kIv, v2, v1, v_0, vp), c, cl[0], top)));
+      d[2] = vmul(J, zd4<true, 8>(w_0, c, cl[2], top));
+      if (low) {  // dstrqc2 (kernel.cu:2564-2767): second-order rates, Cartesian
+        const float km = __shfl_up_sync(kAll, w_0.y, 1);
+        if (lay) {
+          d[0].x = u_p1.x - u_0.x;
+          d[1].x = v_0.x - v1.x;
+          d[2].x = w_0.x - km;
+        }
+      }
     }
     {
       // xy: J12i = 1 / (f g3_c)
@@ -598,22 +679,34 @@ __global__ void __launch_bounds__(kThreads, 2)
       const float2 um = lds2(U0 - kSpan), u1 = lds2(U0 + kSpan), u2 = lds2(U0 + 2 * kSpan);
       const float2 q = dot4(W + kJv, v_m2, v_m1, v_0, v_p1, dot4(W + kJu, um, u_0, u1, u2));
       d[3] = diff4(um, u_0, u1, u2);
-      d[4] = vsub(diff4(v_m2, v_m1, v_0, v_p1), vmul(J, zd7(q, c, cl[0])));
+      d[4] = vsub(diff4(v_m2, v_m1, v_0, v_p1), vmul(J, zd7(q, c, cl[0], top)));
+      if (lay) {
+        d[3].x = u1.x - u_0.x;
+        d[4].x = v_0.x - v_m1.x;
+      }
     }
     {
       // xz: J13i = 1 / (f_1 g3) (:550-598, :1254-1317)
       const float2 J = vmul(W[kF + 2], G(kIg3));
-      const float2 z = zd7(dot4(W + kKw, w_m2, w_m1, w_0, w_p1), c, cl[1]);
-      d[5] = vmul(J, vsub(zd4<false, 7>(u_0, c, cl[3]), vmul(G(kGg), z)));
+      const float2 z = zd7(dot4(W + kKw, w_m2, w_m1, w_0, w_p1), c, cl[1], top);
+      d[5] = vmul(J, vsub(zd4<false, 7>(u_0, c, cl[3], top), vmul(G(kGg), z)));
       d[6] = diff4(w_m2, w_m1, w_0, w_p1);
+      if (lay) {
+        d[5].x = u_0.y - u_0.x;
+        d[6].x = w_0.x - w_m1.x;
+      }
     }
     {
       // yz: J23i = 1 / (f_2 g3) (:600-650, :1319-1380)
       const float2 J = vmul(W[kF + 3], G(kIg3));
       const float2 wm = lds2(W0 - kSpan), w1 = lds2(W0 + kSpan), w2 = lds2(W0 + 2 * kSpan);
-      const float2 z = zd7(dot4(W + kLw, wm, w_0, w1, w2), c, cl[1]);
-      d[7] = vmul(J, vsub(zd4<false, 7>(v_0, c, cl[3]), vmul(G(kGg), z)));
+      const float2 z = zd7(dot4(W + kLw, wm, w_0, w1, w2), c, cl[1], top);
+      d[7] = vmul(J, vsub(zd4<false, 7>(v_0, c, cl[3], top), vmul(G(kGg), z)));
       d[8] = diff4(wm, w_0, w1, w2);
+      if (lay) {
+        d[7].x = v_0.y - v_0.x;
+        d[8].x = w1.x - w_0.x;
+      }
     }
 
     // ---- material coefficients and the update (as the Cartesian dstrqc) -----
@@ -627,6 +720,7 @@ __global__ void __launch_bounds__(kThreads, 2)
       rx.kr2 = make_float2(q2.x, q2.y); rx.kf = make_float2(q2.z, q2.w);
       rx.c0 = make_float2(q3.x, q3.y); rx.c1 = make_float2(q3.z, q3.w);
       rx.c2 = lds2(t + 16);
+      if (lay) rx.c2.x *= 0.5f;
     }
     AwpStrCoef<float2> cf;
     {
@@ -664,11 +758,12 @@ __global__ void __launch_bounds__(kThreads, 2)
       if (!ELASTIC) rr[q] = lds2(O + (6 + q) * kOwn);
     }
     awp_stress_update<ELASTIC>(sg, rr, cf, rx, dcrj, d);
-    if (o0 || o1) {
+    if (o0 || o1) {  // (lay has o1)
+      const bool ox = o0 || lay;
 #pragma unroll
       for (int q = 0; q < 6; ++q) {
-        st2(SG[q] + o, sg[q], o0, o1);
-        if (!ELASTIC) st2(RR[q] + o, rr[q], o0, o1);
+        st2(SG[q] + o, sg[q], ox, o1);
+        if (!ELASTIC) st2(RR[q] + o, rr[q], ox, o1);
       }
     }
     warp_done(pipe.done + cd.slot, c.lane);
@@ -698,24 +793,26 @@ Shape g_shape_vel[kMaxDev], g_shape_str[2][kMaxDev];
 
 }  // namespace
 
-int awp_topo_box(int group, int* bx, int* by) {
+int awp_topo_box(int kernel, int group, int* bx, int* by) {
+  const int nc = kernel == 0 ? VelTile::kCol : StrTile::kCol;
   *bx = kSpan;
-  *by = group == 0 ? kCol + 3 : group == 1 ? kCol + 1 : kCol;
+  *by = group == 0 ? nc + 3 : group == 1 ? nc + 1 : nc;
   return 0;
 }
 
 cudaError_t awp_launch_topo_velocity(const TopoArgs& a, const TmaMaps& tm, int ichunk, int* err,
                                      cudaStream_t st) {
   if (a.nz < 12 || a.nx < 1 || a.ny < 1) return cudaErrorInvalidValue;
-  const dim3 tile(column_tiles(a.nz), cdiv_u(a.ny, kCol));
+  const dim3 tile(column_tiles(a.nz), cdiv_u(a.ny, VelTile::kCol));
   int resident = 0;
-  const cudaError_t e = resident_ctas((const void*)k_topo_velocity, TopoVelCfg::bytes, kThreads,
+  const cudaError_t e = resident_ctas((const void*)k_topo_velocity, TopoVelCfg::bytes,
+                                      VelTile::kThreads,
                                       g_shape_vel, &resident);
   if (e != cudaSuccess) return e;
   const int ch = march_planes((long long)tile.x * tile.y, a.nx, resident, ichunk, kMost);
-  k_topo_velocity<<<dim3(tile.x, tile.y, cdiv_u(a.nx, ch)), kThreads, TopoVelCfg::bytes, st>>>(
-      a, tm, ch, err, awp_pipe_spin_limit);
-  return cudaGetLastError();
+  return launch_after(k_topo_velocity, dim3(tile.x, tile.y, cdiv_u(a.nx, ch)),
+                      dim3(VelTile::kThreads), TopoVelCfg::bytes, st, a, tm, ch, err,
+                      awp_pipe_spin_limit);
 }
 
 cudaError_t awp_launch_topo_stress(const TopoArgs& a, const TmaMaps& tm, bool elastic, int ichunk,
@@ -723,17 +820,14 @@ cudaError_t awp_launch_topo_stress(const TopoArgs& a, const TmaMaps& tm, bool el
   if (a.nz < 12) return cudaErrorInvalidValue;
   const int ni = a.e_i - a.s_i, nj = a.e_j - a.s_j;
   if (ni <= 0 || nj <= 0) return cudaSuccess;
-  const dim3 tile(column_tiles(a.nz), cdiv_u(nj, kCol));
+  const dim3 tile(column_tiles(a.nz), cdiv_u(nj, StrTile::kCol));
   const size_t sm = elastic ? TopoStrCfg<true>::bytes : TopoStrCfg<false>::bytes;
   const void* f = elastic ? (const void*)k_topo_stress<true> : (const void*)k_topo_stress<false>;
   int resident = 0;
-  const cudaError_t e = resident_ctas(f, sm, kThreads, g_shape_str[elastic ? 1 : 0], &resident);
+  const cudaError_t e = resident_ctas(f, sm, StrTile::kThreads, g_shape_str[elastic ? 1 : 0], &resident);
   if (e != cudaSuccess) return e;
   const int ch = march_planes((long long)tile.x * tile.y, ni, resident, ichunk, kMost);
   const dim3 grid(tile.x, tile.y, cdiv_u(ni, ch));
-  if (elastic)
-    k_topo_stress<true><<<grid, kThreads, sm, st>>>(a, tm, ch, err, awp_pipe_spin_limit);
-  else
-    k_topo_stress<false><<<grid, kThreads, sm, st>>>(a, tm, ch, err, awp_pipe_spin_limit);
-  return cudaGetLastError();
+  return launch_after(elastic ? k_topo_stress<true> : k_topo_stress<false>, grid,
+                      dim3(StrTile::kThreads), sm, st, a, tm, ch, err, awp_pipe_spin_limit);
 }

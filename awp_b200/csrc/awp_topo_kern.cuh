@@ -22,13 +22,16 @@ struct TopoArgs {
   float DT, dth, dh1;    // stress: (dt/h)*h, DT/h, 1/h (topo_set_constants)
   unsigned thr;          // Q(f) switch on a pair sum of Q^-1 (StrArgs::thr)
   int s_i, e_i, s_j, e_j;  // stress window, relative indices, ends exclusive
+  // > 0 on a block over a coarser one: level 2, the interface layer, is updated
+  // to second order too (dvelc2; dstrqc2 inside the stress window)
+  int layer;
 };
 
 // dtopo_vel_111_unroll + dtopo_vel_112 (velocity_unroll.cu, optimized_velocity.cu:1040-1629)
 // tensor maps: the TmaMaps groups of the velocity and stress kernels with the
-// boxes of awp_topo_box (group 0: j halo, 1: media, 2: own); ichunk: x planes a
-// CTA marches at most
-int awp_topo_box(int group, int* box_x, int* box_y);
+// boxes of awp_topo_box (kernel 0: velocity, 1: stress; group 0: j halo, 1:
+// media, 2: own); ichunk: x planes a CTA marches at most
+int awp_topo_box(int kernel, int group, int* box_x, int* box_y);
 cudaError_t awp_launch_topo_velocity(const TopoArgs& a, const TmaMaps& tm, int ichunk, int* err,
                                      cudaStream_t st);
 // dtopo_str_111 + dtopo_str_112 (kernels/stress_attenuation.cu:73-1415)
