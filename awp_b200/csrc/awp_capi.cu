@@ -462,7 +462,7 @@ int phase_velocity(awp_ctx* c) {
 
 // Middle band of the NVE = 3 stress split at one rank: xss2..xse2 x
 // yls2..yre2 (pmcl3d.c:573-631; ylsp = yls, yrep = yre at one rank).
-void middle_band(const awp_ctx* c, int* i0, int* i1, int* j0, int* j1) {
+AwpBox middle_band(const awp_ctx* c) {
   const int yls = c->yls, yre = c->yre;
   int yls2 = (int)(yls + (int)(yre - yls) * 0.25);
   if (yls2 % 2 != 0) yls2 += 1;
@@ -470,27 +470,30 @@ void middle_band(const awp_ctx* c, int* i0, int* i1, int* j0, int* j1) {
   if (yre2 % 2 == 0) yre2 -= 1;
   // x range of the whole grid, in this part's indices when it is a sub-domain
   const int x0 = c->sub_nxg ? c->sub_x0 : 0, nxg = c->sub_nxg ? c->sub_nxg : c->g.nxt;
-  *i0 = std::max(AWP_NGSL + 4 - x0, c->sub_nxg ? c->xls : 0);
-  *i1 = std::min(nxg + AWP_NGSL - 1 - x0, c->sub_nxg ? c->xre : INT_MAX);
-  *j0 = std::max(yls2, yls + AWP_NGSL + 2);
-  *j1 = std::min(yre2, yre - AWP_NGSL - 2);
+  return {std::max(AWP_NGSL + 4 - x0, c->sub_nxg ? c->xls : 0),
+          std::min(nxg + AWP_NGSL - 1 - x0, c->sub_nxg ? c->xre : INT_MAX),
+          std::max(yls2, yls + AWP_NGSL + 2), std::min(yre2, yre - AWP_NGSL - 2)};
 }
 
-// Cartesian stress (+ memory variables) over i0..i1 x j0..j1 of the stress
+// Cartesian stress (+ memory variables) over n disjoint boxes of the stress
 // window, with the kernel family the tuning selects.
 // `layer` (TMA kernel): the interface layer too.
-int launch_cart_stress(awp_ctx* c, int i0, int i1, int j0, int j1, bool layer = false) {
-  if (i1 < i0 || j1 < j0) return AWP_OK;
-  const bool tma = awp_tuning_get("tma_str") == 1 && tma_ready(c);
+int launch_cart_stress(awp_ctx* c, const AwpBox* box, int n, bool layer = false) {
   StrArgs s = make_str_args(c);
-  s.i0 = i0; s.i1 = i1; s.j0 = j0; s.j1 = j1;
   s.layer = layer ? 1 : 0;
-  if (tma)
-    CU_TRY(awp_launch_stress_tma(s, c->str_maps, c->elastic, awp_tuning_get("ichunk"),
+  if (awp_tuning_get("tma_str") == 1 && tma_ready(c)) {
+    if (std::all_of(box, box + n, [](const AwpBox& b) { return b.empty(); })) return AWP_OK;
+    CU_TRY(awp_launch_stress_tma(s, box, n, c->str_maps, c->elastic, awp_tuning_get("ichunk"),
                                  c->d_err, c->stream));
-  else
+    c->launches++;
+    return AWP_OK;
+  }
+  for (int q = 0; q < n; ++q) {
+    if (box[q].empty()) continue;
+    s.i0 = box[q].i0; s.i1 = box[q].i1; s.j0 = box[q].j0; s.j1 = box[q].j1;
     CU_TRY(awp_launch_stress(s, c->elastic, c->stream));
-  c->launches++;
+    c->launches++;
+  }
   return AWP_OK;
 }
 
@@ -532,14 +535,14 @@ int phase_stress(awp_ctx* c) {
     return AWP_OK;
   }
   PhaseScope ps(c, 1);
-  if (!stress_split(c))
-    return launch_cart_stress(c, c->xls, c->xre, c->yls, c->yre, stress_layer(c));
-  int i0, i1, j0, j1, st;
-  middle_band(c, &i0, &i1, &j0, &j1);
-  if ((st = launch_cart_stress(c, i0, i1, c->yls, j0 - 1))) return st;  // xss2, front
-  if ((st = launch_cart_stress(c, i0, i1, j1 + 1, c->yre))) return st;  // xss2, back
-  if ((st = launch_cart_stress(c, c->xls, i0 - 1, c->yls, c->yre))) return st;  // xss1
-  return launch_cart_stress(c, i1 + 1, c->xre, c->yls, c->yre);                 // xss3
+  const AwpBox all{c->xls, c->xre, c->yls, c->yre}, m = middle_band(c);
+  if (!stress_split(c)) return launch_cart_stress(c, &all, 1, stress_layer(c));
+  // xss2 in front of and behind the band, xss1, xss3
+  const AwpBox rest[4] = {{m.i0, m.i1, all.j0, m.j0 - 1},
+                          {m.i0, m.i1, m.j1 + 1, all.j1},
+                          {all.i0, m.i0 - 1, all.j0, all.j1},
+                          {m.i1 + 1, all.i1, all.j0, all.j1}};
+  return launch_cart_stress(c, rest, 4);
 }
 
 bool sources_with_fstr(const awp_ctx* c);
@@ -608,9 +611,8 @@ int phase_plasticity(awp_ctx* c) {
   int st;
   if (stress_split(c)) {  // the middle band of the stress split (pmcl3d.c:2139-2148)
     PhaseScope ps(c, 1);
-    int i0, i1, j0, j1;
-    middle_band(c, &i0, &i1, &j0, &j1);
-    if ((st = launch_cart_stress(c, i0, i1, j0, j1))) return st;
+    const AwpBox m = middle_band(c);
+    if ((st = launch_cart_stress(c, &m, 1))) return st;
   }
   PhaseScope ps(c, 3);
   // a sub-domain's ghost planes take the neighbours' updated stresses (the
@@ -1985,9 +1987,8 @@ int decomp_step(awp_decomp* d) {
                            // halo, the return
     for (int p = 0; p < d->n; ++p) {
       if (!stress_split(c[p])) continue;
-      int i0, i1, j0, j1;
-      middle_band(c[p], &i0, &i1, &j0, &j1);
-      if ((st = launch_cart_stress(c[p], i0, i1, j0, j1))) return st;
+      const AwpBox m = middle_band(c[p]);
+      if ((st = launch_cart_stress(c[p], &m, 1))) return st;
     }
     if ((st = decomp_exchange(d, AWP_HALO_STRESS))) return st;
     for (int p = 0; p < d->n; ++p) {

@@ -207,20 +207,25 @@ inline cudaError_t resident_ctas(const void* kernel, size_t smem, int threads,
 // waves takes the chunk with the least waves x (planes + fill), fill being
 // the planes' worth of time a march spends before its first result
 // (48 x 40 x 36: 34 -> 9 us and 60 -> 13 us for the two kernels).
-inline int march_planes(long long tiles, int ni, int resident, int cap, int most) {
+// `ctas(c)`: the grid's CTAs at chunks of c planes, ni its longest extent.
+template <class F>
+inline int march_planes(F ctas, int ni, int resident, int cap, int most) {
   constexpr int kFill = 4, kLeast = 4;
   cap = std::min(std::min(cap, ni), most);
-  if (tiles * cdiv_u(ni, cap) > 4ll * resident) return cap;
+  if (ctas(cap) > 4ll * resident) return cap;
   int best = cap;
   long long cost = -1;
   for (int c = cap; c >= std::min(kLeast, cap); --c) {
-    const long long w = (long long)cdiv_u(tiles * cdiv_u(ni, c), resident) * (c + kFill);
+    const long long w = (long long)cdiv_u(ctas(c), resident) * (c + kFill);
     if (cost < 0 || w < cost) {
       cost = w;
       best = c;
     }
   }
   return best;
+}
+inline int march_planes(long long tiles, int ni, int resident, int cap, int most) {
+  return march_planes([&](int c) { return tiles * cdiv_u(ni, c); }, ni, resident, cap, most);
 }
 
 // Launch a kernel that calls grid_wait: its start-up overlaps the tail of the

@@ -80,21 +80,40 @@ struct StrCfg {
   static constexpr size_t bytes = sizeof(float) * (F_T + kTab) + sizeof(Pipe<NH, NO, NC / 32>);
 };
 
+// The boxes of a launch: one, on the grid's three axes, or several with their
+// CTAs in a row, box by box, in the same order (levels, then j, then chunks).
+// Separate launches for the four boxes around a plasticity section's middle band
+// each end in a wave that is nearly empty and two of them are a few planes wide
+// (240 x 237 x 120: 116 -> 98 us a step).
+struct StrBoxes {
+  AwpBox box[AWP_MAXBOX];
+  int first[AWP_MAXBOX], nj[AWP_MAXBOX];  // first CTA / nk, tiles in j
+  int n, nk;                              // boxes, tiles in k
+};
+
 // LAYER: the launch takes a mesh block's interface layer too (StrArgs::layer).
 template <bool ELASTIC, bool LAYER>
 __global__ void __launch_bounds__(NT, ELASTIC ? 4 : 3)
-    k_stress_tma(const __grid_constant__ StrArgs a, const __grid_constant__ TmaMaps tm, const int ichunk,
-                 int* err, const unsigned spin) {
+    k_stress_tma(const __grid_constant__ StrArgs a, const __grid_constant__ TmaMaps tm,
+                 const __grid_constant__ StrBoxes bx, const int ichunk, int* err,
+                 const unsigned spin) {
   using C = StrCfg<ELASTIC>;
   constexpr int NM = C::NM, NO = C::NO_;
   extern __shared__ __align__(128) float smem[];
   auto& pipe = *reinterpret_cast<Pipe<C::NH, C::NO, NC / 32>*>(smem + C::F_T + C::kTab);
   const int tid = threadIdx.x;
-  const int kb = AWP_ALIGN + blockIdx.x * TZ;
-  const int jb = a.j0 + blockIdx.y * TY;
-  const int ib = a.i0 + blockIdx.z * ichunk;
-  const int ie = min(ib + ichunk - 1, a.i1);
-  const int n = ie - ib + 1;
+  int kt = blockIdx.x, jt = blockIdx.y, it = blockIdx.z, q = 0;
+  if (bx.n > 1) {
+    it = kt / bx.nk;
+    kt -= it * bx.nk;
+    while (q + 1 < bx.n && it >= bx.first[q + 1]) ++q;
+    jt = it - bx.first[q];
+    it = jt / bx.nj[q];
+    jt -= it * bx.nj[q];
+  }
+  const int kb = AWP_ALIGN + kt * TZ, jb = bx.box[q].j0 + jt * TY;
+  const int ib = bx.box[q].i0 + it * ichunk, je = bx.box[q].j1;
+  const int n = min(ichunk, bx.box[q].i1 - ib + 1);
 
   grid_go();
   if (tid == 0) pipe.init();
@@ -146,7 +165,7 @@ __global__ void __launch_bounds__(NT, ELASTIC ? 4 : 3)
 
   const int row = tid >> 4, kp = (tid & 15) * 2;
   const int k = kb + kp, j = jb + row;
-  const bool jin = j <= a.j1;
+  const bool jin = j <= je;
   // the interface layer of a mesh block: second order, weights (1, 0)
   const bool layer = LAYER && k + 1 == a.k0;
   const bool ax = jin && ((k >= a.k0 && k <= a.k1) || layer),
@@ -155,7 +174,7 @@ __global__ void __launch_bounds__(NT, ELASTIC ? 4 : 3)
   const float2 c1 = make_float2(layer ? 1.0f : a.c1, a.c1),
                c2 = make_float2(layer ? 0.0f : a.c2, a.c2);
   const long long col = (long long)j * Y + k;
-  const float dcy = LDG(a.dcrjy + min(j, a.j1));
+  const float dcy = LDG(a.dcrjy + min(j, je));
   const float2 dcz = ldg2(a.dcrjz + k);
   // the pair (ktop - 1, ktop): nzt is even, so the surface is a second level
   const bool top = a.fs && (k + 1 == a.ktop);
@@ -586,11 +605,22 @@ constexpr int kMost = 6;  // planes of a march (march_planes)
 
 }  // namespace
 
-cudaError_t awp_launch_stress_tma(const StrArgs& a, const TmaMaps& tm, bool elastic, int ichunk,
-                                  int* err, cudaStream_t st) {
-  const int nk = a.k1 - AWP_ALIGN + 1, nj = a.j1 - a.j0 + 1, ni = a.i1 - a.i0 + 1;
-  if (nk <= 0 || nj <= 0 || ni <= 0) return cudaSuccess;
-  const dim3 tile(cdiv_u(nk, TZ), cdiv_u(nj, TY));
+cudaError_t awp_launch_stress_tma(const StrArgs& a, const AwpBox* box, int nbox, const TmaMaps& tm,
+                                  bool elastic, int ichunk, int* err, cudaStream_t st) {
+  const int nk = a.k1 - AWP_ALIGN + 1;
+  StrBoxes bx{};
+  int ni = 0;
+  for (int q = 0; q < nbox && bx.n < AWP_MAXBOX; ++q) {
+    if (box[q].empty()) continue;
+    bx.box[bx.n] = box[q];
+    bx.nj[bx.n++] = (int)cdiv_u(box[q].j1 - box[q].j0 + 1, TY);
+    ni = std::max(ni, box[q].i1 - box[q].i0 + 1);
+  }
+  if (nk <= 0 || bx.n == 0) return cudaSuccess;
+  bx.nk = (int)cdiv_u(nk, TZ);
+  auto chunks = [&](int q, int c) {
+    return (long long)cdiv_u(bx.box[q].i1 - bx.box[q].i0 + 1, c);
+  };
   const size_t sm = elastic ? StrCfg<true>::bytes : StrCfg<false>::bytes;
   const auto f = elastic ? (a.layer ? k_stress_tma<true, true> : k_stress_tma<true, false>)
                          : (a.layer ? k_stress_tma<false, true> : k_stress_tma<false, false>);
@@ -598,9 +628,23 @@ cudaError_t awp_launch_stress_tma(const StrArgs& a, const TmaMaps& tm, bool elas
   const cudaError_t e = resident_ctas(
       (const void*)f, sm, NT, g_shape_str[(elastic ? 2 : 0) + (a.layer ? 1 : 0)], &resident);
   if (e != cudaSuccess) return e;
-  const int c = march_planes((long long)tile.x * tile.y, ni, resident, ichunk, kMost);
-  return launch_after(f, dim3(tile.x, tile.y, cdiv_u(ni, c)), dim3(NT), sm, st, a, tm, c,
-                      err, awp_pipe_spin_limit);
+  const int c = march_planes(
+      [&](int c) {
+        long long t = 0;
+        for (int q = 0; q < bx.n; ++q) t += chunks(q, c) * bx.nj[q] * bx.nk;
+        return t;
+      },
+      ni, resident, ichunk, kMost);
+  dim3 grid(bx.nk, bx.nj[0], (unsigned)chunks(0, c));
+  if (bx.n > 1) {
+    long long t = 0;
+    for (int q = 0; q < bx.n; ++q) {
+      bx.first[q] = (int)t;
+      t += chunks(q, c) * bx.nj[q];
+    }
+    grid = dim3((unsigned)(t * bx.nk));
+  }
+  return launch_after(f, grid, dim3(NT), sm, st, a, tm, bx, c, err, awp_pipe_spin_limit);
 }
 
 cudaError_t awp_launch_velocity_tma(const VelArgs& a, const TmaMaps& tm, int ichunk, int* err,

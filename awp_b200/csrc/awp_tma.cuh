@@ -25,8 +25,10 @@ struct TmaMaps {
 int awp_tma_box(int group, int* box_x, int* box_y);
 int awp_tma_encode(CUtensorMap* map, const float* base, const AwpGeom& g, int box_x, int box_y);
 
-cudaError_t awp_launch_stress_tma(const StrArgs& a, const TmaMaps& tm, bool elastic, int ichunk,
-                                  int* err, cudaStream_t st);
+// The stress update over up to AWP_MAXBOX disjoint boxes of columns (a's own i, j
+// range is not read).
+cudaError_t awp_launch_stress_tma(const StrArgs& a, const AwpBox* box, int nbox, const TmaMaps& tm,
+                                  bool elastic, int ichunk, int* err, cudaStream_t st);
 cudaError_t awp_launch_velocity_tma(const VelArgs& a, const TmaMaps& tm, int ichunk, int* err,
                                     cudaStream_t st);
 // Poll limit of the TMA kernels' pipeline waits (0 .. 2^30; default 2^26; 0

@@ -80,6 +80,34 @@ def test_steps_match_float64(case):
         assert float((x.to(y.device) - y).norm()) <= 3e-6 * ref, (name, ref)
 
 
+@pytest.mark.parametrize("nx", [40, 45, 47])
+def test_plastic_return_of_every_cell(nx):
+    """No cohesion and no friction: every cell yields, so the return takes the
+    path of a changed cell on whole planes; widths of a multiple of the planes
+    a thread reads and of remainders, the stress split's narrow boxes with
+    them.  Checked are the fields the return writes (the memory variables'
+    increments are differences of neighbouring velocities, in which the
+    velocities' rounding of 1e-6 weighs several times as much)."""
+    m = cases()
+    inputs = m._yield_inputs
+
+    def weak(*args):
+        s2, cohes, phi = inputs(*args)
+        return s2, 0 * cohes, 0 * phi
+
+    m._yield_inputs = weak
+    case = dict(kind="plastic", nx=nx, ny=41, nz=32, q=True, steps=3)
+    st = m.prepare(case, 5)
+    got = m.run(st)
+    torch.cuda.synchronize()
+    ny, nz = case["ny"], case["nz"]
+    assert int((got["yldfac"] < 1).sum()) > 0.9 * nx * ny * nz
+    want = m.exact(case, 5)
+    for name in ("xx", "yy", "zz", "xy", "xz", "yz", "yldfac", "neta"):
+        x, y = got[name].double(), torch.as_tensor(want[name]).double()
+        assert float((x.to(y.device) - y).norm()) <= 3e-6 * float(y.norm()), name
+
+
 @pytest.mark.parametrize("kind", ["grid", "hill"])
 def test_marches_beside_another_context(kind):
     """Two contexts on their own streams share the SMs; each must leave the
