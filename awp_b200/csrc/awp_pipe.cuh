@@ -198,26 +198,30 @@ inline cudaError_t resident_ctas(const void* kernel, size_t smem, int threads,
   return cudaSuccess;
 }
 
-// x planes a CTA marches, at most `cap` (the tuning value) and `most` (the
-// kernel's).  A grid of many waves takes `most`: the CTAs in flight then stay
-// within a few planes of one another, so the halos of neighbouring tiles and
-// the planes two chunks share are found in L2 (k_stress_tma, 512 x 512 x 256:
-// 1385 us at 6 planes, 1466 at 8 and 1617 at 32 with the wider L2 promotion;
-// the curvilinear kernels have a longer prologue and take 32).  A grid of few
-// waves takes the chunk with the least waves x (planes + fill), fill being
-// the planes' worth of time a march spends before its first result
-// (48 x 40 x 36: 34 -> 9 us and 60 -> 13 us for the two kernels).
+// x planes a CTA marches, at most `cap` (the tuning value).  A grid of many
+// waves takes `most` (the kernel's): the CTAs in flight then stay within a few
+// planes of one another, so the halos of neighbouring tiles and the planes two
+// chunks share are found in L2 (k_stress_tma, 512 x 512 x 256: 1385 us at 6
+// planes, 1466 at 8 and 1617 at 32 with the wider L2 promotion; the
+// curvilinear kernels have a longer prologue and take 32).  A grid of few
+// waves, in flight as a whole, takes the chunk with the least waves x (planes
+// + fill), of equals the shortest; fill is the planes' worth of time a march
+// spends before its first result, mostly hidden behind the SM's other CTAs
+// (ten steps of 128 x 128 x 128, 634 us, and five of a 53 x 41 x 60 mesh, 580,
+// with chunks up to six planes: 604 and 573 with longer ones, 600 and 597
+// with a fill of two planes, 602 and 599 with four; 48 x 40 x 36: 34 -> 9 us
+// and 60 -> 13 us for the two kernels against 32 planes throughout).
 // `ctas(c)`: the grid's CTAs at chunks of c planes, ni its longest extent.
 template <class F>
 inline int march_planes(F ctas, int ni, int resident, int cap, int most) {
-  constexpr int kFill = 4, kLeast = 4;
-  cap = std::min(std::min(cap, ni), most);
-  if (ctas(cap) > 4ll * resident) return cap;
+  constexpr int kFill = 1, kLeast = 4;
+  cap = std::min(cap, ni);
+  if (ctas(std::min(cap, most)) > 4ll * resident) return std::min(cap, most);
   int best = cap;
   long long cost = -1;
   for (int c = cap; c >= std::min(kLeast, cap); --c) {
     const long long w = (long long)cdiv_u(ctas(c), resident) * (c + kFill);
-    if (cost < 0 || w < cost) {
+    if (cost < 0 || w <= cost) {
       cost = w;
       best = c;
     }
