@@ -420,8 +420,8 @@ class Mesh:
 
 class Batch:
     """Many independent single-grid simulations advanced together
-    (awp_batch_*): one persistent launch per half-step over the tiles of every
-    instance, the step replayed as a CUDA graph.  ``solvers`` are ordinary
+    (awp_batch_*): each instance's own launches as parallel branches, replayed
+    as CUDA graphs of up to eight steps.  ``solvers`` are ordinary
     Solvers set up as for ``step``; keep them alive while the batch lives."""
 
     def __init__(self, solvers):
@@ -455,8 +455,8 @@ class Batch:
               "awp_batch_set_graph")
 
     def set_mode(self, mode: int) -> None:
-        """0: persistent tile-queue launches; 1: graph of each instance's own
-        launches as parallel branches."""
+        """0: parallel branches, graphs or direct launches as ``set_graph`` says;
+        1: graphs whatever it says.  Same results."""
         check(self.lib.awp_batch_set_mode(self.batch, int(mode)), "awp_batch_set_mode")
 
     @property
@@ -464,7 +464,7 @@ class Batch:
         return self.lib.awp_batch_get_mode(self.batch)
 
     def set_branches(self, branches: int) -> None:
-        """Mode 1: parallel graph branches the instances are dealt onto
+        """Parallel branches the instances are dealt onto
         (0: one per instance)."""
         check(self.lib.awp_batch_set_branches(self.batch, int(branches)),
               "awp_batch_set_branches")

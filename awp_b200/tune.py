@@ -97,10 +97,10 @@ BATCH_CANDIDATES = {"ty": (8, 4), "ichunk": (8, 16, 32)}
 
 
 def autotune_batch(batch, steps: int = 3, timer=None) -> dict:
-    """Pick the batched execution: the persistent tile-queue mode with its
-    tile shape (ty j rows x ichunk x planes, threads per CTA = 32 ty), or the
-    graph of the instances' own launches, by timing `steps` batched steps per
-    candidate (advancing the instances); `timer(fn)` returns the milliseconds
+    """Pick the batched execution: the mode (both run the instances' own
+    launches as parallel branches; the shape only sets the tile counts that
+    info reports), the kernel family, x chunk and number of branches, by timing
+    `steps` batched steps per candidate (advancing the instances); `timer(fn)` returns the milliseconds
     fn takes.  No choice changes results (each cell is computed by the same
     expression)."""
     table = []

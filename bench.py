@@ -527,8 +527,8 @@ def run_reference(args, rank) -> dict | None:
 def run_batched(args) -> dict:
     """Batched ensemble: the same instances advanced (a) by the plain path,
     one context per simulation, each on its own stream (so independent
-    simulations may overlap on the GPU), and (b) by awp_batch_step (persistent
-    tile-queue launches, one CUDA graph per step).  Both timed on the device
+    simulations may overlap on the GPU), and (b) by awp_batch_step (each
+    instance's launches as a branch of CUDA graphs of several steps).  Both timed on the device
     with CUDA events; value = batched Gcell-updates/s."""
     import torch
     from awp_b200 import Batch, Solver, default_params, scenarios, tune
