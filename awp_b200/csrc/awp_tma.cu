@@ -571,8 +571,12 @@ int awp_tma_get_l2_promotion() { return g_l2_promotion; }
 int awp_tma_encode(CUtensorMap* map, const float* base, const AwpGeom& g, int box_x, int box_y) {
   auto fn = encode_fn();
   if (!fn) return 1;
-  const cuuint64_t dims[3] = {(cuuint64_t)g.nz_pad(), (cuuint64_t)g.ny_pad(),
-                              (cuuint64_t)g.nx_pad()};
+  // The map ends four levels above the surface (the stencils reach two): of the
+  // last tile of a column that is no multiple of 32 levels, the padding beyond
+  // is filled in, not read (five steps of 301 x 223 x 108 1585 -> 1537 us, an
+  // ensemble of 21 uneven grids 2797 -> 2723).
+  const cuuint64_t dims[3] = {(cuuint64_t)std::min<long long>(g.top() + 5, g.nz_pad()),
+                              (cuuint64_t)g.ny_pad(), (cuuint64_t)g.nx_pad()};
   const cuuint64_t strides[2] = {(cuuint64_t)g.yline * 4, (cuuint64_t)g.slice * 4};
   const cuuint32_t box[3] = {(cuuint32_t)box_x, (cuuint32_t)box_y, 1};
   const cuuint32_t estr[3] = {1, 1, 1};
