@@ -460,38 +460,38 @@ int phase_velocity(awp_ctx* c) {
   return AWP_OK;
 }
 
-// Middle band of the NVE = 3 stress split at one rank: xss2..xse2 x
-// yls2..yre2 (pmcl3d.c:573-631; ylsp = yls, yrep = yre at one rank).
+// The NVE = 3 split of the context's stress window (awp::stress_split).
+AwpBox split_window(const awp_ctx* c, AwpBox rest[4]) {
+  const bool sub = c->sub_nxg != 0;
+  AwpBox band;
+  awp::stress_split({c->xls, c->xre, c->yls, c->yre}, sub ? c->sub_x0 : 0,
+                    sub ? c->sub_nxg : c->g.nxt, sub, &band, rest);
+  return band;
+}
 AwpBox middle_band(const awp_ctx* c) {
-  const int yls = c->yls, yre = c->yre;
-  int yls2 = (int)(yls + (int)(yre - yls) * 0.25);
-  if (yls2 % 2 != 0) yls2 += 1;
-  int yre2 = (int)(yls + (int)(yre - yls) * 0.75);
-  if (yre2 % 2 == 0) yre2 -= 1;
-  // x range of the whole grid, in this part's indices when it is a sub-domain
-  const int x0 = c->sub_nxg ? c->sub_x0 : 0, nxg = c->sub_nxg ? c->sub_nxg : c->g.nxt;
-  return {std::max(AWP_NGSL + 4 - x0, c->sub_nxg ? c->xls : 0),
-          std::min(nxg + AWP_NGSL - 1 - x0, c->sub_nxg ? c->xre : INT_MAX),
-          std::max(yls2, yls + AWP_NGSL + 2), std::min(yre2, yre - AWP_NGSL - 2)};
+  AwpBox rest[4];
+  return split_window(c, rest);
 }
 
-// Cartesian stress (+ memory variables) over n disjoint boxes of the stress
-// window, with the kernel family the tuning selects.
+// Cartesian stress (+ memory variables) over n boxes of the stress window, in
+// order, with the kernel family the tuning selects.  The TMA kernel takes
+// disjoint boxes in one launch; a box that meets an earlier one starts the
+// next launch, so its cells are updated after the other's, not beside it.
 // `layer` (TMA kernel): the interface layer too.
 int launch_cart_stress(awp_ctx* c, const AwpBox* box, int n, bool layer = false) {
   StrArgs s = make_str_args(c);
   s.layer = layer ? 1 : 0;
-  if (awp_tuning_get("tma_str") == 1 && tma_ready(c)) {
-    if (std::all_of(box, box + n, [](const AwpBox& b) { return b.empty(); })) return AWP_OK;
-    CU_TRY(awp_launch_stress_tma(s, box, n, c->str_maps, c->elastic, awp_tuning_get("ichunk"),
-                                 c->d_err, c->stream));
-    c->launches++;
-    return AWP_OK;
-  }
-  for (int q = 0; q < n; ++q) {
-    if (box[q].empty()) continue;
-    s.i0 = box[q].i0; s.i1 = box[q].i1; s.j0 = box[q].j0; s.j1 = box[q].j1;
-    CU_TRY(awp_launch_stress(s, c->elastic, c->stream));
+  const bool tma = awp_tuning_get("tma_str") == 1 && tma_ready(c);
+  for (int q = 0, m; q < n; q += m) {
+    m = tma ? awp::disjoint_run(box + q, n - q) : 1;
+    if (std::all_of(box + q, box + q + m, [](const AwpBox& b) { return b.empty(); })) continue;
+    if (tma) {
+      CU_TRY(awp_launch_stress_tma(s, box + q, m, c->str_maps, c->elastic,
+                                   awp_tuning_get("ichunk"), c->d_err, c->stream));
+    } else {
+      s.i0 = box[q].i0; s.i1 = box[q].i1; s.j0 = box[q].j0; s.j1 = box[q].j1;
+      CU_TRY(awp_launch_stress(s, c->elastic, c->stream));
+    }
     c->launches++;
   }
   return AWP_OK;
@@ -535,13 +535,10 @@ int phase_stress(awp_ctx* c) {
     return AWP_OK;
   }
   PhaseScope ps(c, 1);
-  const AwpBox all{c->xls, c->xre, c->yls, c->yre}, m = middle_band(c);
+  const AwpBox all{c->xls, c->xre, c->yls, c->yre};
   if (!stress_split(c)) return launch_cart_stress(c, &all, 1, stress_layer(c));
-  // xss2 in front of and behind the band, xss1, xss3
-  const AwpBox rest[4] = {{m.i0, m.i1, all.j0, m.j0 - 1},
-                          {m.i0, m.i1, m.j1 + 1, all.j1},
-                          {all.i0, m.i0 - 1, all.j0, all.j1},
-                          {m.i1 + 1, all.i1, all.j0, all.j1}};
+  AwpBox rest[4];
+  split_window(c, rest);
   return launch_cart_stress(c, rest, 4);
 }
 

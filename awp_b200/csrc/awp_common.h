@@ -49,6 +49,16 @@ inline AwpGeom awp_make_geom(int nxt, int nyt, int nzt) {
   return g;
 }
 
+// Columns i0..i1 x j0..j1 (inclusive).
+struct AwpBox {
+  int i0, i1, j0, j1;
+  bool empty() const { return i1 < i0 || j1 < j0; }
+  bool meets(const AwpBox& b) const {
+    return !empty() && !b.empty() && i0 <= b.i1 && b.i0 <= i1 && j0 <= b.j1 && b.j0 <= j1;
+  }
+};
+constexpr int AWP_MAXBOX = 4;  // boxes of one stress launch (the split around plasticity)
+
 // Memory-variable parity pattern.  The reference stores vx1/vx2/ww/wwo as four
 // full 3-D arrays (init_texture, mesh.c:1103-1137), but every value is one of
 // eight entries selected by the parity of the visit counters of that loop, so

@@ -5,7 +5,10 @@
 // (checked against the reference's own mesh.c / cerjan.c in the CPU tests).
 #include "awp_host.h"
 
+#include <limits.h>
 #include <math.h>
+
+#include <algorithm>
 
 namespace awp {
 
@@ -148,6 +151,30 @@ void relax_table(const AwpTexture& t, const float coeff16[16], float DT, float d
     out->c1[n] = (float)(0.5 * coeff16[2 * n + 1] / w * K);
     out->c2[n] = (float)(0.5 * K);
   }
+}
+
+void stress_split(const AwpBox& all, int x0, int nxg, bool sub, AwpBox* band, AwpBox rest[4]) {
+  const int yls = all.j0, yre = all.j1;
+  int yls2 = (int)(yls + (int)(yre - yls) * 0.25);
+  if (yls2 % 2 != 0) yls2 += 1;
+  int yre2 = (int)(yls + (int)(yre - yls) * 0.75);
+  if (yre2 % 2 == 0) yre2 -= 1;
+  // x range of the whole grid, in this part's indices when it is a sub-domain
+  const AwpBox m{std::max(AWP_NGSL + 4 - x0, sub ? all.i0 : 0),
+                 std::min(nxg + AWP_NGSL - 1 - x0, sub ? all.i1 : INT_MAX),
+                 std::max(yls2, yls + AWP_NGSL + 2), std::min(yre2, yre - AWP_NGSL - 2)};
+  *band = m;
+  rest[0] = {m.i0, m.i1, all.j0, m.j0 - 1};
+  rest[1] = {m.i0, m.i1, m.j1 + 1, all.j1};
+  rest[2] = {all.i0, m.i0 - 1, all.j0, all.j1};
+  rest[3] = {m.i1 + 1, all.i1, all.j0, all.j1};
+}
+
+int disjoint_run(const AwpBox* box, int n) {
+  for (int q = 1; q < n; ++q)
+    for (int p = 0; p < q; ++p)
+      if (box[p].meets(box[q])) return q;
+  return n;
 }
 
 void inicrj(float arbc, int nxt, int nyt, int nzt, int NX, int NY, int ND,

@@ -30,6 +30,19 @@ void relax_table(const AwpTexture& t, const float coeff16[16], float DT, float d
 void inicrj(float arbc, int nxt, int nyt, int nzt, int NX, int NY, int ND,
             int islowest, int npc, float* dcrjx, float* dcrjy, float* dcrjz);
 
+// The stress window all (xls..xre x yls..yre) of an NVE = 3 step: the middle
+// band xss2..xse2 x yls2..yre2 (pmcl3d.c:573-631; ylsp = yls, yrep = yre at one
+// rank) that runs in the plasticity section, and the boxes around it in the
+// reference's order: xss2 in front of and behind the band, xss1, xss3.  x0, nxg:
+// a sub-domain's first column and its grid's columns (0 and nx for a whole
+// grid, sub false).  Below 20 rows the band is empty and the front and back
+// boxes share rows, which the reference then updates twice.
+void stress_split(const AwpBox& all, int x0, int nxg, bool sub, AwpBox* band, AwpBox rest[4]);
+
+// How many of the n boxes, from the first, share no column: the boxes of one
+// launch, the others following it in stream order.
+int disjoint_run(const AwpBox* box, int n);
+
 // Smallest float x > 0 with 1/(double)x <= 200.0 (the Q(f) branch switch of
 // dstrqc, kernel.cu:974).
 float qf_threshold();

@@ -52,13 +52,6 @@ struct StrArgs {
   int layer;     // TMA kernel: as VelArgs (dstrqc2 on the level below k0)
 };
 
-// Columns i0..i1 x j0..j1 (inclusive).
-struct AwpBox {
-  int i0, i1, j0, j1;
-  bool empty() const { return i1 < i0 || j1 < j0; }
-};
-constexpr int AWP_MAXBOX = 4;  // boxes of one stress launch (the split around plasticity)
-
 // ---------------------------------------------------------------------------
 // Free-surface stress imaging (reference: fstr, kernel.cu:1616-1647).
 // ---------------------------------------------------------------------------

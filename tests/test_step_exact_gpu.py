@@ -151,3 +151,27 @@ def test_march_length_does_not_change_curvilinear_fields():
     finally:
         for k, v in saved.items():
             tune.set_tuning(lib, k, v)
+
+
+@pytest.mark.parametrize("ny", [12, 19, 20])
+def test_overlapping_stress_boxes_follow_one_another(ny):
+    """Below 20 rows the boxes around the plasticity band share rows; the TMA
+    kernel must update them in the order of the read-only-path family, which
+    takes one box a launch, bit for bit."""
+    lib = _lib.load()
+    saved = tune.get_tuning(lib)
+    m = cases()
+    case = dict(kind="plastic", nx=41, ny=ny, nz=36, q=True, steps=3)
+    got = []
+    try:
+        for family in (0, 1):
+            tune.set_tuning(lib, "tma_str", family)
+            st = m.prepare(case, 4)
+            out = m.run(st)
+            torch.cuda.synchronize()
+            got.append({f: v.cpu().numpy().view(np.uint32).copy() for f, v in out.items()})
+    finally:
+        for k, v in saved.items():
+            tune.set_tuning(lib, k, v)
+    for f in got[0]:
+        assert np.array_equal(got[0][f], got[1][f]), f
