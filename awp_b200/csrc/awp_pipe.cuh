@@ -35,12 +35,14 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, unsigned bytes) {
                "r"(bytes)
                : "memory");
 }
-// one arrival per warp (by its lane 0), for all 32 lanes' reads of a step.
-// Called after the step's results are stored: a read of shared memory that is
-// still in flight when the producer refills the slot would see the next
-// plane.  (Arriving as soon as the reads were issued lost that race when
-// another context's kernels shared the SM.)
+// One arrival per warp (by its lane 0), for all 32 lanes' reads of a step.  The
+// refill is a write of the async proxy, which program order alone does not keep
+// behind a lane's plain loads: every lane orders its own with a proxy fence,
+// then the warp meets, then lane 0's arrival releases the slot.  (Without the
+// order a plane was seen to change under its readers when another context's
+// kernels shared the SM.)
 __device__ __forceinline__ void warp_done(uint64_t* bar, int lane) {
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   __syncwarp();
   asm volatile(
       "{\n .reg .pred p;\n setp.eq.s32 p, %1, 0;\n"

@@ -449,15 +449,16 @@ __global__ void __launch_bounds__(NT, 4)
   const float2 dcz = ldg2(a.dcrjz + k);
   long long o = (long long)ib * S + (long long)j * Y + k;
   float2 xx_m2, xx_m1, xx_0, xy_m1, xy_0, xy_p1, xz_m1, xz_0, xz_p1;
-  // density of the current plane: value, and the level below; rows j and j-1
+  // density of the current plane: rows j and j-1; the level below and its sum
+  // over the two rows (formed in the step that reads them)
   float2 d_0, d_0j;
-  float d_0k, d_0jk;
+  float d_0k, d_0s;
   {
     const float *X = a.xx + o, *P = a.xy + o, *Q = a.xz + o, *D = a.d1 + o;
     xx_m2 = ldg2(X - 2 * (long long)S); xx_m1 = ldg2(X - S); xx_0 = ldg2(X);
     xy_m1 = ldg2(P - S); xy_0 = ldg2(P); xy_p1 = ldg2(P + S);
     xz_m1 = ldg2(Q - S); xz_0 = ldg2(Q); xz_p1 = ldg2(Q + S);
-    d_0 = ldg2(D); d_0j = ldg2(D - Y); d_0k = D[-1]; d_0jk = D[-Y - 1];
+    d_0 = ldg2(D); d_0j = ldg2(D - Y); d_0k = D[-1]; d_0s = vadd(d_0k, D[-Y - 1]);
   }
   const int o_own = row * TZ + kp;                    // no halo
   const int o_yy = (row + 1) * TZ + kp;               // j halo from jb - 1
@@ -495,13 +496,13 @@ __global__ void __launch_bounds__(NT, 4)
                  yz_jm2 = lds2(YZ - 2 * HX), yz_jp1 = lds2(YZ + HX);
     const float yz_kp = YZ[2];
     const float2 d_p = lds2(D), d_pj = lds2(D - MX);
-    const float d_pk = D[-1], d_pjk = D[-MX - 1];
+    const float d_pk = D[-1], d_ps = vadd(d_pk, D[-MX - 1]);
     const float2 u_old = lds2(G + C::G_O + o_own), v_old = lds2(G + C::G_O + OTILE + o_own),
                  w_old = lds2(G + C::G_O + 2 * OTILE + o_own);
 
     // density factors: pair sums at the level and at the one below
     const float2 dj = vadd(d_0, d_0j), dx = vadd(d_0, d_p);
-    const float2 fd1 = awp_vel_factor(dth, dj, make_float2(vadd(d_0k, d_0jk), dj.x));
+    const float2 fd1 = awp_vel_factor(dth, dj, make_float2(d_0s, dj.x));
     const float2 fd2 = awp_vel_factor(dth, dx, make_float2(vadd(d_0k, d_pk), dx.x));
     const float2 fd3 = awp_vel_factor(dth, dx, vadd(d_0j, d_pj));
     const float2 dcrj = vscale(LDG(a.dcrjx + ib + s) * dcy, dcz);
@@ -528,7 +529,7 @@ __global__ void __launch_bounds__(NT, 4)
     xx_m2 = xx_m1; xx_m1 = xx_0; xx_0 = xx_p1;
     xy_m1 = xy_0; xy_0 = xy_p1; xy_p1 = xy_p2;
     xz_m1 = xz_0; xz_0 = xz_p1; xz_p1 = xz_p2;
-    d_0 = d_p; d_0j = d_pj; d_0k = d_pk; d_0jk = d_pjk;
+    d_0 = d_p; d_0j = d_pj; d_0k = d_pk; d_0s = d_ps;
     ch.next();
     cd.next();
     ss = ss + 1 == C::DS ? 0 : ss + 1;

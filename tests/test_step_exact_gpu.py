@@ -108,14 +108,24 @@ def test_plastic_return_of_every_cell(nx):
         assert float((x.to(y.device) - y).norm()) <= 3e-6 * float(y.norm()), name
 
 
-@pytest.mark.parametrize("kind", ["grid", "hill"])
-def test_marches_beside_another_context(kind):
+BESIDE = [
+    grid(150, 120, 96, steps=6), grid(150, 120, 96, q=False, steps=6),
+    dict(kind="hill", nx=120, ny=100, nz=96, q=True, steps=4),
+    dict(kind="hill", nx=121, ny=99, nz=68, q=False, steps=4),
+    dict(kind="plastic", nx=130, ny=101, nz=64, q=True, steps=4),
+    dict(kind="mesh", nx=45, ny=40, nz=64, nzc=48, steps=4, hill=False, plastic=False),
+    dict(kind="mesh", nx=40, ny=41, nz=68, nzc=32, steps=4, hill=True, plastic=True),
+]
+
+
+@pytest.mark.parametrize("case", BESIDE, ids=lambda c: f"{c['kind']}-{c['nx']}-{c['nz']}")
+def test_marches_beside_another_context(case):
     """Two contexts on their own streams share the SMs; each must leave the
     fields it leaves alone, bit for bit (the producer may refill a slot only
-    when every lane has its values, however long its warp waits)."""
+    when every lane has its values, however long its warp waits): every
+    variant of the pipelined kernels, the one of several boxes and those that
+    take a mesh block's interface layer among them."""
     m = cases()
-    case = grid(150, 120, 96, steps=6) if kind == "grid" else \
-        dict(kind="hill", nx=120, ny=100, nz=96, q=True, steps=4)
     alone = m.prepare(case, 1)
     m.run(alone)
     torch.cuda.synchronize()
