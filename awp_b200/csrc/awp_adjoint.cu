@@ -373,12 +373,14 @@ __global__ void __launch_bounds__(128) k_adj_stress_gather(const __grid_constant
   const long long q = (long long)ib * S + (long long)j * Y + k;
   const float c1 = a.c1;
   const float2 c2 = vset<float2>(a.c2), zero = make_float2(0.f, 0.f);
-  const float* __restrict__ e1 = a.E[E1] + q;
-  const float* __restrict__ e2 = a.E[E2] + q;
-  const float* __restrict__ e3 = a.E[E3] + q;
-  const float* __restrict__ e4 = a.E[E4] + q;
-  const float* __restrict__ e5 = a.E[E5] + q;
-  const float* __restrict__ e6 = a.E[E6] + q;
+  // (not const __restrict__: this launch starts before the kernel that writes E
+  // ends, so no load of it may take the path for data constant over the launch)
+  const float* e1 = a.E[E1] + q;
+  const float* e2 = a.E[E2] + q;
+  const float* e3 = a.E[E3] + q;
+  const float* e4 = a.E[E4] + q;
+  const float* e5 = a.E[E5] + q;
+  const float* e6 = a.E[E6] + q;
   float* __restrict__ Lu = a.L[LU] + q;
   float* __restrict__ Lv = a.L[LV] + q;
   float* __restrict__ Lw = a.L[LW] + q;
@@ -564,9 +566,10 @@ __global__ void __launch_bounds__(128) k_adj_vel_gather(const __grid_constant__ 
   const long long q = (long long)ib * S + (long long)j * Y + k;
   const float c1 = a.c1;
   const float2 c2 = vset<float2>(a.c2), zero = make_float2(0.f, 0.f);
-  const float* __restrict__ A = a.V[VA] + q;
-  const float* __restrict__ B = a.V[VB] + q;
-  const float* __restrict__ C = a.V[VC] + q;
+  // (inputs qualified as in k_adj_stress_gather)
+  const float* A = a.V[VA] + q;
+  const float* B = a.V[VB] + q;
+  const float* C = a.V[VC] + q;
   float* __restrict__ Lxx = a.L[LXX] + q;
   float* __restrict__ Lxy = a.L[LXY] + q;
   float* __restrict__ Lxz = a.L[LXZ] + q;
@@ -776,10 +779,10 @@ __global__ void k_set_moduli(const float* lambda, const float* mu_, const float*
 
 // padded velocities -> VelBox rows; rows beyond nk (up to ld) are not read
 // level pairs: the box starts on a multiple of four levels
-__global__ void k_pack_vel(const float* __restrict__ u, const float* __restrict__ v,
-                           const float* __restrict__ w, float* __restrict__ du,
-                           float* __restrict__ dv, float* __restrict__ dw, const VelBox b,
-                           long long S, long long Y) {
+// (inputs qualified as in k_adj_stress_gather)
+__global__ void k_pack_vel(const float* u, const float* v, const float* w,
+                           float* __restrict__ du, float* __restrict__ dv,
+                           float* __restrict__ dw, const VelBox b, long long S, long long Y) {
   awp_pipe::grid_start();
   const int np = (b.nk + 1) / 2, idx = blockIdx.x * 128 + threadIdx.x;
   const int jj = idx / np, kk = 2 * (idx % np), ii = blockIdx.y;

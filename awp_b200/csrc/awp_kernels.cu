@@ -985,7 +985,7 @@ inline unsigned cdiv_u(long long a, long long b) { return (unsigned)((a + b - 1)
 
 // Sources of one instance at step *step + 1 + off read from device memory
 // (replayable graphs): the schedule of one_step, IFAULT < 4 while the step is below NST.
-__global__ void k_addsrc_dev(const SrcArgs a, const int* __restrict__ step, const int off,
+__global__ void k_addsrc_dev(const SrcArgs a, const int* step, const int off,
                              const int nst) {
   awp_pipe::grid_start();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -996,7 +996,7 @@ __global__ void k_addsrc_dev(const SrcArgs a, const int* __restrict__ step, cons
   addsrc_cell(b, c);
 }
 
-__global__ void k_addkinsrc_dev(const KinSrcArgs a, const int* __restrict__ step, const int off) {
+__global__ void k_addkinsrc_dev(const KinSrcArgs a, const int* step, const int off) {
   awp_pipe::grid_start();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= a.ncell) return;
