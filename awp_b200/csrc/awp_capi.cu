@@ -68,6 +68,7 @@ struct awp_ctx {
   float qthr = 0.f;
   unsigned thr = 0;    // bits of 2*qthr (StrArgs::thr)
   AwpRelaxTab rel{};   // update constants of the Cartesian stress kernels
+  AwpLayerTab lay{};   // and of the mesh interface layer
   float c1 = 9.0 / 8.0, c2 = -1.0 / 24.0;
   float dth = 0.f, dh1 = 0.f;
   int xls = 0, xre = 0, yls = 0, yre = 0;  // stress / output window (pmcl3d.c:573-631)
@@ -177,6 +178,7 @@ StrArgs make_str_args(awp_ctx* c) {
   a.dcrjx = c->dcrjx; a.dcrjy = c->dcrjy; a.dcrjz = c->dcrjz; a.lam_mu = c->lam_mu;
   a.tex = c->tex;
   a.rel = c->rel;
+  a.lay = c->lay;
   a.slice = c->g.slice;
   a.yline = c->g.yline;
   a.lam_mu_ld = (int)c->g.ny_pad();
@@ -413,6 +415,8 @@ TopoArgs topo_args(awp_ctx* c) {
   a.slice = c->g.slice; a.yline = c->g.yline;
   a.nx = c->g.nxt; a.ny = c->g.nyt; a.nz = c->g.nzt;
   a.layer = mesh_layer(c) ? 1 : 0;
+  a.lay_rel = c->rel; a.lay = c->lay;
+  a.lay_dt = c->p.dt; a.lay_dth = c->dth;
   return a;
 }
 
@@ -836,9 +840,9 @@ int dm_stress(awp_ctx* c) {  // dstrqc2 over xss1..xse3 x yls..yre (pmcl3d.c:193
   a.lam = f[AWP_LAM]; a.mu = f[AWP_MU]; a.qp = f[AWP_QP]; a.qs = f[AWP_QS];
   a.dcrjx = c->dcrjx; a.dcrjy = c->dcrjy; a.dcrjz = c->dcrjz;
   a.tex = c->tex;
-  memcpy(a.coeff, c->coeff, sizeof(a.coeff));
   a.i0 = c->xls; a.i1 = c->xre; a.j0 = c->yls; a.j1 = c->yre;
   a.dth = c->dth; a.dh1 = c->dh1; a.dt = c->p.dt;
+  a.rel = c->rel; a.lay = c->lay;
   a.thr = c->thr;
   a.ex_i0 = a.ex_j0 = 1;
   if (topo_stress_runs(c)) {  // the curvilinear launch took its window's columns
@@ -1084,7 +1088,7 @@ int awp_ctx_create(const awp_params* p, awp_ctx** out) {
     awp::tausub(c->taumin, c->taumax, c->tau8);
     awp::weights_sub(p->ex, p->fac, c->w8, c->coeff);
     awp::texture_tables(c->tau8, c->w8, p->dt, &c->tex);
-    awp::relax_table(c->tex, c->coeff, p->dt, c->dh1, &c->rel);
+    awp::relax_table(c->tex, c->coeff, p->dt, c->dh1, &c->rel, &c->lay);
     c->tex.xls = c->xls;
     c->tex.yls = c->yls;
     c->tex.ny = c->yre - c->yls + 1;

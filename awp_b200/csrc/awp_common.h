@@ -83,6 +83,10 @@ struct AwpTexture {
 struct AwpRelaxTab {
   float vx2[8], wwo[8], kv[8], kr[8], kr2[8], kf[8], c0[8], c1[8], c2[8];
 };
+// What rounding left of c0 and c1 (the mesh interface layer, awp_layer_coef).
+struct AwpLayerTab {
+  float l0[8], l1[8];
+};
 
 // Parity index of init_texture's visit counters (mesh.c:1103-1137) for the
 // cell (di, dj, kk) relative to the loop start: itx = parity of di + 1, ity =

@@ -62,9 +62,6 @@ __global__ void k_dvelc2(const DmVel2Args a) {
 // ===========================================================================
 // dstrqc2 (kernel.cu:2564-2767), anelastic form (ELA2 undefined)
 // ===========================================================================
-// The switch 1/(2q) <= 200 on q = S/4 as one compare of bit patterns and the
-// low-Q polynomial in float, as awp_weight (awp_stencil.cuh); the high-Q
-// branch is wwo*q here where dstrqc has 2*wwo*q, so its constant is halved.
 // Every load is issued before the arithmetic: the kernel's time is the sectors
 // of one level of k-contiguous columns, one 32-byte sector per value (300 x
 // 300: 58 us), so a mesh block leaves it only the ring outside the exclusion
@@ -100,27 +97,22 @@ __global__ void __launch_bounds__(128) k_dstrqc2(const DmStr2Args a) {
   };
   const Mat L = mat(a.lam), M = mat(a.mu), P = mat(a.qp), R = mat(a.qs);
   const float dcrj = __fmul_rn(__fmul_rn(a.dcrjz[k], a.dcrjx[i]), a.dcrjy[j]);
-  float f_vx1, f_vx2, f_wwo;
-  int cidx;
+  AwpRelax<float> rx;
+  AwpLayerOps ops{true, 0.f, 0.f};
   if (a.vx1) {
-    f_vx1 = a.vx1[pos];
-    f_vx2 = a.vx2[pos];
-    f_wwo = a.wwo[pos];
-    cidx = 2 * a.ww[pos] - 2;
+    const float vx1 = a.vx1[pos], wwo = a.wwo[pos];
+    const float *cf = a.coeff_dev + 2 * a.ww[pos] - 2, c0 = cf[0], c1 = cf[1];
+    rx = awp_relax_from(vx1, a.vx2[pos], wwo, c0, c1, a.dt, a.dh1, &ops.l0, &ops.l1);
   } else {
     const int t = awp_tex_index(a.tex, i, j, k);
-    f_vx1 = a.tex.tau1[t];
-    f_vx2 = a.tex.tau2[t];
-    f_wwo = a.tex.wwo8[t];
-    cidx = 2 * t;
+    rx = awp_relax_at(a.rel, t);
+    ops.l0 = a.lay.l0[t];
+    ops.l1 = a.lay.l1[t];
   }
-  const float c0 = a.coeff_dev ? a.coeff_dev[cidx] : a.coeff[cidx];
-  const float c1 = a.coeff_dev ? a.coeff_dev[cidx + 1] : a.coeff[cidx + 1];
-  AwpRelax<float> rx = awp_relax_from(f_vx1, f_vx2, f_wwo, c0, c1, a.dt, a.dh1);
   rx.c2 *= 0.5f;
   const float PM[3] = {M.pk, M.pj, M.pi}, PR[3] = {R.pk, R.pj, R.pi};
   const AwpStrCoef<float> cf =
-      awp_stress_coef<false>(L.s8, M.s8, PM, P.s8, R.s8, PR, rx, a.thr, a.dth, a.dt);
+      awp_stress_coef<false>(L.s8, M.s8, PM, P.s8, R.s8, PR, rx, a.thr, a.dth, a.dt, ops);
   const float d[9] = {__fsub_rn(ux, u0), __fsub_rn(v0, vy), __fsub_rn(w0, wk),  // x, y, z
                       __fsub_rn(uy, u0), __fsub_rn(v0, vx),                     // xy pair
                       __fsub_rn(uk, u0), __fsub_rn(w0, wx),                     // xz pair

@@ -32,8 +32,9 @@ struct DmStr2Args {
   const float *vx1, *vx2, *wwo;
   const int* ww;
   AwpTexture tex;
-  float coeff[16];
-  const float* coeff_dev;
+  AwpRelaxTab rel;  // with the pattern: the update's constants (StrArgs::rel, lay)
+  AwpLayerTab lay;
+  const float* coeff_dev;  // with the arrays: the Q(f) table (8 pairs)
   int i0, i1, j0, j1;
   float dth, dh1, dt;
   unsigned thr;  // Q(f) switch on a pair sum of Q^-1 (StrArgs::thr)

@@ -137,7 +137,7 @@ void texture_tables(const float tau8[8], const float w8[8], float dt, AwpTexture
 }
 
 void relax_table(const AwpTexture& t, const float coeff16[16], float DT, float dh1,
-                 AwpRelaxTab* out) {
+                 AwpRelaxTab* out, AwpLayerTab* lay) {
   for (int n = 0; n < 8; ++n) {
     const double v1 = t.tau1[n], v2 = t.tau2[n], w = t.wwo8[n], dt = DT;
     const double K = -(double)dh1 * v1;
@@ -147,9 +147,14 @@ void relax_table(const AwpTexture& t, const float coeff16[16], float DT, float d
     out->kr2[n] = (float)(dt * v2 * (1.0 - v1));
     out->kr[n] = (float)(dt * (1.0 + v2 * v1) + dt * v2 * (1.0 - v1));
     out->kf[n] = (float)(dt * (w - 1.0));
-    out->c0[n] = (float)(0.25 * coeff16[2 * n] / w * K);
-    out->c1[n] = (float)(0.5 * coeff16[2 * n + 1] / w * K);
+    const double c0 = 0.25 * coeff16[2 * n] / w * K, c1 = 0.5 * coeff16[2 * n + 1] / w * K;
+    out->c0[n] = (float)c0;
+    out->c1[n] = (float)c1;
     out->c2[n] = (float)(0.5 * K);
+    if (lay) {
+      lay->l0[n] = (float)(c0 - out->c0[n]);
+      lay->l1[n] = (float)(c1 - out->c1[n]);
+    }
   }
 }
 

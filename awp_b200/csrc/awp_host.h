@@ -24,7 +24,7 @@ void texture_tables(const float tau8[8], const float w8[8], float dt, AwpTexture
 // memory-variable update uses (AwpRelax of awp_stencil.cuh), in double and
 // rounded once.
 void relax_table(const AwpTexture& t, const float coeff16[16], float DT, float dh1,
-                 AwpRelaxTab* out);
+                 AwpRelaxTab* out, AwpLayerTab* lay = nullptr);
 
 // inicrj (cerjan.c:5-64) for a single rank (coords 0,0).
 void inicrj(float arbc, int nxt, int nyt, int nzt, int NX, int NY, int ND,

@@ -38,6 +38,7 @@ struct StrArgs {
   const int* ww;
   AwpTexture tex;
   AwpRelaxTab rel;         // per texture entry, with the step's DT and 1/h
+  AwpLayerTab lay;         // for the interface layer
   const float* coeff_dev;  // with the explicit arrays: the Q(f) table (8 pairs)
   int slice, yline, lam_mu_ld;
   int i0, i1, j0, j1, k0, k1;

@@ -81,17 +81,26 @@ __device__ __forceinline__ AwpRelax<float> awp_relax_at(const AwpRelaxTab& t, in
 
 // The same constants from explicit arrays (vx1, vx2, wwo) of a caller.
 __device__ __forceinline__ AwpRelax<float> awp_relax_from(float vx1, float vx2, float wwo, float c0,
-                                                          float c1, float DT, float dh1) {
+                                                          float c1, float DT, float dh1,
+                                                          float* l0 = nullptr,
+                                                          float* l1 = nullptr) {
   AwpRelax<float> r;
-  const float K = -(dh1 * vx1);
+  const float K = -__fmul_rn(dh1, vx1);
   r.vx2 = vx2;
   r.wwo = wwo;
-  r.kv = DT * (1.0f + vx2 * vx1);
-  r.kr2 = DT * (vx2 * (1.0f - vx1));
-  r.kr = r.kv + r.kr2;
-  r.kf = DT * (wwo - 1.0f);
-  r.c0 = 0.25f * c0 / wwo * K;
-  r.c1 = 0.5f * c1 / wwo * K;
+  r.kv = __fmul_rn(DT, __fmaf_rn(vx2, vx1, 1.0f));
+  r.kr2 = __fmul_rn(DT, __fmul_rn(vx2, __fsub_rn(1.0f, vx1)));
+  r.kr = __fadd_rn(r.kv, r.kr2);
+  r.kf = __fmul_rn(DT, __fsub_rn(wwo, 1.0f));
+  // c0*S + c1 cancels in part: the two share the factor K/wwo and its error,
+  // and have one rounding each of their own
+  const float g = __fdividef(K, wwo);
+  r.c0 = __fmul_rn(0.25f * c0, g);
+  r.c1 = __fmul_rn(0.5f * c1, g);
+  if (l0) {
+    *l0 = __fmaf_rn(0.25f * c0, g, -r.c0);
+    *l1 = __fmaf_rn(0.5f * c1, g, -r.c1);
+  }
   r.c2 = 0.5f * K;
   return r;
 }
@@ -113,6 +122,67 @@ __device__ __forceinline__ float2 awp_weight(float2 S, float2 c0, float2 c1, flo
   return vmul(s, S);
 }
 
+// Quotient and Q(f) weight of a stress cell's coefficients (awp_stress_coef).
+struct AwpCellOps {
+  template <class V>
+  __device__ __forceinline__ V quot(float n, V d) const { return vquot(n, d); }
+  template <class V>
+  __device__ __forceinline__ V weight(V S, const AwpRelax<V>& t, unsigned thr) const {
+    return awp_weight(S, t.c0, t.c1, t.c2, thr);
+  }
+  template <class V>
+  __device__ __forceinline__ V weight_p(V S, const AwpRelax<V>& t, unsigned thr) const {
+    return awp_weight(S, t.c0, t.c1, t.c2, thr);
+  }
+};
+
+// The same where the first level is a mesh block's interface layer (dstrqc2,
+// kernel.cu:2564-2767), at the precision of the reference, which divides and
+// evaluates the low-Q polynomial in double there: a quotient by the hardware
+// reciprocal is corrected by its remainder (half an ulp then), and c0*S + c1,
+// whose terms may cancel, takes what rounding left of its constants (l0, l1).
+// The switch 1/(2q) <= 200 is in double for Qs, in float for Qp.  The caller
+// halves t.c2: the high-Q branch is wwo*q here where dstrqc has 2*wwo*q.
+struct AwpLayerOps {
+  bool on;
+  float l0, l1;  // zero where off
+  // n a power of two
+  __device__ __forceinline__ float quot(float n, float d) const {
+    const float q = __fdividef(n, d);
+    const float c = __fmaf_rn(__fmaf_rn(-q, d, n), q * (1.0f / n), q);
+    return on && c == c ? c : q;  // d zero or infinite: no remainder
+  }
+  __device__ __forceinline__ float2 quot(float n, float2 d) const {
+    return make_float2(quot(n, d.x), __fdividef(n, d.y));
+  }
+  __device__ __forceinline__ float poly(float S, float c0, float c1) const {
+    return __fadd_rn(__fmaf_rn(c0, S, c1), __fmaf_rn(l0, S, l1));
+  }
+  __device__ __forceinline__ float low(float S, float c0, float c1, float c2, bool b) const {
+    return __fmul_rn(b ? poly(S, c0, c1) : c2, S);
+  }
+  __device__ __forceinline__ float weight(float S, const AwpRelax<float>& t, unsigned thr) const {
+    return low(S, t.c0, t.c1, t.c2, __float_as_uint(S) >= thr);
+  }
+  __device__ __forceinline__ float weight_p(float S, const AwpRelax<float>& t, unsigned) const {
+    return low(S, t.c0, t.c1, t.c2, __fdividef(1.0f, 0.5f * S) <= 200.0f);
+  }
+  __device__ __forceinline__ float2 both(float2 S, const AwpRelax<float2>& t, bool x,
+                                         unsigned thr) const {
+    const float y = __float_as_uint(S.y) >= thr ? __fmaf_rn(t.c0.y, S.y, t.c1.y) : t.c2.y;
+    return make_float2(low(S.x, t.c0.x, t.c1.x, t.c2.x, x), __fmul_rn(y, S.y));
+  }
+  __device__ __forceinline__ float2 weight(float2 S, const AwpRelax<float2>& t,
+                                           unsigned thr) const {
+    return both(S, t, __float_as_uint(S.x) >= thr, thr);
+  }
+  __device__ __forceinline__ float2 weight_p(float2 S, const AwpRelax<float2>& t,
+                                             unsigned thr) const {
+    return both(S, t, on ? __fdividef(1.0f, 0.5f * S.x) <= 200.0f : __float_as_uint(S.x) >= thr,
+                thr);
+  }
+};
+
 // Coefficients of one stress cell (kernel.cu:962-1070): with e_n the strain
 // rates and tr their trace, the elastic increments are A*tr + nxm*(tr - e_n)
 // (normal) and m*e (shear), the memory variables' forcing Q*tr + nh*(tr - e_n)
@@ -128,37 +198,37 @@ struct AwpStrCoef {
 // reciprocal (within two ulp), which keeps the update off the division slow
 // path; the parity tests hold the result to the reference build at relative
 // L2 1e-5.
-template <bool ELASTIC, class V>
+template <bool ELASTIC, class V, class Ops = AwpCellOps>
 __device__ __forceinline__ AwpStrCoef<V> awp_stress_coef(V L8, V M8, const V (&P)[3], V QP8, V QS8,
                                                          const V (&R)[3], const AwpRelax<V>& t,
-                                                         unsigned thr, float dth, float DT) {
+                                                         unsigned thr, V dth, V DT,
+                                                         const Ops& ops = Ops()) {
   AwpStrCoef<V> r;
-  const V nxm = vquot(-16.0f, M8);
-  const V xl = vsub(vquot(8.0f, L8), nxm);
+  const V nxm = ops.quot(-16.0f, M8);
+  const V xl = vsub(ops.quot(8.0f, L8), nxm);
   if (ELASTIC) {
-    r.nxm = vscale(dth, nxm);
-    r.A = vscale(dth, xl);
+    r.nxm = vmul(dth, nxm);
+    r.A = vmul(dth, xl);
     r.Q = r.nh = vset<V>(0.f);
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
-      r.m[q] = vscale(dth, vquot(2.0f, P[q]));
+      r.m[q] = vmul(dth, ops.quot(2.0f, P[q]));
       r.h[q] = vset<V>(0.f);
     }
     return r;
   }
-  const V d = vset<V>(dth), dt = vset<V>(DT);
-  const V hw = awp_weight(vscale(0.25f, QS8), t.c0, t.c1, t.c2, thr);
-  const V qw = awp_weight(vscale(0.25f, QP8), t.c0, t.c1, t.c2, thr);
+  const V hw = ops.weight(vscale(0.25f, QS8), t, thr);
+  const V qw = ops.weight_p(vscale(0.25f, QP8), t, thr);
   r.nh = vmul(nxm, hw);
-  r.nxm = vmul(nxm, vfma(dt, hw, d));
+  r.nxm = vmul(nxm, vfma(DT, hw, dth));
   r.Q = vmul(xl, qw);
-  r.A = vmul(xl, vfma(dt, qw, d));
+  r.A = vmul(xl, vfma(DT, qw, dth));
 #pragma unroll
   for (int q = 0; q < 3; ++q) {
-    const V m = vquot(2.0f, P[q]);
-    const V w = awp_weight(R[q], t.c0, t.c1, t.c2, thr);
+    const V m = ops.quot(2.0f, P[q]);
+    const V w = ops.weight(R[q], t, thr);
     r.h[q] = vmul(m, w);
-    r.m[q] = vmul(m, vfma(dt, w, d));
+    r.m[q] = vmul(m, vfma(DT, w, dth));
   }
   return r;
 }

@@ -277,7 +277,6 @@ __global__ void __launch_bounds__(NT, ELASTIC ? 4 : 3)
         };
         rx = {at(0), at(1), at(2), at(3), at(4), at(5), at(6), at(7), at(8)};
       }
-      if (LAYER && layer) rx.c2.x *= 0.5f;  // dstrqc2's high-Q branch is wwo*q, not 2*wwo*q
     }
     AwpStrCoef<float2> cf;
     {
@@ -294,8 +293,20 @@ __global__ void __launch_bounds__(NT, ELASTIC ? 4 : 3)
         Pq = pn;
         Rq = rn.q; Rt = rn.t; Rm = rn.m; Rk = rn.pk;
       }
-      cf = awp_stress_coef<ELASTIC>(vadd(Lq, Ln), vadd(Mq, mn.q), P, QP8, QS8, R, rx, a.thr,
-                                    a.dth, a.dt);
+      const float2 L8 = vadd(Lq, Ln), M8 = vadd(Mq, mn.q);
+      const float2 dth = vset<float2>(a.dth), DT = vset<float2>(a.dt);
+      if (LAYER) {
+        AwpLayerOps ops{layer, 0.f, 0.f};
+        if (layer) {
+          const int e = odd ? e0[1] : e0[0];
+          ops.l0 = a.lay.l0[e];
+          ops.l1 = a.lay.l1[e];
+          rx.c2.x *= 0.5f;
+        }
+        cf = awp_stress_coef<ELASTIC>(L8, M8, P, QP8, QS8, R, rx, a.thr, dth, DT, ops);
+      } else {
+        cf = awp_stress_coef<ELASTIC>(L8, M8, P, QP8, QS8, R, rx, a.thr, dth, DT);
+      }
       Lq = Ln;
       Mq = mn.q; Mt = mn.t; Mm = mn.m; Mk = mn.pk;
     }

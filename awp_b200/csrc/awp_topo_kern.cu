@@ -485,7 +485,8 @@ struct TopoStrCfg : StrTile {
   static constexpr size_t bytes = sizeof(float) * F_END + sizeof(Pipe<NH, NO, kCol>) + 8;
 };
 
-template <bool ELASTIC>
+// LAYER: on a block over a coarser one (TopoArgs::layer).
+template <bool ELASTIC, bool LAYER>
 __global__ void __launch_bounds__(StrTile::kThreads, 2)
     k_topo_stress(const __grid_constant__ TopoArgs a, const __grid_constant__ TmaMaps tm,
                   const int ichunk, int* err, const unsigned spin) {
@@ -567,7 +568,7 @@ __global__ void __launch_bounds__(StrTile::kThreads, 2)
   const bool o0 = c.out0 && jin, o1 = c.out1 && jin;
   const int S = a.slice, Y = a.yline, FL = a.fld;
   const int ja = jb + warp, jm = min(j, a.ny - 1);
-  const bool low = a.layer && blockIdx.x + 1 == gridDim.x;  // as in k_topo_velocity
+  const bool low = LAYER && blockIdx.x + 1 == gridDim.x;  // as in k_topo_velocity
   const bool lay = low && c.k == 2 && c.lane >= 2 && (c.top || c.lane <= 29) && jin;
   long long o = (long long)ib * S + (long long)ja * Y + (c.ld + AWP_ALIGN);
   float* __restrict__ SG[6] = {a.xx, a.yy, a.zz, a.xy, a.xz, a.yz};
@@ -720,7 +721,6 @@ __global__ void __launch_bounds__(StrTile::kThreads, 2)
       rx.kr2 = make_float2(q2.x, q2.y); rx.kf = make_float2(q2.z, q2.w);
       rx.c0 = make_float2(q3.x, q3.y); rx.c1 = make_float2(q3.z, q3.w);
       rx.c2 = lds2(t + 16);
-      if (lay) rx.c2.x *= 0.5f;
     }
     AwpStrCoef<float2> cf;
     {
@@ -742,8 +742,24 @@ __global__ void __launch_bounds__(StrTile::kThreads, 2)
         Pq = pq;
         Rq = rq; Rt = rt; Rm = rm;
       }
-      cf = awp_stress_coef<ELASTIC>(vadd(Lq, Ln), vadd(Mq, mq), P, QP8, QS8, R, rx, a.thr, a.dth,
-                                    a.DT);
+      const float2 L8 = vadd(Lq, Ln), M8 = vadd(Mq, mq);
+      if (LAYER) {
+        const int e = 2 * ((s & 1) ? e1 : e0);
+        AwpLayerOps ops{lay, 0.f, 0.f};
+        float2 dth = dup(a.dth), DT = dup(a.DT);
+        if (lay) {
+          ops.l0 = a.lay.l0[e];
+          ops.l1 = a.lay.l1[e];
+          const AwpRelax<float> l = awp_relax_at(a.lay_rel, e);
+          rx.kv.x = l.kv; rx.kr.x = l.kr; rx.kr2.x = l.kr2; rx.kf.x = l.kf;
+          rx.c2.x *= 0.5f;
+          dth.x = a.lay_dth;
+          DT.x = a.lay_dt;
+        }
+        cf = awp_stress_coef<ELASTIC>(L8, M8, P, QP8, QS8, R, rx, a.thr, dth, DT, ops);
+      } else {
+        cf = awp_stress_coef<ELASTIC>(L8, M8, P, QP8, QS8, R, rx, a.thr, dup(a.dth), dup(a.DT));
+      }
       Lq = Ln;
       Mq = mq; Mt = mt; Mm = mm;
     }
@@ -789,7 +805,7 @@ unsigned column_tiles(int nz) {
   return 1u + (nz > 63 ? (unsigned)((nz - 63 + kTileOut - 1) / kTileOut) : 0u);
 }
 
-Shape g_shape_vel[kMaxDev], g_shape_str[2][kMaxDev];
+Shape g_shape_vel[kMaxDev], g_shape_str[4][kMaxDev];
 
 }  // namespace
 
@@ -822,12 +838,15 @@ cudaError_t awp_launch_topo_stress(const TopoArgs& a, const TmaMaps& tm, bool el
   if (ni <= 0 || nj <= 0) return cudaSuccess;
   const dim3 tile(column_tiles(a.nz), cdiv_u(nj, StrTile::kCol));
   const size_t sm = elastic ? TopoStrCfg<true>::bytes : TopoStrCfg<false>::bytes;
-  const void* f = elastic ? (const void*)k_topo_stress<true> : (const void*)k_topo_stress<false>;
+  const auto f = elastic ? (a.layer ? k_topo_stress<true, true> : k_topo_stress<true, false>)
+                         : (a.layer ? k_topo_stress<false, true> : k_topo_stress<false, false>);
   int resident = 0;
-  const cudaError_t e = resident_ctas(f, sm, StrTile::kThreads, g_shape_str[elastic ? 1 : 0], &resident);
+  const cudaError_t e =
+      resident_ctas((const void*)f, sm, StrTile::kThreads,
+                    g_shape_str[(elastic ? 2 : 0) + (a.layer ? 1 : 0)], &resident);
   if (e != cudaSuccess) return e;
   const int ch = march_planes((long long)tile.x * tile.y, ni, resident, ichunk, kMost);
   const dim3 grid(tile.x, tile.y, cdiv_u(ni, ch));
-  return launch_after(elastic ? k_topo_stress<true> : k_topo_stress<false>, grid,
-                      dim3(StrTile::kThreads), sm, st, a, tm, ch, err, awp_pipe_spin_limit);
+  return launch_after(f, grid, dim3(StrTile::kThreads), sm, st, a, tm, ch, err,
+                      awp_pipe_spin_limit);
 }

@@ -23,8 +23,12 @@ struct TopoArgs {
   unsigned thr;          // Q(f) switch on a pair sum of Q^-1 (StrArgs::thr)
   int s_i, e_i, s_j, e_j;  // stress window, relative indices, ends exclusive
   // > 0 on a block over a coarser one: level 2, the interface layer, is updated
-  // to second order too (dvelc2; dstrqc2 inside the stress window)
+  // to second order too (dvelc2; dstrqc2 inside the stress window, with the
+  // run's own DT, DT/h and 1/h)
   int layer;
+  AwpRelaxTab lay_rel;
+  AwpLayerTab lay;
+  float lay_dt, lay_dth;
 };
 
 // dtopo_vel_111_unroll + dtopo_vel_112 (velocity_unroll.cu, optimized_velocity.cu:1040-1629)
