@@ -238,7 +238,8 @@ __global__ void __launch_bounds__(kSwThreads) k_swap3(const DmPairArgs a) {
 #pragma unroll
         for (int q = 0; q < kFly; ++q) {
           const int bj = b0 + 4 * q + c4;
-          float s0 = w0 * h[q], s1 = w1 * h[q];
+          // a level outside a window adds nothing to it, whatever it holds
+          float s0 = w0 > 0.f ? w0 * h[q] : 0.f, s1 = w1 > 0.f ? w1 * h[q] : 0.f;
 #pragma unroll
           for (int m = 4; m >= 1; m >>= 1) {
             s0 += __shfl_xor_sync(0xffffffffu, s0, m);

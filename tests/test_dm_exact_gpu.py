@@ -102,3 +102,72 @@ def test_dstrqc2_memory_variables_match_float64():
         assert float(np.median(np.abs(want))) > 0
         err = np.abs(got - want) / np.abs(want)
         assert float(err.max()) <= 14 * EPS, (name, err.max() / EPS)
+
+
+FIELDS = ["xx", "yy", "zz", "xy", "xz", "yz", "u1", "v1", "w1"]
+# level of the first window's centre, windows, shift of the fine columns
+WINDOW = dict(u1=(3, 2, 0, 0), v1=(3, 2, 1, 1), xy=(3, 2, 0, 1), xx=(3, 2, 1, 0),
+              yy=(3, 2, 1, 0), zz=(3, 2, 1, 0), xz=(4, 1, 0, 0), w1=(4, 1, 1, 0),
+              yz=(4, 1, 1, 1))
+
+
+def swap(lib, fine, coarse, nx, ny):
+    st = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    fn = lib.swap_H
+    fn.restype = None
+    fn(*(pointer(coarse[n]) for n in FIELDS), *(pointer(fine[n]) for n in FIELDS), nx, ny,
+       *[None] * 4, -1, ctypes.c_void_p(st.cuda_stream), 0)
+    st.synchronize()
+
+
+def windows(h, nx, ny, kh, di, dj):
+    """(terms [125][i][j] in the reference's order, weights) of every coarse column."""
+    I, J = np.meshgrid(np.arange(NGSL, nx + NGSL + 5), np.arange(NGSL, ny + NGSL + 5),
+                       indexing="ij")
+    ci, cj = 3 * (I - 2 - NGSL) + 2 + NGSL + di, 3 * (J - 2 - NGSL) + 2 + NGSL + dj
+    r = range(-2, 3)
+    t = [((3 - abs(a)) * (3 - abs(b)) * (3 - abs(d)) / 729.0,
+          h[ci + a, cj + b, ALIGN + kh + d].astype(np.float64))
+         for b in r for a in r for d in r]
+    return I, J, t
+
+
+@pytest.mark.parametrize("nx,ny", [(5, 7), (33, 30)])
+def test_swap_windows(nx, ny):
+    """Against float64: 13 roundings a term, and no further off than the
+    reference's chain of 125 sums; an infinite or undefined level stays in the
+    windows that hold it."""
+    lib = _lib.load()
+    nz, nzf = 12, 16
+    grid_constants(lib, [(3 * nx, 3 * ny, nzf), (nx, ny, nz)], [10.0, 30.0], 0.001)
+    g = np.random.default_rng(nx)
+    host = {n: g.standard_normal(padded((3 * nx, 3 * ny, nzf))).astype(np.float32) for n in FIELDS}
+    fine = {n: dev(a) for n, a in host.items()}
+    coarse = {n: torch.zeros(padded((nx, ny, nz)), device="cuda") for n in FIELDS}
+    swap(lib, fine, coarse, nx, ny)
+    for n in FIELDS:
+        kh0, nwin, di, dj = WINDOW[n]
+        got = coarse[n].cpu().numpy()
+        for lev in range(nwin):
+            I, J, t = windows(host[n], nx, ny, 6 if lev else kh0, di, dj)
+            want = sum(w * h for w, h in t)
+            size = sum(w * np.abs(h) for w, h in t)
+            chain = np.zeros(want.shape, np.float32)
+            for w, h in t:
+                chain = (w * h + chain.astype(np.float64)).astype(np.float32)
+            err = got[I, J, ALIGN + nz - 2 + lev] - want
+            assert (np.abs(err) <= 13 * EPS * size).all(), (n, lev)
+            assert np.linalg.norm(err) <= np.linalg.norm(chain - want), (n, lev)
+    clean = {n: coarse[n].clone() for n in FIELDS}
+    for n in FIELDS:  # outside the first window of every field
+        fine[n][:, :, ALIGN + 8] = float("inf")
+        if WINDOW[n][0] == 4:
+            fine[n][:, :, ALIGN + 1] = float("nan")
+    swap(lib, fine, coarse, nx, ny)
+    for n in FIELDS:
+        level = ALIGN + nz - 2
+        assert torch.equal(coarse[n][:, :, level], clean[n][:, :, level]), n
+        if WINDOW[n][1] == 2:
+            inner = coarse[n][NGSL:nx + NGSL + 5, NGSL:ny + NGSL + 5, level + 1]
+            assert bool(torch.isinf(inner).all()), n
