@@ -55,6 +55,11 @@ void awp_internal_set_error(const char* msg) {
 // ===========================================================================
 // Context
 // ===========================================================================
+// Launch-shape tuning of a batch's steps, in place of the process-wide values.
+struct Tune {
+  int tma_vel, tma_str, ichunk, l2_promotion;
+};
+
 struct awp_ctx {
   awp_params p;
   AwpGeom g;
@@ -113,6 +118,7 @@ struct awp_ctx {
   int* d_err = nullptr;           // pipeline-wait error word of the TMA kernels
   bool tma_ok = false;            // tensor maps encoded for this context
   int tma_promo = -1;             // L2 promotion the maps were encoded with
+  const Tune* tune = nullptr;     // while a batch enqueues its steps
   TmaMaps vel_maps{}, str_maps{};
   TmaMaps topo_vel_maps{}, topo_str_maps{};  // of a curvilinear top grid
   long long cur_step = 0;
@@ -337,12 +343,20 @@ bool build_tma_maps(awp_ctx* c) {
 // encoded; a tuning change re-encodes them before the next TMA launch (host
 // only: the fields and boxes stay the same, so results are unchanged).
 bool tma_ready(awp_ctx* c) {
-  const int promo = awp_tuning_get("l2_promotion");
+  const int promo = c->tune ? c->tune->l2_promotion : awp_tuning_get("l2_promotion");
   if (c->tma_promo != promo) {
     c->tma_ok = build_tma_maps(c);
     c->tma_promo = promo;
   }
   return c->tma_ok;
+}
+
+int ichunk(const awp_ctx* c) { return c->tune ? c->tune->ichunk : awp_tuning_get("ichunk"); }
+bool tma_vel(awp_ctx* c) {
+  return (c->tune ? c->tune->tma_vel : awp_tuning_get("tma_vel")) == 1 && tma_ready(c);
+}
+bool tma_str(awp_ctx* c) {
+  return (c->tune ? c->tune->tma_str : awp_tuning_get("tma_str")) == 1 && tma_ready(c);
 }
 
 struct PhaseScope {
@@ -423,6 +437,7 @@ TopoArgs topo_args(awp_ctx* c) {
 VelArgs make_vel_args(awp_ctx* c) {
   float** f = c->f;
   VelArgs v;
+  memset(&v, 0, sizeof(v));
   v.u1 = f[AWP_U1]; v.v1 = f[AWP_V1]; v.w1 = f[AWP_W1];
   v.xx = f[AWP_XX]; v.yy = f[AWP_YY]; v.zz = f[AWP_ZZ];
   v.xy = f[AWP_XY]; v.xz = f[AWP_XZ]; v.yz = f[AWP_YZ];
@@ -447,19 +462,19 @@ int phase_velocity(awp_ctx* c) {
   if (c->topo) {  // topo_velocity_*_H replace dvelc[xy] on the top grid (pmcl3d.c:1661-1698)
     if (!tma_ready(c)) return set_error(AWP_ERR_CUDA, "tensor maps of the curvilinear grid");
     PhaseScope ps(c, 0);
-    CU_TRY(awp_launch_topo_velocity(topo_args(c), c->topo_vel_maps, awp_tuning_get("ichunk"),
+    CU_TRY(awp_launch_topo_velocity(topo_args(c), c->topo_vel_maps, ichunk(c),
                                     c->d_err, c->stream));
     c->launches++;
     return AWP_OK;
   }
-  const bool tma = awp_tuning_get("tma_vel") == 1 && tma_ready(c);
+  const bool tma = tma_vel(c);
   PhaseScope ps(c, 0);
   if (tma) v.layer = mesh_layer(c) ? 1 : 0;
   if (tma)
-    CU_TRY(awp_launch_velocity_tma(v, c->vel_maps, awp_tuning_get("ichunk"), c->d_err,
+    CU_TRY(awp_launch_velocity_tma(v, c->vel_maps, ichunk(c), c->d_err,
                                    c->stream));
   else
-    CU_TRY(awp_launch_velocity(v, c->stream));
+    CU_TRY(awp_launch_velocity(v, ichunk(c), c->stream));
   c->launches++;
   return AWP_OK;
 }
@@ -485,16 +500,16 @@ AwpBox middle_band(const awp_ctx* c) {
 int launch_cart_stress(awp_ctx* c, const AwpBox* box, int n, bool layer = false) {
   StrArgs s = make_str_args(c);
   s.layer = layer ? 1 : 0;
-  const bool tma = awp_tuning_get("tma_str") == 1 && tma_ready(c);
+  const bool tma = tma_str(c);
   for (int q = 0, m; q < n; q += m) {
     m = tma ? awp::disjoint_run(box + q, n - q) : 1;
     if (std::all_of(box + q, box + q + m, [](const AwpBox& b) { return b.empty(); })) continue;
     if (tma) {
       CU_TRY(awp_launch_stress_tma(s, box + q, m, c->str_maps, c->elastic,
-                                   awp_tuning_get("ichunk"), c->d_err, c->stream));
+                                   ichunk(c), c->d_err, c->stream));
     } else {
       s.i0 = box[q].i0; s.i1 = box[q].i1; s.j0 = box[q].j0; s.j1 = box[q].j1;
-      CU_TRY(awp_launch_stress(s, c->elastic, c->stream));
+      CU_TRY(awp_launch_stress(s, c->elastic, ichunk(c), c->stream));
     }
     c->launches++;
   }
@@ -517,11 +532,10 @@ bool stress_split(const awp_ctx* c) {
 // stress is split around the plasticity section (the layer belongs before the
 // sources, whole).
 bool stress_layer(awp_ctx* c) {
-  return mesh_layer(c) && !c->topo && !stress_split(c) && awp_tuning_get("tma_str") == 1 &&
-         tma_ready(c);
+  return mesh_layer(c) && !c->topo && !stress_split(c) && tma_str(c);
 }
 bool velocity_layer(awp_ctx* c) {
-  return mesh_layer(c) && !c->topo && awp_tuning_get("tma_vel") == 1 && tma_ready(c);
+  return mesh_layer(c) && !c->topo && tma_vel(c);
 }
 
 bool topo_stress_runs(const awp_ctx* c) {
@@ -534,7 +548,7 @@ int phase_stress(awp_ctx* c) {
     if (!tma_ready(c)) return set_error(AWP_ERR_CUDA, "tensor maps of the curvilinear grid");
     PhaseScope ps(c, 1);
     CU_TRY(awp_launch_topo_stress(topo_args(c), c->topo_str_maps, c->elastic,
-                                  awp_tuning_get("ichunk"), c->d_err, c->stream));
+                                  ichunk(c), c->d_err, c->stream));
     c->launches++;
     return AWP_OK;
   }
@@ -631,6 +645,7 @@ int phase_plasticity(awp_ctx* c) {
 FstrArgs make_fstr_args(awp_ctx* c) {
   float** f = c->f;
   FstrArgs fs;
+  memset(&fs, 0, sizeof(fs));
   fs.zz = f[AWP_ZZ]; fs.xz = f[AWP_XZ]; fs.yz = f[AWP_YZ];
   fs.slice = c->g.slice; fs.yline = c->g.yline; fs.ktop = c->g.top();
   fs.i0 = c->xls; fs.i1 = c->xre;
@@ -2133,6 +2148,18 @@ int awp_topo_metrics(const char* path, int nx, int ny, int nz, float h, float* o
 // ===========================================================================
 constexpr int kBatchSteps = 8;  // most steps in one graph of parallel branches
 
+// What the launches of an instance bake into a graph: buffers, ranges, sources,
+// the elastic variant.  Compared bytewise (every member is cleared first).
+struct InstKey {
+  VelArgs v;
+  StrArgs s;
+  FstrArgs f;
+  SrcArgs src;
+  KinSrcArgs kin;
+  int elastic, deep;
+  unsigned spin;
+};
+
 struct awp_batch {
   std::vector<awp_ctx*> ctx;
   cudaStream_t stream = nullptr;
@@ -2146,7 +2173,9 @@ struct awp_batch {
   cudaEvent_t fork = nullptr;
   long long launches_per_step = 0;
   bool use_graph = true;
-  bool dirty = true;  // graphs to rebuild
+  bool dirty = true;  // graphs to rebuild, tuning to take
+  Tune tune{};        // process-wide tuning of the first step after that
+  std::vector<InstKey> key;  // the state the graphs were captured in
   long long step = 0;
   long long cells = 0;
   cudaGraphExec_t branch_exec[kBatchSteps + 1] = {};  // n steps of parallel branches
@@ -2187,6 +2216,7 @@ int batch_enqueue_branches(awp_batch* b, int nsteps) {
       const bool prof = c->profile;
       c->stream = b->cs[br];
       c->profile = false;
+      c->tune = &b->tune;
       if (!used[br]) {
         ce = cudaStreamWaitEvent(b->cs[br], b->fork, 0);
         used[br] = 1;
@@ -2215,6 +2245,7 @@ int batch_enqueue_branches(awp_batch* b, int nsteps) {
       if (!st && ce == cudaSuccess && !with_fstr) st = phase_fstr(c);
       c->stream = saved;
       c->profile = prof;
+      c->tune = nullptr;
     }
   for (size_t br = 0; br < nb; ++br) {  // rejoin even after an error (a capture must)
     if (!used[br]) continue;
@@ -2232,12 +2263,12 @@ int batch_enqueue_branches(awp_batch* b, int nsteps) {
 }
 
 int batch_streams(awp_batch* b) {
-  if (!b->cs.empty()) return AWP_OK;
-  b->cs.assign(b->ctx.size(), nullptr);
-  b->join.assign(b->ctx.size(), nullptr);
+  if (b->fork) return AWP_OK;  // made last: a failed call is taken up again
+  b->cs.resize(b->ctx.size(), nullptr);
+  b->join.resize(b->ctx.size(), nullptr);
   for (size_t q = 0; q < b->ctx.size(); ++q) {
-    CU_TRY(cudaStreamCreateWithFlags(&b->cs[q], cudaStreamNonBlocking));
-    CU_TRY(cudaEventCreateWithFlags(&b->join[q], cudaEventDisableTiming));
+    if (!b->cs[q]) CU_TRY(cudaStreamCreateWithFlags(&b->cs[q], cudaStreamNonBlocking));
+    if (!b->join[q]) CU_TRY(cudaEventCreateWithFlags(&b->join[q], cudaEventDisableTiming));
   }
   CU_TRY(cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming));
   return AWP_OK;
@@ -2247,6 +2278,35 @@ long long batch_launches(const awp_batch* b) {
   long long n = 0;
   for (const awp_ctx* c : b->ctx) n += c->launches;
   return n;
+}
+
+InstKey inst_key(awp_ctx* c) {
+  InstKey k;
+  memset(&k, 0, sizeof(k));
+  k.v = make_vel_args(c);
+  k.s = make_str_args(c);
+  k.f = make_fstr_args(c);
+  k.src = make_src_args(c, 0);
+  k.kin = make_kin_args(c, 0);
+  k.elastic = c->elastic;
+  k.deep = c->src_deep;
+  k.spin = (unsigned)awp_tuning_get("spin_limit");
+  return k;
+}
+
+// Graphs captured before an instance's buffers, sources or variant (or the
+// waits' limit) changed go: they hold the old ones.
+void batch_check_graphs(awp_batch* b) {
+  b->key.resize(b->ctx.size());
+  bool same = true;
+  for (size_t q = 0; q < b->ctx.size(); ++q) {
+    const InstKey k = inst_key(b->ctx[q]);
+    if (memcmp(&k, &b->key[q], sizeof(k))) {
+      same = false;
+      memcpy(&b->key[q], &k, sizeof(k));
+    }
+  }
+  if (!same) batch_free_graphs(b);
 }
 
 // The graph of n steps of branches.
@@ -2426,8 +2486,11 @@ int awp_batch_step(awp_batch* b, int nsteps) {
   }
   if (b->dirty) {
     batch_free_graphs(b);
+    b->tune = {awp_tuning_get("tma_vel"), awp_tuning_get("tma_str"), awp_tuning_get("ichunk"),
+               awp_tuning_get("l2_promotion")};
     b->dirty = false;
   }
+  batch_check_graphs(b);
   {
     const int e = batch_step_branches(b, nsteps);
     if (e) return e;

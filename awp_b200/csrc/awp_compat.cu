@@ -111,7 +111,7 @@ void stress_common(float* xx, float* yy, float* zz, float* xy, float* xz, float*
   a.dth = gc.dth; a.dh1 = gc.dh1; a.dt = s.DT; a.c1 = s.c1; a.c2 = s.c2;
   const float thr = 2.0f * s.qthr;
   memcpy(&a.thr, &thr, sizeof(a.thr));
-  check(awp_launch_stress(a, false, St), func);
+  check(awp_launch_stress(a, false, awp_tuning_get("ichunk"), St), func);
 }
 
 DmGrid dm_grid(int d_i, float* u1, float* v1, float* w1, float* xx, float* yy, float* zz,
@@ -241,7 +241,7 @@ void dvelcx_H_opt(float* u1, float* v1, float* w1, float* xx, float* yy, float* 
   if (d_i > 0 && a.k1 > gc.nzt + AWP_ALIGN - 3) a.k1 = gc.nzt + AWP_ALIGN - 3;
   if (d_i < ngrids - 1 && a.k0 < AWP_ALIGN + 3) a.k0 = AWP_ALIGN + 3;
   a.dth = gc.dth; a.c1 = s.c1; a.c2 = s.c2;
-  check(awp_launch_velocity(a, St), "dvelcx_H_opt");
+  check(awp_launch_velocity(a, awp_tuning_get("ichunk"), St), "dvelcx_H_opt");
 }
 
 void dvelcy_H(float* u1, float* v1, float* w1, float* xx, float* yy, float* zz, float* xy,

@@ -1011,37 +1011,37 @@ __global__ void k_step_advance(int* step, const int n) {
 // ===========================================================================
 // launchers
 // ===========================================================================
-cudaError_t awp_launch_velocity(const VelArgs& a, cudaStream_t st) {
+cudaError_t awp_launch_velocity(const VelArgs& a, int ichunk, cudaStream_t st) {
   const int nk = a.k1 - a.k0 + 1, nj = a.j1 - a.j0 + 1, ni = a.i1 - a.i0 + 1;
   if (nk <= 0 || nj <= 0 || ni <= 0) return cudaSuccess;
   const dim3 block(32, 8, 1);
-  const dim3 grid(cdiv_u(nk, 32), cdiv_u(nj, 8), cdiv_u(ni, g_ichunk));
-  k_velocity<8><<<grid, block, 0, st>>>(a, g_ichunk);
+  const dim3 grid(cdiv_u(nk, 32), cdiv_u(nj, 8), cdiv_u(ni, ichunk));
+  k_velocity<8><<<grid, block, 0, st>>>(a, ichunk);
   return cudaGetLastError();
 }
 
 template <int TY>
-static void launch_stress_ty(const StrArgs& a, bool elastic, bool texarr, dim3 grid,
+static void launch_stress_ty(const StrArgs& a, bool elastic, bool texarr, dim3 grid, int ichunk,
                              cudaStream_t st) {
   const dim3 block(32, TY, 1);
   if (elastic) {
     if (texarr)
-      k_stress<true, true, TY><<<grid, block, 0, st>>>(a, g_ichunk);
+      k_stress<true, true, TY><<<grid, block, 0, st>>>(a, ichunk);
     else
-      k_stress<true, false, TY><<<grid, block, 0, st>>>(a, g_ichunk);
+      k_stress<true, false, TY><<<grid, block, 0, st>>>(a, ichunk);
   } else {
     if (texarr)
-      k_stress<false, true, TY><<<grid, block, 0, st>>>(a, g_ichunk);
+      k_stress<false, true, TY><<<grid, block, 0, st>>>(a, ichunk);
     else
-      k_stress<false, false, TY><<<grid, block, 0, st>>>(a, g_ichunk);
+      k_stress<false, false, TY><<<grid, block, 0, st>>>(a, ichunk);
   }
 }
 
-cudaError_t awp_launch_stress(const StrArgs& a, bool elastic, cudaStream_t st) {
+cudaError_t awp_launch_stress(const StrArgs& a, bool elastic, int ichunk, cudaStream_t st) {
   const int nk = a.k1 - a.k0 + 1, nj = a.j1 - a.j0 + 1, ni = a.i1 - a.i0 + 1;
   if (nk <= 0 || nj <= 0 || ni <= 0) return cudaSuccess;
-  const dim3 grid(cdiv_u(nk, 32), cdiv_u(nj, 8), cdiv_u(ni, g_ichunk));
-  launch_stress_ty<8>(a, elastic, a.vx1 != nullptr, grid, st);
+  const dim3 grid(cdiv_u(nk, 32), cdiv_u(nj, 8), cdiv_u(ni, ichunk));
+  launch_stress_ty<8>(a, elastic, a.vx1 != nullptr, grid, ichunk, st);
   return cudaGetLastError();
 }
 

@@ -201,8 +201,9 @@ struct CopySegs {
 cudaError_t awp_launch_copy_segments(const CopySegs& s, cudaStream_t st);
 cudaError_t awp_launch_planesrc(const PlaneSrcArgs& a, cudaStream_t st);
 cudaError_t awp_launch_frcvel(const FrcvelArgs& a, cudaStream_t st);
-cudaError_t awp_launch_velocity(const VelArgs& a, cudaStream_t st);
-cudaError_t awp_launch_stress(const StrArgs& a, bool elastic, cudaStream_t st);
+// ichunk: x planes a CTA marches
+cudaError_t awp_launch_velocity(const VelArgs& a, int ichunk, cudaStream_t st);
+cudaError_t awp_launch_stress(const StrArgs& a, bool elastic, int ichunk, cudaStream_t st);
 cudaError_t awp_launch_fstr(const FstrArgs& a, cudaStream_t st);
 // fstr with the point sources (one of s, k) of the same step in one launch, for
 // sources at least three levels below the surface; step, off, nst as

@@ -317,9 +317,13 @@ int awp_batch_destroy(awp_batch* batch);
  * launches (velocity, stress, sources at the device-held step, free-surface
  * images), replayed as CUDA graphs of up to eight steps in which an instance
  * runs on into its next step without waiting for the others; a batch's first
- * few steps are enqueued directly.  Each instance's arithmetic is that of
- * awp_step, bit for bit.  Ordered after earlier work on the contexts' streams
- * and before later work on them. */
+ * call of up to eight steps is enqueued directly.  Each instance's arithmetic
+ * is that of awp_step, bit for bit.  Ordered after earlier work on the
+ * contexts' streams and before later work on them.  Sources, filters or
+ * materials set on an instance between calls take effect with the next one.
+ * The batch keeps the process-wide tuning (awp_set_tuning; not "spin_limit") in
+ * force at its first step after creation or after an awp_batch_set_graph,
+ * _set_mode or _set_branches that changed something. */
 int awp_batch_step(awp_batch* batch, int nsteps);
 int awp_batch_synchronize(awp_batch* batch);
 /* Tile shape the counts of awp_batch_info refer to (ty = 4 or 8 j rows, ichunk
