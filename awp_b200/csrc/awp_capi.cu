@@ -2165,7 +2165,7 @@ struct awp_batch {
   cudaStream_t stream = nullptr;
   cudaEvent_t ev = nullptr;
   int* d_step = nullptr;  // steps taken (device copy of cur_step)
-  int ty = 8, ichunk = 16;
+  int ty = 8, ichunk = 16;  // tiles that awp_batch_info counts
   int mode = 0;
   int branches = 0;  // parallel branches (0: one per instance)
   std::vector<cudaStream_t> cs;   // one branch stream per instance
@@ -2337,7 +2337,7 @@ int batch_capture_branches(awp_batch* b, int n) {
 int batch_step_branches(awp_batch* b, int nsteps) {
   int e = batch_streams(b);
   if (e) return e;
-  const bool graph = b->use_graph || b->mode == 1;  // mode 1 always replays graphs
+  const bool graph = b->use_graph || b->mode == 1;  // mode 1: whatever set_graph says
   if (!graph || (!b->stepped && nsteps <= kBatchSteps)) {
     b->stepped = true;
     for (int n = 0; n < nsteps; n += kBatchSteps)
@@ -2417,11 +2417,8 @@ int awp_batch_set_shape(awp_batch* b, int ty, int ichunk) {
   if (!b) return set_error(AWP_ERR_ARG, "null batch");
   if ((ty != 4 && ty != 8) || ichunk < 1 || ichunk > 1024)
     return set_error(AWP_ERR_ARG, "tile shape: ty 4 or 8, ichunk 1..1024");
-  if (ty != b->ty || ichunk != b->ichunk) {
-    b->ty = ty;
-    b->ichunk = ichunk;
-    b->dirty = true;
-  }
+  b->ty = ty;
+  b->ichunk = ichunk;
   return AWP_OK;
 }
 

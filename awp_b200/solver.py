@@ -440,6 +440,7 @@ class Batch:
         check(self.lib.awp_batch_synchronize(self.batch), "awp_batch_synchronize")
 
     def set_shape(self, ty: int, ichunk: int) -> None:
+        """Tile shape that ``info`` counts by (no effect on how the batch runs)."""
         check(self.lib.awp_batch_set_shape(self.batch, int(ty), int(ichunk)),
               "awp_batch_set_shape")
 
@@ -456,7 +457,8 @@ class Batch:
 
     def set_mode(self, mode: int) -> None:
         """0: parallel branches, graphs or direct launches as ``set_graph`` says;
-        1: graphs whatever it says.  Same results."""
+        1: graphs whatever it says.  In both, a batch's first call of up to
+        eight steps is launched directly.  Same results."""
         check(self.lib.awp_batch_set_mode(self.batch, int(mode)), "awp_batch_set_mode")
 
     @property
@@ -470,6 +472,8 @@ class Batch:
               "awp_batch_set_branches")
 
     def info(self) -> dict:
+        """Counts of the batch; ``grid_velocity`` and ``grid_stress`` repeat the
+        tile counts (the batch launches no persistent CTAs)."""
         v = (c_longlong * 6)()
         check(self.lib.awp_batch_info(self.batch, v), "awp_batch_info")
         keys = ("instances", "cells", "velocity_tiles", "stress_tiles", "grid_velocity",

@@ -93,66 +93,52 @@ def autotune(solver, steps: int = 3) -> dict:
     return {"chosen": chosen, "table": table}
 
 
-BATCH_CANDIDATES = {"ty": (8, 4), "ichunk": (8, 16, 32)}
+BATCH_CANDIDATES = {"tma_vel": (1, 0), "ichunk": (16, 32, 64)}
+BRANCHES = (32, 16, 8)  # fewer, longer branches than one per instance (0)
 
 
 def autotune_batch(batch, steps: int = 3, timer=None) -> dict:
-    """Pick the batched execution: the mode (both run the instances' own
-    launches as parallel branches; the shape only sets the tile counts that
-    info reports), the kernel family, x chunk and number of branches, by timing
-    `steps` batched steps per candidate (advancing the instances); `timer(fn)` returns the milliseconds
-    fn takes.  No choice changes results (each cell is computed by the same
-    expression)."""
+    """Pick how a batch runs its instances' launches -- the velocity kernel
+    family, the x chunk and the number of branches -- by timing `steps` batched
+    steps per candidate (advancing the instances); `timer(fn)` returns the
+    milliseconds fn takes.  The batch keeps the choice for every later step;
+    the process-wide tuning is left as it was.  No choice changes results (each
+    cell is computed by the same expression)."""
     table = []
-    batch.set_mode(0)
-    for ty, ich in itertools.product(*BATCH_CANDIDATES.values()):
-        batch.set_shape(ty, ich)
-        batch.step(steps)  # build the tile lists or the graphs
-        batch.step(steps)
-        batch.synchronize()
-        ms = timer(lambda: batch.step(steps))
-        table.append({"mode": 0, "ty": ty, "ichunk": ich, "ms_per_step": ms / steps})
-    # mode 1 captures each instance's launches with the process-wide kernel
-    # families and x chunk in force at capture time: try those too, then put
-    # the process-wide values back (the captured graph keeps its own)
     lib = batch.lib
     saved = get_tuning(lib)
-    # the mode-1 rows below are one branch per instance (branches = 0)
-    batch.set_branches(0)
-    for tv, ich in itertools.product((1, 0), (16, 32, 64)):
-        set_tuning(lib, "tma_vel", tv)
-        set_tuning(lib, "ichunk", ich)
-        batch.set_mode(0)
-        batch.set_mode(1)  # recapture
-        batch.step(steps)
-        batch.synchronize()
-        ms = timer(lambda: batch.step(steps))
-        table.append({"mode": 1, "ty": None, "ichunk": ich, "tma_vel": tv,
-                      "ms_per_step": ms / steps})
-    best = min(table, key=lambda r: r["ms_per_step"])
-    if best["mode"] == 1:
-        set_tuning(lib, "tma_vel", best["tma_vel"])
-        set_tuning(lib, "ichunk", best["ichunk"])
-        best["branches"] = 0
-        for nb in (32, 16, 8):  # fewer, longer branches
-            batch.set_branches(nb)
-            batch.step(steps)
-            batch.synchronize()
-            ms = timer(lambda: batch.step(steps))
-            row = {"mode": 1, "ty": None, "ichunk": best["ichunk"], "tma_vel": best["tma_vel"],
-                   "branches": nb, "ms_per_step": ms / steps}
-            table.append(row)
-            if row["ms_per_step"] < best["ms_per_step"]:
-                best = row
-        batch.set_branches(best["branches"])
+
+    def take():  # the batch takes the process-wide tuning at its next step
         batch.set_mode(0)
         batch.set_mode(1)
-        batch.step(1)  # capture with the chosen values
+
+    def timed(row):
+        for _ in range(2):  # a first call runs directly, the next one captures
+            batch.step(steps)
         batch.synchronize()
-    else:
-        batch.set_mode(0)
-        batch.set_shape(best["ty"], best["ichunk"])
-    for k, v in saved.items():
-        set_tuning(lib, k, v)
+        ms = timer(lambda: batch.step(steps))
+        table.append({"mode": 1, "ty": None, **row, "ms_per_step": ms / steps})
+
+    try:
+        batch.set_branches(0)
+        for tv, ich in itertools.product(*BATCH_CANDIDATES.values()):
+            set_tuning(lib, "tma_vel", tv)
+            set_tuning(lib, "ichunk", ich)
+            take()
+            timed({"ichunk": ich, "tma_vel": tv, "branches": 0})
+        best = min(table, key=lambda r: r["ms_per_step"])
+        set_tuning(lib, "tma_vel", best["tma_vel"])
+        set_tuning(lib, "ichunk", best["ichunk"])
+        for nb in BRANCHES:
+            batch.set_branches(nb)
+            timed({"ichunk": best["ichunk"], "tma_vel": best["tma_vel"], "branches": nb})
+        best = min(table, key=lambda r: r["ms_per_step"])
+        batch.set_branches(best["branches"])
+        take()
+        batch.step(1)  # with the chosen values in force
+        batch.synchronize()
+    finally:
+        for k, v in saved.items():
+            set_tuning(lib, k, v)
     return {"chosen": {k: best.get(k) for k in ("mode", "ty", "ichunk", "tma_vel", "branches")},
             "table": table}

@@ -326,14 +326,15 @@ int awp_batch_destroy(awp_batch* batch);
  * _set_mode or _set_branches that changed something. */
 int awp_batch_step(awp_batch* batch, int nsteps);
 int awp_batch_synchronize(awp_batch* batch);
-/* Tile shape the counts of awp_batch_info refer to (ty = 4 or 8 j rows, ichunk
- * x planes per tile; default 8, 16), and graph replay (1, default) or, in mode
- * 0, direct launches (0). */
+/* Tile shape that awp_batch_info counts by (ty = 4 or 8 j rows, ichunk x planes
+ * per tile; default 8, 16): it does not change how the batch runs. */
 int awp_batch_set_shape(awp_batch* batch, int ty, int ichunk);
 int awp_batch_get_shape(const awp_batch* batch, int* ty, int* ichunk);
+/* Graph replay (1, default) or, in mode 0, direct launches (0). */
 int awp_batch_set_graph(awp_batch* batch, int use_graph);
 /* Execution mode: 0 (default) graphs or direct launches as awp_batch_set_graph
- * says; 1 graphs whatever it says.  Same results. */
+ * says; 1 graphs whatever it says (in both, a batch's first call of up to eight
+ * steps is enqueued directly).  Same results. */
 int awp_batch_set_mode(awp_batch* batch, int mode);
 int awp_batch_get_mode(const awp_batch* batch);
 /* The instances' launches are dealt, largest first, round-robin onto

@@ -31,6 +31,7 @@ def make(spec, steps):
     return s
 
 
+# (the tile shape only changes the counts that info reports)
 @pytest.mark.parametrize("mode,ty,ichunk,graph,branches",
                          [(0, 8, 16, True, 0), (0, 4, 8, True, 0), (0, 8, 32, False, 0),
                           (1, 8, 16, True, 0), (1, 8, 16, True, 2), (1, 8, 16, True, 1)])

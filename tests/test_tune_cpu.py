@@ -93,3 +93,51 @@ def test_autotune_keeps_the_promotion_without_a_tma_kernel():
     assert res["chosen"]["tma_vel"] == 0 and res["chosen"]["tma_str"] == 0
     assert res["chosen"]["l2_promotion"] == 2
     assert len(res["table"]) == len(tune.CANDIDATES["tma"]) * len(tune.CANDIDATES["ichunk"])
+
+
+class FakeBatch:
+    """The read-only family at chunk 32 on 16 branches is fastest; a batch takes the
+    process-wide tuning at its first step after a change of mode or branches."""
+
+    def __init__(self, lib):
+        self.lib = lib
+        self.mode, self.branches, self.taken, self.steps = 0, 0, None, 0
+
+    def set_mode(self, m):
+        if m != self.mode:
+            self.mode, self.taken = m, None
+
+    def set_branches(self, n):
+        if n != self.branches:
+            self.branches, self.taken = n, None
+
+    def step(self, n):
+        if self.taken is None:
+            self.taken = (self.lib.v["tma_vel"], self.lib.v["ichunk"])
+        self.steps += n
+
+    def synchronize(self):
+        pass
+
+    def cost(self):
+        tv, ich = self.taken
+        return (2.0 if tv else 1.5) + 0.01 * abs(ich - 32) + 0.1 * abs(self.branches - 16) / 16
+
+
+def test_autotune_batch_leaves_the_choice_with_the_batch():
+    lib = FakeLib()
+    b = FakeBatch(lib)
+
+    def timer(fn):
+        fn()
+        return 3 * b.cost()
+
+    res = tune.autotune_batch(b, steps=3, timer=timer)
+    assert res["chosen"] == {"mode": 1, "ty": None, "ichunk": 32, "tma_vel": 0, "branches": 16}
+    assert b.taken == (0, 32) and b.branches == 16 and b.mode == 1
+    assert tune.get_tuning(lib) == {k: FakeLib.KEYS[k] for k in tune.KEYS}
+    n = len(tune.BATCH_CANDIDATES["tma_vel"]) * len(tune.BATCH_CANDIDATES["ichunk"])
+    assert len(res["table"]) == n + len(tune.BRANCHES)
+    # every row is another configuration
+    rows = [(r["tma_vel"], r["ichunk"], r["branches"]) for r in res["table"]]
+    assert len(set(rows)) == len(rows)
