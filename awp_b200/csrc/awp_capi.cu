@@ -117,6 +117,7 @@ struct awp_ctx {
   unsigned int* d_ext = nullptr;  // media extrema (6 float bit patterns)
   int* d_err = nullptr;           // pipeline-wait error word of the TMA kernels
   bool tma_ok = false;            // tensor maps encoded for this context
+  bool topo_ok = false;           // ... and for its curvilinear kernels
   int tma_promo = -1;             // L2 promotion the maps were encoded with
   const Tune* tune = nullptr;     // while a batch enqueues its steps
   TmaMaps vel_maps{}, str_maps{};
@@ -313,6 +314,7 @@ bool build_tma_maps(awp_ctx* c) {
   for (int q = 0; q < 3; ++q) bad |= awp_tma_encode(&c->str_maps.halo[q], f[vo[q]], c->g, hx, hy);
   for (int q = 0; q < 4; ++q) bad |= awp_tma_encode(&c->str_maps.media[q], f[sm[q]], c->g, mx, my);
   for (int q = 0; q < 12; ++q) bad |= awp_tma_encode(&c->str_maps.own[q], f[so[q]], c->g, ox, oy);
+  int hill = 0;
   if (c->topo) {
     // the curvilinear kernels' tiles: the same fields with their own boxes, and
     // no k halo (the neighbouring levels come from the neighbouring lanes)
@@ -321,21 +323,22 @@ bool build_tma_maps(awp_ctx* c) {
     awp_topo_box(0, 2, &ox, &oy);
     const bool jh[6] = {false, true, false, true, false, true};
     for (int q = 0; q < 6; ++q)
-      bad |= awp_tma_encode(&c->topo_vel_maps.halo[q], f[vh[q]], c->g, jh[q] ? hx : ox,
+      hill |= awp_tma_encode(&c->topo_vel_maps.halo[q], f[vh[q]], c->g, jh[q] ? hx : ox,
                             jh[q] ? hy : oy);
-    bad |= awp_tma_encode(&c->topo_vel_maps.media[0], f[AWP_D1], c->g, mx, my);
+    hill |= awp_tma_encode(&c->topo_vel_maps.media[0], f[AWP_D1], c->g, mx, my);
     for (int q = 0; q < 3; ++q)
-      bad |= awp_tma_encode(&c->topo_vel_maps.own[q], f[vo[q]], c->g, ox, oy);
+      hill |= awp_tma_encode(&c->topo_vel_maps.own[q], f[vo[q]], c->g, ox, oy);
     awp_topo_box(1, 0, &hx, &hy);
     awp_topo_box(1, 1, &mx, &my);
     awp_topo_box(1, 2, &ox, &oy);
     for (int q = 0; q < 3; ++q)
-      bad |= awp_tma_encode(&c->topo_str_maps.halo[q], f[vo[q]], c->g, hx, hy);
+      hill |= awp_tma_encode(&c->topo_str_maps.halo[q], f[vo[q]], c->g, hx, hy);
     for (int q = 0; q < 4; ++q)
-      bad |= awp_tma_encode(&c->topo_str_maps.media[q], f[sm[q]], c->g, mx, my);
+      hill |= awp_tma_encode(&c->topo_str_maps.media[q], f[sm[q]], c->g, mx, my);
     for (int q = 0; q < 12; ++q)
-      bad |= awp_tma_encode(&c->topo_str_maps.own[q], f[so[q]], c->g, ox, oy);
+      hill |= awp_tma_encode(&c->topo_str_maps.own[q], f[so[q]], c->g, ox, oy);
   }
+  c->topo_ok = hill == 0;
   return bad == 0;
 }
 
@@ -349,6 +352,13 @@ bool tma_ready(awp_ctx* c) {
     c->tma_promo = promo;
   }
   return c->tma_ok;
+}
+// The curvilinear kernels have no other form.  Encoding fails only without the
+// driver's entry point or beyond its limits on sizes and strides, which a
+// context's 2^31 cells stay far below.
+bool topo_ready(awp_ctx* c) {
+  (void)tma_ready(c);
+  return c->topo_ok;
 }
 
 int ichunk(const awp_ctx* c) { return c->tune ? c->tune->ichunk : awp_tuning_get("ichunk"); }
@@ -460,7 +470,7 @@ VelArgs make_vel_args(awp_ctx* c) {
 int phase_velocity(awp_ctx* c) {
   VelArgs v = make_vel_args(c);
   if (c->topo) {  // topo_velocity_*_H replace dvelc[xy] on the top grid (pmcl3d.c:1661-1698)
-    if (!tma_ready(c)) return set_error(AWP_ERR_CUDA, "tensor maps of the curvilinear grid");
+    if (!topo_ready(c)) return set_error(AWP_ERR_CUDA, "tensor maps of the curvilinear grid");
     PhaseScope ps(c, 0);
     CU_TRY(awp_launch_topo_velocity(topo_args(c), c->topo_vel_maps, ichunk(c),
                                     c->d_err, c->stream));
@@ -545,7 +555,7 @@ bool topo_stress_runs(const awp_ctx* c) {
 int phase_stress(awp_ctx* c) {
   if (c->topo && !topo_stress_runs(c)) return AWP_OK;
   if (c->topo) {  // topo_stress_*_H replace dstrqc on the top grid (pmcl3d.c:1843-1924)
-    if (!tma_ready(c)) return set_error(AWP_ERR_CUDA, "tensor maps of the curvilinear grid");
+    if (!topo_ready(c)) return set_error(AWP_ERR_CUDA, "tensor maps of the curvilinear grid");
     PhaseScope ps(c, 1);
     CU_TRY(awp_launch_topo_stress(topo_args(c), c->topo_str_maps, c->elastic,
                                   ichunk(c), c->d_err, c->stream));

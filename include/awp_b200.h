@@ -508,7 +508,10 @@ int awp_check_finite_noalloc(const float* const* fields, int nfields, long long 
  * CUDA events around each of its phases on the context's stream.
  * awp_phase_times waits for the stream and returns, per phase, the summed
  * milliseconds and the number of launches since the last call:
- * 0 velocity, 1 stress, 2 sources, 3 plasticity, 4 free-surface stress. */
+ * 0 velocity, 1 stress, 2 sources, 3 plasticity, 4 free-surface stress.  While
+ * it is on, point sources are a launch of their own; otherwise a single grid
+ * without plasticity adds those below the imaged levels in the free-surface
+ * launch. */
 #define AWP_NPHASES 5
 int awp_profile_phases(awp_ctx* ctx, int enable);
 int awp_phase_times(awp_ctx* ctx, double ms[AWP_NPHASES], long long launches[AWP_NPHASES]);
