@@ -235,7 +235,9 @@ inline int march_planes(long long tiles, int ni, int resident, int cap, int most
 }
 
 // Launch a kernel that calls grid_wait: its start-up overlaps the tail of the
-// kernel before it in the stream.  Every kernel of a step is launched so (ten
+// kernel before it in the stream.  The kernels of an ordinary step are launched
+// so; receivers, SOURCEFILE and FORCEFILE adds, halo copies, a batch's sources
+// near the surface and the read-only-path family are plain launches (ten
 // steps of a 48 x 40 x 36 shot: 206 -> 152 us; of a 240 x 237 x 120 grid with
 // plasticity 1312 -> 1265 for three); with some of a step's kernels only, a
 // plain launch behind an overlapped one waits longer than behind a plain one
