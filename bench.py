@@ -149,7 +149,14 @@ def cpu_baseline(workload: str, steps: int = 10, warmup: int = 3, grid=None) -> 
     from oracle import refbind
     scn, _ = build_workload(workload, grid)
     p = scn.params
-    setup = refbind.model_setup(scn)
+    if refbind.have_host():
+        setup = refbind.model_setup(scn)
+    else:  # the same arrays from the product's set-up (not timed)
+        from awp_b200 import Solver, default_params
+        s = Solver(default_params(**p))
+        s.upload_media(scn.media)
+        setup = refbind.product_setup(scn, s)
+        s.close()
     ncores = os.cpu_count() or 1
     sim = orc.OracleSim(scn, setup, precision=32, nthreads=ncores, flush_denormals=True)
     del setup
@@ -165,29 +172,6 @@ def cpu_baseline(workload: str, steps: int = 10, warmup: int = 3, grid=None) -> 
                        f"workload, FP32 with subnormals flushed, {steps} timed steps after "
                        f"{max(1, warmup)} warm-up, {dt:.1f} s"),
             "host": host_cpu()}
-
-
-def texture_arrays(nx, ny, nz, tau1, tau2, w8):
-    """init_texture (mesh.c:1103-1137) arrays from its visit-parity pattern."""
-    shp = (nx + 20, ny + 20, nz + 64)
-    vx1 = np.zeros(shp, np.float32)
-    vx2 = np.zeros(shp, np.float32)
-    wwo = np.zeros(shp, np.float32)
-    ww = np.zeros(shp, np.int32)
-    i = np.arange(nx)[:, None, None]
-    j = np.arange(ny)[None, :, None]
-    k = np.arange(nz)[None, None, :]
-    ij = i * ny + j
-    itx = (i + 1) & 1
-    ity = (ij + 1) & 1
-    itz = (nz * (ij + 1) + k) & 1
-    t = (4 * itx + 2 * ity + itz).astype(np.int64)
-    sl = (slice(10, nx + 10), slice(10, ny + 10), slice(32, nz + 32))
-    vx1[sl] = np.asarray(tau1, np.float32)[t]
-    vx2[sl] = np.asarray(tau2, np.float32)[t]
-    wwo[sl] = (8.0 * np.asarray(w8, np.float64)).astype(np.float32)[t]
-    ww[sl] = (t + 1).astype(np.int32)
-    return vx1, vx2, ww, wwo
 
 
 def reference_gpu(scn, solver, steps=20, warmup=3, topo_path=None, variant="as_shipped") -> dict:
@@ -213,7 +197,7 @@ def reference_gpu(scn, solver, steps=20, warmup=3, topo_path=None, variant="as_s
     solver.lib.awp_q_tau(0.0, 0.005, byref(taumax), byref(taumin), tau8.ctypes.data_as(F))
     solver.lib.awp_q_weights(0.0, 0.005, w8.ctypes.data_as(F), coeff.ctypes.data_as(F))
     tau1, tau2 = refbind.tau12(tau8, p["dt"])
-    vx1, vx2, ww, wwo = texture_arrays(nx, ny, nz, tau1, tau2, w8)
+    vx1, vx2, ww, wwo = refbind.texture_arrays(nx, ny, nz, tau1, tau2, w8)
     dx, dy, dz = host.inicrj(p["arbc"], nx, ny, nz, p["nd"], 1, p["npc"])
     media = {k: solver.field(k) for k in ("d1", "mu", "lam", "qp", "qs")}
     psrc, comps, rs = refbind.map_sources(scn)
@@ -509,8 +493,13 @@ def reference_config(args) -> dict:
 def run_reference(args, rank) -> dict | None:
     """Reference arm: the reference path's CPU restatement on the host cores,
     W warm-up and K timed steps on the workload's full grid."""
+    from oracle import refbind
     if rank != 0:
         return None
+    if not refbind.have_host():
+        return {"impl": "reference",
+                "unavailable": "the reference source tree is absent, so its host set-up code "
+                               "is not built (oracle/_ref)"}
     cb = cpu_baseline(args.workload, steps=args.steps, warmup=args.warmup, grid=args.grid)
     return {"metric": "Gcell-updates/s (whole time step) & %HBM roofline on 1 B200",
             "value": cb["value"], "unit": "Gcell-updates/s", "n_gpus": 1,

@@ -36,6 +36,11 @@ def padded_shape(nx, ny, nz):
     return (nx + 4 + 2 * NGSL, ny + 4 + 2 * NGSL, nz + 2 * ALIGN)
 
 
+def have_host() -> bool:
+    """Whether the reference's host set-up code is built (`make -C oracle ref`)."""
+    return os.path.exists(os.path.join(REF_DIR, "libawpref_host.so"))
+
+
 class RefHost:
     def __init__(self, path=None):
         path = path or os.path.join(REF_DIR, "libawpref_host.so")
@@ -489,6 +494,54 @@ def model_setup(scn, host: RefHost | None = None, fp=2.5, fac=0.005, q0=5.0, ex=
     return dict(media=m, vx1=vx1, vx2=vx2, ww=ww, wwo=wwo, dcrjx=dcrjx, dcrjy=dcrjy,
                 dcrjz=dcrjz, lam_mu=lm, coeff=m["coeff"], psrc=psrc, src=comps,
                 src_stride=rs, tau1=tau1, tau2=tau2)
+
+
+def texture_arrays(nx, ny, nz, tau1, tau2, w8):
+    """init_texture (mesh.c:1103-1137) arrays from its visit-parity pattern."""
+    shp = (nx + 20, ny + 20, nz + 64)
+    vx1 = np.zeros(shp, np.float32)
+    vx2 = np.zeros(shp, np.float32)
+    wwo = np.zeros(shp, np.float32)
+    ww = np.zeros(shp, np.int32)
+    i = np.arange(nx)[:, None, None]
+    j = np.arange(ny)[None, :, None]
+    k = np.arange(nz)[None, None, :]
+    ij = i * ny + j
+    itx = (i + 1) & 1
+    ity = (ij + 1) & 1
+    itz = (nz * (ij + 1) + k) & 1
+    t = (4 * itx + 2 * ity + itz).astype(np.int64)
+    sl = (slice(10, nx + 10), slice(10, ny + 10), slice(32, nz + 32))
+    vx1[sl] = np.asarray(tau1, np.float32)[t]
+    vx2[sl] = np.asarray(tau2, np.float32)[t]
+    wwo[sl] = (8.0 * np.asarray(w8, np.float64)).astype(np.float32)[t]
+    ww[sl] = (t + 1).astype(np.int32)
+    return vx1, vx2, ww, wwo
+
+
+def product_setup(scn, solver):
+    """The arrays of ``model_setup`` from the product's own set-up (the CPU tests hold
+    its tables to the reference's bit for bit), for a check of the time step
+    where the reference's host code is not built.  `solver` has the media."""
+    p = scn.params
+    nx, ny, nz = p["nx"], p["ny"], p["nz"]
+    lib = solver.lib
+    lo, hi = c_float(), c_float()
+    tau8, w8, coeff = np.zeros(8, np.float32), np.zeros(8, np.float32), np.zeros(16, np.float32)
+    if lib.awp_q_tau(0.0, 0.005, ctypes.byref(hi), ctypes.byref(lo), fptr(tau8)) or \
+            lib.awp_q_weights(0.0, 0.005, fptr(w8), fptr(coeff)):
+        raise RuntimeError("Q tables")
+    tau1, tau2 = tau12(tau8, p["dt"])
+    vx1, vx2, ww, wwo = texture_arrays(nx, ny, nz, tau1, tau2, w8)
+    sponge = [np.ones(n, np.float32) for n in padded_shape(nx, ny, nz)]
+    if lib.awp_cerjan(p.get("arbc", 0.92), nx, ny, nz, p.get("nd", 20), 1, p.get("npc", 0),
+                      *[fptr(a) for a in sponge]):
+        raise RuntimeError("sponge")
+    media = {k: solver.field(k) for k in ("d1", "mu", "lam", "qp", "qs")}
+    psrc, comps, rs = map_sources(scn)
+    return dict(media=media, vx1=vx1, vx2=vx2, ww=ww, wwo=wwo, dcrjx=sponge[0], dcrjy=sponge[1],
+                dcrjz=sponge[2], lam_mu=lam_mu_ref(media["lam"], media["mu"], nx, ny, nz),
+                coeff=coeff, psrc=psrc, src=comps, src_stride=rs, tau1=tau1, tau2=tau2)
 
 
 class RefGpuSim:
