@@ -88,9 +88,10 @@ __device__ __forceinline__ float2 dweight(float2 S, const AwpRelax<float2>& t, u
 // cell's own adjoint stresses, memory variables and weight sums (read once and
 // late) come one plane ahead by cp.async, so a plane's copies are in flight
 // while the one before is computed; the next plane's first velocities and media
-// are called into L2 at the same time.  At its traffic (160 x 144 x 96 with Q
-// sums: 110 us); marches of 8 or 16 planes and four CTAs an SM are 5-12 %
-// slower, and without the L2 prefetch a whole gradient is 4 % slower.
+// are called into L2 at the same time.  Without Q sums 109 us at 160 x 144 x 96
+// (0.58 of the copy bandwidth on these bytes): latency at twelve warps an SM.
+// Marches of 8 or 16 planes and four CTAs an SM are 5-12 % slower, and without
+// the L2 prefetch a whole gradient is 4 % slower.
 // ---------------------------------------------------------------------------
 constexpr int kSch = 4;
 
@@ -307,7 +308,7 @@ __global__ void __launch_bounds__(128, 3) k_adj_stress_cell(const __grid_constan
     // chain to the eight-cell sums.  The derivative of a quotient is one division
     // by the square (2.5 ulp), not the approximate quotient squared (twice its
     // error): it is the same in every step and does not average out of the sum
-    // over them.  The time is the traffic's either way.
+    // over them.  The time is the same either way.
     const float2 G_xlraw = vfma(G_qpa, c_q, vmul(G_xl, dthv));
     const float2 G_xmraw = vsub(G_xlraw, vfma(nG_xm, c_xm, vmul(nG_h, c_h)));
     st2(a.E[GL8] + p, vfma(vquot(-8.0f, vmul(L8, L8)), G_xlraw, stg[buf][6][tid]), ax, ay);
