@@ -141,7 +141,8 @@ struct awp_ctx {
   float* adj_slab = nullptr;
   size_t adj_slab_floats = 0;
   // receivers, seismograms and surface scratch of the seismogram and gradient
-  // calls, kept for the next call (grows to the largest one's need)
+  // calls, kept for the next call (the largest one's need); given back when the
+  // adjoint workspace has to grow, and with the context
   char* scratch = nullptr;
   size_t scratch_bytes = 0;
   long long dev_bytes = 0;
@@ -2664,13 +2665,19 @@ struct Scratch {
   awp_ctx* c;
   size_t used = 0;
   static size_t round(size_t bytes) { return (bytes + 255) / 256 * 256; }
-  int reserve(size_t bytes) {
-    if (c->scratch_bytes >= bytes) return AWP_OK;
+  static int release(awp_ctx* c) {
+    if (!c->scratch) return AWP_OK;
     CU_TRY(cudaStreamSynchronize(c->stream));
     cudaFree(c->scratch);
     c->scratch = nullptr;
     c->scratch_bytes = 0;
+    return AWP_OK;
+  }
+  int reserve(size_t bytes) {
+    if (c->scratch_bytes >= bytes) return AWP_OK;
+    if (int e = release(c)) return e;
     if (cudaMalloc((void**)&c->scratch, bytes) != cudaSuccess) {
+      (void)cudaGetLastError();  // reported here, once
       c->scratch = nullptr;
       return set_error(AWP_ERR_NOMEM, "scratch of %zu bytes", bytes);
     }
@@ -2852,7 +2859,8 @@ static int adjoint_plan(awp_ctx* c, int nsteps, int nsnap, AdjPlan* out) {
     size_t freeb = 0, totb = 0;
     CU_TRY(cudaMemGetInfo(&freeb, &totb));
     const double budget =
-        0.9 * (double)(freeb + c->adj_slab_floats * sizeof(float)) - (256u << 20);
+        0.9 * (double)(freeb + c->adj_slab_floats * sizeof(float) + c->scratch_bytes) -
+        (256u << 20);
     int lo = 0, hi = nsteps;  // largest M whose plan fits the budget
     while (lo < hi) {
       const int mid = (lo + hi + 1) / 2;
@@ -2872,6 +2880,7 @@ static int adjoint_plan(awp_ctx* c, int nsteps, int nsnap, AdjPlan* out) {
 // The workspace of a plan: one slab, kept in the context for later calls.
 static int ensure_adjoint_slab(awp_ctx* c, const AdjPlan& pl) {
   if (c->adj_slab_floats >= pl.floats) return AWP_OK;
+  if (int e = Scratch::release(c)) return e;  // an earlier call's, in the way of a larger slab
   cudaFree(c->adj_slab);
   c->adj_slab = nullptr;
   c->adj_slab_floats = 0;
@@ -3179,7 +3188,7 @@ int awp_kernel_launches(const awp_ctx* c, long long* launches) {
 
 int awp_device_bytes(const awp_ctx* c, long long* bytes) {
   if (!c || !bytes) return set_error(AWP_ERR_ARG, "null argument");
-  *bytes = c->dev_bytes;
+  *bytes = c->dev_bytes + (long long)c->scratch_bytes;
   return AWP_OK;
 }
 

@@ -328,3 +328,24 @@ def test_torch_autograd_on_device_tensors():
         assert tt.grad.is_cuda
         assert np.array_equal(tt.grad.cpu().numpy(), g)
     s.close()
+
+
+def test_kept_scratch_does_not_shrink_the_plan():
+    """The seismogram scratch of a large call stays with the context; it counts as
+    free when the workspace is planned, and it is counted in device_bytes."""
+    scn, s, m, xyz, comp, d_obs = setup_case(False, steps=10)
+    before = adjoint.adjoint_plan(s, 4_000_000)["tail_steps"]
+    held = s.device_bytes
+    steps, nrec = 500, 200_000  # 0.4 GB of samples
+    rng = np.random.default_rng(0)
+    p = scn.params
+    pos = np.stack([rng.integers(0, p[n], nrec) for n in ("nx", "ny", "nz")], 1).astype(np.int32)
+    adjoint.seismograms(s, steps, pos, np.zeros(nrec, np.int32))
+    assert s.device_bytes >= held + 4 * steps * nrec
+    after = adjoint.adjoint_plan(s, 4_000_000)["tail_steps"]
+    assert 0 < before < 4_000_000  # the plan is limited by the memory
+    # a few MB of driver allocations aside: 0.4 GB are some thousand steps here
+    assert before - after < 300, (before, after)
+    adjoint.adjoint_reserve(s, 200)  # a larger workspace: the scratch is given back
+    assert s.device_bytes <= held  # (held: with the small scratch of the set-up's call)
+    s.close()

@@ -60,6 +60,7 @@ CASES = [
     dict(kind="mesh", nx=22, ny=20, nz=68, nzc=36, steps=3, hill=True, plastic=True),
     dict(kind="ensemble", n=3, lo=40, hi=70, steps=3, mode=0, draw=3),
     dict(kind="ensemble", n=3, lo=40, hi=70, steps=3, mode=1, draw=4),
+    dict(kind="ensemble", n=2, lo=40, hi=50, steps=11, mode=1, draw=5),  # as graphs of 8 and 3
     dict(kind="gradient", nx=36, ny=33, nz=32, steps=14, q=True, nrec=9, nsnap=0),
     dict(kind="gradient", nx=33, ny=36, nz=36, steps=13, q=False, nrec=9, nsnap=3),
 ]
