@@ -212,7 +212,8 @@ inline cudaError_t resident_ctas(const void* kernel, size_t smem, int threads,
 // (ten steps of 128 x 128 x 128, 634 us, and five of a 53 x 41 x 60 mesh, 580,
 // with chunks up to six planes: 604 and 573 with longer ones, 600 and 597
 // with a fill of two planes, 602 and 599 with four; 48 x 40 x 36: 34 -> 9 us
-// and 60 -> 13 us for the two kernels against 32 planes throughout).
+// and 60 -> 13 us for the two kernels against 32 planes throughout; kFill and
+// the limit of four waves were set on these grids).
 // `ctas(c)`: the grid's CTAs at chunks of c planes, ni its longest extent.
 template <class F>
 inline int march_planes(F ctas, int ni, int resident, int cap, int most) {

@@ -103,7 +103,7 @@ struct ColPos2 {
 // c[31 - lane][p] = the coefficients of levels nz-1-2p (x, y) and nz-2-2p (z,
 // w) in the rows of the lane's two levels (rows 2(31-lane) + 1 and
 // 2(31-lane)).  The shared-memory pipe is the curvilinear kernels' busiest
-// (60 %), and the closures were 29 % of the velocity kernel's traffic as
+// (67 %), and the closures were 29 % of the velocity kernel's traffic as
 // broadcast shuffles: each lane now takes the top ten levels from lanes 27..31
 // as five pairs, and its coefficients four at a time.
 struct Closure {
